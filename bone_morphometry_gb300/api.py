@@ -129,10 +129,14 @@ def _tensor_dims(t):
     return int(w), int(h), int(d)
 
 
+_STREAM_LEGACY = 1  # cudaStreamLegacy: the default stream by handle (NULL means the context's own stream)
+
+
 def _stream_ptr(t):
+    """The tensor's current stream, so that the call runs after the work that produces its inputs."""
     import torch
 
-    return ctypes.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+    return ctypes.c_void_p(torch.cuda.current_stream(t.device).cuda_stream or _STREAM_LEGACY)
 
 
 def euclidean_distance_transform_squared(volume, phase: Phase = Phase.FOREGROUND, ctx: Context | None = None):

@@ -56,6 +56,10 @@ def batch_tbth_tbsp(specimens, feature_mode=FeatureMode.CLASSIC, ctx: Context | 
     if not items:
         return []
     device = _is_cuda_tensor(items[0].bone)
+    if device:  # the workers run on their own streams: the inputs must be complete
+        import torch
+
+        torch.cuda.current_stream(items[0].bone.device).synchronize()
     keep = []
     arr = (BmSpecimen * len(items))()
     for i, sp in enumerate(items):
