@@ -676,8 +676,7 @@ def run_profile_case(args) -> int:
         sp = S.make_specimen((n, n, n), 5.0, 0.15, "cylinder", 0.47 * n, 19.5, 1002)
     ctx = Context(0)
     ctx.set_concurrent_phases(False)
-    # the fill tile shape of the 512^3 and 1024^3 workloads (a 384^3 case alone would get 32-row tiles)
-    ctx.set_fill_tile_rows(64 if args.fill_rows == 0 else args.fill_rows)
+    ctx.set_fill_tile_rows(args.fill_rows)  # 0: the separable fill
     bone = torch.from_numpy(sp.bone).cuda()
     roi = torch.from_numpy(sp.roi).cuda()
     for _ in range(2):

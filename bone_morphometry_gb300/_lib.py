@@ -221,12 +221,12 @@ class Context:
         self.call("bm_ctx_set_concurrent_phases", 1 if on else 0)
 
     def set_site_method(self, method: int = 0) -> None:
-        """How the fill finds the non-selected voxels ridge spheres reach:
-        BM_SITES_AUTO (0), BM_SITES_SPHERES (1) or BM_SITES_CHAINS (2)."""
+        """How the fill finds the non-selected voxels ridge spheres reach: BM_SITES_AUTO
+        (0, the separable fill), BM_SITES_SPHERES (1) or BM_SITES_CHAINS (2)."""
         self.call("bm_ctx_set_site_method", int(method))
 
     def set_fill_tile_rows(self, rows: int = 0) -> None:
-        """Rows of y in the sphere fill's tiles: 0 (by volume size), 16, 32 or 64."""
+        """Rows of y in the tile fill's tiles: 16, 32 or 64; 0 (default): the separable fill."""
         self.call("bm_ctx_set_fill_tile_rows", int(rows))
 
     def set_wait_cycles(self, cycles: int = -1) -> None:

@@ -168,6 +168,14 @@ void ensure_lut(bm_ctx* ctx, uint32_t rmax) {
   float* dia = static_cast<float*>(ensure(ctx, ctx->lutf, ((size_t)target + 1) * sizeof(float), "diameter table"));
   check(ctx, launch_dia_table(static_cast<const uint4*>(p), target + 1, dia, ctx->stream, &ctx->launches),
         "diameter table");
+  const uint32_t nd = (target < kDiscMaxR2 ? target : kDiscMaxR2) + 1;
+  uint2* thr = static_cast<uint2*>(ensure(ctx, ctx->discthr, (size_t)nd * sizeof(uint2), "disc tables"));
+  uint32_t* tmpl = static_cast<uint32_t*>(ensure(ctx, ctx->disctmpl, (size_t)nd * sizeof(uint32_t), "disc tables"));
+  timed(ctx, KF_TEMPLATES, ctx->stream, "disc tables", [&] {
+    return launch_disc_tables(static_cast<const uint4*>(p), nd, thr, tmpl, ctx->stream, &ctx->launches);
+  });
+  // the phase that reads the tables may run on another stream
+  check(ctx, cudaStreamSynchronize(ctx->stream), "template tables");
 }
 
 void ensure_surf(bm_ctx* ctx, uint32_t rmax);
@@ -408,6 +416,67 @@ void run_phase(bm_ctx* ctx, Dims dm, const uint8_t* d_a, const uint8_t* d_b, int
 
   ensure_lut(ctx, hc.rmax);
   const uint4* lut = static_cast<const uint4*>(ctx->lut.ptr);
+  // cleanup, statistics and the readbacks that end the phase, from the r^2 map F
+  auto finish = [&](const uint32_t* F) {
+    StatsAccum* acc = static_cast<StatsAccum*>(ensure(ctx, ctx->accum, sizeof(StatsAccum), "stats"));
+    check(ctx, cudaMemsetAsync(acc, 0, sizeof(StatsAccum), s), "memset");
+    FixedPartial* part = static_cast<FixedPartial*>(
+        ensure(ctx, ctx->cpart, kCleanupMaxGrid * sizeof(FixedPartial), "stats partials"));
+    // every value of the map is at least 2 * scale (diameters are >= 2), so its
+    // f32 exponent is at least that of 2 * scale: the fixed-point base
+    const float two_s = 2.0f * scale;
+    uint32_t tb;
+    std::memcpy(&tb, &two_s, 4);
+    const int e2s = (int)(tb >> 23);
+    const int e_lo = (e2s >= 1 && e2s + kFixedSpan <= 254) ? e2s : 4096;  // 4096: no fixed-point path
+    unsigned cgrid = 0;
+    // the statistics' ordered sums read the f32 map: keep one when the caller wants none
+    float* cmap = (stats && !d_map) ? static_cast<float*>(ensure(ctx, ctx->ordmap, N * 4, "thickness map")) : d_map;
+    timed(ctx, KF_CLEAN_FINAL, s, "cleanup",
+          [&] {
+            return launch_cleanup(F, selbits, dm, static_cast<const float*>(ctx->lutf.ptr), scale, cmap, acc, part,
+                                  e_lo, &ctr->tile_next[1], &cgrid, s, &ctx->launches);
+          });
+    if (stats) ordered_sums(ctx, cmap, (long long)N, scale, acc, s);
+    std::vector<FixedPartial> hpart(cgrid);
+    check(ctx, cudaMemcpyAsync(&res.acc, acc, sizeof(StatsAccum), cudaMemcpyDeviceToHost, s), "stats readback");
+    if (stats)
+      check(ctx, cudaMemcpyAsync(res.osum, ctx->ordout.ptr, 2 * sizeof(double), cudaMemcpyDeviceToHost, s),
+            "stats readback");
+    if (cgrid)
+      check(ctx, cudaMemcpyAsync(hpart.data(), part, cgrid * sizeof(FixedPartial), cudaMemcpyDeviceToHost, s),
+            "stats readback");
+    check(ctx, cudaMemcpyAsync(&hc, ctr, sizeof hc, cudaMemcpyDeviceToHost, s), "counter readback");
+    check(ctx, cudaStreamSynchronize(s), "local thickness");
+    if (e_lo != 4096) fold_fixed_partials(res.acc, hpart.data(), cgrid, e_lo);
+    res.ridges = hc.ridges;
+  };
+  uint32_t* F = d_sq ? d_sq : B;
+  // The separable fill (discs.cu) up to radius 127, where its packed
+  // discs end; a forced site method or tile height asks for the
+  // tile fill.
+  const bool separable = hc.rmax <= kDiscMaxR2 && ctx->site_method == BM_SITES_AUTO && ctx->fill_rows == 0;
+  if (separable) {
+    uint16_t* rmap = static_cast<uint16_t*>(ensure(ctx, ctx->ridgemap, N * sizeof(uint16_t), "ridge map"));
+    const size_t lists = disc_header_count(dm);
+    uint32_t* hdr = static_cast<uint32_t*>(ensure(ctx, ctx->dischdr, lists * 4, "disc lists"));
+    uint2* ent = static_cast<uint2*>(ensure(ctx, ctx->discent, lists * kDiscSlots * sizeof(uint2), "disc lists"));
+    const size_t pool_cap = disc_pool_entries(dm);
+    uint2* pool = static_cast<uint2*>(ensure(ctx, ctx->discpool, pool_cap * sizeof(uint2), "disc lists"));
+    const uint2* thr = static_cast<const uint2*>(ctx->discthr.ptr);
+    const uint32_t* tmpl = static_cast<const uint32_t*>(ctx->disctmpl.ptr);
+    timed(ctx, KF_RIDGE, s, "ridge map", [&] { return launch_ridge_map(E, dm, thr, rmap, s, &ctx->launches); });
+    timed(ctx, KF_FILL_BIN, s, "disc lists", [&] {
+      return launch_disc_lists(rmap, dm, hc.rmax, tmpl, hdr, ent, pool, pool_cap, ctr, s, &ctx->launches);
+    });
+    timed(ctx, KF_FILL, s, "disc painting",
+          [&] { return launch_disc_paint(hdr, ent, pool, dm, hc.rmax, F, s, &ctx->launches); });
+    finish(F);
+    if (!hc.disc_overflow) return;
+    // the lists' pool ran out: again with the tile fill, in the lists' memory
+    for (Buffer* b : {&ctx->ridgemap, &ctx->discent, &ctx->discpool}) release(*b);
+    check(ctx, cudaMemsetAsync(ctr->tile_next, 0, sizeof ctr->tile_next, s), "memset");
+  }
   uint2* ridges = static_cast<uint2*>(ensure(ctx, ctx->ridges, (res.selected + 1) * sizeof(uint2), "ridge list"));
   const size_t rwords = (size_t)hc.rmax + 2;
   uint32_t* occ = static_cast<uint32_t*>(ensure(ctx, ctx->occ, rwords * 4, "r2 flags"));
@@ -417,40 +486,9 @@ void run_phase(bm_ctx* ctx, Dims dm, const uint8_t* d_a, const uint8_t* d_b, int
   timed(ctx, KF_RIDGE, s, "ridge kernel",
         [&] { return launch_ridges(E, selbits, dm, lut, ridges, ctr, occ, rbits, s, &ctx->launches); });
   const bool own_e = E != A && E != d_edt;  // E is the context's map: the chain passes may reuse it
-  uint32_t* F = fill_phase(ctx, dm, ridges, ctr, res.selected, hc.rmax, occ, selbits, A, B, own_e ? E : nullptr,
-                           rbits, d_sq ? d_sq : B, s);
-  StatsAccum* acc = static_cast<StatsAccum*>(ensure(ctx, ctx->accum, sizeof(StatsAccum), "stats"));
-  check(ctx, cudaMemsetAsync(acc, 0, sizeof(StatsAccum), s), "memset");
-  FixedPartial* part = static_cast<FixedPartial*>(
-      ensure(ctx, ctx->cpart, kCleanupMaxGrid * sizeof(FixedPartial), "stats partials"));
-  // every value of the map is at least 2 * scale (diameters are >= 2), so its
-  // f32 exponent is at least that of 2 * scale: the fixed-point base
-  const float two_s = 2.0f * scale;
-  uint32_t tb;
-  std::memcpy(&tb, &two_s, 4);
-  const int e2s = (int)(tb >> 23);
-  const int e_lo = (e2s >= 1 && e2s + kFixedSpan <= 254) ? e2s : 4096;  // 4096: no fixed-point path
-  unsigned cgrid = 0;
-  // the statistics' ordered sums read the f32 map: keep one when the caller wants none
-  float* cmap = (stats && !d_map) ? static_cast<float*>(ensure(ctx, ctx->ordmap, N * 4, "thickness map")) : d_map;
-  timed(ctx, KF_CLEAN_FINAL, s, "cleanup",
-        [&] {
-          return launch_cleanup(F, selbits, dm, static_cast<const float*>(ctx->lutf.ptr), scale, cmap, acc, part,
-                                e_lo, &ctr->tile_next[1], &cgrid, s, &ctx->launches);
-        });
-  if (stats) ordered_sums(ctx, cmap, (long long)N, scale, acc, s);
-  std::vector<FixedPartial> hpart(cgrid);
-  check(ctx, cudaMemcpyAsync(&res.acc, acc, sizeof(StatsAccum), cudaMemcpyDeviceToHost, s), "stats readback");
-  if (stats)
-    check(ctx, cudaMemcpyAsync(res.osum, ctx->ordout.ptr, 2 * sizeof(double), cudaMemcpyDeviceToHost, s),
-          "stats readback");
-  if (cgrid)
-    check(ctx, cudaMemcpyAsync(hpart.data(), part, cgrid * sizeof(FixedPartial), cudaMemcpyDeviceToHost, s),
-          "stats readback");
-  check(ctx, cudaMemcpyAsync(&hc, ctr, sizeof hc, cudaMemcpyDeviceToHost, s), "counter readback");
-  check(ctx, cudaStreamSynchronize(s), "local thickness");
-  if (e_lo != 4096) fold_fixed_partials(res.acc, hpart.data(), cgrid, e_lo);
-  res.ridges = hc.ridges;
+  // (after the separable fill, B no longer holds the y pass output the chain passes need)
+  const bool chains = own_e && !separable;
+  finish(fill_phase(ctx, dm, ridges, ctr, res.selected, hc.rmax, occ, selbits, A, B, chains ? E : nullptr, rbits, F, s));
 }
 
 // nonzero_stats (metrics.rs:228-241; quantile fields NaN) from the reference's
@@ -958,7 +996,7 @@ std::vector<Buffer*> work_buffers(bm_ctx* ctx) {
           &ctx->cpart,     &ctx->outmap,     &ctx->outmap2,     &ctx->occ,     &ctx->rank,   &ctx->rvals,
           &ctx->bincounts, &ctx->binoffsets, &ctx->binentries,  &ctx->scanscratch, &ctx->redo, &ctx->qhist,
           &ctx->qtargets,  &ctx->qmap,       &ctx->rgeo,        &ctx->ordmap,  &ctx->ordscratch, &ctx->ordout,
-          &ctx->tileorder};
+          &ctx->tileorder, &ctx->ridgemap,   &ctx->dischdr,     &ctx->discent, &ctx->discpool};
 }
 
 size_t cached_bytes(const bm_ctx* ctx) {
@@ -1039,6 +1077,8 @@ void bm_ctx_destroy(bm_ctx* ctx) {
     release(ctx->surf_off);
     release(ctx->surf_pts);
     release(ctx->lutf);
+    release(ctx->discthr);
+    release(ctx->disctmpl);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
   }
   delete ctx;

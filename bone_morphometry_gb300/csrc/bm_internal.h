@@ -157,6 +157,9 @@ struct Counters {  // device-side counters of one phase
   unsigned int rmax;
   unsigned int status;          // nonzero: a bounded wait gave up / capacity exceeded
   unsigned int tile_next[2];    // next tile to take: ridge pass, cleanup pass (dynamic tile scheduling)
+  unsigned long long disc_pool; // entries of the disc lists' overflow pool handed out
+  unsigned int disc_overflow;   // nonzero: the pool was too small
+  unsigned int pad;
 };
 
 // Kernel families timed by the context's profiler (bm_profile_*).
@@ -228,6 +231,8 @@ struct bm_ctx {
   bm::Buffer bincounts, binoffsets, binentries, scanscratch;
   // cached sphere lattice-point table for r2 in [0, surf_max]
   bm::Buffer surf_off, surf_pts;
+  // separable fill: u16 ridge map, list headers and disc lists; cached tables by squared radius
+  bm::Buffer ridgemap, dischdr, discent, discpool, discthr, disctmpl;
   bm::Buffer redo;             // per-line flags of the windowed EDT passes
   bm::Buffer qhist, qtargets, qmap;  // quantile histograms, targets, map scratch
   bm::Buffer ordmap, ordscratch, ordout;  // f32 map for the ordered sums, their scratch, their two results

@@ -87,6 +87,33 @@ cudaError_t launch_cleanup(const uint32_t* fillmap, const uint32_t* selbits, Dim
                            unsigned* grid, cudaStream_t s, unsigned long long* launches);
 cudaError_t launch_dia_table(const uint4* lut, uint32_t n, float* dia, cudaStream_t s, unsigned long long* launches);
 
+// Separable fill (discs.cu), for squared radii up to kDiscMaxR2: offsets from a
+// ball's centre are kept in 8 bits.
+constexpr int kDiscMaxHalo = 127;
+constexpr uint32_t kDiscMaxR2 = kDiscMaxHalo * kDiscMaxHalo;
+constexpr int kDiscPX = 32, kDiscPY = 8;   // columns per list patch
+constexpr uint32_t kDiscSlots = 384;       // discs per patch and plane (1.5 per column)
+size_t disc_header_count(Dims dm);
+// thr / tmpl: n entries by squared radius, from the search templates.
+cudaError_t launch_disc_tables(const uint4* lut, uint32_t n, uint2* thr, uint32_t* tmpl, cudaStream_t s,
+                               unsigned long long* launches);
+// The distance ridge as a u16 map (0: not selected, 1: selected, 2 R + 1: ridge of squared radius R).
+cudaError_t launch_ridge_map(const uint32_t* dist, Dims dm, const uint2* thr, uint16_t* rmap, cudaStream_t s,
+                             unsigned long long* launches);
+// Disc lists: hdr[patch] = count | reach << 16 for every 32 x 8 patch of every
+// plane (disc_header_count), its discs {R << 16 | rho, column | (first row +
+// 128) << 8 | (last row + 128) << 16} (rows from the centre's) at
+// ent[patch * kDiscSlots].  A patch with more than kDiscSlots discs has them at
+// pool[ent[patch * kDiscSlots].x]; a pool that is too small (disc_pool_entries)
+// sets ctr->disc_overflow and leaves lists out.  ctr->disc_pool must be 0.
+size_t disc_pool_entries(Dims dm);
+cudaError_t launch_disc_lists(const uint16_t* rmap, Dims dm, uint32_t rmax, const uint32_t* tmpl, uint32_t* hdr,
+                              uint2* ent, uint2* pool, size_t pool_cap, Counters* ctr, cudaStream_t s,
+                              unsigned long long* launches);
+// The u32 r^2 map (selected voxels and the sites that spheres reach, 0 elsewhere).
+cudaError_t launch_disc_paint(const uint32_t* hdr, const uint2* ent, const uint2* pool, Dims dm, uint32_t rmax,
+                              uint32_t* fillmap, cudaStream_t s, unsigned long long* launches);
+
 // Tile-owned fill (fill.cu).
 // Rows of y per fill tile: 64 for volumes of at least kFillTallMinVoxels (fewer
 // ball entries per voxel), 32 from kFillMidMinVoxels, else 16 (more tiles: a

@@ -299,10 +299,12 @@ extern "C" {
 
 uint64_t bm_footprint_bytes(size_t width, size_t height, size_t depth) {
   // per voxel: inputs 2; per phase (the two phases run side by side, each on
-  // its own buffers): four u32 maps 16 (x/y pass, z pass, chain map), envelope
-  // scratch 8, ridge records <= 8, bin entries ~5, f32 thickness map 4 (read by
-  // the statistics' ordered sums, ~0.2 more of their scratch), quantile map 4,
-  // bitmasks ~1; tables 2 x 64 MiB
+  // its own buffers): three u32 maps 12 (x/y pass, z pass), envelope scratch 8,
+  // u16 ridge map 2, disc lists 12.5, f32 thickness map 4 (read by the
+  // statistics' ordered sums, ~0.2 more of their scratch), quantile map 4,
+  // bitmasks ~1; the tile fill (radii above 127) takes a chain map 4, ridge
+  // records <= 8 and bin entries ~5 in place of the ridge map and the lists;
+  // tables 2 x 64 MiB
   const uint64_t n = (uint64_t)width * height * depth;
   return n * 95u + (128ull << 20);
 }

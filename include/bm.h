@@ -285,21 +285,24 @@ int bm_tiff_read(const char* path, unsigned threshold, int accepted, uint8_t* ou
 int bm_ctx_set_concurrent_phases(bm_ctx* ctx, int on);
 
 /* How the sphere fill finds the non-selected voxels a ridge ball reaches
- * (local_thickness.rs:169-202 paints them too): BM_SITES_SPHERES tests every
- * lattice point of every ridge sphere; BM_SITES_CHAINS pushes the ridge r^2
- * backwards along the distance transform's tied argmins (two window passes
- * over the volume, two more u32 maps of device memory); BM_SITES_AUTO (the
- * default) picks chains when the spheres' lattice points would take the site
- * test more than 0.2 half-warp steps per voxel of the volume.  Results are
- * identical either way. */
+ * (local_thickness.rs:169-202 paints them too).  BM_SITES_AUTO (the default)
+ * lets the separable fill paint them with the others, up to a largest radius
+ * of 127 voxels; beyond, and with the other two settings, the tile fill paints
+ * the selected voxels and BM_SITES_SPHERES tests every lattice point of every
+ * ridge sphere, BM_SITES_CHAINS pushes the ridge r^2 backwards along the
+ * distance transform's tied argmins (two window passes over the volume, two
+ * more u32 maps of device memory), BM_SITES_AUTO picks chains when the spheres'
+ * lattice points would take the site test more than 0.2 half-warp steps per
+ * voxel of the volume.  Results are identical either way. */
 enum { BM_SITES_AUTO = 0, BM_SITES_SPHERES = 1, BM_SITES_CHAINS = 2 };
 int bm_ctx_set_site_method(bm_ctx* ctx, int method);
 
-/* Rows of y in the sphere fill's tiles (32 x rows x 16 voxels): 0 (the
- * default) picks 64 for volumes of at least 3 * 2^24 voxels (fewer ball
- * entries and plane tests per voxel), 32 from 2^24 voxels and 16 below (more
- * tiles, shorter serial chains); 16, 32 or 64 forces it.  Results are
- * identical either way. */
+/* Rows of y in the tile fill's tiles (32 x rows x 16 voxels): 16, 32 or 64
+ * makes every fill a tile fill of that height.  0 (the default) leaves the
+ * choice to the largest radius: the separable fill up to 127 voxels, beyond it
+ * the tile fill with 64 rows for volumes of at least 3 * 2^24 voxels (fewer
+ * ball entries and plane tests per voxel), 32 from 2^24 voxels and 16 below
+ * (more tiles, shorter serial chains).  Results are identical either way. */
 int bm_ctx_set_fill_tile_rows(bm_ctx* ctx, int rows);
 
 /* Cycle limit of the device-side bounded waits of this context's kernels (the
