@@ -416,8 +416,11 @@ void run_phase(bm_ctx* ctx, Dims dm, const uint8_t* d_a, const uint8_t* d_b, int
 
   ensure_lut(ctx, hc.rmax);
   const uint4* lut = static_cast<const uint4*>(ctx->lut.ptr);
-  // cleanup, statistics and the readbacks that end the phase, from the r^2 map F
-  auto finish = [&](const uint32_t* F) {
+  const float* dia = static_cast<const float*>(ctx->lutf.ptr);
+  // cleanup, statistics and the readbacks that end the phase, from the fill's diameters and nonzero bits
+  uint32_t* nzbits = static_cast<uint32_t*>(ensure(ctx, ctx->nzbits, bits_bytes, "nonzero bits"));
+  uint32_t* inbits = static_cast<uint32_t*>(ensure(ctx, ctx->inbits, bits_bytes, "interior bits"));
+  auto finish = [&](const float* dmap) {
     StatsAccum* acc = static_cast<StatsAccum*>(ensure(ctx, ctx->accum, sizeof(StatsAccum), "stats"));
     check(ctx, cudaMemsetAsync(acc, 0, sizeof(StatsAccum), s), "memset");
     FixedPartial* part = static_cast<FixedPartial*>(
@@ -434,8 +437,8 @@ void run_phase(bm_ctx* ctx, Dims dm, const uint8_t* d_a, const uint8_t* d_b, int
     float* cmap = (stats && !d_map) ? static_cast<float*>(ensure(ctx, ctx->ordmap, N * 4, "thickness map")) : d_map;
     timed(ctx, KF_CLEAN_FINAL, s, "cleanup",
           [&] {
-            return launch_cleanup(F, selbits, dm, static_cast<const float*>(ctx->lutf.ptr), scale, cmap, acc, part,
-                                  e_lo, &ctr->tile_next[1], &cgrid, s, &ctx->launches);
+            return launch_cleanup(dmap, selbits, nzbits, inbits, dm, scale, cmap, acc, part, e_lo, &cgrid, s,
+                                  &ctx->launches);
           });
     if (stats) ordered_sums(ctx, cmap, (long long)N, scale, acc, s);
     std::vector<FixedPartial> hpart(cgrid);
@@ -451,7 +454,6 @@ void run_phase(bm_ctx* ctx, Dims dm, const uint8_t* d_a, const uint8_t* d_b, int
     if (e_lo != 4096) fold_fixed_partials(res.acc, hpart.data(), cgrid, e_lo);
     res.ridges = hc.ridges;
   };
-  uint32_t* F = d_sq ? d_sq : B;
   // The separable fill (discs.cu) up to radius 127, where its packed
   // discs end; a forced site method or tile height asks for the
   // tile fill.
@@ -469,13 +471,14 @@ void run_phase(bm_ctx* ctx, Dims dm, const uint8_t* d_a, const uint8_t* d_b, int
     timed(ctx, KF_FILL_BIN, s, "disc lists", [&] {
       return launch_disc_lists(rmap, dm, hc.rmax, tmpl, hdr, ent, pool, pool_cap, ctr, s, &ctx->launches);
     });
-    timed(ctx, KF_FILL, s, "disc painting",
-          [&] { return launch_disc_paint(hdr, ent, pool, dm, hc.rmax, F, s, &ctx->launches); });
-    finish(F);
+    float* dmap = reinterpret_cast<float*>(B);  // the y pass output has been read
+    timed(ctx, KF_FILL, s, "disc painting", [&] {
+      return launch_disc_paint(hdr, ent, pool, dm, hc.rmax, dia, dmap, nzbits, d_sq, s, &ctx->launches);
+    });
+    finish(dmap);
     if (!hc.disc_overflow) return;
     // the lists' pool ran out: again with the tile fill, in the lists' memory
     for (Buffer* b : {&ctx->ridgemap, &ctx->discent, &ctx->discpool}) release(*b);
-    check(ctx, cudaMemsetAsync(ctr->tile_next, 0, sizeof ctr->tile_next, s), "memset");
   }
   uint2* ridges = static_cast<uint2*>(ensure(ctx, ctx->ridges, (res.selected + 1) * sizeof(uint2), "ridge list"));
   const size_t rwords = (size_t)hc.rmax + 2;
@@ -488,7 +491,12 @@ void run_phase(bm_ctx* ctx, Dims dm, const uint8_t* d_a, const uint8_t* d_b, int
   const bool own_e = E != A && E != d_edt;  // E is the context's map: the chain passes may reuse it
   // (after the separable fill, B no longer holds the y pass output the chain passes need)
   const bool chains = own_e && !separable;
-  finish(fill_phase(ctx, dm, ridges, ctr, res.selected, hc.rmax, occ, selbits, A, B, chains ? E : nullptr, rbits, F, s));
+  uint32_t* F = fill_phase(ctx, dm, ridges, ctr, res.selected, hc.rmax, occ, selbits, A, B, chains ? E : nullptr,
+                           rbits, d_sq ? d_sq : B, s);
+  float* dmap = reinterpret_cast<float*>(F == d_sq ? B : F);
+  timed(ctx, KF_CLEAN_FINAL, s, "diameters",
+        [&] { return launch_diameters(F, dm, dia, dmap, nzbits, s, &ctx->launches); });
+  finish(dmap);
 }
 
 // nonzero_stats (metrics.rs:228-241; quantile fields NaN) from the reference's
@@ -996,7 +1004,8 @@ std::vector<Buffer*> work_buffers(bm_ctx* ctx) {
           &ctx->cpart,     &ctx->outmap,     &ctx->outmap2,     &ctx->occ,     &ctx->rank,   &ctx->rvals,
           &ctx->bincounts, &ctx->binoffsets, &ctx->binentries,  &ctx->scanscratch, &ctx->redo, &ctx->qhist,
           &ctx->qtargets,  &ctx->qmap,       &ctx->rgeo,        &ctx->ordmap,  &ctx->ordscratch, &ctx->ordout,
-          &ctx->tileorder, &ctx->ridgemap,   &ctx->dischdr,     &ctx->discent, &ctx->discpool};
+          &ctx->tileorder, &ctx->ridgemap,   &ctx->dischdr,     &ctx->discent, &ctx->discpool,
+          &ctx->nzbits,    &ctx->inbits};
 }
 
 size_t cached_bytes(const bm_ctx* ctx) {

@@ -156,7 +156,8 @@ struct Counters {  // device-side counters of one phase
   unsigned long long ridges;
   unsigned int rmax;
   unsigned int status;          // nonzero: a bounded wait gave up / capacity exceeded
-  unsigned int tile_next[2];    // next tile to take: ridge pass, cleanup pass (dynamic tile scheduling)
+  unsigned int tile_next;       // next tile to take in the ridge pass (dynamic tile scheduling)
+  unsigned int pad0;
   unsigned long long disc_pool; // entries of the disc lists' overflow pool handed out
   unsigned int disc_overflow;   // nonzero: the pool was too small
   unsigned int pad;
@@ -217,6 +218,7 @@ struct bm_ctx {
   bm::Buffer stack;            // EDT line scratch
   bm::Buffer fillmap;          // u32 propagated r^2
   bm::Buffer selbits, ridgebits; // row-padded bitmasks: selected voxels, ridge voxels
+  bm::Buffer nzbits, inbits;   // the r^2 map's nonzero voxels, and those without a zero 26-neighbour
   bm::Buffer ridges;           // ridge records
   bm::Buffer counters;         // bm::Counters
   bm::Buffer roicount;         // ROI and bone-in-ROI voxel counts (the bails of bm_tbth_tbsp)

@@ -395,7 +395,8 @@ constexpr int kQueue = 64;                 // discs a warp holds back until 32 a
 template <int TY>
 __global__ void __launch_bounds__(8 * TY, 64 / TY * 2)
 disc_paint_kernel(const uint32_t* __restrict__ hdr, const uint2* __restrict__ ent, const uint2* __restrict__ pool,
-                  Dims dm, int H, int kmax, int npx, int npy, int ntx, int nty, uint32_t* __restrict__ fillmap) {
+                  Dims dm, int H, int kmax, int npx, int npy, int ntx, int nty, const float* __restrict__ dia,
+                  float* __restrict__ dmap, uint32_t* __restrict__ nzbits, uint32_t* __restrict__ fillmap) {
   extern __shared__ __align__(16) uint32_t lev[];  // (kmax + 1) levels of TY rows
   constexpr int kPlane = TY * kPaintStride;
   constexpr int kPaintThreads = 8 * TY, kPaintWarps = kPaintThreads / 32;
@@ -406,7 +407,10 @@ disc_paint_kernel(const uint32_t* __restrict__ hdr, const uint2* __restrict__ en
   const long long bid = blockIdx.x;
   const int tx = (int)(bid % ntx), ty = (int)((bid / ntx) % nty), z = (int)(bid / ((long long)ntx * nty));
   const int x0 = tx * kPaintX, y0 = ty * TY;
-  uint32_t* out = fillmap + ((long long)z * dm.h + y0) * dm.w + x0;
+  const long long first = ((long long)z * dm.h + y0) * dm.w + x0;
+  float* out = dmap + first;
+  const int nw = dm.nw();
+  uint32_t* outbits = nzbits + ((long long)z * dm.h + y0) * nw + (x0 >> 5);
   const int px0 = max(x0 - H, 0) / kDiscPX, px1 = min(x0 + kPaintX - 1 + H, dm.w - 1) / kDiscPX;
   const int py0 = max(y0 - H, 0) / kDiscPY, py1 = min(y0 + TY - 1 + H, dm.h - 1) / kDiscPY;
   const int nhx = px1 - px0 + 1, nh = nhx * (py1 - py0 + 1);
@@ -429,7 +433,11 @@ disc_paint_kernel(const uint32_t* __restrict__ hdr, const uint2* __restrict__ en
   const int vx = min(kPaintX, dm.w - x0), vy = min(TY, dm.h - y0);
   if (patches == 0) {  // no disc in reach: all zero
     for (int y = warp; y < vy; y += kPaintWarps)
-      for (int x = lane; x < vx; x += 32) out[(long long)y * dm.w + x] = 0u;
+      for (int x = lane; x < vx; x += 32) {
+        out[(long long)y * dm.w + x] = 0.0f;
+        if (fillmap) fillmap[first + (long long)y * dm.w + x] = 0u;
+        if (lane == 0) outbits[(long long)y * nw + (x >> 5)] = 0u;
+      }
     return;
   }
   static_assert(kPlane % 4 == 0, "cleared 16 bytes at a time");
@@ -553,8 +561,19 @@ disc_paint_kernel(const uint32_t* __restrict__ hdr, const uint2* __restrict__ en
       a = max3(a, sa, lk[lane]);
       b = max3(b, sb, lk[lane + 32]);
     }
-    if (lane < vx) out[(long long)y * dm.w + lane] = a;
-    if (lane + 32 < vx) out[(long long)y * dm.w + lane + 32] = b;
+    const long long at = (long long)y * dm.w + lane;
+    if (lane < vx) {
+      out[at] = __ldg(dia + a);
+      if (fillmap) fillmap[first + at] = a;
+    }
+    if (lane + 32 < vx) {
+      out[at + 32] = __ldg(dia + b);
+      if (fillmap) fillmap[first + at + 32] = b;
+    }
+    const unsigned ma = __ballot_sync(0xffffffffu, lane < vx && a != 0u);
+    const unsigned mb = __ballot_sync(0xffffffffu, lane + 32 < vx && b != 0u);
+    if (lane == 0) outbits[(long long)y * nw] = ma;
+    if (lane == 0 && vx > 32) outbits[(long long)y * nw + 1] = mb;
   }
 }
 
@@ -624,8 +643,8 @@ cudaError_t launch_disc_lists(const uint16_t* rmap, Dims dm, uint32_t rmax, cons
 
 namespace {
 template <int TY>
-cudaError_t paint_rows(const uint32_t* hdr, const uint2* ent, const uint2* pool, Dims dm, int H, uint32_t* fillmap,
-                       cudaStream_t s) {
+cudaError_t paint_rows(const uint32_t* hdr, const uint2* ent, const uint2* pool, Dims dm, int H, const float* dia,
+                       float* dmap, uint32_t* nzbits, uint32_t* fillmap, cudaStream_t s) {
   int kmax = 0;  // largest level a chord of at most min(2 H + 1, 64) voxels writes (two cells of 32 cover 64)
   while (kmax < 5 && (2 << kmax) <= 2 * H + 1) ++kmax;
   const int npx = (dm.w + kDiscPX - 1) / kDiscPX, npy = (dm.h + kDiscPY - 1) / kDiscPY;
@@ -637,17 +656,18 @@ cudaError_t paint_rows(const uint32_t* hdr, const uint2* ent, const uint2* pool,
                                        (int)(6 * level));
   if (e != cudaSuccess) return e;
   disc_paint_kernel<TY><<<(unsigned)((long long)ntx * nty * dm.d), 8 * TY, (kmax + 1) * level, s>>>(
-      hdr, ent, pool, dm, H, kmax, npx, npy, ntx, nty, fillmap);
+      hdr, ent, pool, dm, H, kmax, npx, npy, ntx, nty, dia, dmap, nzbits, fillmap);
   return cudaGetLastError();
 }
 }  // namespace
 
 cudaError_t launch_disc_paint(const uint32_t* hdr, const uint2* ent, const uint2* pool, Dims dm, uint32_t rmax,
-                              uint32_t* fillmap, cudaStream_t s, unsigned long long* launches) {
+                              const float* dia, float* dmap, uint32_t* nzbits, uint32_t* fillmap, cudaStream_t s,
+                              unsigned long long* launches) {
   ++*launches;
   const int H = halo_of(rmax);
-  return dm.n() >= (1ll << 22) ? paint_rows<64>(hdr, ent, pool, dm, H, fillmap, s)
-                               : paint_rows<32>(hdr, ent, pool, dm, H, fillmap, s);
+  return dm.n() >= (1ll << 22) ? paint_rows<64>(hdr, ent, pool, dm, H, dia, dmap, nzbits, fillmap, s)
+                               : paint_rows<32>(hdr, ent, pool, dm, H, dia, dmap, nzbits, fillmap, s);
 }
 
 }  // namespace bm

@@ -75,16 +75,20 @@ cudaError_t launch_chain_y(const uint32_t* f, const uint32_t* g, const uint32_t*
 cudaError_t launch_fill(const uint2* ridges, const Counters* ctr, unsigned long long max_ridges, Dims dm,
                         uint32_t* fillmap, cudaStream_t s, unsigned long long* launches);
 
-// Fused cleanup passes 1 and 2, phase mask, optional f32 map, exact statistics.
-// dia: f32 diameters 2*sqrt(r2) by r2 (launch_dia_table).
+// Cleanup passes 1 and 2, phase mask, optional f32 map, exact statistics.
+// dmap: the fill's diameters 2*sqrt(r2) (0 where no ball reaches); nzbits: its
+// nonzero voxels as a row-padded bitmask; inbits: scratch of its size.  The
+// separable fill writes both; launch_diameters makes them of an r2 map (dmap
+// may be the map's memory).  dia: f32 diameters by r2 (launch_dia_table).
 // Values whose f32 exponent lies in [e_lo, e_lo + kFixedSpan] are summed in
 // fixed point, one FixedPartial per CTA in part[0 .. *grid); the others go to
 // acc's per-exponent sums.  At most kCleanupMaxGrid CTAs.
 constexpr unsigned kCleanupMaxGrid = 4096;
-// tile_next: a zeroed counter the CTAs take tiles from.
-cudaError_t launch_cleanup(const uint32_t* fillmap, const uint32_t* selbits, Dims dm, const float* dia, float scale,
-                           float* outmap, StatsAccum* acc, FixedPartial* part, int e_lo, unsigned* tile_next,
-                           unsigned* grid, cudaStream_t s, unsigned long long* launches);
+cudaError_t launch_diameters(const uint32_t* fillmap, Dims dm, const float* dia, float* dmap, uint32_t* nzbits,
+                             cudaStream_t s, unsigned long long* launches);
+cudaError_t launch_cleanup(const float* dmap, const uint32_t* selbits, const uint32_t* nzbits, uint32_t* inbits, Dims dm,
+                           float scale, float* outmap, StatsAccum* acc, FixedPartial* part, int e_lo, unsigned* grid,
+                           cudaStream_t s, unsigned long long* launches);
 cudaError_t launch_dia_table(const uint4* lut, uint32_t n, float* dia, cudaStream_t s, unsigned long long* launches);
 
 // Separable fill (discs.cu), for squared radii up to kDiscMaxR2: offsets from a
@@ -110,9 +114,12 @@ size_t disc_pool_entries(Dims dm);
 cudaError_t launch_disc_lists(const uint16_t* rmap, Dims dm, uint32_t rmax, const uint32_t* tmpl, uint32_t* hdr,
                               uint2* ent, uint2* pool, size_t pool_cap, Counters* ctr, cudaStream_t s,
                               unsigned long long* launches);
-// The u32 r^2 map (selected voxels and the sites that spheres reach, 0 elsewhere).
+// The fill's diameters (selected voxels and the sites that spheres reach, 0
+// elsewhere; dia: diameters by r^2), their nonzero voxels as a row-padded
+// bitmask and, when fillmap is not null, the r^2 map.
 cudaError_t launch_disc_paint(const uint32_t* hdr, const uint2* ent, const uint2* pool, Dims dm, uint32_t rmax,
-                              uint32_t* fillmap, cudaStream_t s, unsigned long long* launches);
+                              const float* dia, float* dmap, uint32_t* nzbits, uint32_t* fillmap, cudaStream_t s,
+                              unsigned long long* launches);
 
 // Tile-owned fill (fill.cu).
 // Rows of y per fill tile: 64 for volumes of at least kFillTallMinVoxels (fewer
