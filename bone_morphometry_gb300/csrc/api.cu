@@ -538,65 +538,27 @@ int finish_stats(bm_ctx* ctx, const StatsAccum& a, const double* osum, bm_stats*
 void quantiles(bm_ctx* ctx, const float* d_map, long long n, unsigned long long count, double scale,
                bm_stats* out, cudaStream_t s) {
   static const double kQ[5] = {0.5, 0.1, 0.25, 0.75, 0.9};  // metrics.rs:247-251
-  unsigned long long ranks[10];
+  QuantileState qs{};
   double frac[5];
   for (int i = 0; i < 5; ++i) {
     const double position = kQ[i] * (double)(count - 1);
     const double lo = std::floor(position), hi = std::ceil(position);
-    ranks[2 * i] = (unsigned long long)lo;
-    ranks[2 * i + 1] = (unsigned long long)hi;
+    qs.rank[2 * i] = (unsigned long long)lo;
+    qs.rank[2 * i + 1] = (unsigned long long)hi;
     frac[i] = position - lo;
   }
-  uint32_t* hist = static_cast<uint32_t*>(ensure(ctx, ctx->qhist, (size_t)17 * 65536 * 4, "quantile histograms"));
-  uint32_t* dtargets = static_cast<uint32_t*>(ensure(ctx, ctx->qtargets, 16 * 4, "quantile targets"));
-  check(ctx, cudaMemsetAsync(hist, 0, (size_t)65536 * 4, s), "memset");
-  timed(ctx, KF_QUANTILE, s, "quantile histogram", [&] { return launch_hist_hi(d_map, n, hist, s, &ctx->launches); });
-  std::vector<uint32_t> hh(65536);
-  check(ctx, cudaMemcpyAsync(hh.data(), hist, 65536 * 4, cudaMemcpyDeviceToHost, s), "histogram readback");
-  check(ctx, cudaStreamSynchronize(s), "quantile histogram");
-  // locate every rank's high-16 bin and its rank inside that bin
-  uint32_t tgt[10];
-  unsigned long long resid[10];
-  for (int r = 0; r < 10; ++r) {
-    unsigned long long cum = 0;
-    uint32_t b = 0;
-    for (; b < 65536; ++b) {
-      if (cum + hh[b] > ranks[r]) break;
-      cum += hh[b];
-    }
-    if (b == 65536) fail(ctx, BM_ERR_CUDA, "quantile rank %llu beyond %llu values", ranks[r], cum);
-    tgt[r] = b;
-    resid[r] = ranks[r] - cum;
-  }
-  uint32_t uniq[10];
-  int nu = 0;
-  int slot_of[10];
-  for (int r = 0; r < 10; ++r) {
-    int j = 0;
-    while (j < nu && uniq[j] != tgt[r]) ++j;
-    if (j == nu) uniq[nu++] = tgt[r];
-    slot_of[r] = j;
-  }
-  uint32_t* lo = hist + 65536;
-  check(ctx, cudaMemcpyAsync(dtargets, uniq, (size_t)nu * 4, cudaMemcpyHostToDevice, s), "targets upload");
-  check(ctx, cudaMemsetAsync(lo, 0, (size_t)nu * 65536 * 4, s), "memset");
-  timed(ctx, KF_QUANTILE, s, "quantile histogram",
-        [&] { return launch_hist_lo(d_map, n, dtargets, nu, lo, s, &ctx->launches); });
-  std::vector<uint32_t> hl((size_t)nu * 65536);
-  check(ctx, cudaMemcpyAsync(hl.data(), lo, hl.size() * 4, cudaMemcpyDeviceToHost, s), "histogram readback");
-  check(ctx, cudaStreamSynchronize(s), "quantile histogram");
-  double v[10];
-  for (int r = 0; r < 10; ++r) {
-    const uint32_t* h = hl.data() + (size_t)slot_of[r] * 65536;
-    unsigned long long cum = 0;
-    uint32_t b = 0;
-    for (; b < 65536; ++b) {
-      if (cum + h[b] > resid[r]) break;
-      cum += h[b];
-    }
-    const uint32_t bits = (tgt[r] << 16) | b;
+  uint32_t* hist = static_cast<uint32_t*>(ensure(ctx, ctx->qhist, quantile_scratch_words() * 4, "quantile histograms"));
+  QuantileState* dq = static_cast<QuantileState*>(ensure(ctx, ctx->qtargets, sizeof(QuantileState), "quantile ranks"));
+  check(ctx, cudaMemcpyAsync(dq, &qs, sizeof qs, cudaMemcpyHostToDevice, s), "ranks upload");
+  timed(ctx, KF_QUANTILE, s, "quantiles", [&] { return launch_quantiles(d_map, n, hist, dq, s, &ctx->launches); });
+  check(ctx, cudaMemcpyAsync(&qs, dq, sizeof qs, cudaMemcpyDeviceToHost, s), "quantile readback");
+  check(ctx, cudaStreamSynchronize(s), "quantiles");
+  double v[kQuantileRanks];
+  for (int r = 0; r < kQuantileRanks; ++r) {
+    if (qs.bits[r] == 0xffffffffu)
+      fail(ctx, BM_ERR_CUDA, "quantile rank %llu beyond the %llu values", qs.rank[r], count);
     float f;
-    std::memcpy(&f, &bits, 4);
+    std::memcpy(&f, &qs.bits[r], 4);
     v[r] = (double)f;
   }
   const float sf = (float)scale;

@@ -170,11 +170,20 @@ cudaError_t launch_ordered_sums(const float* map, long long n, float scale, cons
 // Exact moment sums of f32(raw * scale) over the finite positive raw values.
 cudaError_t launch_moments(const float* map, long long n, float scale, StatsAccum* acc, cudaStream_t s,
                            unsigned long long* launches);
-// Quantiles (quantile.cu): histogram of the high 16 bits of the positive finite
-// f32 values, and of the low 16 bits for values whose high bits equal one of
-// ntarget (<= 16) targets (hist laid out [target][65536]).
-cudaError_t launch_hist_hi(const float* map, long long n, uint32_t* hist, cudaStream_t s, unsigned long long* launches);
-cudaError_t launch_hist_lo(const float* map, long long n, const uint32_t* targets, int ntarget, uint32_t* hist,
-                           cudaStream_t s, unsigned long long* launches);
+// Exact order statistics (quantile.cu): q->bits[r] = the f32 bits of the value
+// of rank q->rank[r] (0-based) among the finite positive values of map[0 .. n);
+// 0xffffffff when there is none.  scratch: quantile_scratch_words() words.
+constexpr int kQuantileRanks = 10;
+struct QuantileState {
+  unsigned long long rank[kQuantileRanks];   // in
+  unsigned long long resid[kQuantileRanks];  // rank inside its high bin
+  uint32_t target[kQuantileRanks];           // the distinct high bins
+  uint32_t slot[kQuantileRanks];             // each rank's index into target
+  uint32_t targets;
+  uint32_t bits[kQuantileRanks];             // out
+};
+size_t quantile_scratch_words();
+cudaError_t launch_quantiles(const float* map, long long n, uint32_t* scratch, QuantileState* q, cudaStream_t s,
+                             unsigned long long* launches);
 
 }  // namespace bm
