@@ -20,28 +20,36 @@
 // reached 2^(E+1) exactly, which both roundings agree on); otherwise the run
 // crossed into the next binade and its elements are replayed.
 //
-// The pipeline.  The map is cut into chunks of kChunk voxels in index order.
+// The pipeline.  The map is cut into chunks of kChunk voxels in index order,
+// 32 chunks make a block.
 //   1. approximate sums of v and v*v per chunk (f32, on values scaled by a
-//      power of two) and per block of 32 chunks (fixed point);
-//   2. an exclusive scan of the block sums: approximate prefix sums;
-//   3. per chunk, the binade the running sum is predicted to stay in (from the
-//      approximate prefix, with a relative margin), and the chunk's function
-//      for that binade, folded value by value by one thread; per block of 32
-//      chunks, the composition when all its chunks share one binade;
-//   4. compositions of 32 blocks at each further level;
-//   5. a walker (one warp per sum) that follows the sequence from s = 0: it
-//      skips empty runs before the first value, applies the largest aligned
-//      run whose predicted binade is the one s is in and whose result stays
-//      in it (32 entries of a level at a time, composed by a warp
-//      reduction), and replays a chunk where no prediction holds -- at the
-//      ~30 binade crossings of each sum: lanes fold their values, a warp
-//      scan finds the lane whose values leave the binade, and that lane adds
-//      them one by one (integer increments of s/U, and a hardware f64
-//      addition, the reference's own operation, for the value that crosses).
-// Every step the walker takes is checked against the exact state, so a wrong
-// prediction costs time, never exactness.  No per-value f64 arithmetic: the
-// GB300's f64 rate is a small fraction of its f32 and integer rates.  Not a
-// reference function: the reference's loop is serial (metrics.rs:215-226).
+//      power of two), per block and per 32, 1024 and 32768 blocks (fixed point);
+//   2. per chunk, the binade the running sum is predicted to stay in (from the
+//      approximate prefix, with a relative margin) and the chunk's function for
+//      that binade.  Without a tie a value's increment does not depend on the
+//      parity, and increments add up in any order: the lanes sum them.  A chunk
+//      with a tie (or +inf) is folded in order.  Per block of 32 chunks, and on
+//      further levels of 32, the composition when all share one binade;
+//   3. a walker per sum.  The blocks whose composition is invalid -- the ~30
+//      binade crossings -- are listed by step 2; the walker's warps compose the
+//      runs of blocks between them, and inside each of them the chunks before
+//      the first and after the last unpredicted chunk.  One warp then follows
+//      the sequence from s = 0: a composed run is one integer addition, an
+//      unpredicted chunk is replayed: lanes sum their increments, a warp scan
+//      finds the lane whose values leave the binade, and that lane adds its
+//      eight values with f64 additions, the reference's own operation.
+// Every step the walker takes is checked against the exact state, and where a
+// prediction does not hold it goes through the levels and, at worst, replays
+// every chunk: a wrong prediction costs time, never exactness.  No per-value
+// f64 arithmetic outside the crossings: the GB300's f64 rate is a small
+// fraction of its f32 and integer rates.  Not a reference function: the
+// reference's loop is serial (metrics.rs:215-226).
+//
+// Per map, against the earlier form (a serial fold per chunk, a one-CTA scan,
+// a walker that went through the levels alone): 0.11 against 0.22 ms on
+// 64 x 56 x 72, 0.35 against 0.50 ms on 33.5 M values, 0.69 against 0.90 ms on
+// 512^3.  The second step is bound by the integer ALU pipe, the walker by the
+// latency of its replays.
 #include <climits>
 #include <cstdint>
 
@@ -59,11 +67,11 @@ constexpr unsigned long long kSat = 1ull << 54;  // saturated increment: never v
 // shrinking relative to the prefix as it grows); the sequential sum differs
 // from the exact prefix by ~sqrt(k) 2^-53.  A miss only sends a chunk to the
 // replay.
-constexpr double kMargin = 1.0 / 16777216.0;  // 2^-24
+constexpr int kMarginBits = 24;
 // Fixed-point scale of the approximate sums (values scaled into [1, 2)):
 // 2^24 units per unit, so a 2^32-voxel map's sums of squares fit 64 bits.
+constexpr int kFixBits = 24;
 constexpr float kFix = 16777216.0f;
-constexpr double kUnfix = 1.0 / 16777216.0;
 
 // meta word of a function: 0 = invalid (no prediction); bit 2 = identity valid
 // in every binade; else bits 3.. hold E + 2048; bits 0, 1 = out parity for
@@ -169,6 +177,21 @@ __device__ __forceinline__ double term_value(float raw, float scale, bool sq) {
   return sq ? __dmul_rn(v, v) : v;
 }
 
+// The increment of an element M * 2^k (M < 2^MBITS) in the binade whose ulp is
+// 2^em52, when it does not depend on the parity; odd is set for a tie, and for
+// an increment of 2^54 or more, which need the ordered fold.  Without branches:
+// with M moved up to 54 bits, every increment is one right shift (of a whole
+// number of ulps, one rounded, or one that loses the element).
+template <int MBITS>
+__device__ __forceinline__ unsigned long long plain_increment(unsigned long long M, int k, int em52, bool& odd) {
+  constexpr int kUp = 54 - MBITS;
+  const int r = em52 - k + kUp;
+  const unsigned s = (unsigned)min(max(r, 0), 55);
+  const unsigned long long half = (1ull << s) >> 1, t = (M << kUp) + half;
+  odd = odd || (r < 0 && M != 0ull) || (s != 0u && (t & (2ull * half - 1ull)) == 0ull);  // a remainder of exactly half an ulp
+  return t >> s;
+}
+
 __device__ __forceinline__ int binade_of(double s) {
   return (int)((__double_as_longlong(s) >> 52) & 0x7ff) - 1023;
 }
@@ -224,113 +247,102 @@ __device__ __forceinline__ unsigned long long to_fixed(float x) {
   return (unsigned long long)__fmul_rn(x, kFix);
 }
 
-// 1. Approximate sums per chunk of v and v^2 (scaled by norm_factor, in f32)
-// and per block of 32 chunks (fixed point); one warp per block, lane j keeps chunk j.
-__global__ void __launch_bounds__(256)
+constexpr int kSumLevels = 4;      // approximate sums: blocks, and groups of 32, 1024 and 32768 blocks
+// Chunks per warp (32 / CPW warps take the 32 chunks of a block): 4, or 1 for
+// maps of fewer than kSmallMap values, which are bound by a warp's latency.
+constexpr long long kSmallMap = 1ll << 22;
+constexpr float kEmptyChunk = -0.0f;  // approximate sum of a chunk without values (others have no sign)
+
+struct Sums {
+  unsigned long long* s[kSumLevels];
+  unsigned long long* q[kSumLevels];
+};
+
+// 1. Approximate sums per chunk of v and v^2 (scaled by norm_factor, in f32),
+// and per block and group of blocks (fixed point; the groups' sums start at 0).
+// One CTA per block; all loads of a warp's chunks are in flight together.
+template <int CPW>
+__global__ void __launch_bounds__(1024 / CPW)
 osum_chunk_kernel(const float* __restrict__ map, long long n, float scale, long long nchunks,
-                  const uint32_t* __restrict__ maxbits, float* __restrict__ cs, float* __restrict__ cq,
-                  unsigned long long* __restrict__ bs, unsigned long long* __restrict__ bq) {
-  const int lane = threadIdx.x & 31;
-  const long long blk = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const long long c0 = blk * 32;
-  if (c0 >= nchunks) return;
+                  const uint32_t* __restrict__ maxbits, float* __restrict__ cs, float* __restrict__ cq, Sums sums) {
+  __shared__ unsigned long long sh_s, sh_q;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long blk = blockIdx.x, c0 = blk * 32 + warp * CPW;
+  if (threadIdx.x == 0) sh_s = sh_q = 0ull;
+  __syncthreads();
   const float nf = norm_factor(*maxbits);
-  float my_s = 0.0f, my_q = 0.0f;
-  for (int j = 0; j < 32 && c0 + j < nchunks; ++j) {
-    float v[8];
-    load8(map, n, (c0 + j) * kChunk + lane * 8, v);
+  float v[CPW][8];
+#pragma unroll
+  for (int j = 0; j < CPW; ++j) load8(map, n, (c0 + j) * kChunk + lane * 8, v[j]);
+  unsigned long long ts = 0, tq = 0;
+#pragma unroll
+  for (int j = 0; j < CPW; ++j) {
     float s = 0.0f, q = 0.0f;
+    bool any = false;
 #pragma unroll
     for (int t = 0; t < 8; ++t) {
-      const float raw = v[t];
-      const float x = (raw > 0.0f && isfinite(raw)) ? __fmul_rn(__fmul_rn(raw, scale), nf) : 0.0f;
+      const float raw = v[j][t];
+      const bool ok = raw > 0.0f && isfinite(raw);
+      const float x = ok ? __fmul_rn(__fmul_rn(raw, scale), nf) : 0.0f;
+      any = any || ok;
       s += x;
       q += x * x;
     }
+    const bool some = __any_sync(0xffffffffu, any);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       s += __shfl_xor_sync(0xffffffffu, s, o);
       q += __shfl_xor_sync(0xffffffffu, q, o);
     }
-    if (lane == j) {
-      my_s = s;
-      my_q = q;
+    if (lane == 0 && c0 + j < nchunks) {
+      cs[c0 + j] = some ? s : kEmptyChunk;
+      cq[c0 + j] = q;
     }
-  }
-  if (c0 + lane < nchunks) {
-    cs[c0 + lane] = my_s;
-    cq[c0 + lane] = my_q;
-  }
-  unsigned long long ts = c0 + lane < nchunks ? to_fixed(my_s) : 0ull;
-  unsigned long long tq = c0 + lane < nchunks ? to_fixed(my_q) : 0ull;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    ts += __shfl_xor_sync(0xffffffffu, ts, o);
-    tq += __shfl_xor_sync(0xffffffffu, tq, o);
+    ts += to_fixed(s);
+    tq += to_fixed(q);
   }
   if (lane == 0) {
-    bs[blk] = ts;
-    bq[blk] = tq;
+    if (ts) atomicAdd(&sh_s, ts);
+    if (tq) atomicAdd(&sh_q, tq);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int L = 0; L < kSumLevels; ++L) {
+    if (threadIdx.x != L) continue;
+    if (L == 0) {
+      sums.s[0][blk] = sh_s;
+      sums.q[0][blk] = sh_q;
+    } else {
+      if (sh_s) atomicAdd(sums.s[L] + (blk >> (5 * L)), sh_s);
+      if (sh_q) atomicAdd(sums.q[L] + (blk >> (5 * L)), sh_q);
+    }
   }
 }
 
-// 2. Exclusive scan of the block sums in place, fixed point (one CTA of 1024 threads).
-__global__ void __launch_bounds__(1024) osum_scan_kernel(unsigned long long* __restrict__ bs,
-                                                         unsigned long long* __restrict__ bq, long long nb) {
-  __shared__ unsigned long long ws[32], wq[32];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const long long per = (nb + 1023) / 1024;
-  const long long b0 = (long long)tid * per, b1 = b0 + per < nb ? b0 + per : nb;
-  unsigned long long ls = 0, lq = 0;
-  for (long long b = b0; b < b1; ++b) {
-    ls += bs[b];
-    lq += bq[b];
-  }
-  unsigned long long is = ls, iq = lq;  // inclusive scan of the threads' totals
+// Sum of everything before block blk (whole warp; the same in all lanes).
+__device__ __forceinline__ unsigned long long prefix_of(unsigned long long* const (&lv)[kSumLevels], long long blk,
+                                                        int lane) {
+  unsigned long long t = 0;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned long long us = __shfl_up_sync(0xffffffffu, is, o), uq = __shfl_up_sync(0xffffffffu, iq, o);
-    if (lane >= o) {
-      is += us;
-      iq += uq;
-    }
+  for (int L = 0; L < kSumLevels; ++L) {
+    const long long at = blk >> (5 * L), first = L + 1 < kSumLevels ? at & ~31ll : 0ll;
+    for (long long i = first + lane; i < at; i += 32) t += lv[L][i];  // at most once below the top level
   }
-  if (lane == 31) {
-    ws[warp] = is;
-    wq[warp] = iq;
-  }
-  __syncthreads();
-  if (warp == 0) {
-    unsigned long long a = ws[lane], b = wq[lane];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned long long ua = __shfl_up_sync(0xffffffffu, a, o), ub = __shfl_up_sync(0xffffffffu, b, o);
-      if (lane >= o) {
-        a += ua;
-        b += ub;
-      }
-    }
-    ws[lane] = a - ws[lane];
-    wq[lane] = b - wq[lane];
-  }
-  __syncthreads();
-  unsigned long long rs = ws[warp] + is - ls, rq = wq[warp] + iq - lq;
-  for (long long b = b0; b < b1; ++b) {
-    const unsigned long long ts = bs[b], tq = bq[b];
-    bs[b] = rs;
-    bq[b] = rq;
-    rs += ts;
-    rq += tq;
-  }
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return t;
 }
 
-// Binade the running sum is predicted to stay in over [P, P + A] * 2^eshift
-// (INT_MIN: none).  P and A are approximate (f32 chunk sums), hence the margin.
-__device__ __forceinline__ int predict(double P, double A, int eshift) {
-  const double lo = P * (1.0 - kMargin), hi = (P + A) * (1.0 + kMargin);
-  if (!(lo > 0.0) || !(hi < 1e300)) return INT_MIN;
-  const int e0 = binade_of(lo), e1 = binade_of(hi);
-  return e0 == e1 ? e0 + eshift : INT_MIN;
+// Binade the running sum is predicted to stay in from P to S, both approximate
+// (f32 chunk sums in fixed point, hence the margin); 2^(eshift - kFixBits) is
+// their unit.  INT_MIN: none.  Integers only: GB300 retires two f64 operations
+// per SM and clock.
+__device__ __forceinline__ int predict(unsigned long long P, unsigned long long S, int eshift) {
+  if (P == 0ull) return INT_MIN;
+  const unsigned long long lo = P - (P >> kMarginBits) - 1ull, hi = S + (S >> kMarginBits) + 1ull;
+  if (lo == 0ull) return INT_MIN;
+  const int e0 = 63 - __clzll((long long)lo), e1 = 63 - __clzll((long long)hi);
+  return e0 == e1 ? e0 - kFixBits + eshift : INT_MIN;
 }
 
 struct Level {
@@ -385,98 +397,217 @@ __device__ __forceinline__ void acc_elem(Acc& A, unsigned long long M, int k, in
   A.o1 ^= (uint32_t)(c & 1ull);
 }
 
+// A run whose total increment does not depend on the parity.
+__device__ __forceinline__ Fn plain_fn(unsigned long long inc, int E) {
+  if (E == INT_MIN) return Fn{0ull, 0ull, 0u};
+  const uint32_t p = (uint32_t)(inc & 1ull);
+  if (inc > kSat) inc = kSat;
+  return Fn{inc, inc, meta_of(E, p, p ^ 1u)};
+}
+
 __device__ __forceinline__ Fn acc_fn(const Acc& A, bool any, int E) {
   if (!any) return fn_identity();
   if (E == INT_MIN) return Fn{0ull, 0ull, 0u};
   return Fn{A.i0 >= kSat ? kSat : A.i0, A.i1 >= kSat ? kSat : A.i1, meta_of(E, A.o0, A.o1)};
 }
 
-constexpr int kTileStride = 33;  // words per row of a warp's transpose tile (conflict-free column reads)
+constexpr int kMaxLevels = 8;
+constexpr int kMaxMixed = 256;  // blocks with a crossing the walker prepares (more: it goes through all levels)
 
-// 3. Predicted binade and function of every chunk, for both sums, and the
-// first aggregate level.  One warp per block of 32 chunks; lane j owns chunk
-// j and folds its 256 values in order.  The values reach the lanes through a
-// shared-memory transpose of 32 values of each chunk at a time, so the
-// global loads stay coalesced.
-__global__ void __launch_bounds__(256)
+struct Walk {
+  Level lv[kMaxLevels];  // lv[0]: chunks; lv[L]: blocks of 32^L chunks
+  long long cnt[kMaxLevels];
+  int nlev;
+  uint32_t* mixed;  // [0]: number of blocks without a valid composition, then their indexes (any order)
+};
+
+// The functions of chunk c folded in order (whole warp; the same in all lanes):
+// lane l folds values 8 l .. 8 l + 7, then the lanes' functions are composed.
+struct FnPair {
+  Fn s, q;
+};
+__device__ __noinline__ FnPair ordered_fold(const float* __restrict__ map, long long n, float scale, long long c, int es,
+                                            int eq, int lane) {
+  float w[8];
+  load8(map, n, c * kChunk + lane * 8, w);
+  Acc a{0ull, 0ull, 0u, 1u}, q{0ull, 0ull, 0u, 1u};
+  bool has = false;
+#pragma unroll 1
+  for (int t = 0; t < 8; ++t) {
+    float v = w[0];
+#pragma unroll
+    for (int j = 1; j < 8; ++j) v = t == j ? w[j] : v;
+    const Term x = term(v, scale, false);
+    if (!x.M) continue;
+    has = true;
+    const bool inf = x.k == INT_MAX;
+    if (es != INT_MIN) acc_elem(a, x.M, x.k, es - 52, 24);
+    if (eq != INT_MIN) acc_elem(q, inf ? x.M : x.M * x.M, inf ? INT_MAX : 2 * x.k, eq - 52, 48);
+  }
+  return FnPair{shfl_fn(warp_reduce_fn(acc_fn(a, has, es), lane), 0),
+                shfl_fn(warp_reduce_fn(acc_fn(q, has, eq), lane), 0)};
+}
+
+// 2. Functions of every chunk, for both sums, and of every block.  One CTA per
+// block; a chunk without values is not read again.
+template <int CPW>
+__global__ void __launch_bounds__(1024 / CPW)
 osum_fn_kernel(const float* __restrict__ map, long long n, float scale, long long nchunks,
                const uint32_t* __restrict__ maxbits, const float* __restrict__ cs, const float* __restrict__ cq,
-               const unsigned long long* __restrict__ bps, const unsigned long long* __restrict__ bpq, Level s0,
-               Level q0, Level s1, Level q1) {
-  __shared__ float tile[8][32 * kTileStride];
+               Sums sums, Walk ws, Walk wq) {
+  __shared__ Fn sh[2][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long blk = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const long long c0 = blk * 32;
-  if (c0 >= nchunks) return;
-  float* T = tile[warp];
-  const bool mine = c0 + lane < nchunks;
-  const unsigned long long as = mine ? to_fixed(cs[c0 + lane]) : 0ull, aq = mine ? to_fixed(cq[c0 + lane]) : 0ull;
-  unsigned long long ps = as, pq = aq;  // inclusive scan within the block
+  const long long blk = blockIdx.x, b0 = blk * 32;
+  const float my_s = b0 + lane < nchunks ? cs[b0 + lane] : kEmptyChunk;
+  const unsigned filled = __ballot_sync(0xffffffffu, __float_as_uint(my_s) != __float_as_uint(kEmptyChunk));
+  const bool vec = (reinterpret_cast<uintptr_t>(map) & 15u) == 0;
+  auto load = [&](int j, float (&x)[8]) {  // any order within the chunk: coalesced
+    const int c = warp * CPW + j;
+    const long long at = (b0 + c) * kChunk + lane * 4;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned long long us = __shfl_up_sync(0xffffffffu, ps, o), uq = __shfl_up_sync(0xffffffffu, pq, o);
-    if (lane >= o) {
-      ps += us;
-      pq += uq;
+    for (int h = 0; h < 2; ++h) {
+      const long long i = at + h * 128;
+      if (!((filled >> c) & 1u)) {
+        x[4 * h] = x[4 * h + 1] = x[4 * h + 2] = x[4 * h + 3] = 0.0f;
+      } else if (vec && i + 4 <= n) {
+        const float4 y = *reinterpret_cast<const float4*>(map + i);
+        x[4 * h] = y.x; x[4 * h + 1] = y.y; x[4 * h + 2] = y.z; x[4 * h + 3] = y.w;
+      } else {
+#pragma unroll
+        for (int t = 0; t < 4; ++t) x[4 * h + t] = i + t < n ? map[i + t] : 0.0f;
+      }
     }
+  };
+  float next[8];
+  load(0, next);
+  // lane j: chunk j's predicted binades
+  int es_mine = INT_MIN, eq_mine = INT_MIN;
+  if (filled) {
+    const unsigned long long as = to_fixed(my_s), aq = b0 + lane < nchunks ? to_fixed(cq[b0 + lane]) : 0ull;
+    unsigned long long ps = as, pq = aq;  // inclusive scan within the block
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long us = __shfl_up_sync(0xffffffffu, ps, o), uq = __shfl_up_sync(0xffffffffu, pq, o);
+      if (lane >= o) {
+        ps += us;
+        pq += uq;
+      }
+    }
+    ps += prefix_of(sums.s, blk, lane);
+    pq += prefix_of(sums.q, blk, lane);
+    // the approximate sums are of values scaled by 2^(127 - ef): undo it in the binade
+    const int shift = max_exponent_field(*maxbits) - 127;
+    es_mine = predict(ps - as, ps, shift);
+    eq_mine = predict(pq - aq, pq, 2 * shift);
   }
-  // the approximate sums are of values scaled by 2^(127 - ef): undo it in the binade
-  const int shift = max_exponent_field(*maxbits) - 127;
-  const int es = predict((double)(bps[blk] + ps - as) * kUnfix, (double)as * kUnfix, shift);
-  const int eq = predict((double)(bpq[blk] + pq - aq) * kUnfix, (double)aq * kUnfix, 2 * shift);
-  const int ems = es == INT_MIN ? 0 : es - 52, emq = eq == INT_MIN ? 0 : eq - 52;
-  Acc A{0ull, 0ull, 0u, 1u}, Q{0ull, 0ull, 0u, 1u};
-  bool any = false;
-  const long long base0 = c0 * kChunk;
-  const bool vec = (reinterpret_cast<uintptr_t>(map) & 15u) == 0 && base0 + 32ll * kChunk <= n;
-  for (int t = 0; t < kChunk / 32; ++t) {
-    // T[j][x] = value t*32 + x of chunk j
-    if (vec) {
+#pragma unroll 1
+  for (int j = 0; j < CPW; ++j) {
+    float v[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int j = 4 * i + (lane >> 3), x = 4 * (lane & 7);
-        const float4 v = *reinterpret_cast<const float4*>(map + base0 + (long long)j * kChunk + t * 32 + x);
-        float* r = T + j * kTileStride + x;
-        r[0] = v.x;
-        r[1] = v.y;
-        r[2] = v.z;
-        r[3] = v.w;
-      }
-    } else {
-      for (int j = 0; j < 32; ++j) {
-        const long long idx = base0 + (long long)j * kChunk + t * 32 + lane;
-        T[j * kTileStride + lane] = idx < n ? map[idx] : 0.0f;
-      }
-    }
-    __syncwarp();
-    if (mine) {
-#pragma unroll 4
-      for (int x = 0; x < 32; ++x) {
-        const Term a = term(T[lane * kTileStride + x], scale, false);
-        if (a.M) {
-          any = true;
-          if (es != INT_MIN) acc_elem(A, a.M, a.k, ems, 24);
-          if (eq != INT_MIN)
-            acc_elem(Q, a.k == INT_MAX ? a.M : a.M * a.M, a.k == INT_MAX ? INT_MAX : 2 * a.k, emq, 48);
+    for (int t = 0; t < 8; ++t) v[t] = next[t];
+    if (j + 1 < CPW) load(j + 1, next);
+    const int c = warp * CPW + j;
+    if (!((filled >> c) & 1u)) {
+      if (lane == 0) {
+        sh[0][c] = sh[1][c] = fn_identity();
+        if (b0 + c < nchunks) {
+          store_fn(ws.lv[0], b0 + c, fn_identity());
+          store_fn(wq.lv[0], b0 + c, fn_identity());
         }
       }
+      continue;
     }
-    __syncwarp();
+    const int es = __shfl_sync(0xffffffffu, es_mine, c), eq = __shfl_sync(0xffffffffu, eq_mine, c);
+    // M = 0 (an increment of 0) for the entries that are skipped
+    uint32_t bits[8], top = 0u, low = ~0u;
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+      const bool ok = v[t] > 0.0f && isfinite(v[t]);
+      bits[t] = ok ? __float_as_uint(__fmul_rn(v[t], scale)) : 0u;
+      top = max(top, bits[t]);
+      low = min(low, bits[t] - 1u);  // (the skipped ones go to the top)
+    }
+    top = __reduce_max_sync(0xffffffffu, top) >> 23;
+    low = (__reduce_min_sync(0xffffffffu, low) + 1u) >> 23;
+    // The usual chunk: normal values over at most 8 binades.  In units of the
+    // lowest one's ulp 2^k a value is a 31-bit integer m, and all are rounded
+    // at the same bit: m at bit sha, m^2 (one multiplication that adds half an
+    // ulp too) at bit shq.
+    const int k = (int)low - 150;
+    const int sha = es == INT_MIN ? 0 : es - 52 - k, shq = eq == INT_MIN ? 40 : eq - 52 - 2 * k;
+    Fn fs, fq;
+    bool odd = true;
+    unsigned long long A = 0, Q = 0;
+    if (low > 0u && top < 255u && top - low <= 7u && sha >= -23 && sha <= 31 && shq >= 1 && shq <= 62) {
+      const unsigned ra = (unsigned)max(sha, 0);
+      const uint32_t half_a = (1u << ra) >> 1, mask_a = (1u << ra) - 1u, tie_a = ra ? 0u : 1u;
+      const unsigned long long half_q = 1ull << (shq - 1);
+      const uint32_t base = low << 23;
+      odd = false;
+      auto sum = [&](auto&& shift_q) {
+#pragma unroll
+        for (int t = 0; t < 8; ++t) {
+          const uint32_t m = bits[t] ? ((bits[t] & 0x7fffffu) | 0x800000u) << ((bits[t] - base) >> 23) : 0u;
+          const uint32_t ta = m + half_a;
+          odd = odd || (ta & mask_a) == tie_a;
+          A += ta >> ra;
+          shift_q((unsigned long long)m * m + half_q);
+        }
+      };
+      if (shq >= 32) {
+        const unsigned rq = (unsigned)shq - 32u;
+        const uint32_t mask = (1u << rq) - 1u;
+        sum([&](unsigned long long tq) {
+          const uint32_t hi = (uint32_t)(tq >> 32);
+          odd = odd || ((hi & mask) | (uint32_t)tq) == 0u;
+          Q += hi >> rq;
+        });
+      } else {
+        const unsigned rq = (unsigned)shq;
+        const uint32_t mask = (1u << rq) - 1u;
+        sum([&](unsigned long long tq) {
+          odd = odd || ((uint32_t)tq & mask) == 0u;
+          Q += tq >> rq;
+        });
+      }
+      if (sha < 0) A <<= -sha;
+    }
+    if (!__any_sync(0xffffffffu, odd)) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        A += __shfl_xor_sync(0xffffffffu, A, o);
+        Q += __shfl_xor_sync(0xffffffffu, Q, o);
+      }
+      fs = plain_fn(A, es);
+      fq = plain_fn(Q, eq);
+    } else {
+      const FnPair f = ordered_fold(map, n, scale, b0 + c, es, eq, lane);
+      fs = f.s;
+      fq = f.q;
+    }
+    if (lane == 0) {
+      sh[0][c] = b0 + c < nchunks ? fs : fn_identity();
+      sh[1][c] = b0 + c < nchunks ? fq : fn_identity();
+      if (b0 + c < nchunks) {
+        store_fn(ws.lv[0], b0 + c, fs);
+        store_fn(wq.lv[0], b0 + c, fq);
+      }
+    }
   }
-  const Fn my_s = acc_fn(A, any, es), my_q = acc_fn(Q, any, eq);
-  if (mine) {
-    store_fn(s0, c0 + lane, my_s);
-    store_fn(q0, c0 + lane, my_q);
-  }
-  const Fn as_ = warp_reduce_fn(mine ? my_s : fn_identity(), lane);
-  const Fn aq_ = warp_reduce_fn(mine ? my_q : fn_identity(), lane);
-  if (lane == 0) {
-    store_fn(s1, blk, as_);
-    store_fn(q1, blk, aq_);
+  __syncthreads();
+  if (warp > 1) return;
+  // warp 0 composes the sum's block function, warp 1 that of the squares
+  const Walk& W = warp ? wq : ws;
+  const Fn f = warp_reduce_fn(sh[warp][lane], lane);
+  if (lane > 0) return;
+  store_fn(W.lv[1], blk, f);
+  if (f.meta == 0u) {
+    const uint32_t p = atomicAdd(&W.mixed[0], 1u);
+    if (p < kMaxMixed) W.mixed[1 + p] = (uint32_t)blk;
   }
 }
 
-// 4. Next aggregate level: compositions of 32 consecutive entries.
+// Next aggregate level: compositions of 32 consecutive entries.
 __global__ void __launch_bounds__(256) osum_level_kernel(Level s_in, Level q_in, long long n_in, Level s_out,
                                                          Level q_out) {
   const int lane = threadIdx.x & 31;
@@ -489,60 +620,6 @@ __global__ void __launch_bounds__(256) osum_level_kernel(Level s_in, Level q_in,
     store_fn(s_out, blk, fs);
     store_fn(q_out, blk, fq);
   }
-}
-
-constexpr int kMaxLevels = 8;
-
-struct Walk {
-  Level lv[kMaxLevels];  // lv[0]: chunks; lv[L]: blocks of 32^L chunks
-  long long cnt[kMaxLevels];
-  int nlev;
-};
-
-// Adds values vals[j0 .. 8) to s one after the other as the reference does
-// (one thread): s kept as an integer count of its binade's ulps plus each
-// value's rounded increment (round half to even on that count), a hardware
-// f64 addition -- the reference's own operation -- for the first value
-// (s = 0), for a value that leaves the binade, and for +inf.
-__device__ double add_serially(double s, const float (&vals)[8], int j0, float scale, bool sq) {
-  bool in_units = isfinite(s) && s > 0.0;
-  int E = in_units ? binade_of(s) : 0;
-  unsigned long long u = in_units ? units_of(s) : 0ull;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    if (j < j0) continue;
-    const Term t = term(vals[j], scale, sq);
-    if (!t.M) continue;  // skipped (metrics.rs:216-218) or zero
-    if (in_units && t.k != INT_MAX) {
-      const int sh = (E - 52) - t.k;
-      unsigned long long a = 0;
-      bool tie = false, fits = true;
-      if (sh <= 0) {
-        fits = sh > -54 && (t.M >> (54 + sh)) == 0;
-        a = fits ? t.M << -sh : 0;
-      } else if (sh < 64) {
-        const unsigned long long rem = t.M & ((1ull << sh) - 1ull), half = 1ull << (sh - 1);
-        a = (t.M >> sh) + (rem > half ? 1ull : 0ull);
-        tie = rem == half;
-      }
-      if (fits && u + a < kTwo53) {  // the exact sum stays below 2^(E+1): the binade's grid
-        u += tie ? (a + ((u + a) & 1ull)) : a;
-        if (u == kTwo53) {  // a tie rounded up to 2^(E+1): the next binade
-          u = 1ull << 52;
-          ++E;
-        }
-        continue;
-      }
-      s = from_units(u, E);
-    }
-    s = __dadd_rn(s, term_value(vals[j], scale, sq));  // metrics.rs:223-224
-    in_units = isfinite(s) && s > 0.0;
-    if (in_units) {
-      E = binade_of(s);
-      u = units_of(s);
-    }
-  }
-  return in_units ? from_units(u, E) : s;
 }
 
 __device__ __forceinline__ Fn shfl_up_fn(const Fn& f, int o) {
@@ -564,44 +641,69 @@ __device__ __forceinline__ Fn warp_scan_fn(Fn f, int lane) {
 }
 
 // Replays chunk c from state s exactly as the reference adds.  Lane l holds
-// values 8l .. 8l+7.  In s's binade every lane folds its values into one
-// function and a warp scan composes them in order; the first lane whose
-// prefix leaves the binade (or the lane holding the first value, s = 0)
-// adds its values serially with add_serially, and the lanes after it are
-// folded again in the new binade.  s is broadcast back.
-__device__ void replay_chunk(const float* __restrict__ map, long long n, float scale, bool sq, long long c, double& s,
-                             int lane) {
+// values 8l .. 8l+7.  In s's binade every lane sums its values' increments and
+// a warp scan adds them up (or, when a value ties, folds and composes them in
+// order); the first lane whose prefix leaves the binade (or the lane holding
+// the first value, s = 0) adds its values with f64 additions, the reference's
+// own operation (metrics.rs:223-224), and the lanes after it go on in the new
+// binade.  s is broadcast back.
+__device__ __noinline__ double replay_chunk(const float* __restrict__ map, long long n, float scale, bool sq,
+                                            long long c, double s, int lane) {
   float vals[8];
   load8(map, n, c * kChunk + lane * 8, vals);
+  unsigned long long M[8];
+  int k[8];
+  bool inf = false, any = false;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const Term t = term(vals[j], scale, sq);
+    const bool is_inf = t.k == INT_MAX;
+    M[j] = is_inf ? 0ull : t.M;
+    k[j] = is_inf ? 0 : t.k;
+    inf = inf || is_inf;
+    any = any || t.M != 0ull;
+  }
   int start = 0;  // first lane not yet added
-  const int mbits = sq ? 48 : 24;
   while (start < 32) {
     if (!isfinite(s)) break;  // +inf stays +inf
     int b;                    // the lane that adds serially
     if (s == 0.0) {
-      bool any = false;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) any = any || term(vals[j], scale, sq).M != 0;
       const unsigned m = __ballot_sync(0xffffffffu, lane >= start && any);
       if (!m) break;
       b = __ffs(m) - 1;
     } else {
       const int E = binade_of(s);
       const unsigned long long u0 = units_of(s);
-      Acc A{0ull, 0ull, 0u, 1u};
-      bool any = false;
-      if (lane >= start) {
+      unsigned long long inc = 0;
+      bool odd = inf;
+      if (sq) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const Term t = term(vals[j], scale, sq);
-          if (t.M) {
-            any = true;
-            acc_elem(A, t.M, t.k, E - 52, mbits);
-          }
-        }
+        for (int j = 0; j < 8; ++j) inc += plain_increment<48>(M[j], k[j], E - 52, odd);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) inc += plain_increment<24>(M[j], k[j], E - 52, odd);
       }
-      const Fn pre = warp_scan_fn(acc_fn(A, any, E), lane);
-      const unsigned long long after = sat_add(u0, (u0 & 1ull) ? pre.i1 : pre.i0);
+      if (lane < start) inc = 0ull;
+      unsigned long long after;
+      if (!__any_sync(0xffffffffu, odd && lane >= start)) {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const unsigned long long u = __shfl_up_sync(0xffffffffu, inc, o);
+          if (lane >= o) inc += u;
+        }
+        after = sat_add(u0, inc);
+      } else {
+        Acc A{0ull, 0ull, 0u, 1u};
+        const bool has = any && lane >= start;
+        if (has) {
+          if (inf) A.i0 = A.i1 = kSat;
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (M[j]) acc_elem(A, M[j], k[j], E - 52, 48);
+        }
+        const Fn pre = warp_scan_fn(acc_fn(A, has, E), lane);
+        after = sat_add(u0, (u0 & 1ull) ? pre.i1 : pre.i0);
+      }
       const unsigned bad = __ballot_sync(0xffffffffu, lane >= start && after > kTwo53);
       if (!bad) {
         s = from_units(__shfl_sync(0xffffffffu, after, 31), E);
@@ -612,73 +714,70 @@ __device__ void replay_chunk(const float* __restrict__ map, long long n, float s
       const unsigned long long ub = __shfl_sync(0xffffffffu, after, b > 0 ? b - 1 : 0);
       if (b > start) s = from_units(ub, E);
     }
-    double sb = 0.0;
-    if (lane == b) sb = add_serially(s, vals, 0, scale, sq);
-    s = __shfl_sync(0xffffffffu, sb, b);
+    if (lane == b) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (vals[j] > 0.0f && isfinite(vals[j])) s = __dadd_rn(s, term_value(vals[j], scale, sq));
+    }
+    s = __shfl_sync(0xffffffffu, s, b);
     start = b + 1;
   }
-  s = __shfl_sync(0xffffffffu, s, 0);
+  return __shfl_sync(0xffffffffu, s, 0);
 }
 
-// Largest total of aggregate-level entries the walker keeps in shared memory.
-constexpr size_t kWalkSmemBytes = 96 * 1024;
-constexpr int kEntryBytes = 20;  // i0, i1, meta
-
-// The lowest level (>= 1) from which all levels fit kWalkSmemBytes.
-__host__ __device__ __forceinline__ int cached_from(const long long* cnt, int nlev) {
-  long long bytes = 0;
-  int L = nlev;
-  while (L - 1 >= 1 && bytes + cnt[L - 1] * kEntryBytes <= (long long)kWalkSmemBytes) {
-    --L;
-    bytes += cnt[L] * kEntryBytes;
-  }
-  return L;
-}
-
-// 5. The walker: block 0 follows the sum of values, block 1 the sum of squares.
-// The small aggregate levels are copied to shared memory first, so that the
-// walker's level probes near a crossing cost shared-memory latency; level 0
-// (and level 1 when large) stay in global memory.
-__global__ void __launch_bounds__(32) osum_walk_kernel(const float* __restrict__ map, long long n, float scale,
-                                                       Walk ws, Walk wq, double* __restrict__ out) {
-  extern __shared__ __align__(16) unsigned char walk_smem[];
-  const bool sq = blockIdx.x == 1;
-  Walk W = sq ? wq : ws;
-  const int lane = threadIdx.x;
-  const long long nchunks = W.cnt[0];
-  {
-    const int Lc = cached_from(W.cnt, W.nlev);
-    unsigned char* p = walk_smem;
-    for (int L = Lc; L < W.nlev; ++L) {
-      const long long c = W.cnt[L];
-      unsigned long long* i0 = reinterpret_cast<unsigned long long*>(p);
-      unsigned long long* i1 = i0 + c;
-      uint32_t* meta = reinterpret_cast<uint32_t*>(i1 + c);
-      for (long long i = lane; i < c; i += 32) {
-        i0[i] = W.lv[L].i0[i];
-        i1[i] = W.lv[L].i1[i];
-        meta[i] = W.lv[L].meta[i];
+// Follows the sequence through one block whose chunk functions the lanes hold
+// (lane j: chunk c0 + j; identity past the map's end), from lane p to lane e.
+__device__ __noinline__ double walk_block(const float* __restrict__ map, long long n, float scale, bool sq,
+                                          long long c0, const Fn& f, int p, int e, double s, int lane) {
+  while (p <= e) {
+    if (!isfinite(s)) break;
+    const int E = s == 0.0 ? INT_MIN : binade_of(s);
+    const bool ok = (f.meta & 4u) || (E != INT_MIN && f.meta != 0u && (int)(f.meta >> 3) - 2048 == E);
+    const unsigned stop = __ballot_sync(0xffffffffu, lane >= p && (!ok || lane > e));
+    const int t = stop ? __ffs(stop) - 1 : 32;  // chunks p .. t - 1 qualify
+    if (t > p) {
+      const bool run = lane >= p && lane < t;
+      double s2 = s;
+      bool moved = E == INT_MIN;  // empty chunks before the first value
+      if (!moved) {
+        const Fn r = shfl_fn(warp_reduce_fn(run ? f : fn_identity(), lane), 0);
+        moved = apply_fn(r, s2);
       }
-      W.lv[L] = Level{i0, i1, meta};
-      p += ((size_t)c * kEntryBytes + 15) & ~(size_t)15;
+      if (moved) {
+        s = s2;
+        p = t;
+        continue;
+      }
+      const Fn f0 = shfl_fn(f, p);  // the run left the binade somewhere: its first chunk alone
+      if (t > p + 1 && apply_fn(f0, s)) {
+        ++p;
+        continue;
+      }
     }
-    __syncwarp();
+    s = replay_chunk(map, n, scale, sq, c0 + p, s, lane);
+    ++p;
   }
-  double s = 0.0;
-  long long c = 0;
-  while (c < nchunks) {
+  return s;
+}
+
+// Follows the sequence over chunks c .. end - 1 from state s: the highest level
+// whose entry starts at c, does not pass `end` and applies, up to 32 entries of
+// it at a time, or a replay of one chunk.
+__device__ __noinline__ double walk_range(const float* __restrict__ map, long long n, float scale, bool sq,
+                                          const Walk& W, long long c, long long end, double s, int lane) {
+  while (c < end) {
     if (!isfinite(s)) break;  // a value overflowed to +inf: the sum stays +inf
-    // the highest level whose block starts at c and whose first entry applies:
-    // before the first value (s = 0) only empty runs, after it runs in s's binade
     bool moved = false;
     for (int L = W.nlev - 1; L >= 0 && !moved; --L) {
       const int lg = 5 * L;
       const long long span = 1ll << lg;
       if (c & (span - 1)) continue;
       const long long q = c >> lg;
-      // up to 32 entries of this level, but not past the next block of level L + 1
-      const long long lim = (L + 1 < W.nlev) ? ((q / 32) + 1) * 32 : W.cnt[L];
-      const long long qe = lim < W.cnt[L] ? lim : W.cnt[L];
+      // up to 32 entries of this level, but not past the next block of level
+      // L + 1, and only whole ones before `end` (the map's last entry may be short)
+      long long qe = min((q / 32 + 1) * 32, end >= W.cnt[0] ? W.cnt[L] : end >> lg);
+      if (L + 1 == W.nlev) qe = min(q + 32, end >= W.cnt[0] ? W.cnt[L] : end >> lg);
+      if (q >= qe) continue;
       const long long i = q + lane;
       const Fn f = i < qe ? load_fn(W.lv[L], i) : Fn{0ull, 0ull, 0u};
       const int E = s == 0.0 ? INT_MIN : binade_of(s);
@@ -687,7 +786,7 @@ __global__ void __launch_bounds__(32) osum_walk_kernel(const float* __restrict__
       const int t = (~okm) ? __ffs(~okm) - 1 : 32;  // entries 0 .. t-1 qualify
       if (t == 0) continue;
       if (E == INT_MIN) {  // empty chunks before the first value
-        c = (q + t) * span < nchunks ? (q + t) * span : nchunks;
+        c = min((q + t) * span, end);
         moved = true;
         break;
       }
@@ -696,7 +795,7 @@ __global__ void __launch_bounds__(32) osum_walk_kernel(const float* __restrict__
       double s2 = s;
       if (apply_fn(r, s2)) {
         s = s2;
-        c = (q + t) * span < nchunks ? (q + t) * span : nchunks;
+        c = min((q + t) * span, end);
         moved = true;
       } else if (t > 1) {
         // the run left the binade somewhere: take its first entry alone
@@ -704,15 +803,123 @@ __global__ void __launch_bounds__(32) osum_walk_kernel(const float* __restrict__
         s2 = s;
         if (apply_fn(f0, s2)) {
           s = s2;
-          c = (q + 1) * span < nchunks ? (q + 1) * span : nchunks;
+          c = min((q + 1) * span, end);
           moved = true;
         }
       }
     }
     if (!moved) {
-      replay_chunk(map, n, scale, sq, c, s, lane);
+      s = replay_chunk(map, n, scale, sq, c, s, lane);
       ++c;
     }
+  }
+  return s;
+}
+
+// Composition of level-1 entries a .. b - 1 (whole warp), through the levels.
+__device__ Fn compose_blocks(const Walk& W, long long a, long long b, int lane) {
+  Fn front = fn_identity(), back = fn_identity();
+  for (int L = 1; a < b; ++L) {
+    const bool top = L + 1 >= W.nlev;
+    const long long head = top ? b : min((a + 31) & ~31ll, b);  // entries up to the next whole group
+    for (; a < head; a += 32) {
+      const Fn f = a + lane < head ? load_fn(W.lv[L], a + lane) : fn_identity();
+      front = compose(front, shfl_fn(warp_reduce_fn(f, lane), 0));
+      if (head - a < 32) {
+        a = head;
+        break;
+      }
+    }
+    if (a >= b) break;
+    const long long tail = b & ~31ll;  // a is a multiple of 32 and below b
+    if (tail < b) {
+      const Fn f = tail + lane < b ? load_fn(W.lv[L], tail + lane) : fn_identity();
+      back = compose(shfl_fn(warp_reduce_fn(f, lane), 0), back);
+      b = tail;
+    }
+    a >>= 5;
+    b >>= 5;
+  }
+  return compose(front, back);
+}
+
+constexpr int kWalkWarps = 16;
+
+// 3. The walker: block 0 follows the sum of values, block 1 the sum of squares.
+__global__ void __launch_bounds__(kWalkWarps * 32)
+osum_walk_kernel(const float* __restrict__ map, long long n, float scale, Walk ws, Walk wq, double* __restrict__ out) {
+  __shared__ uint32_t at[kMaxMixed];                  // the mixed blocks in order
+  __shared__ Fn gap[kMaxMixed + 1];                   // the blocks before each of them (and after the last)
+  __shared__ Fn pre[kMaxMixed], suf[kMaxMixed];       // their chunks before the first / after the last unpredicted one
+  __shared__ uint8_t first[kMaxMixed], last[kMaxMixed];
+  const bool sq = blockIdx.x == 1;
+  const Walk& W = sq ? wq : ws;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const long long nchunks = W.cnt[0], nblocks = W.cnt[1];
+  const int nm = (int)W.mixed[0];
+  if (nm > kMaxMixed) {  // many wrong predictions: through all levels
+    if (warp == 0) {
+      const double s = walk_range(map, n, scale, sq, W, 0, nchunks, 0.0, lane);
+      if (lane == 0) out[sq ? 1 : 0] = s;
+    }
+    return;
+  }
+  for (int i = tid; i < nm; i += kWalkWarps * 32) {
+    const uint32_t me = W.mixed[1 + i];
+    int r = 0;
+    for (int j = 0; j < nm; ++j) r += W.mixed[1 + j] < me ? 1 : 0;
+    at[r] = me;
+  }
+  __syncthreads();
+  for (int t = warp; t < 2 * nm + 1; t += kWalkWarps) {
+    const int i = t >> 1;
+    if (t & 1) {  // inside mixed block i
+      const long long c = (long long)at[i] * 32 + lane;
+      const Fn f = c < nchunks ? load_fn(W.lv[0], c) : fn_identity();
+      const unsigned bad = __ballot_sync(0xffffffffu, f.meta == 0u);
+      const int a = bad ? __ffs(bad) - 1 : 32, b = bad ? 31 - __clz(bad) : 31;
+      const Fn p = warp_reduce_fn(lane < a ? f : fn_identity(), lane);
+      const Fn q = warp_reduce_fn(lane > b ? f : fn_identity(), lane);
+      if (lane == 0) {
+        pre[i] = p;
+        suf[i] = q;
+        first[i] = (uint8_t)a;
+        last[i] = (uint8_t)b;
+      }
+      for (unsigned left = bad; left; left &= left - 1u) {  // the values about to be replayed
+        const long long v = ((long long)at[i] * 32 + __ffs(left) - 1) * kChunk + lane * 8;
+        if (v < n) asm volatile("prefetch.global.L1 [%0];" ::"l"(map + v));
+      }
+    } else {  // between mixed blocks i - 1 and i
+      const long long a = i ? (long long)at[i - 1] + 1 : 0, b = i < nm ? (long long)at[i] : nblocks;
+      const Fn f = compose_blocks(W, a, b, lane);
+      if (lane == 0) gap[i] = f;
+    }
+  }
+  __syncthreads();
+  if (warp > 0) return;
+  double s = 0.0;
+  long long block = 0;
+  for (int i = 0; i <= nm; ++i) {
+    const long long m = i < nm ? (long long)at[i] : nblocks;
+    if (m > block && !apply_fn(gap[i], s))
+      s = walk_range(map, n, scale, sq, W, block * 32, min(m * 32, nchunks), s, lane);
+    if (i == nm) break;
+    const long long c0 = m * 32;
+    const int a = first[i], b = last[i];
+    if (a == b && apply_fn(pre[i], s)) {  // the usual case: one unpredicted chunk
+      s = replay_chunk(map, n, scale, sq, c0 + a, s, lane);
+      if (apply_fn(suf[i], s)) {
+        block = m + 1;
+        continue;
+      }
+      const Fn f = c0 + lane < nchunks ? load_fn(W.lv[0], c0 + lane) : fn_identity();
+      s = walk_block(map, n, scale, sq, c0, f, b + 1, 31, s, lane);
+    } else {
+      const Fn f = c0 + lane < nchunks ? load_fn(W.lv[0], c0 + lane) : fn_identity();
+      s = walk_block(map, n, scale, sq, c0, f, 0, 31, s, lane);
+    }
+    block = m + 1;
   }
   if (lane == 0) out[sq ? 1 : 0] = s;
 }
@@ -732,64 +939,85 @@ int level_counts(long long nchunks, long long* cnt) {
 
 }  // namespace
 
-size_t ordered_sum_scratch_bytes(long long n) {
-  const long long nchunks = n > 0 ? (n + kChunk - 1) / kChunk : 1;
-  const long long nblocks = (nchunks + 31) / 32;
-  auto rnd = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  size_t bytes = 2 * rnd((size_t)nchunks * 4) + 2 * rnd((size_t)nblocks * 8);
+namespace {
+
+// The scratch memory's parts, in order; base null: sizes only.
+struct Parts {
+  char* base;
+  size_t used = 0;
+  template <class T>
+  T* take(long long count) {
+    char* r = base ? base + used : nullptr;
+    used += ((size_t)count * sizeof(T) + 255) & ~(size_t)255;
+    return reinterpret_cast<T*>(r);
+  }
+};
+
+struct Plan {
+  float *cs, *cq;
+  Sums sums;
+  Walk ws, wq;
+  size_t zero_at, zero_bytes;  // the part that starts at 0: group sums, mixed lists
+  size_t bytes;
+};
+
+Plan plan_of(long long n, void* scratch) {
+  const long long nchunks = n > 0 ? (n + kChunk - 1) / kChunk : 1, nblocks = (nchunks + 31) / 32;
+  Parts p{static_cast<char*>(scratch)};
+  Plan r{};
+  r.cs = p.take<float>(nchunks);
+  r.cq = p.take<float>(nchunks);
+  r.sums.s[0] = p.take<unsigned long long>(nblocks);
+  r.sums.q[0] = p.take<unsigned long long>(nblocks);
   long long cnt[kMaxLevels];
   const int nlev = level_counts(nchunks, cnt);
-  for (int L = 0; L < nlev; ++L) bytes += 2 * (2 * rnd((size_t)cnt[L] * 8) + rnd((size_t)cnt[L] * 4));
-  return bytes;
+  r.ws.nlev = r.wq.nlev = nlev;
+  for (int L = 0; L < nlev; ++L)
+    for (Walk* w : {&r.ws, &r.wq}) {
+      w->lv[L].i0 = p.take<unsigned long long>(cnt[L]);
+      w->lv[L].i1 = p.take<unsigned long long>(cnt[L]);
+      w->lv[L].meta = p.take<uint32_t>(cnt[L]);
+      w->cnt[L] = cnt[L];
+    }
+  r.zero_at = p.used;
+  for (int L = 1; L < kSumLevels; ++L) {
+    const long long groups = ((nblocks - 1) >> (5 * L)) + 1;
+    r.sums.s[L] = p.take<unsigned long long>(groups);
+    r.sums.q[L] = p.take<unsigned long long>(groups);
+  }
+  r.ws.mixed = p.take<uint32_t>(1 + kMaxMixed);
+  r.wq.mixed = p.take<uint32_t>(1 + kMaxMixed);
+  r.zero_bytes = p.used - r.zero_at;
+  r.bytes = p.used;
+  return r;
 }
+
+}  // namespace
+
+size_t ordered_sum_scratch_bytes(long long n) { return plan_of(n, nullptr).bytes; }
 
 cudaError_t launch_ordered_sums(const float* map, long long n, float scale, const uint32_t* maxbits, void* scratch,
                                 double* out, cudaStream_t s, unsigned long long* launches) {
   if (n <= 0) return cudaMemsetAsync(out, 0, 2 * sizeof(double), s);
-  const long long nchunks = (n + kChunk - 1) / kChunk;
-  const long long nblocks = (nchunks + 31) / 32;
-  char* p = static_cast<char*>(scratch);
-  auto take = [&](size_t bytes) {
-    char* r = p;
-    p += (bytes + 255) & ~(size_t)255;
-    return r;
-  };
-  float* cs = reinterpret_cast<float*>(take((size_t)nchunks * 4));
-  float* cq = reinterpret_cast<float*>(take((size_t)nchunks * 4));
-  unsigned long long* bs = reinterpret_cast<unsigned long long*>(take((size_t)nblocks * 8));
-  unsigned long long* bq = reinterpret_cast<unsigned long long*>(take((size_t)nblocks * 8));
-  Walk ws{}, wq{};
-  long long cnt[kMaxLevels];
-  const int nlev = level_counts(nchunks, cnt);
-  for (int L = 0; L < nlev; ++L) {
-    for (Walk* w : {&ws, &wq}) {
-      w->lv[L].i0 = reinterpret_cast<unsigned long long*>(take((size_t)cnt[L] * 8));
-      w->lv[L].i1 = reinterpret_cast<unsigned long long*>(take((size_t)cnt[L] * 8));
-      w->lv[L].meta = reinterpret_cast<uint32_t*>(take((size_t)cnt[L] * 4));
-      w->cnt[L] = cnt[L];
-    }
+  const Plan p = plan_of(n, scratch);
+  const long long nchunks = p.ws.cnt[0];
+  const unsigned blocks = (unsigned)p.ws.cnt[1];
+  cudaError_t e = cudaMemsetAsync(static_cast<char*>(scratch) + p.zero_at, 0, p.zero_bytes, s);
+  if (e != cudaSuccess) return e;
+  if (n < kSmallMap) {
+    osum_chunk_kernel<1><<<blocks, 1024, 0, s>>>(map, n, scale, nchunks, maxbits, p.cs, p.cq, p.sums);
+    osum_fn_kernel<1><<<blocks, 1024, 0, s>>>(map, n, scale, nchunks, maxbits, p.cs, p.cq, p.sums, p.ws, p.wq);
+  } else {
+    osum_chunk_kernel<4><<<blocks, 256, 0, s>>>(map, n, scale, nchunks, maxbits, p.cs, p.cq, p.sums);
+    osum_fn_kernel<4><<<blocks, 256, 0, s>>>(map, n, scale, nchunks, maxbits, p.cs, p.cq, p.sums, p.ws, p.wq);
   }
-  ws.nlev = wq.nlev = nlev;
-  const unsigned warps_per_cta = 8;
-  const unsigned g1 = (unsigned)((nblocks + warps_per_cta - 1) / warps_per_cta);
-  osum_chunk_kernel<<<g1, 32 * warps_per_cta, 0, s>>>(map, n, scale, nchunks, maxbits, cs, cq, bs, bq);
-  osum_scan_kernel<<<1, 1024, 0, s>>>(bs, bq, nblocks);
-  osum_fn_kernel<<<g1, 32 * warps_per_cta, 0, s>>>(map, n, scale, nchunks, maxbits, cs, cq, bs, bq, ws.lv[0],
-                                                   wq.lv[0], ws.lv[1], wq.lv[1]);
   *launches += 3;
-  for (int L = 2; L < nlev; ++L) {
-    const unsigned g = (unsigned)((cnt[L] + warps_per_cta - 1) / warps_per_cta);
-    osum_level_kernel<<<g, 32 * warps_per_cta, 0, s>>>(ws.lv[L - 1], wq.lv[L - 1], cnt[L - 1], ws.lv[L], wq.lv[L]);
+  for (int L = 2; L < p.ws.nlev; ++L) {
+    osum_level_kernel<<<(unsigned)((p.ws.cnt[L] + 7) / 8), 256, 0, s>>>(p.ws.lv[L - 1], p.wq.lv[L - 1], p.ws.cnt[L - 1],
+                                                                       p.ws.lv[L], p.wq.lv[L]);
     ++*launches;
   }
-  const int Lc = cached_from(cnt, nlev);
-  size_t wsmem = 0;
-  for (int L = Lc; L < nlev; ++L) wsmem += ((size_t)cnt[L] * kEntryBytes + 15) & ~(size_t)15;
-  cudaError_t e = cudaFuncSetAttribute(osum_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)kWalkSmemBytes + 1024);
-  if (e != cudaSuccess) return e;
-  osum_walk_kernel<<<2, 32, wsmem, s>>>(map, n, scale, ws, wq, out);
-  ++*launches;
+  osum_walk_kernel<<<2, kWalkWarps * 32, 0, s>>>(map, n, scale, p.ws, p.wq, out);
   return cudaGetLastError();
 }
 
