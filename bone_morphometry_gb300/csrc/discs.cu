@@ -199,7 +199,8 @@ disc_list_kernel(const uint16_t* __restrict__ rmap, Dims dm, int H, const uint32
   uint32_t* largest = smem;  // kListZ x kPlaneCells: rho << 16 | R
   uint2* centres = reinterpret_cast<uint2*>(largest + kListZ * kPlaneCells);  // kCentres
   uint2* queues = centres + kCentres;
-  __shared__ uint32_t s_count[kListZ], s_full, s_centres;
+  static_assert(kListZ == 32, "a bit per plane");
+  __shared__ uint32_t s_count[kListZ], s_full, s_centres;  // s_full: planes whose list goes to the pool
   __shared__ uint2* s_dst[kListZ];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned below = (1u << lane) - 1u;
@@ -229,6 +230,7 @@ disc_list_kernel(const uint16_t* __restrict__ rmap, Dims dm, int H, const uint32
   for (int pass = 0; pass < 3; ++pass) {
     const int kept = pass ? (int)s_centres : 0;
     const bool cached = pass && kept <= kCentres;  // else the columns are walked again
+    const uint32_t planes = pass == 2 ? s_full : ~0u;
     int n = 0, nr = 0, z = w0, ci = warp * 32;
     uint32_t v[kWalk + 2];  // planes z - 1 .. z + kWalk
     auto at = [&](int z) -> uint32_t { return in && z >= 0 && z < dm.d ? src[(long long)z * slice] : 0u; };
@@ -291,17 +293,17 @@ disc_list_kernel(const uint16_t* __restrict__ rmap, Dims dm, int H, const uint32
         }
         // runs {R | column << 16 | length << 24, first plane | (first plane - centre's + 128) << 8}
         for (bool last = false; !last;) {
-          const bool more = lo <= hi;
-          const unsigned m = __ballot_sync(0xffffffffu, more);
-          if (more)
+          const int run = min(kRunLen, hi - lo + 1);
+          const unsigned m = __ballot_sync(0xffffffffu, run > 0 && (planes >> lo & ((1u << run) - 1u)) != 0u);
+          if (m >> lane & 1u)
             rq[nr + __popc(m & below)] = make_uint2(
-                (uint32_t)R | (cc << 16) | ((uint32_t)min(kRunLen, hi - lo + 1) << 24),
+                (uint32_t)R | (cc << 16) | ((uint32_t)run << 24),
                 (uint32_t)lo | ((uint32_t)(lo - k + 128) << 8));
           nr += __popc(m);
           lo += kRunLen;
           __syncwarp();
           // a full warp of runs, or what is left at the very end
-          last = m == 0u;
+          last = !__any_sync(0xffffffffu, lo <= hi);
           const bool flush = last && n == 0 && final;
           if (nr < 32 && !(flush && nr > 0)) continue;
           const int rtake = min(nr, 32);
@@ -332,7 +334,7 @@ disc_list_kernel(const uint16_t* __restrict__ rmap, Dims dm, int H, const uint32
               const int h = (int)floor_sqrt((uint32_t)rho), ra = (int)(a & 0xffffu), rb = (int)(b & 0xffffu);
               yhi = ra >= Rr ? min(h, cut_above((int)(a >> 16) - rho, ra > Rr)) : h;
               ylo = rb >= Rr ? max(-h, cut_below((int)(b >> 16) - rho)) : -h;
-              keep = !covered && ylo <= yhi && (pass == 1 || s_dst[kk] != nullptr);
+              keep = !covered && ylo <= yhi && (planes >> kk & 1u);
             }
             // one counter update per plane and warp
             const unsigned grp = __match_any_sync(0xffffffffu, keep ? kk : -1);
@@ -368,7 +370,7 @@ disc_list_kernel(const uint16_t* __restrict__ rmap, Dims dm, int H, const uint32
             list[0].x = (uint32_t)first;
             s_dst[k] = pool + first;
             s_count[k] = 0u;
-            s_full = 1u;
+            atomicOr(&s_full, 1u << k);
           } else {
             ctr->disc_overflow = 1u;
             h = 0u;
@@ -505,34 +507,46 @@ disc_paint_kernel(const uint32_t* __restrict__ hdr, const uint2* __restrict__ en
       while (nq >= 32 || (done && nq > 0)) {
         const int take = min(nq, 32);
         nq -= take;
-        // the rows of the discs one after the other, 32 at a time: a lane's disc is
-        // the last one that starts at or before its row
+        // the rows of the discs one after the other, two to a lane: a lane's disc
+        // is the last one that starts at or before its rows
         const uint2 it = q[nq + min(lane, take - 1)];
-        const int rows = lane < take ? (int)(it.y >> 26) - (int)((it.y >> 20) & 63u) + 1 : 0;
-        int end = rows;
+        const int ya = (int)((it.y >> 20) & 63u);
+        const int pairs = lane < take ? ((int)(it.y >> 26) - ya + 2) >> 1 : 0;
+        int end = pairs;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
           const int u = __shfl_up_sync(0xffffffffu, end, o);
           if (lane >= o) end += u;
         }
-        const int start = end - rows, total = __shfl_sync(0xffffffffu, end, 31);
-        const int first = (int)((it.y >> 20) & 63u) - start;  // row = first + position
-        int before = 0;                                       // discs that start before s
+        const int start = end - pairs, total = __shfl_sync(0xffffffffu, end, 31);
+        const int first = ya - 2 * start;  // row = first + 2 * position
+        int before = 0;                    // discs that start before s
         for (int s = 0; s < total; s += 32) {
           const unsigned at = (unsigned)(start - s);
-          const unsigned starts = __reduce_or_sync(0xffffffffu, rows > 0 && at < 32u ? 1u << at : 0u);
+          const unsigned starts = __reduce_or_sync(0xffffffffu, pairs > 0 && at < 32u ? 1u << at : 0u);
           const int owner = before + __popc(starts & (2u * below + 1u)) - 1;
           before += __popc(starts);
           const uint32_t ox = __shfl_sync(0xffffffffu, it.x, owner), oy = __shfl_sync(0xffffffffu, it.y, owner);
-          const int y = __shfl_sync(0xffffffffu, first, owner) + s + lane;
+          const int y = __shfl_sync(0xffffffffu, first, owner) + 2 * (s + lane);
           if (s + lane < total) {
             const uint32_t R = ox >> 16;
             const int cx = (int)(oy & 1023u) - 256, dy = y - (int)((oy >> 10) & 1023u) + 256;
-            const int hw = (int)floor_sqrt((ox & 0xffffu) - (uint32_t)(dy * dy));
-            const int xa = max(cx - hw, 0), len = min(cx + hw, kPaintX - 1) - xa + 1;
-            if (len > 0) {
-              const uint2 off = chord[len];
-              uint32_t* p = lev + off.x + y * kPaintStride + xa;
+            const int t0 = (int)(ox & 0xffffu) - dy * dy, t1 = t0 - 2 * dy - 1;
+            const bool two = y < (int)(oy >> 26);
+            const int h0 = (int)floor_sqrt((uint32_t)t0), h1 = (int)floor_sqrt((uint32_t)max(t1, 0));
+            const int xa0 = max(cx - h0, 0), len0 = min(cx + h0, kPaintX - 1) - xa0 + 1;
+            const int xa1 = max(cx - h1, 0), len1 = two ? min(cx + h1, kPaintX - 1) - xa1 + 1 : 0;
+            uint32_t* row = lev + y * kPaintStride;
+            if (len0 > 0) {
+              const uint2 off = chord[len0];
+              uint32_t* p = row + off.x + xa0;
+              uint32_t* p2 = p + off.y;
+              if (*p < R) atomicMax(p, R);
+              if (*p2 < R) atomicMax(p2, R);
+            }
+            if (len1 > 0) {
+              const uint2 off = chord[len1];
+              uint32_t* p = row + kPaintStride + off.x + xa1;
               uint32_t* p2 = p + off.y;
               if (*p < R) atomicMax(p, R);
               if (*p2 < R) atomicMax(p2, R);
