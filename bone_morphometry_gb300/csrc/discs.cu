@@ -44,9 +44,8 @@ __device__ __forceinline__ uint32_t floor_sqrt(uint32_t t) {
 __device__ __forceinline__ uint32_t max3(uint32_t a, uint32_t b, uint32_t c) { return max(max(a, b), c); }
 
 // ---- ridge map --------------------------------------------------------------
-// Distance ridge (local_thickness.rs:104-167) as a u16 map: 0 for a
-// non-selected voxel, 2 R + 1 for a ridge voxel of squared radius R, 1 for any
-// other selected voxel.  A warp owns 30 x (its outer lanes hold the x
+// Distance ridge (local_thickness.rs:104-167) as a u16 map: twice the squared
+// distance (0 for a non-selected voxel), plus 1 for a ridge voxel.  A warp owns 30 x (its outer lanes hold the x
 // neighbours) and ROWS rows and walks NZ planes upwards; each plane's rows are
 // loaded once and reduced to the maxima that the face, edge and corner tests of
 // three planes share, in registers.
@@ -110,7 +109,7 @@ ridge_map_kernel(const uint32_t* __restrict__ dist, Dims dm, const uint2* __rest
         const uint2 t = __ldg(thr + R);  // {face | edge << 16, corner}
         const bool ridge = max(face[r], hi[r].c) < (t.x & 0xffffu) && max(edge[r], hi[r].m) < (t.x >> 16) &&
                            max(corner[r], hi[r].s) < t.y;
-        v = ridge ? 2u * R + 1u : 1u;
+        v = 2u * R + (ridge ? 1u : 0u);
       }
       if (xout && y0 + r < dm.h) dst[(long long)z * slice + r * dm.w] = (uint16_t)v;
       face[r] = max(hi[r].m, mid[r].c);
@@ -146,8 +145,8 @@ constexpr int kListZ = 32;                 // planes per CTA
 constexpr int kCols = kDiscPX * kDiscPY;   // columns of the patch
 constexpr int kRowPad = kDiscPX + 2;       // per-plane table with an empty border of one cell
 constexpr int kPlaneCells = (kDiscPY + 2) * kRowPad;
-constexpr int kRunLen = 4;                 // planes per run
-constexpr int kWalk = 4;                   // planes a thread walks per step
+constexpr int kRunLen = 3;                 // planes per run
+constexpr int kWalk = 6;                   // planes a thread walks per step
 constexpr int kCentres = 4096;             // ball centres a CTA keeps from its first walk
 // centres and runs a warp holds back until 32 are ready
 constexpr int kCentreQueue = 32 + 32 * kWalk, kRunQueue = 64;
@@ -170,24 +169,26 @@ __device__ __forceinline__ int cell_of(uint32_t c) { return (int)(c >> 5) * kRow
 // ball centres they meet are collected per warp, handled 32 at a time, and kept
 // for the second step (up to kCentres; beyond, the columns are walked again).
 //
-// Cut along z: the planes of a centre's discs end where one of its two
-// neighbours in the column covers them.  For the centre above, with R' >= R,
-// rho' - rho grows along z, so it covers this one's discs from some plane on,
-// and the one below up to some plane (of two equal discs the lower centre's
-// stays).  First step: every disc left enters a table of the largest rho of its
+// Cut along z: the planes of a centre's discs end where the ball of one of its
+// two neighbours in the column covers them, ridge voxel or not (a ball that is
+// not on the ridge lies in a larger one that is).  For the neighbour above, with
+// R' >= R, rho' - rho grows along z, so it covers this centre's discs from some
+// plane on, and the one below up to some plane (of two equal discs the lower
+// one stays).  First step: every disc left enters a table of the largest rho of its
 // column and plane.  Second step, a thread per run of up to kRunLen discs:
 //   - a disc that its own column's largest disc covers (R' >= R, rho' >= rho)
 //     or that of one of the six neighbouring columns at x -+ 1 is left out;
 //   - the rows of the others are cut at the largest discs of the columns at
 //     y -+ 1, as the planes were along z.
-// At any row, each of these tests leaves a chord out only for one with R' >= R
-// and a larger squared half-length (or an equal one and a lower centre), so no
-// chain of them closes and the last of a chain is painted.
+// At any row, each of these tests leaves a chord out only for one with R' > R, or
+// with R' = R and a larger squared half-length (or an equal one and a lower
+// centre).  So of the chords of the largest R that contain a voxel one is left:
+// no chain of tests among them closes.
 //
-// Per selected voxel of the 192^3 marrow phase: 1.9 discs enter the table, 0.87
-// discs with 7.5 rows are listed.  Cutting the planes at every centre of the
-// column enters 1.5 and lists as many; testing the six columns at x -+ 2 too
-// lists 0.79 with 6.7 rows.
+// Per selected voxel of the 192^3 marrow phase: 1.55 discs enter the table, 0.85
+// discs with 7.4 rows are listed.  Cutting at ridge voxels alone enters 2.0,
+// at every centre of the column 1.5, and lists as many; testing the six columns
+// at x -+ 2 too lists 0.79 with 6.7 rows, for as much time as it saves.
 //
 // A plane with more than kDiscSlots discs gets a segment of the overflow pool
 // and a third step.
@@ -234,9 +235,12 @@ disc_list_kernel(const uint16_t* __restrict__ rmap, Dims dm, int H, const uint32
     int n = 0, nr = 0, z = w0, ci = warp * 32;
     uint32_t v[kWalk + 2];  // planes z - 1 .. z + kWalk
     auto at = [&](int z) -> uint32_t { return in && z >= 0 && z < dm.d ? src[(long long)z * slice] : 0u; };
+    uint32_t ahead[kWalk];  // the next step's planes, in flight during this one
     if (!cached) {
       v[0] = at(w0 - 1);
       v[1] = at(w0);
+#pragma unroll
+      for (int j = 0; j < kWalk; ++j) ahead[j] = at(w0 + 1 + j);
     }
     for (bool final = false; !final;) {
       if (cached) {
@@ -244,11 +248,15 @@ disc_list_kernel(const uint16_t* __restrict__ rmap, Dims dm, int H, const uint32
         final = ci + kListThreads >= kept;
       } else {
 #pragma unroll
-        for (int j = 0; j < kWalk; ++j) v[2 + j] = at(z + 1 + j);
+        for (int j = 0; j < kWalk; ++j) v[2 + j] = ahead[j];
+        if (z + kWalk < w1) {
+#pragma unroll
+          for (int j = 0; j < kWalk; ++j) ahead[j] = at(z + kWalk + 1 + j);
+        }
 #pragma unroll
         for (int j = 0; j < kWalk; ++j) {
           const int k = z + j - z0;
-          const uint32_t R = v[1 + j] >> 1;
+          const uint32_t R = v[1 + j] & 1u ? v[1 + j] >> 1 : 0u;
           const int far = k < 0 ? -k : max(k - (nz - 1), 0);
           const bool have = z + j < w1 && R != 0u && (int)R >= far * far;  // a centre whose ball meets the planes
           const unsigned m = __ballot_sync(0xffffffffu, have);
@@ -541,15 +549,15 @@ disc_paint_kernel(const uint32_t* __restrict__ hdr, const uint2* __restrict__ en
               const uint2 off = chord[len0];
               uint32_t* p = row + off.x + xa0;
               uint32_t* p2 = p + off.y;
-              if (*p < R) atomicMax(p, R);
-              if (*p2 < R) atomicMax(p2, R);
+              atomicMax(p, R);
+              atomicMax(p2, R);
             }
             if (len1 > 0) {
               const uint2 off = chord[len1];
               uint32_t* p = row + kPaintStride + off.x + xa1;
               uint32_t* p2 = p + off.y;
-              if (*p < R) atomicMax(p, R);
-              if (*p2 < R) atomicMax(p2, R);
+              atomicMax(p, R);
+              atomicMax(p2, R);
             }
           }
         }

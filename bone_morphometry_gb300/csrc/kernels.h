@@ -101,7 +101,7 @@ size_t disc_header_count(Dims dm);
 // thr / tmpl: n entries by squared radius, from the search templates.
 cudaError_t launch_disc_tables(const uint4* lut, uint32_t n, uint2* thr, uint32_t* tmpl, cudaStream_t s,
                                unsigned long long* launches);
-// The distance ridge as a u16 map (0: not selected, 1: selected, 2 R + 1: ridge of squared radius R).
+// The distance ridge as a u16 map: twice the squared distance, plus 1 for ridge voxels.
 cudaError_t launch_ridge_map(const uint32_t* dist, Dims dm, const uint2* thr, uint16_t* rmap, cudaStream_t s,
                              unsigned long long* launches);
 // Disc lists: hdr[patch] = count | reach << 16 for every 32 x 8 patch of every
