@@ -33,11 +33,11 @@
 //   3. a walker per sum.  The blocks whose composition is invalid -- the ~30
 //      binade crossings -- are listed by step 2; the walker's warps compose the
 //      runs of blocks between them, and inside each of them the chunks before
-//      the first and after the last unpredicted chunk.  One warp then follows
-//      the sequence from s = 0: a composed run is one integer addition, an
-//      unpredicted chunk is replayed: lanes sum their increments, a warp scan
-//      finds the lane whose values leave the binade, and that lane adds its
-//      eight values with f64 additions, the reference's own operation.
+//      the first and after the last unpredicted chunk.  Then they follow the
+//      sequence from s = 0 together: a composed run is one integer addition, an
+//      unpredicted chunk is replayed, a value per thread: a scan of the
+//      increments finds the value that leaves the binade, and that one is added
+//      with an f64 addition, the reference's own operation.
 // Every step the walker takes is checked against the exact state, and where a
 // prediction does not hold it goes through the levels and, at worst, replays
 // every chunk: a wrong prediction costs time, never exactness.  No per-value
@@ -45,11 +45,12 @@
 // fraction of its f32 and integer rates.  Not a reference function: the
 // reference's loop is serial (metrics.rs:215-226).
 //
-// Per map, against the earlier form (a serial fold per chunk, a one-CTA scan,
-// a walker that went through the levels alone): 0.11 against 0.22 ms on
-// 64 x 56 x 72, 0.35 against 0.50 ms on 33.5 M values, 0.69 against 0.90 ms on
+// Per map, against an earlier form (a serial fold per chunk, a one-CTA scan, a
+// one-warp walker that went through the levels): 0.08 against 0.22 ms on
+// 64 x 56 x 72, 0.30 against 0.50 ms on 33.5 M values, 0.64 against 0.90 ms on
 // 512^3.  The second step is bound by the integer ALU pipe, the walker by the
-// latency of its replays.
+// latency of its replays (about 1.5 us each; 3.7 us by one warp of 8 values a
+// lane).
 #include <climits>
 #include <cstdint>
 
@@ -175,21 +176,6 @@ __device__ __forceinline__ Term term(float raw, float scale, bool sq) {
 __device__ __forceinline__ double term_value(float raw, float scale, bool sq) {
   const double v = (double)__fmul_rn(raw, scale);
   return sq ? __dmul_rn(v, v) : v;
-}
-
-// The increment of an element M * 2^k (M < 2^MBITS) in the binade whose ulp is
-// 2^em52, when it does not depend on the parity; odd is set for a tie, and for
-// an increment of 2^54 or more, which need the ordered fold.  Without branches:
-// with M moved up to 54 bits, every increment is one right shift (of a whole
-// number of ulps, one rounded, or one that loses the element).
-template <int MBITS>
-__device__ __forceinline__ unsigned long long plain_increment(unsigned long long M, int k, int em52, bool& odd) {
-  constexpr int kUp = 54 - MBITS;
-  const int r = em52 - k + kUp;
-  const unsigned s = (unsigned)min(max(r, 0), 55);
-  const unsigned long long half = (1ull << s) >> 1, t = (M << kUp) + half;
-  odd = odd || (r < 0 && M != 0ull) || (s != 0u && (t & (2ull * half - 1ull)) == 0ull);  // a remainder of exactly half an ulp
-  return t >> s;
 }
 
 __device__ __forceinline__ int binade_of(double s) {
@@ -622,113 +608,108 @@ __global__ void __launch_bounds__(256) osum_level_kernel(Level s_in, Level q_in,
   }
 }
 
-__device__ __forceinline__ Fn shfl_up_fn(const Fn& f, int o) {
-  Fn r;
-  r.i0 = __shfl_up_sync(0xffffffffu, f.i0, o);
-  r.i1 = __shfl_up_sync(0xffffffffu, f.i1, o);
-  r.meta = __shfl_up_sync(0xffffffffu, f.meta, o);
-  return r;
-}
+// Shared memory of a replay.
+struct Replay {
+  unsigned long long total[kChunk / 32];
+  uint32_t parity[kChunk / 32];
+  int first;
+  unsigned long long units;
+  double s;
+};
 
-// Inclusive in-order scan: lane j gets the composition of lanes 0 .. j.
-__device__ __forceinline__ Fn warp_scan_fn(Fn f, int lane) {
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const Fn g = shfl_up_fn(f, o);
-    if (lane >= o) f = compose(g, f);
-  }
-  return f;
-}
-
-// Replays chunk c from state s exactly as the reference adds.  Lane l holds
-// values 8l .. 8l+7.  In s's binade every lane sums its values' increments and
-// a warp scan adds them up (or, when a value ties, folds and composes them in
-// order); the first lane whose prefix leaves the binade (or the lane holding
-// the first value, s = 0) adds its values with f64 additions, the reference's
-// own operation (metrics.rs:223-224), and the lanes after it go on in the new
-// binade.  s is broadcast back.
+// Replays chunk c from state s exactly as the reference adds, by a CTA of kChunk
+// threads that all hold s, a value per thread.  In s's binade every value is an
+// increment; a scan of them gives the state after each value, and the first
+// value that leaves the binade (or the first value at all, s = 0) is added with
+// an f64 addition, the reference's own operation (metrics.rs:223-224); the
+// values after it go on in the new binade.  A tie is rounded to even by the
+// parity before it, from a scan of its own: a value flips the parity or, after
+// a tie, leaves it even.
 __device__ __noinline__ double replay_chunk(const float* __restrict__ map, long long n, float scale, bool sq,
-                                            long long c, double s, int lane) {
-  float vals[8];
-  load8(map, n, c * kChunk + lane * 8, vals);
-  unsigned long long M[8];
-  int k[8];
-  bool inf = false, any = false;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const Term t = term(vals[j], scale, sq);
-    const bool is_inf = t.k == INT_MAX;
-    M[j] = is_inf ? 0ull : t.M;
-    k[j] = is_inf ? 0 : t.k;
-    inf = inf || is_inf;
-    any = any || t.M != 0ull;
-  }
-  int start = 0;  // first lane not yet added
-  while (start < 32) {
-    if (!isfinite(s)) break;  // +inf stays +inf
-    int b;                    // the lane that adds serially
+                                            long long c, double s, Replay& sh) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const long long at = c * kChunk + tid;
+  const float raw = at < n ? map[at] : 0.0f;
+  const Term t = term(raw, scale, sq);
+  const bool has = t.M != 0ull, inf = t.k == INT_MAX;
+  const double x = has ? term_value(raw, scale, sq) : 0.0;
+  for (int start = 0; start < kChunk;) {  // the first value not yet added
+    if (!isfinite(s)) return s;           // +inf stays +inf
+    int b;                                // the value added in f64
+    double before = s;
     if (s == 0.0) {
-      const unsigned m = __ballot_sync(0xffffffffu, lane >= start && any);
-      if (!m) break;
-      b = __ffs(m) - 1;
+      if (tid == 0) sh.first = kChunk;
+      __syncthreads();
+      if (has && tid >= start) atomicMin(&sh.first, tid);
+      __syncthreads();
+      b = sh.first;
+      if (b == kChunk) return s;
     } else {
-      const int E = binade_of(s);
+      const int E = binade_of(s), sft = E - 52 - (inf ? 0 : t.k);
       const unsigned long long u0 = units_of(s);
       unsigned long long inc = 0;
-      bool odd = inf;
-      if (sq) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) inc += plain_increment<48>(M[j], k[j], E - 52, odd);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) inc += plain_increment<24>(M[j], k[j], E - 52, odd);
+      bool tie = false;
+      if (has && tid >= start) {
+        if (inf || sft <= -54 || (sft < 0 && (t.M >> (54 + sft)) != 0ull)) {
+          inc = kSat;  // leaves the binade
+        } else if (sft <= 0) {
+          inc = t.M << -sft;
+        } else if (sft <= 48) {
+          const unsigned long long rem = t.M & ((1ull << sft) - 1ull), half = 1ull << (sft - 1);
+          tie = rem == half;
+          inc = (t.M >> sft) + (rem > half ? 1ull : 0ull);
+        }
       }
-      if (lane < start) inc = 0ull;
-      unsigned long long after;
-      if (!__any_sync(0xffffffffu, odd && lane >= start)) {
+      if (__syncthreads_or(tie)) {
+        // bit 1: the parity is set (to bit 0), else flipped by bit 0
+        auto then = [](uint32_t f, uint32_t g) { return g & 2u ? g : (f & 2u) | ((f ^ g) & 1u); };
+        uint32_t f = tie ? 2u : (uint32_t)(inc & 1ull);
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-          const unsigned long long u = __shfl_up_sync(0xffffffffu, inc, o);
-          if (lane >= o) inc += u;
+          const uint32_t g = __shfl_up_sync(0xffffffffu, f, o);
+          if (lane >= o) f = then(g, f);
         }
-        after = sat_add(u0, inc);
-      } else {
-        Acc A{0ull, 0ull, 0u, 1u};
-        const bool has = any && lane >= start;
-        if (has) {
-          if (inf) A.i0 = A.i1 = kSat;
-#pragma unroll
-          for (int j = 0; j < 8; ++j)
-            if (M[j]) acc_elem(A, M[j], k[j], E - 52, 48);
-        }
-        const Fn pre = warp_scan_fn(acc_fn(A, has, E), lane);
-        after = sat_add(u0, (u0 & 1ull) ? pre.i1 : pre.i0);
+        if (lane == 31) sh.parity[warp] = f;
+        __syncthreads();
+        uint32_t p = 2u | (uint32_t)(u0 & 1ull);  // the parity before the warp
+        for (int w = 0; w < warp; ++w) p = then(p, sh.parity[w]);
+        const uint32_t g = __shfl_up_sync(0xffffffffu, f, 1);
+        if (lane > 0) p = then(p, g);
+        if (tie) inc += (inc + p) & 1ull;
       }
-      const unsigned bad = __ballot_sync(0xffffffffu, lane >= start && after > kTwo53);
-      if (!bad) {
-        s = from_units(__shfl_sync(0xffffffffu, after, 31), E);
-        break;
-      }
-      b = __ffs(bad) - 1;
-      // lanes start .. b-1 stay in the binade: s after them
-      const unsigned long long ub = __shfl_sync(0xffffffffu, after, b > 0 ? b - 1 : 0);
-      if (b > start) s = from_units(ub, E);
-    }
-    if (lane == b) {
+      unsigned long long incl = inc;
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (vals[j] > 0.0f && isfinite(vals[j])) s = __dadd_rn(s, term_value(vals[j], scale, sq));
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long g = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += g;
+      }
+      if (lane == 31) sh.total[warp] = incl;
+      __syncthreads();
+      unsigned long long after = u0 + incl;
+      for (int w = 0; w < warp; ++w) after += sh.total[w];
+      b = __syncthreads_count(after <= kTwo53);  // the states only grow
+      if (b == kChunk) {
+        if (tid == kChunk - 1) sh.units = after;
+        __syncthreads();
+        return from_units(sh.units, E);
+      }
+      before = from_units(after - inc, E);
     }
-    s = __shfl_sync(0xffffffffu, s, b);
+    if (tid == b) sh.s = __dadd_rn(before, x);
+    __syncthreads();
+    s = sh.s;
     start = b + 1;
   }
-  return __shfl_sync(0xffffffffu, s, 0);
+  return s;
 }
 
+// The walker's state is the same in all its threads: every warp makes the same
+// steps, and the replays are theirs together.
+//
 // Follows the sequence through one block whose chunk functions the lanes hold
 // (lane j: chunk c0 + j; identity past the map's end), from lane p to lane e.
 __device__ __noinline__ double walk_block(const float* __restrict__ map, long long n, float scale, bool sq,
-                                          long long c0, const Fn& f, int p, int e, double s, int lane) {
+                                          long long c0, const Fn& f, int p, int e, double s, int lane, Replay& sh) {
   while (p <= e) {
     if (!isfinite(s)) break;
     const int E = s == 0.0 ? INT_MIN : binade_of(s);
@@ -754,7 +735,7 @@ __device__ __noinline__ double walk_block(const float* __restrict__ map, long lo
         continue;
       }
     }
-    s = replay_chunk(map, n, scale, sq, c0 + p, s, lane);
+    s = replay_chunk(map, n, scale, sq, c0 + p, s, sh);
     ++p;
   }
   return s;
@@ -764,7 +745,7 @@ __device__ __noinline__ double walk_block(const float* __restrict__ map, long lo
 // whose entry starts at c, does not pass `end` and applies, up to 32 entries of
 // it at a time, or a replay of one chunk.
 __device__ __noinline__ double walk_range(const float* __restrict__ map, long long n, float scale, bool sq,
-                                          const Walk& W, long long c, long long end, double s, int lane) {
+                                          const Walk& W, long long c, long long end, double s, int lane, Replay& sh) {
   while (c < end) {
     if (!isfinite(s)) break;  // a value overflowed to +inf: the sum stays +inf
     bool moved = false;
@@ -809,7 +790,7 @@ __device__ __noinline__ double walk_range(const float* __restrict__ map, long lo
       }
     }
     if (!moved) {
-      s = replay_chunk(map, n, scale, sq, c, s, lane);
+      s = replay_chunk(map, n, scale, sq, c, s, sh);
       ++c;
     }
   }
@@ -843,7 +824,7 @@ __device__ Fn compose_blocks(const Walk& W, long long a, long long b, int lane) 
   return compose(front, back);
 }
 
-constexpr int kWalkWarps = 16;
+constexpr int kWalkWarps = kChunk / 32;
 
 // 3. The walker: block 0 follows the sum of values, block 1 the sum of squares.
 __global__ void __launch_bounds__(kWalkWarps * 32)
@@ -852,16 +833,15 @@ osum_walk_kernel(const float* __restrict__ map, long long n, float scale, Walk w
   __shared__ Fn gap[kMaxMixed + 1];                   // the blocks before each of them (and after the last)
   __shared__ Fn pre[kMaxMixed], suf[kMaxMixed];       // their chunks before the first / after the last unpredicted one
   __shared__ uint8_t first[kMaxMixed], last[kMaxMixed];
+  __shared__ Replay replay;
   const bool sq = blockIdx.x == 1;
   const Walk& W = sq ? wq : ws;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const long long nchunks = W.cnt[0], nblocks = W.cnt[1];
   const int nm = (int)W.mixed[0];
   if (nm > kMaxMixed) {  // many wrong predictions: through all levels
-    if (warp == 0) {
-      const double s = walk_range(map, n, scale, sq, W, 0, nchunks, 0.0, lane);
-      if (lane == 0) out[sq ? 1 : 0] = s;
-    }
+    const double s = walk_range(map, n, scale, sq, W, 0, nchunks, 0.0, lane, replay);
+    if (tid == 0) out[sq ? 1 : 0] = s;
     return;
   }
   for (int i = tid; i < nm; i += kWalkWarps * 32) {
@@ -897,31 +877,30 @@ osum_walk_kernel(const float* __restrict__ map, long long n, float scale, Walk w
     }
   }
   __syncthreads();
-  if (warp > 0) return;
   double s = 0.0;
   long long block = 0;
   for (int i = 0; i <= nm; ++i) {
     const long long m = i < nm ? (long long)at[i] : nblocks;
     if (m > block && !apply_fn(gap[i], s))
-      s = walk_range(map, n, scale, sq, W, block * 32, min(m * 32, nchunks), s, lane);
+      s = walk_range(map, n, scale, sq, W, block * 32, min(m * 32, nchunks), s, lane, replay);
     if (i == nm) break;
     const long long c0 = m * 32;
     const int a = first[i], b = last[i];
     if (a == b && apply_fn(pre[i], s)) {  // the usual case: one unpredicted chunk
-      s = replay_chunk(map, n, scale, sq, c0 + a, s, lane);
+      s = replay_chunk(map, n, scale, sq, c0 + a, s, replay);
       if (apply_fn(suf[i], s)) {
         block = m + 1;
         continue;
       }
       const Fn f = c0 + lane < nchunks ? load_fn(W.lv[0], c0 + lane) : fn_identity();
-      s = walk_block(map, n, scale, sq, c0, f, b + 1, 31, s, lane);
+      s = walk_block(map, n, scale, sq, c0, f, b + 1, 31, s, lane, replay);
     } else {
       const Fn f = c0 + lane < nchunks ? load_fn(W.lv[0], c0 + lane) : fn_identity();
-      s = walk_block(map, n, scale, sq, c0, f, 0, 31, s, lane);
+      s = walk_block(map, n, scale, sq, c0, f, 0, 31, s, lane, replay);
     }
     block = m + 1;
   }
-  if (lane == 0) out[sq ? 1 : 0] = s;
+  if (tid == 0) out[sq ? 1 : 0] = s;
 }
 
 // Entry counts of the levels: chunks, then blocks of 32 per level up to a
