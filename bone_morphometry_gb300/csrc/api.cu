@@ -308,157 +308,160 @@ void ensure_surf(bm_ctx* ctx, uint32_t rmax) {
   ctx->surf_max = target;
 }
 
-struct PhaseResult {
-  unsigned long long sites = 0, selected = 0, ridges = 0;
-  uint32_t rmax = 0;
-  StatsAccum acc;
-  double osum[2] = {0.0, 0.0};  // the reference's sequential sum and sum of squares
+// Page-locked readback area of a context: copies into it return at once, so a
+// phase's work is queued to its end without a wait.
+struct Readback {
+  Counters ctr;                   // after the distance transform
+  PhaseOut out;                   // at the end of the phase
+  unsigned long long counts[3];   // ROI counts; volume counts
+  QuantileState quantile;
 };
+
+Readback& readback(bm_ctx* ctx) { return *static_cast<Readback*>(ctx->pinned); }
+
+PhaseOut* phase_out(bm_ctx* ctx, size_t flags = 0) {
+  return static_cast<PhaseOut*>(ensure(ctx, ctx->phaseout, sizeof(PhaseOut) + flags, "phase results"));
+}
 
 // The reference's sequential f64 sums of the calibrated map values
-// (metrics.rs:215-224), on stream s, after the statistics accumulator acc has
-// its maximum; results land in ctx->ordout.
-void ordered_sums(bm_ctx* ctx, const float* d_map, long long n, float scale, const StatsAccum* acc, cudaStream_t s) {
+// (metrics.rs:215-224) into out->osum, on stream s, after out->acc has its
+// maximum.
+void ordered_sums(bm_ctx* ctx, const float* d_map, long long n, float scale, PhaseOut* out, cudaStream_t s) {
   void* scratch = ensure(ctx, ctx->ordscratch, ordered_sum_scratch_bytes(n), "ordered-sum scratch");
-  double* out = static_cast<double*>(ensure(ctx, ctx->ordout, 2 * sizeof(double), "ordered sums"));
   timed(ctx, KF_STATS_ORDER, s, "ordered sums", [&] {
-    return launch_ordered_sums(d_map, n, scale, &acc->max_bits, scratch, out, s, &ctx->launches);
-  });
-}
-
-// The buffers of one phase's distance transform.
-struct EdtBufs {
-  uint32_t* A;        // x pass output (kept for the chain passes), y pass input
-  uint32_t* B;        // y pass output
-  void* scratch;      // envelope scratch of the flagged lines
-  uint32_t* selbits;  // selection bits
-  Counters* ctr;
-  uint8_t* redo;      // per-line flags of the windowed passes
-};
-
-EdtBufs edt_buffers(bm_ctx* ctx, Dims dm) {
-  const size_t N = (size_t)dm.n();
-  const size_t bits_bytes = (size_t)dm.nw() * dm.h * dm.d * sizeof(uint32_t);
-  EdtBufs b;
-  b.A = static_cast<uint32_t*>(ensure(ctx, ctx->dist, N * 4, "distance map"));
-  b.B = static_cast<uint32_t*>(ensure(ctx, ctx->dist2, N * 4, "distance map"));
-  b.scratch = ensure(ctx, ctx->stack, edt_scratch_bytes(dm), "envelope scratch");
-  b.selbits = static_cast<uint32_t*>(ensure(ctx, ctx->selbits, bits_bytes, "selection bits"));
-  b.ctr = static_cast<Counters*>(ensure(ctx, ctx->counters, sizeof(Counters), "counters"));
-  const size_t redo_bytes = (size_t)dm.w * (dm.h > dm.d ? dm.h : dm.d);
-  b.redo = static_cast<uint8_t*>(ensure(ctx, ctx->redo, redo_bytes, "line flags"));
-  return b;
-}
-
-// The x and y passes of planes z0 .. z1-1: both work within a plane, so a slab
-// of planes is a volume of its own (every offset is a whole number of planes,
-// which keeps the 16-byte alignment of rows whose width is a multiple of 4).
-// The counters accumulate over slabs.
-void edt_xy(bm_ctx* ctx, Dims dm, const uint8_t* d_a, const uint8_t* d_b, int mode, const EdtBufs& b, int z0, int z1,
-            cudaStream_t s) {
-  const Dims sd{dm.w, dm.h, z1 - z0};
-  const long long off = (long long)z0 * dm.w * dm.h;
-  const uint8_t* a = d_a + off;
-  const uint8_t* bb = d_b ? d_b + off : nullptr;
-  uint32_t* A = b.A + off;
-  uint32_t* B = b.B + off;
-  uint32_t* sel = b.selbits + (long long)z0 * dm.h * dm.nw();
-  timed(ctx, KF_EDT_X, s, "edt x pass",
-        [&] { return launch_edt_x(a, bb, mode, sd, A, sel, b.ctr, s, &ctx->launches); });
-  timed(ctx, KF_EDT_Y, s, "edt y pass", [&] {
-    return launch_edt_window(1, A, B, sd, b.scratch, b.redo, b.ctr, ctx->wait_cycles, s, &ctx->launches);
+    return launch_ordered_sums(d_map, n, scale, &out->acc.max_bits, scratch, out->osum, s, &ctx->launches);
   });
 }
 
 // One phase: EDT (+ local thickness unless edt_only, + the reference-order
 // statistics sums when stats).  d_a / d_b are the device inputs for `mode`;
 // results optionally go to d_edt (u32 EDT), d_map (f32 masked diameters) and
-// d_sq (u32 propagated r^2).  xy_done: the x and y passes have already run on
-// this context's buffers (slab by slab, as the inputs arrived), with its
-// counters cleared before them.
-void run_phase(bm_ctx* ctx, Dims dm, const uint8_t* d_a, const uint8_t* d_b, int mode, bool edt_only,
-               uint32_t* d_edt, float* d_map, uint32_t* d_sq, float scale, bool stats, cudaStream_t s,
-               PhaseResult& res, bool xy_done = false) {
-  const size_t N = (size_t)dm.n();
-  const size_t bits_bytes = (size_t)dm.nw() * dm.h * dm.d * sizeof(uint32_t);
-  const EdtBufs eb = edt_buffers(ctx, dm);
-  uint32_t* A = eb.A;
-  uint32_t* B = eb.B;
-  void* scratch = eb.scratch;
-  uint32_t* selbits = eb.selbits;
-  Counters* ctr = eb.ctr;
-  uint8_t* redo = eb.redo;
-  if (!xy_done) {
-    check(ctx, cudaMemsetAsync(ctr, 0, sizeof(Counters), s), "memset");
-    edt_xy(ctx, dm, d_a, d_b, mode, eb, 0, dm.d, s);
-  }
-  // local thickness keeps the x pass output (the chain passes read it): the z
-  // pass then writes its own map
-  uint32_t* E = d_edt ? d_edt
-                      : (edt_only ? A : static_cast<uint32_t*>(ensure(ctx, ctx->edtmap, N * 4, "distance map")));
-  timed(ctx, KF_EDT_Z, s, "edt z pass",
-        [&] { return launch_edt_window(2, B, E, dm, scratch, redo, ctr, ctx->wait_cycles, s, &ctx->launches); });
+// d_sq (u32 propagated r^2).
+//
+// The steps only queue work, but for the two waits: prepare, xy (slab by slab
+// where the inputs arrive so), z; wait_edt, whose largest radius sizes and
+// chooses what follows; fill; finish, which waits for the results.  The two
+// phases of a call are stepped in turn by one host thread, each on its own
+// context.  64^3 device inputs: 272 us, against 383 with a thread started per
+// call, pageable readbacks and a wait for the ROI counts before either phase
+// (128^3 host inputs with quantiles: 547 against 688).
+struct Phase {
+  // set by the caller
+  bm_ctx* ctx;
+  Dims dm;
+  const uint8_t* d_a;
+  const uint8_t* d_b;
+  int mode;
+  cudaStream_t s;
+  bool edt_only = false, stats = false;
+  uint32_t* d_edt = nullptr;
+  float* d_map = nullptr;
+  uint32_t* d_sq = nullptr;
+  float scale = 1.0f;
 
-  Counters hc;
-  check(ctx, cudaMemcpyAsync(&hc, ctr, sizeof hc, cudaMemcpyDeviceToHost, s), "counter readback");
-  check(ctx, cudaStreamSynchronize(s), "edt");
-  if (hc.status) fail(ctx, BM_ERR_TIMEOUT, "a bounded device-side wait of the distance transform ran out");
-  res.sites = hc.sites;
-  res.selected = N - hc.sites;
-  res.rmax = hc.rmax;
-  if (hc.sites == 0) {
-    const int phase = (mode == SEL_BACKGROUND) ? BM_PHASE_BACKGROUND : BM_PHASE_FOREGROUND;
-    fail(ctx, BM_ERR_ALL_SELECTED,
-         "distance transform is undefined for an all-%s volume unless an exterior convention is specified",
-         phase_name(phase));
-  }
-  if (edt_only) return;
+  // results
+  Counters hc{};
+  StatsAccum acc;
+  double osum[2] = {0.0, 0.0};
 
-  ensure_lut(ctx, hc.rmax);
-  const uint4* lut = static_cast<const uint4*>(ctx->lut.ptr);
-  const float* dia = static_cast<const float*>(ctx->lutf.ptr);
-  // cleanup, statistics and the readbacks that end the phase, from the fill's diameters and nonzero bits
-  uint32_t* nzbits = static_cast<uint32_t*>(ensure(ctx, ctx->nzbits, bits_bytes, "nonzero bits"));
-  uint32_t* inbits = static_cast<uint32_t*>(ensure(ctx, ctx->inbits, bits_bytes, "interior bits"));
-  auto finish = [&](const float* dmap) {
-    StatsAccum* acc = static_cast<StatsAccum*>(ensure(ctx, ctx->accum, sizeof(StatsAccum), "stats"));
-    check(ctx, cudaMemsetAsync(acc, 0, sizeof(StatsAccum), s), "memset");
-    FixedPartial* part = static_cast<FixedPartial*>(
-        ensure(ctx, ctx->cpart, kCleanupMaxGrid * sizeof(FixedPartial), "stats partials"));
-    // every value of the map is at least 2 * scale (diameters are >= 2), so its
-    // f32 exponent is at least that of 2 * scale: the fixed-point base
-    const float two_s = 2.0f * scale;
-    uint32_t tb;
-    std::memcpy(&tb, &two_s, 4);
-    const int e2s = (int)(tb >> 23);
-    const int e_lo = (e2s >= 1 && e2s + kFixedSpan <= 254) ? e2s : 4096;  // 4096: no fixed-point path
-    unsigned cgrid = 0;
-    // the statistics' ordered sums read the f32 map: keep one when the caller wants none
-    float* cmap = (stats && !d_map) ? static_cast<float*>(ensure(ctx, ctx->ordmap, N * 4, "thickness map")) : d_map;
-    timed(ctx, KF_CLEAN_FINAL, s, "cleanup",
-          [&] {
-            return launch_cleanup(dmap, selbits, nzbits, inbits, dm, scale, cmap, acc, part, e_lo, &cgrid, s,
-                                  &ctx->launches);
-          });
-    if (stats) ordered_sums(ctx, cmap, (long long)N, scale, acc, s);
-    std::vector<FixedPartial> hpart(cgrid);
-    check(ctx, cudaMemcpyAsync(&res.acc, acc, sizeof(StatsAccum), cudaMemcpyDeviceToHost, s), "stats readback");
-    if (stats)
-      check(ctx, cudaMemcpyAsync(res.osum, ctx->ordout.ptr, 2 * sizeof(double), cudaMemcpyDeviceToHost, s),
-            "stats readback");
-    if (cgrid)
-      check(ctx, cudaMemcpyAsync(hpart.data(), part, cgrid * sizeof(FixedPartial), cudaMemcpyDeviceToHost, s),
-            "stats readback");
-    check(ctx, cudaMemcpyAsync(&hc, ctr, sizeof hc, cudaMemcpyDeviceToHost, s), "counter readback");
-    check(ctx, cudaStreamSynchronize(s), "local thickness");
-    if (e_lo != 4096) fold_fixed_partials(res.acc, hpart.data(), cgrid, e_lo);
-    res.ridges = hc.ridges;
-  };
-  // The separable fill (discs.cu) up to radius 127, where its packed
-  // discs end; a forced site method or tile height asks for the
-  // tile fill.
-  const bool separable = hc.rmax <= kDiscMaxR2 && ctx->site_method == BM_SITES_AUTO && ctx->fill_rows == 0;
-  if (separable) {
+  uint32_t* A = nullptr;        // x pass output (kept for the chain passes), y pass input
+  uint32_t* B = nullptr;        // y pass output
+  uint32_t* E = nullptr;        // z pass output
+  void* scratch = nullptr;      // envelope scratch of the flagged lines
+  uint32_t* selbits = nullptr;  // selection bits
+  PhaseOut* out = nullptr;
+  uint8_t* yflags = nullptr;    // per-line flags of the windowed passes
+  uint8_t* zflags = nullptr;
+  bool separable = false;
+  int e_lo = 0;
+
+  size_t voxels() const { return (size_t)dm.n(); }
+  size_t bits_bytes() const { return (size_t)dm.nw() * dm.h * dm.d * sizeof(uint32_t); }
+
+  // Buffers, and everything the phase accumulates into zeroed.
+  void prepare() {
+    const size_t N = voxels();
+    A = static_cast<uint32_t*>(ensure(ctx, ctx->dist, N * 4, "distance map"));
+    B = static_cast<uint32_t*>(ensure(ctx, ctx->dist2, N * 4, "distance map"));
+    scratch = ensure(ctx, ctx->stack, edt_scratch_bytes(dm), "envelope scratch");
+    selbits = static_cast<uint32_t*>(ensure(ctx, ctx->selbits, bits_bytes(), "selection bits"));
+    const size_t ny = (size_t)dm.w * dm.d, nz = (size_t)dm.w * dm.h;
+    out = phase_out(ctx, ny + nz);
+    yflags = reinterpret_cast<uint8_t*>(out + 1);
+    zflags = yflags + ny;
+    // local thickness keeps the x pass output (the chain passes read it): the z
+    // pass then writes its own map
+    E = d_edt ? d_edt : (edt_only ? A : static_cast<uint32_t*>(ensure(ctx, ctx->edtmap, N * 4, "distance map")));
+    check(ctx, cudaMemsetAsync(out, 0, sizeof(PhaseOut) + ny + nz, s), "memset");
+  }
+
+  // The x and y passes of planes z0 .. z1-1: both work within a plane, so a slab
+  // of planes is a volume of its own (every offset is a whole number of planes,
+  // which keeps the 16-byte alignment of rows whose width is a multiple of 4).
+  // The counters accumulate over slabs.
+  void xy(int z0, int z1) {
+    const Dims sd{dm.w, dm.h, z1 - z0};
+    const long long off = (long long)z0 * dm.w * dm.h;
+    const uint8_t* a = d_a + off;
+    const uint8_t* b = d_b ? d_b + off : nullptr;
+    uint32_t* sel = selbits + (long long)z0 * dm.h * dm.nw();
+    uint8_t* flags = yflags + (long long)z0 * dm.w;
+    timed(ctx, KF_EDT_X, s, "edt x pass",
+          [&] { return launch_edt_x(a, b, mode, sd, A + off, sel, &out->ctr, s, &ctx->launches); });
+    timed(ctx, KF_EDT_Y, s, "edt y pass", [&] {
+      const cudaError_t e =
+          launch_edt_window(1, A + off, B + off, sd, flags, &out->ctr, ctx->wait_cycles, s, &ctx->launches);
+      if (e != cudaSuccess) return e;
+      return launch_edt_redo(1, A + off, B + off, sd, scratch, flags, &out->ctr, s, &ctx->launches);
+    });
+  }
+
+  void z() {
+    timed(ctx, KF_EDT_Z, s, "edt z pass", [&] {
+      return launch_edt_window(2, B, E, dm, zflags, &out->ctr, ctx->wait_cycles, s, &ctx->launches);
+    });
+    read_counters();
+  }
+
+  void read_counters() {
+    check(ctx, cudaMemcpyAsync(&readback(ctx).ctr, &out->ctr, sizeof(Counters), cudaMemcpyDeviceToHost, s),
+          "counter readback");
+  }
+
+  void wait_edt() {
+    check(ctx, cudaStreamSynchronize(s), "edt");
+    hc = readback(ctx).ctr;
+    if (hc.z_redo) {
+      timed(ctx, KF_EDT_Z, s, "edt z lines",
+            [&] { return launch_edt_redo(2, B, E, dm, scratch, zflags, &out->ctr, s, &ctx->launches); });
+      read_counters();
+      check(ctx, cudaStreamSynchronize(s), "edt");
+      hc = readback(ctx).ctr;
+    }
+    if (hc.status) fail(ctx, BM_ERR_TIMEOUT, "a bounded device-side wait of the distance transform ran out");
+    if (hc.sites == 0) {
+      const int phase = (mode == SEL_BACKGROUND) ? BM_PHASE_BACKGROUND : BM_PHASE_FOREGROUND;
+      fail(ctx, BM_ERR_ALL_SELECTED,
+           "distance transform is undefined for an all-%s volume unless an exterior convention is specified",
+           phase_name(phase));
+    }
+    // The separable fill (discs.cu) up to radius 127, where its packed
+    // discs end; a forced site method or tile height asks for the
+    // tile fill.
+    separable = hc.rmax <= kDiscMaxR2 && ctx->site_method == BM_SITES_AUTO && ctx->fill_rows == 0;
+  }
+
+  // Local thickness, after wait_edt: queued to its end, but for the tile
+  // fill's own waits.
+  void fill() {
+    ensure_lut(ctx, hc.rmax);
+    if (separable) disc_fill();
+    else tile_fill();
+  }
+
+  void disc_fill() {
+    const size_t N = voxels();
+    uint32_t* nzbits = static_cast<uint32_t*>(ensure(ctx, ctx->nzbits, bits_bytes(), "nonzero bits"));
     uint16_t* rmap = static_cast<uint16_t*>(ensure(ctx, ctx->ridgemap, N * sizeof(uint16_t), "ridge map"));
     const size_t lists = disc_header_count(dm);
     uint32_t* hdr = static_cast<uint32_t*>(ensure(ctx, ctx->dischdr, lists * 4, "disc lists"));
@@ -467,36 +470,88 @@ void run_phase(bm_ctx* ctx, Dims dm, const uint8_t* d_a, const uint8_t* d_b, int
     uint2* pool = static_cast<uint2*>(ensure(ctx, ctx->discpool, pool_cap * sizeof(uint2), "disc lists"));
     const uint2* thr = static_cast<const uint2*>(ctx->discthr.ptr);
     const uint32_t* tmpl = static_cast<const uint32_t*>(ctx->disctmpl.ptr);
+    const float* dia = static_cast<const float*>(ctx->lutf.ptr);
     timed(ctx, KF_RIDGE, s, "ridge map", [&] { return launch_ridge_map(E, dm, thr, rmap, s, &ctx->launches); });
     timed(ctx, KF_FILL_BIN, s, "disc lists", [&] {
-      return launch_disc_lists(rmap, dm, hc.rmax, tmpl, hdr, ent, pool, pool_cap, ctr, s, &ctx->launches);
+      return launch_disc_lists(rmap, dm, hc.rmax, tmpl, hdr, ent, pool, pool_cap, &out->ctr, s, &ctx->launches);
     });
     float* dmap = reinterpret_cast<float*>(B);  // the y pass output has been read
     timed(ctx, KF_FILL, s, "disc painting", [&] {
       return launch_disc_paint(hdr, ent, pool, dm, hc.rmax, dia, dmap, nzbits, d_sq, s, &ctx->launches);
     });
-    finish(dmap);
-    if (!hc.disc_overflow) return;
-    // the lists' pool ran out: again with the tile fill, in the lists' memory
-    for (Buffer* b : {&ctx->ridgemap, &ctx->discent, &ctx->discpool}) release(*b);
+    cleanup(dmap, nzbits);
   }
-  uint2* ridges = static_cast<uint2*>(ensure(ctx, ctx->ridges, (res.selected + 1) * sizeof(uint2), "ridge list"));
-  const size_t rwords = (size_t)hc.rmax + 2;
-  uint32_t* occ = static_cast<uint32_t*>(ensure(ctx, ctx->occ, rwords * 4, "r2 flags"));
-  check(ctx, cudaMemsetAsync(occ, 0, rwords * 4, s), "memset");
-  uint32_t* rbits = static_cast<uint32_t*>(ensure(ctx, ctx->ridgebits, bits_bytes, "ridge bits"));
-  check(ctx, cudaMemsetAsync(rbits, 0, bits_bytes, s), "memset");
-  timed(ctx, KF_RIDGE, s, "ridge kernel",
-        [&] { return launch_ridges(E, selbits, dm, lut, ridges, ctr, occ, rbits, s, &ctx->launches); });
-  const bool own_e = E != A && E != d_edt;  // E is the context's map: the chain passes may reuse it
-  // (after the separable fill, B no longer holds the y pass output the chain passes need)
-  const bool chains = own_e && !separable;
-  uint32_t* F = fill_phase(ctx, dm, ridges, ctr, res.selected, hc.rmax, occ, selbits, A, B, chains ? E : nullptr,
-                           rbits, d_sq ? d_sq : B, s);
-  float* dmap = reinterpret_cast<float*>(F == d_sq ? B : F);
-  timed(ctx, KF_CLEAN_FINAL, s, "diameters",
-        [&] { return launch_diameters(F, dm, dia, dmap, nzbits, s, &ctx->launches); });
-  finish(dmap);
+
+  void tile_fill() {
+    const uint4* lut = static_cast<const uint4*>(ctx->lut.ptr);
+    const float* dia = static_cast<const float*>(ctx->lutf.ptr);
+    const unsigned long long selected = voxels() - hc.sites;
+    uint32_t* nzbits = static_cast<uint32_t*>(ensure(ctx, ctx->nzbits, bits_bytes(), "nonzero bits"));
+    uint2* ridges = static_cast<uint2*>(ensure(ctx, ctx->ridges, (selected + 1) * sizeof(uint2), "ridge list"));
+    const size_t rwords = (size_t)hc.rmax + 2;
+    uint32_t* occ = static_cast<uint32_t*>(ensure(ctx, ctx->occ, rwords * 4, "r2 flags"));
+    check(ctx, cudaMemsetAsync(occ, 0, rwords * 4, s), "memset");
+    uint32_t* rbits = static_cast<uint32_t*>(ensure(ctx, ctx->ridgebits, bits_bytes(), "ridge bits"));
+    check(ctx, cudaMemsetAsync(rbits, 0, bits_bytes(), s), "memset");
+    timed(ctx, KF_RIDGE, s, "ridge kernel",
+          [&] { return launch_ridges(E, selbits, dm, lut, ridges, &out->ctr, occ, rbits, s, &ctx->launches); });
+    const bool own_e = E != A && E != d_edt;  // E is the context's map: the chain passes may reuse it
+    // (after the separable fill, B no longer holds the y pass output the chain passes need)
+    const bool chains = own_e && !separable;
+    uint32_t* F = fill_phase(ctx, dm, ridges, &out->ctr, selected, hc.rmax, occ, selbits, A, B, chains ? E : nullptr,
+                             rbits, d_sq ? d_sq : B, s);
+    float* dmap = reinterpret_cast<float*>(F == d_sq ? B : F);
+    timed(ctx, KF_CLEAN_FINAL, s, "diameters",
+          [&] { return launch_diameters(F, dm, dia, dmap, nzbits, s, &ctx->launches); });
+    cleanup(dmap, nzbits);
+  }
+
+  // Cleanup, statistics and the readback that ends the phase, from the fill's
+  // diameters and nonzero bits.
+  void cleanup(const float* dmap, const uint32_t* nzbits) {
+    uint32_t* inbits = static_cast<uint32_t*>(ensure(ctx, ctx->inbits, bits_bytes(), "interior bits"));
+    // every value of the map is at least 2 * scale (diameters are >= 2), so its
+    // f32 exponent is at least that of 2 * scale: the fixed-point base
+    const float two_s = 2.0f * scale;
+    uint32_t tb;
+    std::memcpy(&tb, &two_s, 4);
+    const int e2s = (int)(tb >> 23);
+    e_lo = (e2s >= 1 && e2s + kFixedSpan <= 254) ? e2s : 4096;  // 4096: no fixed-point path
+    // the statistics' ordered sums read the f32 map: keep one when the caller wants none
+    float* cmap = (stats && !d_map) ? static_cast<float*>(ensure(ctx, ctx->ordmap, voxels() * 4, "thickness map")) : d_map;
+    timed(ctx, KF_CLEAN_FINAL, s, "cleanup", [&] {
+      return launch_cleanup(dmap, selbits, nzbits, inbits, dm, scale, cmap, &out->acc, e_lo, s, &ctx->launches);
+    });
+    if (stats) ordered_sums(ctx, cmap, dm.n(), scale, out, s);
+    check(ctx, cudaMemcpyAsync(&readback(ctx).out, out, sizeof(PhaseOut), cudaMemcpyDeviceToHost, s), "stats readback");
+  }
+
+  void finish() {
+    check(ctx, cudaStreamSynchronize(s), "local thickness");
+    if (separable && readback(ctx).out.ctr.disc_overflow) {
+      // the lists' pool ran out: again with the tile fill, in the lists' memory
+      for (Buffer* b : {&ctx->ridgemap, &ctx->discent, &ctx->discpool}) release(*b);
+      check(ctx, cudaMemsetAsync(&out->acc, 0, sizeof(StatsAccum), s), "memset");
+      tile_fill();
+      check(ctx, cudaStreamSynchronize(s), "local thickness");
+    }
+    const PhaseOut& r = readback(ctx).out;
+    acc = r.acc;
+    if (e_lo != 4096) acc.fx_elo = e_lo;
+    osum[0] = r.osum[0];
+    osum[1] = r.osum[1];
+  }
+};
+
+// A whole phase, one step after the other.
+void run_phase(Phase& p) {
+  p.prepare();
+  p.xy(0, p.dm.d);
+  p.z();
+  p.wait_edt();
+  if (p.edt_only) return;
+  p.fill();
+  p.finish();
 }
 
 // nonzero_stats (metrics.rs:228-241; quantile fields NaN) from the reference's
@@ -538,7 +593,8 @@ int finish_stats(bm_ctx* ctx, const StatsAccum& a, const double* osum, bm_stats*
 void quantiles(bm_ctx* ctx, const float* d_map, long long n, unsigned long long count, double scale,
                bm_stats* out, cudaStream_t s) {
   static const double kQ[5] = {0.5, 0.1, 0.25, 0.75, 0.9};  // metrics.rs:247-251
-  QuantileState qs{};
+  QuantileState& qs = readback(ctx).quantile;
+  qs = QuantileState{};
   double frac[5];
   for (int i = 0; i < 5; ++i) {
     const double position = kQ[i] * (double)(count - 1);
@@ -576,6 +632,22 @@ void quantiles(bm_ctx* ctx, const float* d_map, long long n, unsigned long long 
   out->interquartile_range = q[3] - q[2];
 }
 
+int nonzero_stats_impl(bm_ctx* ctx, const float* d_values, size_t n, double scale, unsigned flags, bm_stats* out,
+                       cudaStream_t s) {
+  PhaseOut* po = phase_out(ctx);
+  check(ctx, cudaMemsetAsync(po, 0, sizeof(PhaseOut), s), "memset");
+  timed(ctx, KF_QUANTILE, s, "moments kernel",
+        [&] { return launch_moments(d_values, (long long)n, (float)scale, &po->acc, s, &ctx->launches); });
+  ordered_sums(ctx, d_values, (long long)n, (float)scale, po, s);
+  PhaseOut& r = readback(ctx).out;
+  check(ctx, cudaMemcpyAsync(&r, po, sizeof(PhaseOut), cudaMemcpyDeviceToHost, s), "stats readback");
+  check(ctx, cudaStreamSynchronize(s), "moments kernel");
+  const int st = finish_stats(ctx, r.acc, r.osum, out);
+  if (st) return st;
+  if (flags & BM_FLAG_QUANTILES) quantiles(ctx, d_values, (long long)n, r.acc.count, scale, out, s);
+  return BM_OK;
+}
+
 template <class F>
 int guarded(bm_ctx* ctx, F&& f) {
   if (!ctx) return BM_ERR_INVALID;
@@ -601,17 +673,19 @@ cudaStream_t pick_stream(bm_ctx* ctx, void* stream) {
 }
 
 int edt_device_impl(bm_ctx* ctx, const uint8_t* d_vol, Dims dm, int phase, uint32_t* d_out, cudaStream_t s) {
-  PhaseResult r;
-  run_phase(ctx, dm, d_vol, nullptr, phase == BM_PHASE_BACKGROUND ? SEL_BACKGROUND : SEL_FOREGROUND, true, d_out,
-            nullptr, nullptr, 1.0f, false, s, r);
+  Phase p{ctx, dm, d_vol, nullptr, phase == BM_PHASE_BACKGROUND ? SEL_BACKGROUND : SEL_FOREGROUND, s};
+  p.edt_only = true;
+  p.d_edt = d_out;
+  run_phase(p);
   return BM_OK;
 }
 
 int lt_device_impl(bm_ctx* ctx, const uint8_t* d_vol, Dims dm, int phase, float* d_out, uint32_t* d_sq,
                    cudaStream_t s) {
-  PhaseResult r;
-  run_phase(ctx, dm, d_vol, nullptr, phase == BM_PHASE_BACKGROUND ? SEL_BACKGROUND : SEL_FOREGROUND, false,
-            nullptr, d_out, d_sq, 1.0f, false, s, r);
+  Phase p{ctx, dm, d_vol, nullptr, phase == BM_PHASE_BACKGROUND ? SEL_BACKGROUND : SEL_FOREGROUND, s};
+  p.d_map = d_out;
+  p.d_sq = d_sq;
+  run_phase(p);
   return BM_OK;
 }
 
@@ -808,7 +882,7 @@ int volume_metrics_impl(bm_ctx* ctx, const uint8_t* d_bone, const uint8_t* d_roi
   for (int i = 0; i < 3; ++i)
     if (!std::isfinite(sp[i]) || sp[i] <= 0.0)
       fail(ctx, BM_ERR_SPACING, "voxel spacings must be finite and positive; got [%g, %g, %g]", sp[0], sp[1], sp[2]);
-  unsigned long long* dc = static_cast<unsigned long long*>(ensure(ctx, ctx->counters, sizeof(Counters), "counters"));
+  unsigned long long* dc = reinterpret_cast<unsigned long long*>(phase_out(ctx));
   check(ctx, cudaMemsetAsync(dc, 0, 24, s), "memset");
   timed(ctx, KF_COUNT_ROI, s, "volume counts", [&] {
     if (((reinterpret_cast<uintptr_t>(d_bone) | reinterpret_cast<uintptr_t>(d_roi)) & 3u) == 0)
@@ -818,7 +892,7 @@ int volume_metrics_impl(bm_ctx* ctx, const uint8_t* d_bone, const uint8_t* d_roi
     ++ctx->launches;
     return cudaGetLastError();
   });
-  unsigned long long hc[3];
+  unsigned long long* hc = readback(ctx).counts;
   check(ctx, cudaMemcpyAsync(hc, dc, 24, cudaMemcpyDeviceToHost, s), "count readback");
   check(ctx, cudaStreamSynchronize(s), "volume counts");
   const double voxel_volume = ((1.0 * sp[0]) * sp[1]) * sp[2];  // metrics.rs:123 (product)
@@ -856,109 +930,190 @@ void check_call(bm_ctx* ctx, double spacing, unsigned flags) {
     fail(ctx, BM_ERR_INVALID, "unknown flags 0x%x", flags);
 }
 
-// Work already done by the upload pipeline of bm_tbth_tbsp: the ROI counts, and
-// the x and y passes of either phase.
-struct Prestaged {
-  unsigned long long roi = 0, bone_in_roi = 0;
-  bool bone_xy = false, marrow_xy = false;
-};
-
 bool phases_side_by_side(const bm_ctx* ctx, Dims dm) { return ctx->split_phases && dm.n() <= kSplitMaxVoxels; }
 
-int tbth_device_impl(bm_ctx* ctx, const uint8_t* d_bone, const uint8_t* d_roi, Dims dm, double spacing,
-                     unsigned flags, bm_stats* th, bm_stats* sp, float* d_thmap, float* d_spmap, cudaStream_t s,
-                     const Prestaged* pre = nullptr) {
-  check_call(ctx, spacing, flags);
-  const long long N = dm.n();
-  unsigned long long hc[2];
-  if (pre) {
-    hc[0] = pre->roi;
-    hc[1] = pre->bone_in_roi;
-  } else {
-    unsigned long long* dcnt =
-        static_cast<unsigned long long*>(ensure(ctx, ctx->roicount, 2 * sizeof(unsigned long long), "counts"));
-    check(ctx, cudaMemsetAsync(dcnt, 0, 16, s), "memset");
-    timed(ctx, KF_COUNT_ROI, s, "count kernel", [&] {
-      count_roi_kernel<<<152 * 8, 256, 0, s>>>(d_bone, d_roi, N, dcnt);
-      ++ctx->launches;
-      return cudaGetLastError();
-    });
-    check(ctx, cudaMemcpyAsync(hc, dcnt, 16, cudaMemcpyDeviceToHost, s), "count readback");
-    check(ctx, cudaStreamSynchronize(s), "count kernel");
-  }
-  if (hc[0] == 0) fail(ctx, BM_ERR_ROI_EMPTY, "ROI mask contains no included voxels");
-  if ((flags & BM_FLAG_BONEJ_ROI) && hc[0] == (unsigned long long)N)
-    fail(ctx, BM_ERR_ROI_FULL, "BoneJ compatibility mode requires an ROI mask with both inside and outside voxels");
-  if (hc[1] == 0) fail(ctx, BM_ERR_NO_BONE, "ROI contains no bone voxels");
-  if (hc[1] == hc[0]) fail(ctx, BM_ERR_NO_MARROW, "ROI contains no marrow voxels");
+void count_roi(bm_ctx* ctx, const uint8_t* d_bone, const uint8_t* d_roi, long long n, PhaseOut* out, cudaStream_t s) {
+  timed(ctx, KF_COUNT_ROI, s, "count kernel", [&] {
+    count_roi_kernel<<<152 * 8, 256, 0, s>>>(d_bone, d_roi, n, out->roi);
+    ++ctx->launches;
+    return cudaGetLastError();
+  });
+}
 
-  const float scale = (float)spacing;  // metrics.rs:213
+void read_roi_counts(bm_ctx* ctx, const PhaseOut* out, cudaStream_t s) {
+  check(ctx, cudaMemcpyAsync(readback(ctx).counts, out->roi, sizeof out->roi, cudaMemcpyDeviceToHost, s),
+        "count readback");
+  check(ctx, cudaEventRecord(ctx->counted, s), "event record");
+}
+
+// Waits for the ROI counts; the bails of metrics.rs:79-99.
+void check_roi_counts(bm_ctx* ctx, long long n, unsigned flags) {
+  check(ctx, cudaEventSynchronize(ctx->counted), "count kernel");
+  const unsigned long long roi = readback(ctx).counts[0], bone = readback(ctx).counts[1];
+  if (roi == 0) fail(ctx, BM_ERR_ROI_EMPTY, "ROI mask contains no included voxels");
+  if ((flags & BM_FLAG_BONEJ_ROI) && roi == (unsigned long long)n)
+    fail(ctx, BM_ERR_ROI_FULL, "BoneJ compatibility mode requires an ROI mask with both inside and outside voxels");
+  if (bone == 0) fail(ctx, BM_ERR_NO_BONE, "ROI contains no bone voxels");
+  if (bone == roi) fail(ctx, BM_ERR_NO_MARROW, "ROI contains no marrow voxels");
+}
+
+// Runs steps of the twin's phase; its error is reported on this context.
+template <class F>
+void on_twin(bm_ctx* ctx, bm_ctx* tw, F&& f) {
+  try {
+    f();
+  } catch (const CallError&) {
+    ctx->last_error = tw->last_error;
+    throw;
+  }
+}
+
+// On every exit from bm_tbth_tbsp: nothing of the call is left in flight (no
+// copy from the caller's buffers, no pass reading the inputs), and the twin's
+// launches count as this context's.
+struct CallFence {
+  bm_ctx* ctx;
+  bm_ctx* twin;
+  cudaStream_t s;
+  bool done = false;  // everything has been waited for
+  ~CallFence() {
+    if (!done) {
+      if (ctx->upload_stream) cudaStreamSynchronize(ctx->upload_stream);
+      cudaStreamSynchronize(s);
+      if (twin) cudaStreamSynchronize(twin->stream);
+    }
+    if (twin) {
+      ctx->launches += twin->launches;
+      twin->launches = 0;
+    }
+  }
+};
+
+int report_phase(Phase& p, bm_ctx* ctx, cudaStream_t s, bool want_q, const float* map, double spacing, bm_stats* out) {
+  const int st = finish_stats(ctx, p.acc, p.osum, out);
+  if (st == BM_OK && want_q && out) quantiles(ctx, map, p.dm.n(), p.acc.count, spacing, out, s);
+  return st;
+}
+
+// bm_tbth_tbsp on device inputs.  feed: queues the ROI counts (into the bone
+// phase's out) and the x and y passes of the bone phase and, side by side, of
+// the marrow phase; the bails are checked once the z passes are queued behind
+// them (the passes only write the phases' own buffers).
+template <class Feed>
+int tbth_phases(bm_ctx* ctx, const uint8_t* d_bone, const uint8_t* d_roi, Dims dm, double spacing, unsigned flags,
+                bm_stats* th, bm_stats* sp, float* d_thmap, float* d_spmap, cudaStream_t s, Feed&& feed) {
+  const long long N = dm.n();
   const bool want_q = (flags & BM_FLAG_QUANTILES) != 0;
-  float* qm = nullptr;
-  if (want_q && (!d_thmap || !d_spmap))
-    qm = static_cast<float*>(ensure(ctx, ctx->qmap, (size_t)N * 4, "quantile map"));
   // The two phases are independent: the marrow phase runs on the twin context
-  // (its own stream and buffers, on a second host thread) while this thread
-  // runs the bone phase, so their kernels overlap on the GPU.  Results and
-  // errors are reported in the reference's order (bone first).
-  PhaseResult rb, rm;
+  // (its own stream and buffers), so that their kernels overlap on the GPU.
+  // Results and errors are reported in the reference's order (bone first).
   // Side by side only while one phase cannot fill the GPU: on 1024^3 the two
   // phases' kernels compete (174 ms against 159 ms one after the other), on
   // 512^3 and below they fill each other's gaps.
-  const bool bone_xy = pre && pre->bone_xy, marrow_xy = pre && pre->marrow_xy;
-  if (!phases_side_by_side(ctx, dm)) {
-    float* mb = d_thmap ? d_thmap : qm;
-    run_phase(ctx, dm, d_bone, d_roi, SEL_BONE_IN_ROI, false, nullptr, mb, nullptr, scale, true, s, rb, bone_xy);
-    int st = finish_stats(ctx, rb.acc, rb.osum, th);
-    if (st) return st;
-    if (want_q && th) quantiles(ctx, mb, N, rb.acc.count, spacing, th, s);
-    float* mm = d_spmap ? d_spmap : qm;
-    run_phase(ctx, dm, d_bone, d_roi, SEL_MARROW_IN_ROI, false, nullptr, mm, nullptr, scale, true, s, rm, marrow_xy);
-    st = finish_stats(ctx, rm.acc, rm.osum, sp);
-    if (st) return st;
-    if (want_q && sp) quantiles(ctx, mm, N, rm.acc.count, spacing, sp, s);
-    return BM_OK;
+  bm_ctx* tw = phases_side_by_side(ctx, dm) ? twin_of(ctx) : nullptr;
+  bm_ctx* mctx = tw ? tw : ctx;
+  CallFence fence{ctx, tw, s};
+  Phase bone{ctx, dm, d_bone, d_roi, SEL_BONE_IN_ROI, s};
+  Phase marrow{mctx, dm, d_bone, d_roi, SEL_MARROW_IN_ROI, tw ? tw->stream : s};
+  bone.stats = marrow.stats = true;
+  bone.scale = marrow.scale = (float)spacing;  // metrics.rs:213
+  auto map_of = [&](bm_ctx* c, float* caller) {
+    return caller || !want_q ? caller : static_cast<float*>(ensure(c, c->qmap, (size_t)N * 4, "quantile map"));
+  };
+  if (tw) {
+    check(ctx, cudaEventRecord(ctx->inputs_ready, s), "event record");
+    check(ctx, cudaStreamWaitEvent(tw->stream, ctx->inputs_ready, 0), "stream wait");
   }
-  bm_ctx* tw = twin_of(ctx);
-  float* mb = d_thmap ? d_thmap : qm;
-  float* mm = d_spmap ? d_spmap
-                      : (want_q ? static_cast<float*>(ensure(tw, tw->qmap, (size_t)N * 4, "quantile map")) : nullptr);
-  check(ctx, cudaEventRecord(ctx->inputs_ready, s), "event record");
+  bone.prepare();
+  if (tw) on_twin(ctx, tw, [&] { marrow.prepare(); });
+  feed(bone, tw ? &marrow : nullptr);
+  bone.z();
+  if (tw) on_twin(ctx, tw, [&] { marrow.z(); });
+  check_roi_counts(ctx, N, flags);
+
+  bone.d_map = map_of(ctx, d_thmap);
+  bone.wait_edt();
+  if (!tw) {
+    bone.fill();
+    bone.finish();
+    int st = report_phase(bone, ctx, s, want_q, bone.d_map, spacing, th);
+    if (st) return st;
+    marrow.d_map = map_of(ctx, d_spmap);
+    run_phase(marrow);
+    fence.done = true;
+    return report_phase(marrow, ctx, s, want_q, marrow.d_map, spacing, sp);
+  }
   int twin_status = BM_OK;
-  std::thread marrow([&] {
+  auto try_twin = [&](auto&& f) {
+    if (twin_status != BM_OK) return;
     try {
-      cudaSetDevice(tw->device);
-      check(tw, cudaStreamWaitEvent(tw->stream, ctx->inputs_ready, 0), "stream wait");
-      run_phase(tw, dm, d_bone, d_roi, SEL_MARROW_IN_ROI, false, nullptr, mm, nullptr, scale, true, tw->stream, rm,
-                marrow_xy);
+      f();
     } catch (const CallError& e) {
       twin_status = e.status;
     } catch (const std::bad_alloc&) {
       tw->last_error = "host allocation failed";
       twin_status = BM_ERR_OOM;
     }
+  };
+  try_twin([&] {
+    marrow.d_map = map_of(tw, d_spmap);
+    marrow.wait_edt();
   });
-  int bone_status = BM_OK;
-  try {
-    run_phase(ctx, dm, d_bone, d_roi, SEL_BONE_IN_ROI, false, nullptr, mb, nullptr, scale, true, s, rb, bone_xy);
-  } catch (const CallError& e) {
-    bone_status = e.status;
+  if (twin_status == BM_OK && !(bone.separable && marrow.separable)) {
+    // the tile fill waits for its own counts: a host thread for each phase
+    std::thread thread([&] {
+      try_twin([&] {
+        const cudaError_t e = cudaSetDevice(tw->device);
+        check(tw, e, "cudaSetDevice");
+        marrow.fill();
+        marrow.finish();
+      });
+    });
+    struct Join {
+      std::thread& t;
+      ~Join() { t.join(); }
+    } join{thread};
+    bone.fill();
+    bone.finish();
+  } else {
+    bone.fill();
+    try_twin([&] { marrow.fill(); });
+    bone.finish();
   }
-  marrow.join();
-  ctx->launches += tw->launches;
-  tw->launches = 0;
-  if (bone_status != BM_OK) throw CallError{bone_status};
-  int st = finish_stats(ctx, rb.acc, rb.osum, th);
+  int st = report_phase(bone, ctx, s, want_q, bone.d_map, spacing, th);
   if (st) return st;
-  if (want_q && th) quantiles(ctx, mb, N, rb.acc.count, spacing, th, s);
+  if (marrow.separable && bone.separable) try_twin([&] { marrow.finish(); });
   if (twin_status != BM_OK) {
     ctx->last_error = tw->last_error;
     throw CallError{twin_status};
   }
-  st = finish_stats(ctx, rm.acc, rm.osum, sp);
-  if (st) return st;
-  if (want_q && sp) quantiles(ctx, mm, N, rm.acc.count, spacing, sp, s);
-  return BM_OK;
+  fence.done = true;
+  return report_phase(marrow, ctx, s, want_q, marrow.d_map, spacing, sp);
+}
+
+int tbth_device_impl(bm_ctx* ctx, const uint8_t* d_bone, const uint8_t* d_roi, Dims dm, double spacing,
+                     unsigned flags, bm_stats* th, bm_stats* sp, float* d_thmap, float* d_spmap, cudaStream_t s) {
+  check_call(ctx, spacing, flags);
+  auto feed = [&](Phase& bone, Phase* marrow) {
+    count_roi(ctx, d_bone, d_roi, dm.n(), bone.out, s);
+    read_roi_counts(ctx, bone.out, s);
+    bone.xy(0, dm.d);
+    if (marrow) on_twin(ctx, marrow->ctx, [&] { marrow->xy(0, dm.d); });
+  };
+  try {
+    return tbth_phases(ctx, d_bone, d_roi, dm, spacing, flags, th, sp, d_thmap, d_spmap, s, feed);
+  } catch (const CallError& e) {
+    if (e.status != BM_ERR_OOM) throw;
+    // a bail comes before a failed allocation of the phases' buffers
+    const std::string message = ctx->last_error;
+    PhaseOut* out = phase_out(ctx);
+    check(ctx, cudaMemsetAsync(out, 0, sizeof(PhaseOut), s), "memset");
+    count_roi(ctx, d_bone, d_roi, dm.n(), out, s);
+    read_roi_counts(ctx, out, s);
+    check_roi_counts(ctx, dm.n(), flags);
+    ctx->last_error = message;
+    throw;
+  }
 }
 
 uint8_t* stage_input(bm_ctx* ctx, Buffer& b, const uint8_t* host, size_t n, cudaStream_t s) {
@@ -976,17 +1131,6 @@ uint8_t* stage_input(bm_ctx* ctx, Buffer& b, const uint8_t* host, size_t n, cuda
 constexpr long long kPipeMinVoxels = 1ll << 22;
 constexpr int kPipeSlabs = 8;
 
-// On every exit: no copy from the caller's buffers, and no pass reading the
-// uploaded inputs, is left in flight.
-struct UploadFence {
-  bm_ctx* ctx;
-  bm_ctx* twin;
-  ~UploadFence() {
-    if (ctx->upload_stream) cudaStreamSynchronize(ctx->upload_stream);
-    if (twin) cudaStreamSynchronize(twin->stream);
-  }
-};
-
 int tbth_host_pipelined(bm_ctx* ctx, const uint8_t* bone, const uint8_t* roi, Dims dm, double spacing, unsigned flags,
                         bm_stats* th, bm_stats* sp, float* d_th, float* d_sp, cudaStream_t s) {
   check_call(ctx, spacing, flags);
@@ -1000,58 +1144,27 @@ int tbth_host_pipelined(bm_ctx* ctx, const uint8_t* bone, const uint8_t* roi, Di
     check(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event create");
     ctx->slab_ready.push_back(e);
   }
-  bm_ctx* tw = phases_side_by_side(ctx, dm) ? twin_of(ctx) : nullptr;
-  UploadFence fence{ctx, tw};
-  const EdtBufs eb = edt_buffers(ctx, dm);
-  check(ctx, cudaMemsetAsync(eb.ctr, 0, sizeof(Counters), s), "memset");
-  unsigned long long* dcnt =
-      static_cast<unsigned long long*>(ensure(ctx, ctx->roicount, 2 * sizeof(unsigned long long), "counts"));
-  check(ctx, cudaMemsetAsync(dcnt, 0, 16, s), "memset");
-  // the twin's calls report their errors on this context
-  auto on_twin = [&](auto&& f) {
-    try {
-      f();
-    } catch (const CallError&) {
-      ctx->last_error = tw->last_error;
-      throw;
+  return tbth_phases(ctx, d_bone, d_roi, dm, spacing, flags, th, sp, d_th, d_sp, s, [&](Phase& bp, Phase* mp) {
+    const int K = dm.d < kPipeSlabs ? dm.d : kPipeSlabs;
+    const size_t plane = (size_t)dm.w * dm.h;
+    for (int k = 0; k < K; ++k) {
+      const int z0 = (int)((long long)dm.d * k / K), z1 = (int)((long long)dm.d * (k + 1) / K);
+      const size_t off = (size_t)z0 * plane, len = (size_t)(z1 - z0) * plane;
+      check(ctx, cudaMemcpyAsync(d_bone + off, bone + off, len, cudaMemcpyHostToDevice, ctx->upload_stream),
+            "input upload");
+      check(ctx, cudaMemcpyAsync(d_roi + off, roi + off, len, cudaMemcpyHostToDevice, ctx->upload_stream),
+            "input upload");
+      check(ctx, cudaEventRecord(ctx->slab_ready[k], ctx->upload_stream), "event record");
+      check(ctx, cudaStreamWaitEvent(s, ctx->slab_ready[k], 0), "stream wait");
+      count_roi(ctx, d_bone + off, d_roi + off, (long long)len, bp.out, s);
+      bp.xy(z0, z1);
+      if (mp) on_twin(ctx, mp->ctx, [&] {
+        check(mp->ctx, cudaStreamWaitEvent(mp->s, ctx->slab_ready[k], 0), "stream wait");
+        mp->xy(z0, z1);
+      });
     }
-  };
-  EdtBufs et{};
-  if (tw) on_twin([&] {
-    et = edt_buffers(tw, dm);
-    check(tw, cudaMemsetAsync(et.ctr, 0, sizeof(Counters), tw->stream), "memset");
+    read_roi_counts(ctx, bp.out, s);
   });
-  const int K = dm.d < kPipeSlabs ? dm.d : kPipeSlabs;
-  const size_t plane = (size_t)dm.w * dm.h;
-  for (int k = 0; k < K; ++k) {
-    const int z0 = (int)((long long)dm.d * k / K), z1 = (int)((long long)dm.d * (k + 1) / K);
-    const size_t off = (size_t)z0 * plane, len = (size_t)(z1 - z0) * plane;
-    check(ctx, cudaMemcpyAsync(d_bone + off, bone + off, len, cudaMemcpyHostToDevice, ctx->upload_stream),
-          "input upload");
-    check(ctx, cudaMemcpyAsync(d_roi + off, roi + off, len, cudaMemcpyHostToDevice, ctx->upload_stream),
-          "input upload");
-    check(ctx, cudaEventRecord(ctx->slab_ready[k], ctx->upload_stream), "event record");
-    check(ctx, cudaStreamWaitEvent(s, ctx->slab_ready[k], 0), "stream wait");
-    timed(ctx, KF_COUNT_ROI, s, "count kernel", [&] {
-      count_roi_kernel<<<152 * 8, 256, 0, s>>>(d_bone + off, d_roi + off, (long long)len, dcnt);
-      ++ctx->launches;
-      return cudaGetLastError();
-    });
-    edt_xy(ctx, dm, d_bone, d_roi, SEL_BONE_IN_ROI, eb, z0, z1, s);
-    if (tw) on_twin([&] {
-      check(tw, cudaStreamWaitEvent(tw->stream, ctx->slab_ready[k], 0), "stream wait");
-      edt_xy(tw, dm, d_bone, d_roi, SEL_MARROW_IN_ROI, et, z0, z1, tw->stream);
-    });
-  }
-  unsigned long long hc[2];
-  check(ctx, cudaMemcpyAsync(hc, dcnt, 16, cudaMemcpyDeviceToHost, s), "count readback");
-  check(ctx, cudaStreamSynchronize(s), "count kernel");
-  Prestaged pre;
-  pre.roi = hc[0];
-  pre.bone_in_roi = hc[1];
-  pre.bone_xy = true;
-  pre.marrow_xy = tw != nullptr;
-  return tbth_device_impl(ctx, d_bone, d_roi, dm, spacing, flags, th, sp, d_th, d_sp, s, &pre);
 }
 
 }  // namespace
@@ -1065,10 +1178,10 @@ void set_thread_error(const char* msg) { g_create_error = msg; }
 // cached tables stay).
 std::vector<Buffer*> work_buffers(bm_ctx* ctx) {
   return {&ctx->in_a,      &ctx->in_b,       &ctx->dist,        &ctx->dist2,   &ctx->stack,  &ctx->edtmap,
-          &ctx->chainmap,  &ctx->fillmap,    &ctx->selbits,     &ctx->ridgebits, &ctx->ridges, &ctx->accum,
-          &ctx->cpart,     &ctx->outmap,     &ctx->outmap2,     &ctx->occ,     &ctx->rank,   &ctx->rvals,
-          &ctx->bincounts, &ctx->binoffsets, &ctx->binentries,  &ctx->scanscratch, &ctx->redo, &ctx->qhist,
-          &ctx->qtargets,  &ctx->qmap,       &ctx->rgeo,        &ctx->ordmap,  &ctx->ordscratch, &ctx->ordout,
+          &ctx->chainmap,  &ctx->fillmap,    &ctx->selbits,     &ctx->ridgebits, &ctx->ridges, &ctx->phaseout,
+          &ctx->outmap,    &ctx->outmap2,     &ctx->occ,     &ctx->rank,   &ctx->rvals,
+          &ctx->bincounts, &ctx->binoffsets, &ctx->binentries,  &ctx->scanscratch, &ctx->qhist,
+          &ctx->qtargets,  &ctx->qmap,       &ctx->rgeo,        &ctx->ordmap,  &ctx->ordscratch,
           &ctx->tileorder, &ctx->ridgemap,   &ctx->dischdr,     &ctx->discent, &ctx->discpool,
           &ctx->nzbits,    &ctx->inbits};
 }
@@ -1103,8 +1216,12 @@ int bm_ctx_create(int device, bm_ctx** out) {
   e = cudaSetDevice(device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->counted, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaMallocHost(&ctx->pinned, sizeof(Readback));
   if (e != cudaSuccess) {
     cudaGetLastError();
+    if (ctx->counted) cudaEventDestroy(ctx->counted);
+    if (ctx->stream) cudaStreamDestroy(ctx->stream);
     set_err(nullptr, "context creation failed: %s", cudaGetErrorString(e));
     delete ctx;
     return BM_ERR_CUDA;
@@ -1136,13 +1253,15 @@ void bm_ctx_destroy(bm_ctx* ctx) {
     if (ctx->twin) bm_ctx_destroy(ctx->twin);
     ctx->twin = nullptr;
     if (ctx->inputs_ready) cudaEventDestroy(ctx->inputs_ready);
+    if (ctx->counted) cudaEventDestroy(ctx->counted);
+    if (ctx->pinned) cudaFreeHost(ctx->pinned);
     if (ctx->upload_stream) {
       cudaStreamSynchronize(ctx->upload_stream);
       cudaStreamDestroy(ctx->upload_stream);
     }
     for (cudaEvent_t e : ctx->slab_ready) cudaEventDestroy(e);
     for (Buffer* b : work_buffers(ctx)) release(*b);
-    for (Buffer* b : {&ctx->lut, &ctx->counters, &ctx->roicount, &ctx->host_pinned, &ctx->fillinfo}) release(*b);
+    for (Buffer* b : {&ctx->lut, &ctx->fillinfo}) release(*b);
     for (const ProfRec& r : ctx->prof) {
       cudaEventDestroy(r.start);
       cudaEventDestroy(r.stop);
@@ -1333,20 +1452,7 @@ int bm_nonzero_stats_device(bm_ctx* ctx, const float* d_values, size_t n, double
     if (!d_values || !out) fail(ctx, BM_ERR_INVALID, "null pointer");
     if (flags & ~(unsigned)BM_FLAG_QUANTILES) fail(ctx, BM_ERR_INVALID, "unknown flags 0x%x", flags);
     cudaStream_t s = pick_stream(ctx, stream);
-    StatsAccum* acc = static_cast<StatsAccum*>(ensure(ctx, ctx->accum, sizeof(StatsAccum), "stats"));
-    check(ctx, cudaMemsetAsync(acc, 0, sizeof(StatsAccum), s), "memset");
-    timed(ctx, KF_QUANTILE, s, "moments kernel",
-          [&] { return launch_moments(d_values, (long long)n, (float)scale, acc, s, &ctx->launches); });
-    ordered_sums(ctx, d_values, (long long)n, (float)scale, acc, s);
-    StatsAccum ha;
-    double osum[2];
-    check(ctx, cudaMemcpyAsync(&ha, acc, sizeof ha, cudaMemcpyDeviceToHost, s), "stats readback");
-    check(ctx, cudaMemcpyAsync(osum, ctx->ordout.ptr, sizeof osum, cudaMemcpyDeviceToHost, s), "stats readback");
-    check(ctx, cudaStreamSynchronize(s), "moments kernel");
-    int st = finish_stats(ctx, ha, osum, out);
-    if (st) return st;
-    if (flags & BM_FLAG_QUANTILES) quantiles(ctx, d_values, (long long)n, ha.count, scale, out, s);
-    return BM_OK;
+    return nonzero_stats_impl(ctx, d_values, n, scale, flags, out, s);
   });
 }
 
@@ -1357,20 +1463,7 @@ int bm_nonzero_stats(bm_ctx* ctx, const float* values, size_t n, double scale, u
     cudaStream_t s = ctx->stream;
     float* d = static_cast<float*>(ensure(ctx, ctx->qmap, (n ? n : 1) * 4, "values"));
     if (n) check(ctx, cudaMemcpyAsync(d, values, n * 4, cudaMemcpyHostToDevice, s), "values upload");
-    StatsAccum* acc = static_cast<StatsAccum*>(ensure(ctx, ctx->accum, sizeof(StatsAccum), "stats"));
-    check(ctx, cudaMemsetAsync(acc, 0, sizeof(StatsAccum), s), "memset");
-    timed(ctx, KF_QUANTILE, s, "moments kernel",
-          [&] { return launch_moments(d, (long long)n, (float)scale, acc, s, &ctx->launches); });
-    ordered_sums(ctx, d, (long long)n, (float)scale, acc, s);
-    StatsAccum ha;
-    double osum[2];
-    check(ctx, cudaMemcpyAsync(&ha, acc, sizeof ha, cudaMemcpyDeviceToHost, s), "stats readback");
-    check(ctx, cudaMemcpyAsync(osum, ctx->ordout.ptr, sizeof osum, cudaMemcpyDeviceToHost, s), "stats readback");
-    check(ctx, cudaStreamSynchronize(s), "moments kernel");
-    int st = finish_stats(ctx, ha, osum, out);
-    if (st) return st;
-    if (flags & BM_FLAG_QUANTILES) quantiles(ctx, d, (long long)n, ha.count, scale, out, s);
-    return BM_OK;
+    return nonzero_stats_impl(ctx, d, n, scale, flags, out, s);
   });
 }
 

@@ -96,9 +96,9 @@ struct StatsAccum {
   unsigned long long count;
   unsigned int max_bits;
   unsigned int pad;
-  // Fixed-point totals (filled on the host from FixedPartial records):
-  // sum of m * 2^(e - e_lo) and of m^2 * 2^(2 (e - e_lo)) over the values
-  // whose exponent e lies in [e_lo, e_lo + kFixedSpan]; fx_elo = 0: none.
+  // Fixed-point totals: sum of m * 2^(e - e_lo) and of m^2 * 2^(2 (e - e_lo))
+  // over the values whose exponent e lies in [e_lo, e_lo + kFixedSpan];
+  // fx_elo (set on the host) = 0: none.
   unsigned long long fx_s1[2];
   unsigned long long fx_s2[3];
   int fx_elo;
@@ -108,14 +108,6 @@ struct StatsAccum {
 // Exponent span of the fixed-point statistics path (values of one map lie
 // within 2^16 of their smallest possible value).
 constexpr int kFixedSpan = 20;
-
-// One CTA's fixed-point statistics: s1 (sum of shifted mantissas) and the
-// 128-bit sum of their squares.
-struct FixedPartial {
-  unsigned long long s1;
-  unsigned long long s2lo, s2hi;
-  unsigned long long pad;
-};
 
 // Tile of the tile-owned sphere fill: 32 x (16, 32 or 64) x 16 voxels (x, y, z).
 constexpr int kFillTX = 32;
@@ -160,7 +152,16 @@ struct Counters {  // device-side counters of one phase
   unsigned int pad0;
   unsigned long long disc_pool; // entries of the disc lists' overflow pool handed out
   unsigned int disc_overflow;   // nonzero: the pool was too small
-  unsigned int pad;
+  unsigned int z_redo;          // nonzero: the windowed z pass flagged lines
+};
+
+// What a phase leaves for the host (one copy to page-locked memory), zeroed in
+// one piece with the line flags that follow it.
+struct PhaseOut {
+  unsigned long long roi[2];  // ROI voxels and ROI-clipped bone voxels (the bails of bm_tbth_tbsp)
+  Counters ctr;
+  StatsAccum acc;
+  double osum[2];             // the reference's sequential sum and sum of squares
 };
 
 // Kernel families timed by the context's profiler (bm_profile_*).
@@ -194,6 +195,8 @@ void pool_destroy(Pool* p);
 struct bm_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
+  void* pinned = nullptr;      // page-locked readback area (bm::Readback)
+  cudaEvent_t counted = nullptr;  // the ROI counts have been copied
   // second context (own stream and buffers) that runs the marrow phase of
   // bm_tbth_tbsp while this one runs the bone phase; created on first use
   bm_ctx* twin = nullptr;
@@ -220,13 +223,9 @@ struct bm_ctx {
   bm::Buffer selbits, ridgebits; // row-padded bitmasks: selected voxels, ridge voxels
   bm::Buffer nzbits, inbits;   // the r^2 map's nonzero voxels, and those without a zero 26-neighbour
   bm::Buffer ridges;           // ridge records
-  bm::Buffer counters;         // bm::Counters
-  bm::Buffer roicount;         // ROI and bone-in-ROI voxel counts (the bails of bm_tbth_tbsp)
-  bm::Buffer accum;            // bm::StatsAccum
-  bm::Buffer cpart;            // bm::FixedPartial per cleanup CTA
+  bm::Buffer phaseout;         // bm::PhaseOut, then the line flags of the windowed y and z passes
   bm::Buffer outmap;           // f32 output staging
   bm::Buffer outmap2;
-  bm::Buffer host_pinned;      // pinned staging for small readbacks
   bm::Buffer occ, rank, rvals; // per-r^2 flags, ranks, rank -> r^2
   bm::Buffer rgeo;             // rank -> {r^2, ceil sqrt, floor sqrt, 0}
   bm::Buffer fillinfo;         // bm::FillInfo
@@ -235,9 +234,8 @@ struct bm_ctx {
   bm::Buffer surf_off, surf_pts;
   // separable fill: u16 ridge map, list headers and disc lists; cached tables by squared radius
   bm::Buffer ridgemap, dischdr, discent, discpool, discthr, disctmpl;
-  bm::Buffer redo;             // per-line flags of the windowed EDT passes
   bm::Buffer qhist, qtargets, qmap;  // quantile histograms, targets, map scratch
-  bm::Buffer ordmap, ordscratch, ordout;  // f32 map for the ordered sums, their scratch, their two results
+  bm::Buffer ordmap, ordscratch;  // f32 map for the ordered sums, and their scratch
   bm::Buffer tileorder;        // the fill's tile order (heaviest first) and its bucket counts
   uint32_t surf_max = 0;
 

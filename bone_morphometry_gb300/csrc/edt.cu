@@ -459,7 +459,10 @@ edt_window_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, i
     if (m > 3) op[3 * stride] = b3;
     localmax = max(localmax, mx);
   }
-  if (bad) redo[orow * (long long)w + x] = 1u;
+  if (bad) {
+    redo[orow * (long long)w + x] = 1u;
+    if (track_max) ctr->z_redo = 1u;
+  }
   if (track_max) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) localmax = max(localmax, __shfl_xor_sync(0xffffffffu, localmax, o));
@@ -596,7 +599,10 @@ edt_window_tma_kernel(const __grid_constant__ CUtensorMap tin, uint32_t* __restr
     if (m > 3) op[3 * stride] = b3;
     localmax = max(localmax, mx);
   }
-  if (bad) redo[(long long)orow * w + x] = 1u;
+  if (bad) {
+    redo[(long long)orow * w + x] = 1u;
+    if (track_max) ctr->z_redo = 1u;
+  }
   if (track_max) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) localmax = max(localmax, __shfl_xor_sync(0xffffffffu, localmax, o));
@@ -716,50 +722,51 @@ bool window_map(CUtensorMap* map, const uint32_t* vol, Dims dm, int axis, unsign
 
 }  // namespace
 
-cudaError_t launch_edt_window(int axis, const uint32_t* in, uint32_t* out, Dims dm, void* scratch, uint8_t* redo,
-                              Counters* ctr, long long wait_cycles, cudaStream_t s, unsigned long long* launches) {
-  int n;
-  long long stride, outer, nlines, orows;
-  if (axis == 1) {
-    n = dm.h;
-    stride = dm.w;
-    outer = (long long)dm.w * dm.h;
-    nlines = (long long)dm.w * dm.d;
-    orows = dm.d;
-  } else {
-    n = dm.d;
-    stride = (long long)dm.w * dm.h;
-    outer = dm.w;
-    nlines = (long long)dm.w * dm.h;
-    orows = dm.h;
-  }
-  cudaError_t e = cudaMemsetAsync(redo, 0, (size_t)nlines, s);
-  if (e != cudaSuccess) return e;
+namespace {
+
+struct Lines {  // the lines along an axis
+  int n;                          // length
+  long long stride, outer, rows;  // step along a line, step between rows of lines, rows
+  long long count;                // lines
+};
+
+Lines lines_of(int axis, Dims dm) {
+  const long long w = dm.w, wh = w * dm.h;
+  return axis == 1 ? Lines{dm.h, w, wh, dm.d, w * dm.d} : Lines{dm.d, wh, w, dm.h, wh};
+}
+
+}  // namespace
+
+cudaError_t launch_edt_window(int axis, const uint32_t* in, uint32_t* out, Dims dm, uint8_t* redo, Counters* ctr,
+                              long long wait_cycles, cudaStream_t s, unsigned long long* launches) {
+  const Lines l = lines_of(axis, dm);
   const int nxt = (dm.w + 31) / 32;
-  const int nchunk = (n + kWinTL - 1) / kWinTL;
-  const long long blocks = (long long)nxt * nchunk * orows;
+  const int nchunk = (l.n + kWinTL - 1) / kWinTL;
+  const long long blocks = (long long)nxt * nchunk * l.rows;
   // TMA staging for the y pass only: a z-pass box spans 256 rows a whole
   // slice apart (a different page each), which the copy engine translates one
   // by one; there the per-thread loads measured faster (2.2 against 3.0 ms on
   // 1024^3 bone).
   CUtensorMap map;
   if (axis == 1 && window_map(&map, in, dm, axis, kTmaRows)) {
-    edt_window_tma_kernel<<<(unsigned)blocks, kWinThreads, 0, s>>>(map, out, axis, n, stride, dm.w, outer, nxt,
+    edt_window_tma_kernel<<<(unsigned)blocks, kWinThreads, 0, s>>>(map, out, axis, l.n, l.stride, dm.w, l.outer, nxt,
                                                                    nchunk, redo, ctr, axis == 2 ? 1 : 0,
                                                                    wait_cycles < 0 ? kWaitCycles : wait_cycles);
   } else {
-    edt_window_kernel<<<(unsigned)blocks, kWinThreads, 0, s>>>(in, out, n, stride, dm.w, outer, nxt, nchunk, redo,
+    edt_window_kernel<<<(unsigned)blocks, kWinThreads, 0, s>>>(in, out, l.n, l.stride, dm.w, l.outer, nxt, nchunk, redo,
                                                                ctr, axis == 2 ? 1 : 0);
   }
   ++*launches;
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  // exact lower envelope for the lines the window could not cover
+  return cudaGetLastError();
+}
+
+cudaError_t launch_edt_redo(int axis, const uint32_t* in, uint32_t* out, Dims dm, void* scratch, const uint8_t* redo,
+                            Counters* ctr, cudaStream_t s, unsigned long long* launches) {
+  const Lines l = lines_of(axis, dm);
   uint32_t* spos = static_cast<uint32_t*>(scratch);
-  uint32_t* sf = spos + (size_t)nlines * n;
-  edt_line_kernel<<<(unsigned)((nlines + 255) / 256), 256, 0, s>>>(in, out, n, stride, dm.w,
-                                                                  axis == 1 ? (long long)dm.w * dm.h : dm.w, nlines,
-                                                                  spos, sf, ctr, axis == 2 ? 1 : 0, redo);
+  uint32_t* sf = spos + (size_t)l.count * l.n;
+  edt_line_kernel<<<(unsigned)((l.count + 255) / 256), 256, 0, s>>>(in, out, l.n, l.stride, dm.w, l.outer, l.count, spos,
+                                                                   sf, ctr, axis == 2 ? 1 : 0, redo);
   ++*launches;
   return cudaGetLastError();
 }

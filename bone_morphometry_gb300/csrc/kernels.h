@@ -1,19 +1,30 @@
 // Host-side launchers of the device kernels (one declaration per kernel family).
 #pragma once
 
+#include <atomic>
+
 #include "bm_internal.h"
 
 namespace bm {
 
 // Grid of a persistent (tile-looping) kernel: as many CTAs as the current
-// device keeps resident at once, at most one per tile.
-template <typename Kernel>
-inline unsigned resident_grid(Kernel kernel, int threads, size_t smem, long long tiles) {
-  int dev = 0, sms = 0, per = 0;
+// device keeps resident at once, at most one per tile.  A kernel is always
+// launched with the same block size and no dynamic shared memory, so the number
+// is looked up once per device (its constant, kept for the process).
+template <auto kKernel>
+inline unsigned resident_grid(int threads, long long tiles) {
+  constexpr int kDevices = 64;
+  static std::atomic<long long> known[kDevices];
+  int dev = 0;
   cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem);
-  long long g = (long long)(per > 0 ? per : 1) * (sms > 0 ? sms : 1);
+  long long g = dev < kDevices ? known[dev].load(std::memory_order_relaxed) : 0;
+  if (g == 0) {
+    int sms = 0, per = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kKernel, threads, 0);
+    g = (long long)(per > 0 ? per : 1) * (sms > 0 ? sms : 1);
+    if (dev < kDevices) known[dev].store(g, std::memory_order_relaxed);
+  }
   if (g > tiles) g = tiles;
   if (g < 1) g = 1;
   return (unsigned)g;
@@ -33,12 +44,16 @@ cudaError_t launch_edt_x(const uint8_t* a, const uint8_t* b, int mode, Dims dm, 
 cudaError_t launch_edt_line(int axis, const uint32_t* in, uint32_t* out, Dims dm, void* scratch,
                             Counters* ctr, cudaStream_t s, unsigned long long* launches);
 
-// Windowed y (axis 1) / z (axis 2) pass; lines it cannot bound are recomputed
-// by the lower-envelope kernel (redo: one byte per line, scratch as above).
-// wait_cycles: limit of the TMA copy's first bounded wait (< 0: the default,
-// about 2 s); a block that gives up sets ctr->status.
-cudaError_t launch_edt_window(int axis, const uint32_t* in, uint32_t* out, Dims dm, void* scratch, uint8_t* redo,
-                              Counters* ctr, long long wait_cycles, cudaStream_t s, unsigned long long* launches);
+// Windowed y (axis 1) / z (axis 2) pass.  Lines it cannot bound are flagged in
+// redo (one byte per line, zeroed by the caller; the z pass also sets
+// ctr->z_redo) and left to launch_edt_redo.  wait_cycles: limit of the TMA
+// copy's first bounded wait (< 0: the default, about 2 s); a block that gives up
+// sets ctr->status.
+cudaError_t launch_edt_window(int axis, const uint32_t* in, uint32_t* out, Dims dm, uint8_t* redo, Counters* ctr,
+                              long long wait_cycles, cudaStream_t s, unsigned long long* launches);
+// The exact lower envelope of the flagged lines (scratch: edt_scratch_bytes).
+cudaError_t launch_edt_redo(int axis, const uint32_t* in, uint32_t* out, Dims dm, void* scratch, const uint8_t* redo,
+                            Counters* ctr, cudaStream_t s, unsigned long long* launches);
 
 // Search-template table entries lut[r2] for r2 in [lo, hi]:
 // {scan_cube(1,0,0), scan_cube(1,1,0), scan_cube(1,1,1), f32 bits of 2*sqrt(r2)}.
@@ -81,14 +96,12 @@ cudaError_t launch_fill(const uint2* ridges, const Counters* ctr, unsigned long 
 // separable fill writes both; launch_diameters makes them of an r2 map (dmap
 // may be the map's memory).  dia: f32 diameters by r2 (launch_dia_table).
 // Values whose f32 exponent lies in [e_lo, e_lo + kFixedSpan] are summed in
-// fixed point, one FixedPartial per CTA in part[0 .. *grid); the others go to
-// acc's per-exponent sums.  At most kCleanupMaxGrid CTAs.
-constexpr unsigned kCleanupMaxGrid = 4096;
+// fixed point (acc->fx_s1, fx_s2); the others go to acc's per-exponent sums.
 cudaError_t launch_diameters(const uint32_t* fillmap, Dims dm, const float* dia, float* dmap, uint32_t* nzbits,
                              cudaStream_t s, unsigned long long* launches);
 cudaError_t launch_cleanup(const float* dmap, const uint32_t* selbits, const uint32_t* nzbits, uint32_t* inbits, Dims dm,
-                           float scale, float* outmap, StatsAccum* acc, FixedPartial* part, int e_lo, unsigned* grid,
-                           cudaStream_t s, unsigned long long* launches);
+                           float scale, float* outmap, StatsAccum* acc, int e_lo, cudaStream_t s,
+                           unsigned long long* launches);
 cudaError_t launch_dia_table(const uint4* lut, uint32_t n, float* dia, cudaStream_t s, unsigned long long* launches);
 
 // Separable fill (discs.cu), for squared radii up to kDiscMaxR2: offsets from a

@@ -226,10 +226,18 @@ struct Moments {
   }
 };
 
+// limb[at ..] += v with carries, by atomics (the total is the same in any order).
+__device__ __forceinline__ void add_limbs(unsigned long long* limb, int limbs, int at, unsigned long long v) {
+  for (; v && at < limbs; ++at) {
+    const unsigned long long old = atomicAdd(&limb[at], v);
+    v = old + v < old ? 1ull : 0ull;
+  }
+}
+
 __global__ void __launch_bounds__(kCleanThreads, 4)
 cleanup_kernel(const float* __restrict__ dmap, const uint32_t* __restrict__ selbits,
                const uint32_t* __restrict__ inbits, Dims dm, VoxelDecoder vd, float scale,
-               float* __restrict__ outmap, StatsAccum* __restrict__ acc, FixedPartial* __restrict__ part, int e_lo,
+               float* __restrict__ outmap, StatsAccum* __restrict__ acc, int e_lo,
                int nyt, long long units) {
   __shared__ StatsAccum sacc;
   __shared__ uint32_t queue[kCleanWarps][32 + 32 * kCleanRows];  // skin voxels a warp holds back until 32 are ready
@@ -345,7 +353,7 @@ cleanup_kernel(const float* __restrict__ dmap, const uint32_t* __restrict__ selb
   mom.flush(sacc, e_lo);
   if (count) atomicAdd(&sacc.count, (unsigned long long)count);
   if (mom.mx) atomicMax(&sacc.max_bits, mom.mx);
-  // this CTA's fixed-point sums: warp reduction, then one record per CTA
+  // this CTA's fixed-point sums
   unsigned long long fx1 = mom.fx1, f2lo = (unsigned long long)mom.fx2, f2hi = (unsigned long long)(mom.fx2 >> 64);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -364,14 +372,15 @@ cleanup_kernel(const float* __restrict__ dmap, const uint32_t* __restrict__ selb
   }
   __syncthreads();
   if (tid == 0) {
-    FixedPartial r{0ull, 0ull, 0ull, 0ull};
-    for (int w = 0; w < kCleanWarps; ++w) {
-      r.s1 += s_fx[w][0];
-      const unsigned long long lo = r.s2lo + s_fx[w][1];
-      r.s2hi += s_fx[w][2] + (lo < r.s2lo ? 1u : 0u);
-      r.s2lo = lo;
+    for (int w = 1; w < kCleanWarps; ++w) {
+      s_fx[0][0] += s_fx[w][0];
+      const unsigned long long lo = s_fx[0][1] + s_fx[w][1];
+      s_fx[0][2] += s_fx[w][2] + (lo < s_fx[0][1] ? 1u : 0u);
+      s_fx[0][1] = lo;
     }
-    part[blockIdx.x] = r;
+    add_limbs(acc->fx_s1, 2, 0, s_fx[0][0]);
+    add_limbs(acc->fx_s2, 3, 0, s_fx[0][1]);
+    add_limbs(acc->fx_s2, 3, 1, s_fx[0][2]);
   }
   for (int i = tid; i < 256; i += kCleanThreads) {
     if (sacc.sum_m[i]) atomicAdd(&acc->sum_m[i], sacc.sum_m[i]);
@@ -543,8 +552,8 @@ cudaError_t launch_ridges(const uint32_t* dist, const uint32_t* selbits, Dims dm
                           unsigned long long* launches) {
   const int ntx = (dm.w + kRTX - 1) / kRTX, nty = (dm.h + kRTY - 1) / kRTY, ntz = (dm.d + kRTZ - 1) / kRTZ;
   const long long tiles = (long long)ntx * nty * ntz;
-  ridge_tile_kernel<<<resident_grid(ridge_tile_kernel, 256, 0, tiles), 256, 0, s>>>(dist, selbits, dm, lut, ridges,
-                                                                                    ctr, occ, ridgebits, ntx, nty, ntz);
+  ridge_tile_kernel<<<resident_grid<ridge_tile_kernel>(256, tiles), 256, 0, s>>>(dist, selbits, dm, lut, ridges, ctr,
+                                                                                 occ, ridgebits, ntx, nty, ntz);
   ++*launches;
   return cudaGetLastError();
 }
@@ -565,18 +574,16 @@ cudaError_t launch_diameters(const uint32_t* fillmap, Dims dm, const float* dia,
 }
 
 cudaError_t launch_cleanup(const float* dmap, const uint32_t* selbits, const uint32_t* nzbits, uint32_t* inbits, Dims dm,
-                           float scale, float* outmap, StatsAccum* acc, FixedPartial* part, int e_lo, unsigned* grid,
-                           cudaStream_t s, unsigned long long* launches) {
+                           float scale, float* outmap, StatsAccum* acc, int e_lo, cudaStream_t s,
+                           unsigned long long* launches) {
   const long long cols = (long long)dm.nw() * dm.h;
   interior_kernel<<<dim3((unsigned)((cols + 255) / 256), (unsigned)((dm.d + kErodeZ - 1) / kErodeZ)), 256, 0, s>>>(
       nzbits, dm, inbits);
   const int nyt = (dm.h + kCleanRows - 1) / kCleanRows;
   const long long units = (long long)dm.nw() * nyt * dm.d;
-  unsigned g = resident_grid(cleanup_kernel, kCleanThreads, 0, (units + kCleanWarps - 1) / kCleanWarps);
-  if (g > kCleanupMaxGrid) g = kCleanupMaxGrid;
-  *grid = g;
-  cleanup_kernel<<<g, kCleanThreads, 0, s>>>(dmap, selbits, inbits, dm, VoxelDecoder::of(dm), scale, outmap, acc, part,
-                                             e_lo, nyt, units);
+  const unsigned g = resident_grid<cleanup_kernel>(kCleanThreads, (units + kCleanWarps - 1) / kCleanWarps);
+  cleanup_kernel<<<g, kCleanThreads, 0, s>>>(dmap, selbits, inbits, dm, VoxelDecoder::of(dm), scale, outmap, acc, e_lo,
+                                             nyt, units);
   *launches += 2;
   return cudaGetLastError();
 }
