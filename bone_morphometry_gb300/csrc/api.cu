@@ -1,6 +1,7 @@
 // C ABI of libbm_gb300 (include/bm.h): context, buffer cache, the per-phase
 // pipeline and the drop-in entry points for edt.rs / local_thickness.rs /
 // metrics.rs.
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -372,17 +373,26 @@ struct Phase {
   PhaseOut* out = nullptr;
   uint8_t* yflags = nullptr;    // per-line flags of the windowed passes
   uint8_t* zflags = nullptr;
+  bool near = false;            // the 16-bit passes first
   bool separable = false;
   int e_lo = 0;
 
   size_t voxels() const { return (size_t)dm.n(); }
   size_t bits_bytes() const { return (size_t)dm.nw() * dm.h * dm.d * sizeof(uint32_t); }
 
+  // A forced site method or tile height asks for the tile fill.
+  bool tiles_asked() const { return ctx->site_method != BM_SITES_AUTO || ctx->fill_rows != 0; }
+
   // Buffers, and everything the phase accumulates into zeroed.
   void prepare() {
     const size_t N = voxels();
-    A = static_cast<uint32_t*>(ensure(ctx, ctx->dist, N * 4, "distance map"));
-    B = static_cast<uint32_t*>(ensure(ctx, ctx->dist2, N * 4, "distance map"));
+    // the 16-bit passes, but where the caller has asked for the tile fill (its
+    // chain passes read the 32-bit maps)
+    near = edt_only || !tiles_asked();
+    const size_t narrow = near ? (size_t)edt_near_pitch(dm.w) * dm.h * dm.d * 2 : 0;
+    const size_t map = std::max(N * 4, narrow);
+    A = static_cast<uint32_t*>(ensure(ctx, ctx->dist, map, "distance map"));
+    B = static_cast<uint32_t*>(ensure(ctx, ctx->dist2, map, "distance map"));
     scratch = ensure(ctx, ctx->stack, edt_scratch_bytes(dm), "envelope scratch");
     selbits = static_cast<uint32_t*>(ensure(ctx, ctx->selbits, bits_bytes(), "selection bits"));
     const size_t ny = (size_t)dm.w * dm.d, nz = (size_t)dm.w * dm.h;
@@ -405,12 +415,28 @@ struct Phase {
     const uint8_t* a = d_a + off;
     const uint8_t* b = d_b ? d_b + off : nullptr;
     uint32_t* sel = selbits + (long long)z0 * dm.h * dm.nw();
-    uint8_t* flags = yflags + (long long)z0 * dm.w;
+    if (near) {
+      const long long off16 = (long long)z0 * edt_near_pitch(dm.w) * dm.h;
+      uint16_t* xmap = reinterpret_cast<uint16_t*>(A) + off16;
+      uint16_t* ymap = reinterpret_cast<uint16_t*>(B) + off16;
+      for (const bool x_pass : {true, false})
+        timed(ctx, x_pass ? KF_EDT_X : KF_EDT_Y, s, x_pass ? "edt x pass" : "edt y pass", [&] {
+          return launch_edt_near_xy(a, b, mode, sd, xmap, ymap, sel, &out->ctr, ctx->wait_cycles, x_pass, s,
+                                    &ctx->launches);
+        });
+      return;
+    }
+    wide_xy(sd, a, b, sel, off, yflags + (long long)z0 * dm.w, nullptr);
+  }
+
+  // The 32-bit x and y passes; only: the z lines whose tiles the y pass is for (null: all).
+  void wide_xy(Dims sd, const uint8_t* a, const uint8_t* b, uint32_t* sel, long long off, uint8_t* flags,
+               const uint8_t* only) {
     timed(ctx, KF_EDT_X, s, "edt x pass",
           [&] { return launch_edt_x(a, b, mode, sd, A + off, sel, &out->ctr, s, &ctx->launches); });
     timed(ctx, KF_EDT_Y, s, "edt y pass", [&] {
       const cudaError_t e =
-          launch_edt_window(1, A + off, B + off, sd, flags, &out->ctr, ctx->wait_cycles, s, &ctx->launches);
+          launch_edt_window(1, A + off, B + off, sd, flags, &out->ctr, ctx->wait_cycles, only, s, &ctx->launches);
       if (e != cudaSuccess) return e;
       return launch_edt_redo(1, A + off, B + off, sd, scratch, flags, &out->ctr, s, &ctx->launches);
     });
@@ -418,7 +444,9 @@ struct Phase {
 
   void z() {
     timed(ctx, KF_EDT_Z, s, "edt z pass", [&] {
-      return launch_edt_window(2, B, E, dm, zflags, &out->ctr, ctx->wait_cycles, s, &ctx->launches);
+      if (near)
+        return launch_edt_near_z(reinterpret_cast<const uint16_t*>(B), E, dm, zflags, &out->ctr, s, &ctx->launches);
+      return launch_edt_window(2, B, E, dm, zflags, &out->ctr, ctx->wait_cycles, nullptr, s, &ctx->launches);
     });
     read_counters();
   }
@@ -431,12 +459,16 @@ struct Phase {
   void wait_edt() {
     check(ctx, cudaStreamSynchronize(s), "edt");
     hc = readback(ctx).ctr;
-    if (hc.z_redo) {
+    if (hc.z_redo && !hc.status) {
+      // the flagged lines, from 32-bit x and y passes
+      const unsigned long long sites = hc.sites;
+      if (near) wide_xy(dm, d_a, d_b, selbits, 0, yflags, zflags);
       timed(ctx, KF_EDT_Z, s, "edt z lines",
             [&] { return launch_edt_redo(2, B, E, dm, scratch, zflags, &out->ctr, s, &ctx->launches); });
       read_counters();
       check(ctx, cudaStreamSynchronize(s), "edt");
       hc = readback(ctx).ctr;
+      hc.sites = sites;  // counted twice by two x passes
     }
     if (hc.status) fail(ctx, BM_ERR_TIMEOUT, "a bounded device-side wait of the distance transform ran out");
     if (hc.sites == 0) {
@@ -445,10 +477,8 @@ struct Phase {
            "distance transform is undefined for an all-%s volume unless an exterior convention is specified",
            phase_name(phase));
     }
-    // The separable fill (discs.cu) up to radius 127, where its packed
-    // discs end; a forced site method or tile height asks for the
-    // tile fill.
-    separable = hc.rmax <= kDiscMaxR2 && ctx->site_method == BM_SITES_AUTO && ctx->fill_rows == 0;
+    // The separable fill (discs.cu) up to radius 127, where its packed discs end.
+    separable = hc.rmax <= kDiscMaxR2 && !tiles_asked();
   }
 
   // Local thickness, after wait_edt: queued to its end, but for the tile

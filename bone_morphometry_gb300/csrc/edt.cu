@@ -32,6 +32,7 @@ __device__ __forceinline__ bool selected_at(const uint8_t* __restrict__ a, const
 }
 
 constexpr int kXWarps = 8;
+constexpr int kXMaxSmem = kXWarps * 3 * 1024 * 4;  // rows of 32768 voxels
 constexpr int kNoLeft = -(1 << 20);  // sentinels: no site on that side (w <= 32768)
 constexpr int kNoRight = 1 << 21;
 
@@ -256,8 +257,15 @@ edt_line_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, int
     int k = -1;
     long long p1 = 0, F1 = 0;  // stack top
     long long p0 = 0, F0 = 0;  // entry below the top (valid when k >= 1)
+    constexpr int kAhead = 4;  // inputs in flight
+    uint32_t next[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) next[u] = u < n ? in[base + (long long)u * stride] : kInfSq;
     for (int q = 0; q < n; ++q) {
-      const uint32_t fq = in[base + (long long)q * stride];
+      const uint32_t fq = next[0];
+#pragma unroll
+      for (int u = 0; u + 1 < kAhead; ++u) next[u] = next[u + 1];
+      next[kAhead - 1] = q + kAhead < n ? in[base + (long long)(q + kAhead) * stride] : kInfSq;
       if (fq == kInfSq) continue;
       const long long Fq = (long long)fq + (long long)q * q;
       while (k >= 1 && (Fq - F1) * (p1 - p0) <= (F1 - F0) * ((long long)q - p1)) {
@@ -355,10 +363,19 @@ __device__ __forceinline__ void win_step(uint32_t L, uint32_t R, uint32_t e, uin
   b3 = __viaddmin_u32(L, s3, __viaddmin_u32(R, s0, b3));
 }
 
+// Whether a flag of rows q0 .. q0 + kWinTL - 1 (of n, w flags each) is set in
+// the block's 32 columns, x being the thread's own (block-wide vote).
+__device__ __forceinline__ bool any_flag(const uint8_t* __restrict__ only, int q0, int n, int x, int w) {
+  bool any = false;
+  for (int q = q0 + (int)(threadIdx.x >> 5); q < min(q0 + kWinTL, n); q += kWinWarps)
+    any = any || (x < w && only[(long long)q * w + x]);
+  return __syncthreads_or(any);
+}
+
 __global__ void __launch_bounds__(kWinThreads)
 edt_window_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, int n, long long stride, int w,
                   long long outer_stride, int nxt, int nchunk, uint8_t* __restrict__ redo, Counters* __restrict__ ctr,
-                  int track_max) {
+                  int track_max, const uint8_t* __restrict__ only) {
   __shared__ uint32_t buf[(kWinTL + 2 * kWinHalo) * 32];
   __shared__ uint32_t s_need;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -370,6 +387,7 @@ edt_window_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, i
   const bool xin = x < w;
   const long long base = orow * outer_stride + x;
   const int q0 = chunk * kWinTL;
+  if (only && !any_flag(only, q0, n, x, w)) return;
   if (threadIdx.x == 0) s_need = 0u;
   __syncthreads();
   // centre rows (loads of the warp's 16 rows issued before their use)
@@ -506,7 +524,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long lo
 __global__ void __launch_bounds__(kWinThreads)
 edt_window_tma_kernel(const __grid_constant__ CUtensorMap tin, uint32_t* __restrict__ out, int axis, int n,
                       long long stride, int w, long long outer_stride, int nxt, int nchunk,
-                      uint8_t* __restrict__ redo, Counters* __restrict__ ctr, int track_max, long long wait_limit) {
+                      uint8_t* __restrict__ redo, Counters* __restrict__ ctr, int track_max, long long wait_limit,
+                      const uint8_t* __restrict__ only) {
   __shared__ alignas(128) uint32_t buf[kTmaRows * 32];
   __shared__ alignas(8) unsigned long long bar;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -517,6 +536,7 @@ edt_window_tma_kernel(const __grid_constant__ CUtensorMap tin, uint32_t* __restr
   const int x = xt * 32 + lane;
   const bool xin = x < w;
   const int q0 = chunk * kWinTL;
+  if (only && !any_flag(only, q0, n, x, w)) return;
   const uint32_t b = smem_u32(&bar);
   if (threadIdx.x == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b) : "memory");
@@ -610,6 +630,357 @@ edt_window_tma_kernel(const __grid_constant__ CUtensorMap tin, uint32_t* __restr
   }
 }
 
+// ---- 16-bit passes ----------------------------------------------------------
+// The transform while every squared distance is at most kNearMax = 65^2: the
+// x and y results in 16 bits at a padded row pitch, two adjacent voxels of x
+// per register, so that the maps between the passes are half as large and a
+// scan step serves eight outputs instead of four.  A value up to kNearMax is
+// exact in every pass, and a larger one only says that the true value is at
+// least kNearMax: the row distance is cut at kReach, rows outside the volume
+// read kFar16, and the y pass stores what it has once it has tried its 64 rows
+// on either side (a candidate beyond them adds at least 65^2).  A minimum of at
+// most kNearMax can only have come from exact candidates, so the z pass' outputs
+// up to kNearMax are exact too; it flags the lines that hold others, and the
+// 32-bit passes compute those (launch_edt_far).
+//
+// 512^3, 15 % foreground: 754 us with 32-bit passes, 476 here (x 121, y 129,
+// z 184; the maps' bytes alone take 260 at the copy rate, the rest is issue).
+// 417 x 333 x 379 (rows that no vector load fits): 726 us, 387 here (129, 102,
+// 119).  Where 36 to 94 % of the volume lies beyond 65 voxels of a site, so
+// that the 32-bit passes run as well, 1.23-2.70 ms before and 1.18-2.68 here.
+constexpr uint32_t kNearMax = (kWinHalo + 1) * (kWinHalo + 1);
+constexpr uint32_t kFar16 = 40000;
+constexpr int kReach = 190;
+constexpr uint32_t kPair = 0x10001u;
+static_assert((kReach + 7) * (kReach + 7) <= (int)kFar16 && kReach * kReach > (int)kNearMax, "far rows stay far");
+static_assert(kFar16 + (kWinHalo + 6) * (kWinHalo + 6) < 65536, "the window scan adds distance^2 to kFar16");
+
+// The x pass: a warp per row, eight voxels per lane.  A voxel's distance is the
+// least of three: to a site among its lane's eight voxels (a table by their
+// bits), to the nearest site left of them and right of them.
+template <int MODE, bool VEC>
+__global__ void __launch_bounds__(kXWarps * 32, 6)
+edt_x_near_kernel(const uint8_t* __restrict__ a, const uint8_t* __restrict__ b, Dims dm, int pitch,
+                  uint16_t* __restrict__ out, uint32_t* __restrict__ selbits, Counters* __restrict__ ctr) {
+  extern __shared__ uint32_t smem[];
+  __shared__ uint4 s_inside[256];
+  static_assert(kXWarps * 32 == 256, "a table entry per thread");
+  const int lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5;
+  const int nw = dm.nw();
+  uint32_t* mask = smem + (size_t)warp * 3 * nw;
+  int* lastpos = reinterpret_cast<int*>(mask + nw);
+  int* firstpos = lastpos + nw;
+  const long long rows = (long long)dm.h * dm.d;
+  const bool two = MODE == SEL_BONE_IN_ROI || MODE == SEL_MARROW_IN_ROI;
+  unsigned long long sites = 0;
+  {
+    const uint32_t t = threadIdx.x;
+    uint32_t v[4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t lo = t & ((2u << i) - 1u), hi = t >> i;  // bits at or below, at or above
+      const int l = lo ? i - (31 - __clz(lo)) : 255, r = hi ? __ffs(hi) - 1 : 255;
+      const uint32_t g = (uint32_t)min(l, r);
+      if (i & 1) v[i >> 1] |= g << 16;
+      else v[i >> 1] = g;
+    }
+    s_inside[t] = make_uint4(v[0], v[1], v[2], v[3]);
+  }
+  __syncthreads();
+
+  for (long long row = (long long)blockIdx.x * kXWarps + warp; row < rows;
+       row += (long long)gridDim.x * kXWarps) {
+    const long long base = row * dm.w;
+    if (VEC) {
+      const uint4* av = reinterpret_cast<const uint4*>(a + base);
+      const uint4* bv = two ? reinterpret_cast<const uint4*>(b + base) : nullptr;
+      const int nvec = dm.w >> 4;  // 16 voxels per uint4
+      for (int v0 = 0; v0 < nvec; v0 += 32) {
+        const int v = v0 + lane;
+        uint32_t s16 = 0, t16 = 0;
+        if (v < nvec) {
+          const uint4 A = av[v];
+          const uint4 B = two ? bv[v] : make_uint4(0u, 0u, 0u, 0u);
+          s16 = sel4<MODE>(A.x, B.x) | (sel4<MODE>(A.y, B.y) << 4) | (sel4<MODE>(A.z, B.z) << 8) |
+                (sel4<MODE>(A.w, B.w) << 12);
+          t16 = ~s16 & 0xffffu;  // all 16 voxels lie inside the row
+        }
+        const uint32_t s_hi = __shfl_down_sync(0xffffffffu, s16, 1);
+        const uint32_t t_hi = __shfl_down_sync(0xffffffffu, t16, 1);
+        if (!(lane & 1) && v < nvec) {
+          const int c = v >> 1;  // word index: voxels 32c .. 32c + 31
+          // a row of 16k voxels with k odd ends on a half word: its upper half is empty
+          const bool full = v + 1 < nvec;
+          const uint32_t tw = t16 | (full ? t_hi << 16 : 0u);
+          mask[c] = tw;
+          selbits[row * nw + c] = s16 | (full ? s_hi << 16 : 0u);
+          sites += __popc(tw);
+        }
+      }
+    } else {
+      constexpr int kAhead = 8;  // words whose bytes are in flight
+      for (int c0 = 0; c0 < nw; c0 += kAhead) {
+        uint32_t av[kAhead], bv[kAhead];
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) {
+          const int x = (c0 + j) * 32 + lane;
+          av[j] = x < dm.w ? a[base + x] : 0u;
+          bv[j] = two && x < dm.w ? b[base + x] : 0u;
+        }
+        uint32_t sw = 0, tw = 0;
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) {
+          const bool in = (c0 + j) * 32 + lane < dm.w;
+          const bool s = in && (MODE == SEL_FOREGROUND    ? av[j] != 0
+                                : MODE == SEL_BACKGROUND  ? av[j] == 0
+                                : MODE == SEL_BONE_IN_ROI ? bv[j] != 0 && av[j] != 0
+                                                          : bv[j] != 0 && av[j] == 0);
+          const uint32_t t = __ballot_sync(0xffffffffu, in && !s), u = __ballot_sync(0xffffffffu, s);
+          if (lane == j) tw = t, sw = u;
+        }
+        if (lane < kAhead && c0 + lane < nw) {
+          mask[c0 + lane] = tw;
+          selbits[row * nw + c0 + lane] = sw;
+          sites += __popc(tw);
+        }
+      }
+    }
+    __syncwarp();
+    x_row_scans(mask, lastpos, firstpos, nw, lane);
+    const int bit = (lane & 3) * 8;  // first bit of this lane's voxels in their word
+    const uint32_t below = (1u << bit) - 1u, above = ~((2u << (bit + 7)) - 1u);  // bit + 7 = 31: above = 0
+    uint4* orow = reinterpret_cast<uint4*>(out + row * pitch);
+#pragma unroll 1
+    for (int x0 = 0; x0 < dm.w; x0 += 256) {
+      const int x = x0 + 8 * lane;
+      if (x < dm.w) {
+        const int c = x >> 5;
+        const uint32_t m = mask[c];
+        const uint32_t lo = m & below, hi = m & above;
+        const int left = lo ? c * 32 + 31 - __clz(lo) : (c > 0 ? lastpos[c - 1] : kNoLeft);
+        const int right = hi ? c * 32 + __ffs(hi) - 1 : (c + 1 < nw ? firstpos[c + 1] : kNoRight);
+        const uint32_t dl = (uint32_t)min(x - left, kReach) * kPair, dr = (uint32_t)min(right - x - 7, kReach) * kPair;
+        const uint4 in8 = s_inside[(m >> bit) & 0xffu];
+        auto square = [&](uint32_t inside, uint32_t i) {  // of voxels i and i + 1 of the eight
+          const uint32_t g = __viaddmin_u16x2(dl, i * kPair + 0x10000u,
+                                              __viaddmin_u16x2(dr, (7u - i) * kPair - 0x10000u, inside));
+          const uint32_t g0 = g & 0xffffu, g1 = g >> 16;
+          return g1 * (g & 0xffff0000u) + g0 * g0;
+        };
+        uint4 v = make_uint4(square(in8.x, 0), square(in8.y, 2), square(in8.z, 4), square(in8.w, 6));
+        if (x + 8 > dm.w) {  // the padding holds zeros
+          const int k = dm.w - x;
+          auto cut = [&](uint32_t p, int i) { return k >= i + 2 ? p : k == i + 1 ? p & 0xffffu : 0u; };
+          v = make_uint4(cut(v.x, 0), cut(v.y, 2), cut(v.z, 4), cut(v.w, 6));
+        }
+        orow[x >> 3] = v;
+        if (x + 8 < pitch && x + 8 >= dm.w) orow[(x >> 3) + 1] = make_uint4(0u, 0u, 0u, 0u);
+      }
+    }
+    __syncwarp();
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sites += __shfl_xor_sync(0xffffffffu, sites, o);
+  if (lane == 0 && sites) atomicAdd(&ctr->sites, sites);
+}
+
+// Four adjacent outputs of a lane's two columns (col: the group's first row in
+// shared memory, 32 pairs per row); m: how many lie inside the line; halo: rows
+// staged on either side, a multiple of 4.  Returns the largest of the outputs.
+__device__ __forceinline__ uint32_t near_group(const uint32_t* col, int m, int halo, uint32_t (&b)[4]) {
+  const uint32_t c0 = col[0], c1 = col[32], c2 = col[64], c3 = col[96];
+  b[0] = __viaddmin_u16x2(c1, kPair, __viaddmin_u16x2(c2, 4 * kPair, __viaddmin_u16x2(c3, 9 * kPair, c0)));
+  b[1] = __viaddmin_u16x2(c0, kPair, __viaddmin_u16x2(c2, kPair, __viaddmin_u16x2(c3, 4 * kPair, c1)));
+  b[2] = __viaddmin_u16x2(c0, 4 * kPair, __viaddmin_u16x2(c1, kPair, __viaddmin_u16x2(c3, kPair, c2)));
+  b[3] = __viaddmin_u16x2(c0, 9 * kPair, __viaddmin_u16x2(c1, 4 * kPair, __viaddmin_u16x2(c2, kPair, c3)));
+  if (m < 4) {  // outputs past the line end take no part in the stopping test
+    b[3] = 0u;
+    if (m < 3) b[2] = 0u;
+    if (m < 2) b[1] = 0u;
+  }
+  // after offsets 1 .. e-1 every candidate within distance e of every output
+  // has been tried, so the scan stops once e^2 reaches the largest minimum
+  uint32_t mx = __vmaxu2(__vimax3_u16x2(b[0], b[1], b[2]), b[3]);
+  const uint32_t *lp = col - 32, *rp = col + 4 * 32;
+#pragma unroll 1
+  for (uint32_t e = 1, t = kPair; e <= (uint32_t)halo && __vmaxu2(mx, t) != t; e += 4, lp -= 4 * 32, rp += 4 * 32) {
+    uint32_t sq[8];  // (e + k)^2
+    sq[0] = t;
+#pragma unroll
+    for (uint32_t k = 0; k < 7; ++k) sq[k + 1] = sq[k] + 2u * e * kPair + (2u * k + 1u) * kPair;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint32_t L = lp[-u * 32], R = rp[u * 32];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        b[k] = __viaddmin_u16x2(L, sq[u + k], __viaddmin_u16x2(R, sq[u + 3 - k], b[k]));
+    }
+    t = sq[4];
+    mx = __vmaxu2(__vimax3_u16x2(b[0], b[1], b[2]), b[3]);
+  }
+  return mx;
+}
+
+// The y (Z = false) or z pass over 64 columns and kWinTL outputs per block, the
+// input staged by every thread, with a halo as wide as the largest value needs.
+// in: pairs; strides in pairs.  The z pass writes the 32-bit result at the
+// volume's own pitch.
+template <bool Z>
+__global__ void __launch_bounds__(kWinThreads)
+edt_near_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, int n, long long stride, int pairs,
+                long long outer, int nxt, int nchunk, int w, long long out_stride, uint8_t* __restrict__ redo,
+                Counters* __restrict__ ctr) {
+  __shared__ uint32_t buf[(kWinTL + 2 * kWinHalo) * 32];
+  __shared__ uint32_t s_max[kWinWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long bid = blockIdx.x;
+  const int xt = (int)(bid % nxt);
+  const int chunk = (int)((bid / nxt) % nchunk);
+  const long long orow = bid / ((long long)nxt * nchunk);
+  const int px = xt * 32 + lane;
+  const bool pin = px < pairs;
+  const long long base = orow * outer + px;
+  const int q0 = chunk * kWinTL;
+  constexpr int kPer = kWinTL / kWinWarps;  // 16
+  uint32_t f[kPer];
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    const int q = q0 + warp + kWinWarps * j;
+    f[j] = q < n ? (pin ? in[base + (long long)q * stride] : 0u) : kFar16 * kPair;
+  }
+  uint32_t top = 0;
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    if (q0 + warp + kWinWarps * j < n) top = __vmaxu2(top, f[j]);
+    buf[(kWinHalo + warp + kWinWarps * j) * 32 + lane] = f[j];
+  }
+  top = __reduce_max_sync(0xffffffffu, max(top & 0xffffu, top >> 16));
+  if (lane == 0) s_max[warp] = top;
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kWinWarps; ++k) top = max(top, s_max[k]);
+  const int halo = top ? (int)min((halo_need(top) + 3u) & ~3u, (uint32_t)kWinHalo) : 0;
+  uint32_t least = kFar16 * kPair;
+  if (Z && top > kNearMax)
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) least = __vminu2(least, f[j]);
+  for (int i = warp; i < halo; i += kWinWarps) {
+    const int ql = q0 - 1 - i, qr = q0 + kWinTL + i;
+    const uint32_t l = ql >= 0 ? (pin ? in[base + (long long)ql * stride] : 0u) : kFar16 * kPair;
+    const uint32_t r = qr < n ? (pin ? in[base + (long long)qr * stride] : 0u) : kFar16 * kPair;
+    buf[(kWinHalo - 1 - i) * 32 + lane] = l;
+    buf[(kWinHalo + kWinTL + i) * 32 + lane] = r;
+    least = __vminu2(least, __vminu2(l, r));
+  }
+  const int x = 2 * px;
+  uint32_t localmax = 0;
+  uint32_t far = 0;  // the lane's columns with an output beyond kNearMax
+  // a block that stages nothing up to kNearMax holds no output up to it either
+  // (columns of the padding stage zeros)
+  const bool some = !Z || top <= kNearMax || (pin && min(least & 0xffffu, x + 1 < w ? least >> 16 : kFar16) <= kNearMax);
+  if (!__syncthreads_or(some)) {
+    if (x < w) redo[orow * w + x] = 1u;
+    if (x + 1 < w) redo[orow * w + x + 1] = 1u;
+    if (threadIdx.x == 0) ctr->z_redo = 1u;
+    return;
+  }
+#pragma unroll 1
+  for (int j = 0; j < kPer / kWinGroup; ++j) {
+    const int i = kWinGroup * (warp + kWinWarps * j);
+    const int q = q0 + i;
+    if (!pin || q >= n) continue;
+    const int m = min(kWinGroup, n - q);
+    uint32_t b[4];
+    const uint32_t mx = near_group(buf + (kWinHalo + i) * 32 + lane, m, halo, b);
+    if (Z) {
+      const uint32_t m0 = mx & 0xffffu, m1 = mx >> 16;
+      if (m0 > kNearMax) far |= 1u;
+      else localmax = max(localmax, m0);
+      if (m1 > kNearMax) far |= 2u;
+      else localmax = max(localmax, m1);
+      uint32_t* op = out + orow * w + x + (long long)q * out_stride;
+#pragma unroll
+      for (int k = 0; k < kWinGroup; ++k, op += out_stride) {
+        if (k >= m) break;
+        if (x < w) op[0] = b[k] & 0xffffu;
+        if (x + 1 < w) op[1] = b[k] >> 16;
+      }
+    } else {
+      uint32_t* op = out + base + (long long)q * stride;
+#pragma unroll
+      for (int k = 0; k < kWinGroup; ++k)
+        if (k < m) op[k * stride] = b[k];
+    }
+  }
+  if (Z) {
+    if (far) {
+      if (far & 1u) redo[orow * w + x] = 1u;
+      if (far & 2u) redo[orow * w + x + 1] = 1u;
+      ctr->z_redo = 1u;
+    }
+    localmax = __reduce_max_sync(0xffffffffu, localmax);
+    if (lane == 0 && localmax) atomicMax(&ctr->rmax, localmax);
+  }
+}
+
+// The y pass staged by one TMA copy per block, as edt_window_tma_kernel.
+__global__ void __launch_bounds__(kWinThreads)
+edt_near_tma_kernel(const __grid_constant__ CUtensorMap tin, uint32_t* __restrict__ out, int n, int pairs, int nxt,
+                    int nchunk, Counters* __restrict__ ctr, long long wait_limit) {
+  __shared__ alignas(128) uint32_t buf[kTmaRows * 32];
+  __shared__ alignas(8) unsigned long long bar;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long bid = blockIdx.x;
+  const int xt = (int)(bid % nxt);
+  const int chunk = (int)((bid / nxt) % nchunk);
+  const int plane = (int)(bid / ((long long)nxt * nchunk));
+  const int px = xt * 32 + lane;
+  const int q0 = chunk * kWinTL;
+  const uint32_t b = smem_u32(&bar);
+  if (threadIdx.x == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(kTmaRows * 32 * 4)
+                 : "memory");
+    // x start: 64 16-bit values, a multiple of 128 bytes; rows may start below 0
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+        ::"r"(smem_u32(buf)), "l"(reinterpret_cast<unsigned long long>(&tin)), "r"(xt * 64), "r"(q0 - kWinHalo),
+        "r"(plane), "r"(b)
+        : "memory");
+  }
+  const bool landed = mbar_wait(b, 0u, wait_limit);
+  if (!__syncthreads_and(landed)) {  // as in edt_window_tma_kernel
+    if (threadIdx.x == 0) atomicOr(&ctr->status, 1u);
+    mbar_wait(b, 0u, kWaitCycles);
+    return;
+  }
+  const int before = kWinHalo - q0, inside = n - q0 + kWinHalo;  // the box's rows before the line; up to its end
+  if (before > 0 || inside < kTmaRows) {
+    for (int k = threadIdx.x; k < before * 32; k += kWinThreads) buf[k] = kFar16 * kPair;
+    for (int k = inside * 32 + threadIdx.x; k < kTmaRows * 32; k += kWinThreads) buf[k] = kFar16 * kPair;
+    __syncthreads();
+  }
+  if (px >= pairs) return;
+#pragma unroll 1
+  for (int j = 0; j < kWinTL / (kWinGroup * kWinWarps); ++j) {
+    const int i = kWinGroup * (warp + kWinWarps * j);
+    const int q = q0 + i;
+    if (q >= n) continue;
+    const int m = min(kWinGroup, n - q);
+    uint32_t v[4];
+    near_group(buf + (kWinHalo + i) * 32 + lane, m, kWinHalo, v);
+    uint32_t* op = out + ((long long)plane * n + q) * pairs + px;
+#pragma unroll
+    for (int k = 0; k < kWinGroup; ++k)
+      if (k < m) op[(long long)k * pairs] = v[k];
+  }
+}
+
 }  // namespace
 
 size_t edt_scratch_bytes(Dims dm) {
@@ -628,13 +999,13 @@ cudaError_t launch_edt_x_mode(const uint8_t* a, const uint8_t* b, Dims dm, uint3
   if (vec) {
     if (smem > 48 * 1024) {
       cudaError_t e =
-          cudaFuncSetAttribute(edt_x_vec_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+          cudaFuncSetAttribute(edt_x_vec_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kXMaxSmem);
       if (e != cudaSuccess) return e;
     }
     edt_x_vec_kernel<MODE><<<blocks, kXWarps * 32, smem, s>>>(a, b, dm, out, selbits, ctr);
   } else {
     if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(edt_x_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaError_t e = cudaFuncSetAttribute(edt_x_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kXMaxSmem);
       if (e != cudaSuccess) return e;
     }
     edt_x_kernel<MODE><<<blocks, kXWarps * 32, smem, s>>>(a, b, dm, out, selbits, ctr);
@@ -720,6 +1091,20 @@ bool window_map(CUtensorMap* map, const uint32_t* vol, Dims dm, int axis, unsign
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Tensor map of a 16-bit map of pitch edt_near_pitch(w): boxes of 64 x by kTmaRows y.
+bool near_map(CUtensorMap* map, const uint16_t* vol, Dims dm) {
+  const PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
+  if (!enc || (reinterpret_cast<uintptr_t>(vol) & 15u) != 0) return false;
+  const cuuint64_t pitch = (cuuint64_t)edt_near_pitch(dm.w);
+  const cuuint64_t dims[3] = {pitch, (cuuint64_t)dm.h, (cuuint64_t)dm.d};
+  const cuuint64_t strides[2] = {pitch * 2, pitch * dm.h * 2};
+  const cuuint32_t box[3] = {64u, (cuuint32_t)kTmaRows, 1u};
+  const cuuint32_t unit[3] = {1u, 1u, 1u};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, const_cast<uint16_t*>(vol), dims, strides, box, unit,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 }  // namespace
 
 namespace {
@@ -738,7 +1123,8 @@ Lines lines_of(int axis, Dims dm) {
 }  // namespace
 
 cudaError_t launch_edt_window(int axis, const uint32_t* in, uint32_t* out, Dims dm, uint8_t* redo, Counters* ctr,
-                              long long wait_cycles, cudaStream_t s, unsigned long long* launches) {
+                              long long wait_cycles, const uint8_t* only, cudaStream_t s,
+                              unsigned long long* launches) {
   const Lines l = lines_of(axis, dm);
   const int nxt = (dm.w + 31) / 32;
   const int nchunk = (l.n + kWinTL - 1) / kWinTL;
@@ -751,10 +1137,10 @@ cudaError_t launch_edt_window(int axis, const uint32_t* in, uint32_t* out, Dims 
   if (axis == 1 && window_map(&map, in, dm, axis, kTmaRows)) {
     edt_window_tma_kernel<<<(unsigned)blocks, kWinThreads, 0, s>>>(map, out, axis, l.n, l.stride, dm.w, l.outer, nxt,
                                                                    nchunk, redo, ctr, axis == 2 ? 1 : 0,
-                                                                   wait_cycles < 0 ? kWaitCycles : wait_cycles);
+                                                                   wait_cycles < 0 ? kWaitCycles : wait_cycles, only);
   } else {
     edt_window_kernel<<<(unsigned)blocks, kWinThreads, 0, s>>>(in, out, l.n, l.stride, dm.w, l.outer, nxt, nchunk, redo,
-                                                               ctr, axis == 2 ? 1 : 0);
+                                                               ctr, axis == 2 ? 1 : 0, only);
   }
   ++*launches;
   return cudaGetLastError();
@@ -767,6 +1153,70 @@ cudaError_t launch_edt_redo(int axis, const uint32_t* in, uint32_t* out, Dims dm
   uint32_t* sf = spos + (size_t)l.count * l.n;
   edt_line_kernel<<<(unsigned)((l.count + 255) / 256), 256, 0, s>>>(in, out, l.n, l.stride, dm.w, l.outer, l.count, spos,
                                                                    sf, ctr, axis == 2 ? 1 : 0, redo);
+  ++*launches;
+  return cudaGetLastError();
+}
+
+int edt_near_pitch(int w) { return (w + 15) & ~15; }
+
+template <int MODE>
+cudaError_t launch_edt_x_near_mode(const uint8_t* a, const uint8_t* b, Dims dm, uint16_t* out, uint32_t* selbits,
+                                   Counters* ctr, unsigned blocks, cudaStream_t s) {
+  const bool two = MODE == SEL_BONE_IN_ROI || MODE == SEL_MARROW_IN_ROI;
+  const size_t smem = (size_t)kXWarps * 3 * dm.nw() * sizeof(uint32_t);
+  const bool vec = dm.w % 16 == 0 && (reinterpret_cast<uintptr_t>(a) & 15u) == 0 &&
+                   (!two || (reinterpret_cast<uintptr_t>(b) & 15u) == 0);
+  auto kernel = vec ? edt_x_near_kernel<MODE, true> : edt_x_near_kernel<MODE, false>;
+  if (smem > 44 * 1024) {  // with the table's 4 KB
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kXMaxSmem);
+    if (e != cudaSuccess) return e;
+  }
+  kernel<<<blocks, kXWarps * 32, smem, s>>>(a, b, dm, edt_near_pitch(dm.w), out, selbits, ctr);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_edt_near_xy(const uint8_t* a, const uint8_t* b, int mode, Dims dm, uint16_t* xmap, uint16_t* ymap,
+                               uint32_t* selbits, Counters* ctr, long long wait_cycles, bool x_pass, cudaStream_t s,
+                               unsigned long long* launches) {
+  ++*launches;
+  if (x_pass) {
+    // enough rows per warp that the table is not what a block spends its time on
+    long long blocks = ((long long)dm.h * dm.d + kXWarps - 1) / kXWarps;
+    if (blocks > 152 * 12) blocks = 152 * 12;
+    switch (mode) {
+      case SEL_FOREGROUND:
+        return launch_edt_x_near_mode<SEL_FOREGROUND>(a, b, dm, xmap, selbits, ctr, (unsigned)blocks, s);
+      case SEL_BACKGROUND:
+        return launch_edt_x_near_mode<SEL_BACKGROUND>(a, b, dm, xmap, selbits, ctr, (unsigned)blocks, s);
+      case SEL_BONE_IN_ROI:
+        return launch_edt_x_near_mode<SEL_BONE_IN_ROI>(a, b, dm, xmap, selbits, ctr, (unsigned)blocks, s);
+      default:
+        return launch_edt_x_near_mode<SEL_MARROW_IN_ROI>(a, b, dm, xmap, selbits, ctr, (unsigned)blocks, s);
+    }
+  }
+  const int pairs = edt_near_pitch(dm.w) / 2;
+  const int nxt = (pairs + 31) / 32, nchunk = (dm.h + kWinTL - 1) / kWinTL;
+  const unsigned blocks = (unsigned)((long long)nxt * nchunk * dm.d);
+  const uint32_t* in = reinterpret_cast<const uint32_t*>(xmap);
+  uint32_t* out = reinterpret_cast<uint32_t*>(ymap);
+  CUtensorMap map;
+  if (near_map(&map, xmap, dm)) {
+    edt_near_tma_kernel<<<blocks, kWinThreads, 0, s>>>(map, out, dm.h, pairs, nxt, nchunk, ctr,
+                                                       wait_cycles < 0 ? kWaitCycles : wait_cycles);
+  } else {
+    edt_near_kernel<false><<<blocks, kWinThreads, 0, s>>>(in, out, dm.h, pairs, pairs, (long long)pairs * dm.h, nxt,
+                                                          nchunk, dm.w, 0, nullptr, ctr);
+  }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_edt_near_z(const uint16_t* ymap, uint32_t* out, Dims dm, uint8_t* redo, Counters* ctr,
+                              cudaStream_t s, unsigned long long* launches) {
+  const int pairs = edt_near_pitch(dm.w) / 2;
+  const int nxt = (pairs + 31) / 32, nchunk = (dm.d + kWinTL - 1) / kWinTL;
+  edt_near_kernel<true><<<(unsigned)((long long)nxt * nchunk * dm.h), kWinThreads, 0, s>>>(
+      reinterpret_cast<const uint32_t*>(ymap), out, dm.d, (long long)pairs * dm.h, pairs, pairs, nxt, nchunk, dm.w,
+      (long long)dm.w * dm.h, redo, ctr);
   ++*launches;
   return cudaGetLastError();
 }

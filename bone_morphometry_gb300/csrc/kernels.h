@@ -48,12 +48,25 @@ cudaError_t launch_edt_line(int axis, const uint32_t* in, uint32_t* out, Dims dm
 // redo (one byte per line, zeroed by the caller; the z pass also sets
 // ctr->z_redo) and left to launch_edt_redo.  wait_cycles: limit of the TMA
 // copy's first bounded wait (< 0: the default, about 2 s); a block that gives up
-// sets ctr->status.
+// sets ctr->status.  only (the y pass; may be null): the flags of the z pass; the
+// blocks whose columns have none are left out.
 cudaError_t launch_edt_window(int axis, const uint32_t* in, uint32_t* out, Dims dm, uint8_t* redo, Counters* ctr,
-                              long long wait_cycles, cudaStream_t s, unsigned long long* launches);
+                              long long wait_cycles, const uint8_t* only, cudaStream_t s,
+                              unsigned long long* launches);
 // The exact lower envelope of the flagged lines (scratch: edt_scratch_bytes).
 cudaError_t launch_edt_redo(int axis, const uint32_t* in, uint32_t* out, Dims dm, void* scratch, const uint8_t* redo,
                             Counters* ctr, cudaStream_t s, unsigned long long* launches);
+
+// The 16-bit passes (squared distances up to 65^2): x (x_pass) or y of a volume
+// or slab of planes, and z.  Maps of edt_near_pitch(w) * h * d values, 16-byte
+// aligned.  The z pass flags the lines that hold larger distances in redo and
+// ctr->z_redo; the 32-bit passes compute those.
+int edt_near_pitch(int w);
+cudaError_t launch_edt_near_xy(const uint8_t* a, const uint8_t* b, int mode, Dims dm, uint16_t* xmap, uint16_t* ymap,
+                               uint32_t* selbits, Counters* ctr, long long wait_cycles, bool x_pass, cudaStream_t s,
+                               unsigned long long* launches);
+cudaError_t launch_edt_near_z(const uint16_t* ymap, uint32_t* out, Dims dm, uint8_t* redo, Counters* ctr,
+                              cudaStream_t s, unsigned long long* launches);
 
 // Search-template table entries lut[r2] for r2 in [lo, hi]:
 // {scan_cube(1,0,0), scan_cube(1,1,0), scan_cube(1,1,1), f32 bits of 2*sqrt(r2)}.

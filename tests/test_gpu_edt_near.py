@@ -1,0 +1,56 @@
+"""The 16-bit distance passes against the oracle at the edges of their eights of
+x, 64-column tiles, 128-row chunks and 64-row halos, around the largest distance
+they hold (65 voxels) and beyond it, where the 32-bit passes compute the flagged
+lines.  Squared distances are whole numbers: the comparison is exact."""
+
+import numpy as np
+import pytest
+
+import oracle as O
+from bone_morphometry_gb300 import Phase
+from bone_morphometry_gb300 import euclidean_distance_transform_squared as edt
+
+pytestmark = pytest.mark.gpu
+
+
+def sites(shape, at):
+    vol = np.ones(shape, np.uint8)
+    for p in at:
+        vol[p] = 0
+    return vol
+
+
+def noise(shape, p, seed):
+    return (np.random.default_rng(seed).random(shape) < p).astype(np.uint8)
+
+
+def near_and_far(shape, seed):  # most columns near a site, one corner far from any
+    vol = noise(shape, 0.97, seed)
+    vol[: shape[0] // 2, : shape[1] // 2, : shape[2] // 2] = 1
+    return vol
+
+
+CASES = [("noise-%d-%d-%d" % s, lambda s=s: noise(s, 0.96, sum(s)))
+         for s in [(3, 5, 2), (4, 3, 7), (127, 9, 8), (128, 129, 9), (129, 127, 17), (5, 64, 63), (6, 65, 65),
+                   (3, 4, 255), (4, 5, 256), (5, 6, 257), (260, 3, 31), (3, 260, 129), (2, 2, 1100)]]
+# one site: the largest squared distance lies just below, at and above 65^2 along each axis
+for n in (65, 66, 67, 130, 199, 257):
+    CASES += [("x-%d" % n, lambda n=n: sites((3, 4, n), [(0, 0, 0)])),
+              ("y-%d" % n, lambda n=n: sites((3, n, 5), [(2, 0, 4)])),
+              ("z-%d" % n, lambda n=n: sites((n, 3, 4), [(n - 1, 2, 0)]))]
+CASES += [
+    ("diagonal", lambda: sites((50, 60, 70), [(0, 0, 0)])),
+    ("two-far", lambda: sites((150, 140, 97), [(3, 5, 7), (149, 100, 90)])),
+    ("part-far", lambda: near_and_far((160, 150, 140), 1)),
+    ("part-far-odd", lambda: near_and_far((141, 153, 167), 2)),
+    ("row-reach", lambda: sites((2, 2, 600), [(0, 0, 0), (0, 0, 400), (1, 1, 590)])),
+]
+
+
+@pytest.mark.parametrize("name,make", CASES, ids=[c[0] for c in CASES])
+@pytest.mark.parametrize("phase", [Phase.FOREGROUND, Phase.BACKGROUND])
+def test_edt_bitwise(gpu_ctx, name, make, phase):
+    vol = make()
+    if phase == Phase.BACKGROUND:
+        vol = 1 - vol
+    assert np.array_equal(edt(vol, phase, ctx=gpu_ctx), O.edt_sq(vol, int(phase)))
