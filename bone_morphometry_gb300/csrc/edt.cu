@@ -240,6 +240,8 @@ edt_x_vec_kernel(const uint8_t* __restrict__ a, const uint8_t* __restrict__ b, D
     __syncwarp();
     x_row_distances4(mask, lastpos, firstpos, nw, dm.w, lane, out + base);
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sites += __shfl_xor_sync(0xffffffffu, sites, o);
   if (lane == 0 && sites) atomicAdd(&ctr->sites, sites);
 }
 

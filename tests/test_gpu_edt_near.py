@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 import oracle as O
-from bone_morphometry_gb300 import Phase
+from bone_morphometry_gb300 import Phase, local_thickness
 from bone_morphometry_gb300 import euclidean_distance_transform_squared as edt
 
 pytestmark = pytest.mark.gpu
@@ -54,3 +54,18 @@ def test_edt_bitwise(gpu_ctx, name, make, phase):
     if phase == Phase.BACKGROUND:
         vol = 1 - vol
     assert np.array_equal(edt(vol, phase, ctx=gpu_ctx), O.edt_sq(vol, int(phase)))
+
+
+@pytest.mark.parametrize("w", [64, 112, 1040])
+@pytest.mark.parametrize("tiles", [False, True])
+def test_sites_outside_the_first_word(gpu_ctx, w, tiles):
+    """No site in the first 32 of any 512 columns: both forms of the x pass count the others."""
+    vol = noise((9, 11, w), 0.9, w)
+    for x in range(0, w, 512):
+        vol[:, :, x : x + 32] = 1
+    gpu_ctx.set_fill_tile_rows(16 if tiles else 0)
+    try:
+        got = local_thickness(vol, Phase.FOREGROUND, ctx=gpu_ctx)
+    finally:
+        gpu_ctx.set_fill_tile_rows(0)
+    assert np.array_equal(got.view(np.uint32), O.local_thickness(vol, 0).thickness.view(np.uint32))
