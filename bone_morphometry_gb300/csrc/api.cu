@@ -375,6 +375,9 @@ struct Phase {
   uint8_t* zflags = nullptr;
   bool near = false;            // the 16-bit passes first
   bool separable = false;
+  uint32_t* hdr = nullptr;      // disc lists
+  uint2* ent = nullptr;
+  uint2* pool = nullptr;
   int e_lo = 0;
 
   size_t voxels() const { return (size_t)dm.n(); }
@@ -481,30 +484,33 @@ struct Phase {
     separable = hc.rmax <= kDiscMaxR2 && !tiles_asked();
   }
 
-  // Local thickness, after wait_edt: queued to its end, but for the tile
-  // fill's own waits.
-  void fill() {
+  // Local thickness, after wait_edt: lists, then paint, queued to their end (but
+  // for the tile fill's own waits).
+  void lists() {
     ensure_lut(ctx, hc.rmax);
-    if (separable) disc_fill();
-    else tile_fill();
-  }
-
-  void disc_fill() {
+    if (!separable) return;
     const size_t N = voxels();
-    uint32_t* nzbits = static_cast<uint32_t*>(ensure(ctx, ctx->nzbits, bits_bytes(), "nonzero bits"));
     uint16_t* rmap = static_cast<uint16_t*>(ensure(ctx, ctx->ridgemap, N * sizeof(uint16_t), "ridge map"));
-    const size_t lists = disc_header_count(dm);
-    uint32_t* hdr = static_cast<uint32_t*>(ensure(ctx, ctx->dischdr, lists * 4, "disc lists"));
-    uint2* ent = static_cast<uint2*>(ensure(ctx, ctx->discent, lists * kDiscSlots * sizeof(uint2), "disc lists"));
+    const size_t count = disc_header_count(dm);
+    hdr = static_cast<uint32_t*>(ensure(ctx, ctx->dischdr, count * 4, "disc lists"));
+    ent = static_cast<uint2*>(ensure(ctx, ctx->discent, count * kDiscSlots * sizeof(uint2), "disc lists"));
     const size_t pool_cap = disc_pool_entries(dm);
-    uint2* pool = static_cast<uint2*>(ensure(ctx, ctx->discpool, pool_cap * sizeof(uint2), "disc lists"));
+    pool = static_cast<uint2*>(ensure(ctx, ctx->discpool, pool_cap * sizeof(uint2), "disc lists"));
     const uint2* thr = static_cast<const uint2*>(ctx->discthr.ptr);
     const uint32_t* tmpl = static_cast<const uint32_t*>(ctx->disctmpl.ptr);
-    const float* dia = static_cast<const float*>(ctx->lutf.ptr);
     timed(ctx, KF_RIDGE, s, "ridge map", [&] { return launch_ridge_map(E, dm, thr, rmap, s, &ctx->launches); });
     timed(ctx, KF_FILL_BIN, s, "disc lists", [&] {
       return launch_disc_lists(rmap, dm, hc.rmax, tmpl, hdr, ent, pool, pool_cap, &out->ctr, s, &ctx->launches);
     });
+  }
+
+  void paint() {
+    if (!separable) {
+      tile_fill();
+      return;
+    }
+    uint32_t* nzbits = static_cast<uint32_t*>(ensure(ctx, ctx->nzbits, bits_bytes(), "nonzero bits"));
+    const float* dia = static_cast<const float*>(ctx->lutf.ptr);
     float* dmap = reinterpret_cast<float*>(B);  // the y pass output has been read
     timed(ctx, KF_FILL, s, "disc painting", [&] {
       return launch_disc_paint(hdr, ent, pool, dm, hc.rmax, dia, dmap, nzbits, d_sq, s, &ctx->launches);
@@ -580,7 +586,8 @@ void run_phase(Phase& p) {
   p.z();
   p.wait_edt();
   if (p.edt_only) return;
-  p.fill();
+  p.lists();
+  p.paint();
   p.finish();
 }
 
@@ -1064,7 +1071,8 @@ int tbth_phases(bm_ctx* ctx, const uint8_t* d_bone, const uint8_t* d_roi, Dims d
   bone.d_map = map_of(ctx, d_thmap);
   bone.wait_edt();
   if (!tw) {
-    bone.fill();
+    bone.lists();
+    bone.paint();
     bone.finish();
     int st = report_phase(bone, ctx, s, want_q, bone.d_map, spacing, th);
     if (st) return st;
@@ -1095,7 +1103,8 @@ int tbth_phases(bm_ctx* ctx, const uint8_t* d_bone, const uint8_t* d_roi, Dims d
       try_twin([&] {
         const cudaError_t e = cudaSetDevice(tw->device);
         check(tw, e, "cudaSetDevice");
-        marrow.fill();
+        marrow.lists();
+        marrow.paint();
         marrow.finish();
       });
     });
@@ -1103,11 +1112,21 @@ int tbth_phases(bm_ctx* ctx, const uint8_t* d_bone, const uint8_t* d_roi, Dims d
       std::thread& t;
       ~Join() { t.join(); }
     } join{thread};
-    bone.fill();
+    bone.lists();
+    bone.paint();
     bone.finish();
   } else {
-    bone.fill();
-    try_twin([&] { marrow.fill(); });
+    // Small volumes in turns and the marrow phase, whose balls are larger as a
+    // rule, first: neither phase's kernels wait for all the other's launches (64^3
+    // 240 us, 268 with the bone phase queued whole and first).  Where kernels
+    // outlast launches the bone phase first, so that the phases are at different
+    // kernels (128^3 536 us, 543 in turns; 512^3 10.10 ms, 10.32).
+    const bool turns = N < (1ll << 20);
+    if (turns) try_twin([&] { marrow.lists(); });
+    bone.lists();
+    if (turns) try_twin([&] { marrow.paint(); });
+    bone.paint();
+    if (!turns) try_twin([&] { marrow.lists(), marrow.paint(); });
     bone.finish();
   }
   int st = report_phase(bone, ctx, s, want_q, bone.d_map, spacing, th);

@@ -141,7 +141,6 @@ __global__ void disc_tables_kernel(const uint4* __restrict__ lut, uint32_t n, ui
 // ---- disc lists -------------------------------------------------------------
 constexpr int kListThreads = 512;
 constexpr int kListWarps = kListThreads / 32;
-constexpr int kListZ = 32;                 // planes per CTA
 constexpr int kCols = kDiscPX * kDiscPY;   // columns of the patch
 constexpr int kRowPad = kDiscPX + 2;       // per-plane table with an empty border of one cell
 constexpr int kPlaneCells = (kDiscPY + 2) * kRowPad;
@@ -150,7 +149,6 @@ constexpr int kWalk = 6;                   // planes a thread walks per step
 constexpr int kCentres = 4096;             // ball centres a CTA keeps from its first walk
 // centres and runs a warp holds back until 32 are ready
 constexpr int kCentreQueue = 32 + 32 * kWalk, kRunQueue = 64;
-static_assert(kListZ <= 64, "run encoding");
 
 // The last t with a disc (or chord) of squared radius rho - t^2 not covered by
 // that of the neighbour one step up, rho' - (t - 1)^2, gain = rho' - rho: covered
@@ -164,7 +162,7 @@ __device__ __forceinline__ int cut_below(int gain) { return (gain + 1) >> 1; }
 // Cell of patch column c in a plane of the padded table.
 __device__ __forceinline__ int cell_of(uint32_t c) { return (int)(c >> 5) * kRowPad + kRowPad + (int)(c & 31u) + 1; }
 
-// One CTA per patch of 32 x 8 columns and kListZ planes.  Its threads walk the
+// One CTA per patch of 32 x 8 columns and NZ planes.  Its threads walk the
 // ridge map's columns through the planes and a halo of the largest radius; the
 // ball centres they meet are collected per warp, handled 32 at a time, and kept
 // for the second step (up to kCentres; beyond, the columns are walked again).
@@ -192,22 +190,23 @@ __device__ __forceinline__ int cell_of(uint32_t c) { return (int)(c >> 5) * kRow
 //
 // A plane with more than kDiscSlots discs gets a segment of the overflow pool
 // and a third step.
+template <int NZ>
 __global__ void __launch_bounds__(kListThreads, 2)
 disc_list_kernel(const uint16_t* __restrict__ rmap, Dims dm, int H, const uint32_t* __restrict__ tmpl, int npx, int npy,
                  uint32_t* __restrict__ hdr, uint2* __restrict__ ent, uint2* __restrict__ pool,
                  unsigned long long pool_cap, Counters* __restrict__ ctr) {
   extern __shared__ uint32_t smem[];
-  uint32_t* largest = smem;  // kListZ x kPlaneCells: rho << 16 | R
-  uint2* centres = reinterpret_cast<uint2*>(largest + kListZ * kPlaneCells);  // kCentres
+  uint32_t* largest = smem;  // NZ x kPlaneCells: rho << 16 | R
+  uint2* centres = reinterpret_cast<uint2*>(largest + NZ * kPlaneCells);  // kCentres
   uint2* queues = centres + kCentres;
-  static_assert(kListZ == 32, "a bit per plane");
-  __shared__ uint32_t s_count[kListZ], s_full, s_centres;  // s_full: planes whose list goes to the pool
-  __shared__ uint2* s_dst[kListZ];
+  static_assert(NZ <= 32, "a bit per plane");
+  __shared__ uint32_t s_count[NZ], s_full, s_centres;  // s_full: planes whose list goes to the pool
+  __shared__ uint2* s_dst[NZ];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned below = (1u << lane) - 1u;
   const long long bid = blockIdx.x;
   const int px = (int)(bid % npx), py = (int)((bid / npx) % npy), pz = (int)(bid / ((long long)npx * npy));
-  const int z0 = pz * kListZ, nz = min(kListZ, dm.d - z0);
+  const int z0 = pz * NZ, nz = min(NZ, dm.d - z0);
   const long long slice = (long long)dm.w * dm.h;
   const long long plane_hdrs = (long long)npx * npy;
   const long long first_hdr = (long long)z0 * plane_hdrs + (long long)py * npx + px;
@@ -221,8 +220,8 @@ disc_list_kernel(const uint16_t* __restrict__ rmap, Dims dm, int H, const uint32
   const int w0 = za + part * per, w1 = min(w0 + per, zb);  // planes this thread walks
   uint2* cq = queues + warp * (kCentreQueue + kRunQueue);
   uint2* rq = cq + kCentreQueue;
-  for (int i = tid; i < kListZ * kPlaneCells; i += kListThreads) largest[i] = 0u;
-  if (tid < kListZ) {
+  for (int i = tid; i < NZ * kPlaneCells; i += kListThreads) largest[i] = 0u;
+  if (tid < NZ) {
     s_count[tid] = 0u;
     s_dst[tid] = ent + (first_hdr + (long long)tid * plane_hdrs) * kDiscSlots;
   }
@@ -644,8 +643,18 @@ int halo_of(uint32_t rmax) {
   return h;
 }
 
-constexpr size_t kListSmem = (size_t)kListZ * kPlaneCells * sizeof(uint32_t) +
-                             ((size_t)kCentres + kListWarps * (kCentreQueue + kRunQueue)) * sizeof(uint2);
+template <int NZ>
+cudaError_t list_planes(const uint16_t* rmap, Dims dm, int H, const uint32_t* tmpl, int npx, int npy, uint32_t* hdr,
+                        uint2* ent, uint2* pool, size_t pool_cap, Counters* ctr, cudaStream_t s) {
+  constexpr size_t smem = (size_t)NZ * kPlaneCells * sizeof(uint32_t) +
+                          ((size_t)kCentres + kListWarps * (kCentreQueue + kRunQueue)) * sizeof(uint2);
+  const long long blocks = (long long)npx * npy * ((dm.d + NZ - 1) / NZ);
+  cudaError_t e = cudaFuncSetAttribute(disc_list_kernel<NZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  disc_list_kernel<NZ><<<(unsigned)blocks, kListThreads, smem, s>>>(rmap, dm, H, tmpl, npx, npy, hdr, ent, pool,
+                                                                    pool_cap, ctr);
+  return cudaGetLastError();
+}
 
 }  // namespace
 
@@ -654,13 +663,14 @@ cudaError_t launch_disc_lists(const uint16_t* rmap, Dims dm, uint32_t rmax, cons
                               unsigned long long* launches) {
   const int H = halo_of(rmax);
   const int npx = (dm.w + kDiscPX - 1) / kDiscPX, npy = (dm.h + kDiscPY - 1) / kDiscPY;
-  const long long blocks = (long long)npx * npy * ((dm.d + kListZ - 1) / kListZ);
-  cudaError_t e = cudaFuncSetAttribute(disc_list_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kListSmem);
-  if (e != cudaSuccess) return e;
-  disc_list_kernel<<<(unsigned)blocks, kListThreads, kListSmem, s>>>(rmap, dm, H, tmpl, npx, npy, hdr, ent, pool,
-                                                                     pool_cap, ctr);
   ++*launches;
-  return cudaGetLastError();
+  // 32 planes per CTA share the walk through the halo.  Where such CTAs would
+  // leave half of the SMs idle, 8: lists of both phases of 56 x 64 x 72 (42
+  // CTAs) 47 us with 32 planes, 36 with 16, 28 with 8; 72 x 81 x 97 (132 CTAs) 23 with any of
+  // them; 128^3 (256 CTAs) 78, 73, 82; 200 x 180 x 251 191, 225, 311.
+  if ((long long)npx * npy * ((dm.d + 31) / 32) <= 76)
+    return list_planes<8>(rmap, dm, H, tmpl, npx, npy, hdr, ent, pool, pool_cap, ctr, s);
+  return list_planes<32>(rmap, dm, H, tmpl, npx, npy, hdr, ent, pool, pool_cap, ctr, s);
 }
 
 namespace {

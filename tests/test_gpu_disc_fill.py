@@ -56,3 +56,13 @@ def test_separable_fill_bitwise(gpu_ctx, name, make, phase):
     got, sq = local_thickness(vol, phase, ctx=gpu_ctx, return_squared=True)
     assert np.array_equal(sq, ref.propagated)
     assert np.array_equal(got.view(np.uint32), ref.thickness.view(np.uint32))
+
+
+@pytest.mark.parametrize("d,w", [(7, 70), (8, 70), (9, 70), (17, 33), (31, 1300), (32, 1300), (33, 1300), (65, 1000)])
+def test_plane_runs_bitwise(gpu_ctx, d, w):
+    """Runs of 8 planes (narrow volumes) and of 32 (wide ones), at their edges."""
+    vol = blobs((d, 17, w), 2.0, 0.6, d + w)
+    ref = O.local_thickness(vol, 0)
+    got, sq = local_thickness(vol, Phase.FOREGROUND, ctx=gpu_ctx, return_squared=True)
+    assert np.array_equal(sq, ref.propagated)
+    assert np.array_equal(got.view(np.uint32), ref.thickness.view(np.uint32))
