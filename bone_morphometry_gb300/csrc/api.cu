@@ -383,6 +383,8 @@ struct Phase {
   size_t voxels() const { return (size_t)dm.n(); }
   size_t bits_bytes() const { return (size_t)dm.nw() * dm.h * dm.d * sizeof(uint32_t); }
 
+  size_t narrow_bytes() const { return (size_t)edt_near_pitch(dm.w) * dm.h * dm.d * 2; }
+
   // A forced site method or tile height asks for the tile fill.
   bool tiles_asked() const { return ctx->site_method != BM_SITES_AUTO || ctx->fill_rows != 0; }
 
@@ -392,10 +394,8 @@ struct Phase {
     // the 16-bit passes, but where the caller has asked for the tile fill (its
     // chain passes read the 32-bit maps)
     near = edt_only || !tiles_asked();
-    const size_t narrow = near ? (size_t)edt_near_pitch(dm.w) * dm.h * dm.d * 2 : 0;
-    const size_t map = std::max(N * 4, narrow);
-    A = static_cast<uint32_t*>(ensure(ctx, ctx->dist, map, "distance map"));
-    B = static_cast<uint32_t*>(ensure(ctx, ctx->dist2, map, "distance map"));
+    A = static_cast<uint32_t*>(ensure(ctx, ctx->dist, near ? narrow_bytes() : N * 4, "distance map"));
+    B = static_cast<uint32_t*>(ensure(ctx, ctx->dist2, std::max(N * 4, near ? narrow_bytes() : 0), "distance map"));
     scratch = ensure(ctx, ctx->stack, edt_scratch_bytes(dm), "envelope scratch");
     selbits = static_cast<uint32_t*>(ensure(ctx, ctx->selbits, bits_bytes(), "selection bits"));
     const size_t ny = (size_t)dm.w * dm.d, nz = (size_t)dm.w * dm.h;
@@ -403,8 +403,9 @@ struct Phase {
     yflags = reinterpret_cast<uint8_t*>(out + 1);
     zflags = yflags + ny;
     // local thickness keeps the x pass output (the chain passes read it): the z
-    // pass then writes its own map
-    E = d_edt ? d_edt : (edt_only ? A : static_cast<uint32_t*>(ensure(ctx, ctx->edtmap, N * 4, "distance map")));
+    // pass then writes its own map, in 16 bits for the separable fill
+    E = d_edt ? d_edt
+              : static_cast<uint32_t*>(ensure(ctx, ctx->edtmap, near ? narrow_bytes() : N * 4, "distance map"));
     check(ctx, cudaMemsetAsync(out, 0, sizeof(PhaseOut) + ny + nz, s), "memset");
   }
 
@@ -435,6 +436,7 @@ struct Phase {
   // The 32-bit x and y passes; only: the z lines whose tiles the y pass is for (null: all).
   void wide_xy(Dims sd, const uint8_t* a, const uint8_t* b, uint32_t* sel, long long off, uint8_t* flags,
                const uint8_t* only) {
+    A = static_cast<uint32_t*>(ensure(ctx, ctx->dist, voxels() * 4, "distance map"));
     timed(ctx, KF_EDT_X, s, "edt x pass",
           [&] { return launch_edt_x(a, b, mode, sd, A + off, sel, &out->ctr, s, &ctx->launches); });
     timed(ctx, KF_EDT_Y, s, "edt y pass", [&] {
@@ -448,7 +450,8 @@ struct Phase {
   void z() {
     timed(ctx, KF_EDT_Z, s, "edt z pass", [&] {
       if (near)
-        return launch_edt_near_z(reinterpret_cast<const uint16_t*>(B), E, dm, zflags, &out->ctr, s, &ctx->launches);
+        return launch_edt_near_z(reinterpret_cast<const uint16_t*>(B), d_edt, reinterpret_cast<uint16_t*>(E), dm,
+                                 zflags, &out->ctr, s, &ctx->launches);
       return launch_edt_window(2, B, E, dm, zflags, &out->ctr, ctx->wait_cycles, nullptr, s, &ctx->launches);
     });
     read_counters();
@@ -466,8 +469,12 @@ struct Phase {
       // the flagged lines, from 32-bit x and y passes
       const unsigned long long sites = hc.sites;
       if (near) wide_xy(dm, d_a, d_b, selbits, 0, yflags, zflags);
-      timed(ctx, KF_EDT_Z, s, "edt z lines",
-            [&] { return launch_edt_redo(2, B, E, dm, scratch, zflags, &out->ctr, s, &ctx->launches); });
+      timed(ctx, KF_EDT_Z, s, "edt z lines", [&] {
+        if (near && !d_edt)
+          return launch_edt_near_redo(B, reinterpret_cast<uint16_t*>(E), dm, scratch, zflags, &out->ctr, s,
+                                      &ctx->launches);
+        return launch_edt_redo(2, B, E, dm, scratch, zflags, &out->ctr, s, &ctx->launches);
+      });
       read_counters();
       check(ctx, cudaStreamSynchronize(s), "edt");
       hc = readback(ctx).ctr;
@@ -489,8 +496,7 @@ struct Phase {
   void lists() {
     ensure_lut(ctx, hc.rmax);
     if (!separable) return;
-    const size_t N = voxels();
-    uint16_t* rmap = static_cast<uint16_t*>(ensure(ctx, ctx->ridgemap, N * sizeof(uint16_t), "ridge map"));
+    uint16_t* rmap = static_cast<uint16_t*>(ensure(ctx, ctx->ridgemap, narrow_bytes(), "ridge map"));
     const size_t count = disc_header_count(dm);
     hdr = static_cast<uint32_t*>(ensure(ctx, ctx->dischdr, count * 4, "disc lists"));
     ent = static_cast<uint2*>(ensure(ctx, ctx->discent, count * kDiscSlots * sizeof(uint2), "disc lists"));
@@ -498,7 +504,9 @@ struct Phase {
     pool = static_cast<uint2*>(ensure(ctx, ctx->discpool, pool_cap * sizeof(uint2), "disc lists"));
     const uint2* thr = static_cast<const uint2*>(ctx->discthr.ptr);
     const uint32_t* tmpl = static_cast<const uint32_t*>(ctx->disctmpl.ptr);
-    timed(ctx, KF_RIDGE, s, "ridge map", [&] { return launch_ridge_map(E, dm, thr, rmap, s, &ctx->launches); });
+    timed(ctx, KF_RIDGE, s, "ridge map", [&] {
+      return launch_ridge_map(reinterpret_cast<const uint16_t*>(E), dm, thr, rmap, s, &ctx->launches);
+    });
     timed(ctx, KF_FILL_BIN, s, "disc lists", [&] {
       return launch_disc_lists(rmap, dm, hc.rmax, tmpl, hdr, ent, pool, pool_cap, &out->ctr, s, &ctx->launches);
     });
@@ -518,7 +526,25 @@ struct Phase {
     cleanup(dmap, nzbits);
   }
 
+  // The whole transform in 32 bits, for the tile fill after the 16-bit passes.
+  void widen() {
+    E = static_cast<uint32_t*>(ensure(ctx, ctx->edtmap, voxels() * 4, "distance map"));
+    check(ctx, cudaMemsetAsync(yflags, 0, (size_t)dm.w * (dm.d + dm.h), s), "memset");
+    wide_xy(dm, d_a, d_b, selbits, 0, yflags, nullptr);
+    timed(ctx, KF_EDT_Z, s, "edt z pass", [&] {
+      const cudaError_t e =
+          launch_edt_window(2, B, E, dm, zflags, &out->ctr, ctx->wait_cycles, nullptr, s, &ctx->launches);
+      if (e != cudaSuccess) return e;
+      return launch_edt_redo(2, B, E, dm, scratch, zflags, &out->ctr, s, &ctx->launches);
+    });
+    read_counters();
+    check(ctx, cudaStreamSynchronize(s), "edt");
+    if (readback(ctx).ctr.status)
+      fail(ctx, BM_ERR_TIMEOUT, "a bounded device-side wait of the distance transform ran out");
+  }
+
   void tile_fill() {
+    if (near) widen();
     const uint4* lut = static_cast<const uint4*>(ctx->lut.ptr);
     const float* dia = static_cast<const float*>(ctx->lutf.ptr);
     const unsigned long long selected = voxels() - hc.sites;
@@ -531,11 +557,9 @@ struct Phase {
     check(ctx, cudaMemsetAsync(rbits, 0, bits_bytes(), s), "memset");
     timed(ctx, KF_RIDGE, s, "ridge kernel",
           [&] { return launch_ridges(E, selbits, dm, lut, ridges, &out->ctr, occ, rbits, s, &ctx->launches); });
-    const bool own_e = E != A && E != d_edt;  // E is the context's map: the chain passes may reuse it
-    // (after the separable fill, B no longer holds the y pass output the chain passes need)
-    const bool chains = own_e && !separable;
-    uint32_t* F = fill_phase(ctx, dm, ridges, &out->ctr, selected, hc.rmax, occ, selbits, A, B, chains ? E : nullptr,
-                             rbits, d_sq ? d_sq : B, s);
+    // E is the context's map: the chain passes may reuse it
+    uint32_t* F = fill_phase(ctx, dm, ridges, &out->ctr, selected, hc.rmax, occ, selbits, A, B, E, rbits,
+                             d_sq ? d_sq : B, s);
     float* dmap = reinterpret_cast<float*>(F == d_sq ? B : F);
     timed(ctx, KF_CLEAN_FINAL, s, "diameters",
           [&] { return launch_diameters(F, dm, dia, dmap, nzbits, s, &ctx->launches); });

@@ -45,44 +45,52 @@ __device__ __forceinline__ uint32_t max3(uint32_t a, uint32_t b, uint32_t c) { r
 
 // ---- ridge map --------------------------------------------------------------
 // Distance ridge (local_thickness.rs:104-167) as a u16 map: twice the squared
-// distance (0 for a non-selected voxel), plus 1 for a ridge voxel.  A warp owns 30 x (its outer lanes hold the x
-// neighbours) and ROWS rows and walks NZ planes upwards; each plane's rows are
+// distance (0 for a non-selected voxel), plus 1 for a ridge voxel.  Two
+// adjacent voxels of x per register.  A warp owns 60 x (its outer lanes hold the
+// x neighbours) and ROWS rows and walks NZ planes upwards; each plane's rows are
 // loaded once and reduced to the maxima that the face, edge and corner tests of
 // three planes share, in registers.
-constexpr int kMapX = 30;
+//
+// Bound by issue and by the gather of the bounds (two per register of selected
+// voxels): both phases of 512^3 595 us with a voxel per lane from a 32-bit map,
+// 412 here (bytes alone: 160).
+constexpr int kMapPairs = 30;
 constexpr int kMapWarps = 4;
 
 template <int ROWS, int NZ>
 __global__ void __launch_bounds__(kMapWarps * 32)
-ridge_map_kernel(const uint32_t* __restrict__ dist, Dims dm, const uint2* __restrict__ thr, uint16_t* __restrict__ out,
-                 int nxt, int nyt, int nzt) {
+ridge_map_kernel(const uint32_t* __restrict__ dist, int pairs, int h, int d, const uint2* __restrict__ thr,
+                 uint32_t* __restrict__ out, int nxt, int nyt, int nzt) {
   const int lane = threadIdx.x & 31;
   const long long wid = (long long)blockIdx.x * kMapWarps + (threadIdx.x >> 5);
   if (wid >= (long long)nxt * nyt * nzt) return;
   const int xt = (int)(wid % nxt), yt = (int)((wid / nxt) % nyt), zt = (int)(wid / ((long long)nxt * nyt));
-  const int x = xt * kMapX - 1 + lane, y0 = yt * ROWS, z0 = zt * NZ;
-  const int z1 = min(z0 + NZ, dm.d);
-  const bool xin = x >= 0 && x < dm.w, xout = lane >= 1 && lane <= kMapX && x < dm.w;
-  const long long slice = (long long)dm.w * dm.h;
-  const uint32_t* src = dist + (long long)(y0 - 1) * dm.w + x;
-  uint16_t* dst = out + (long long)y0 * dm.w + x;
+  const int x = xt * kMapPairs - 1 + lane, y0 = yt * ROWS, z0 = zt * NZ;
+  const int z1 = min(z0 + NZ, d);
+  const bool xin = x >= 0 && x < pairs, xout = lane >= 1 && lane <= kMapPairs && x < pairs;
+  const long long slice = (long long)pairs * h;
+  const uint32_t* src = dist + (long long)(y0 - 1) * pairs + x;
+  uint32_t* dst = out + (long long)y0 * pairs + x;
   auto load = [&](int z, uint32_t (&c)[ROWS + 2]) {
-    const bool zin = xin && z >= 0 && z < dm.d;
+    const bool zin = xin && z >= 0 && z < d;
     const uint32_t* p = src + (long long)z * slice;
 #pragma unroll
-    for (int r = 0; r < ROWS + 2; ++r) c[r] = zin && y0 - 1 + r >= 0 && y0 - 1 + r < dm.h ? p[r * dm.w] : 0u;
+    for (int r = 0; r < ROWS + 2; ++r) c[r] = zin && y0 - 1 + r >= 0 && y0 - 1 + r < h ? p[r * pairs] : 0u;
   };
-  // of a voxel and its plane: itself, its in-plane face neighbours, its in-plane corner neighbours
+  // of two voxels and their plane: themselves, their in-plane face neighbours, their in-plane corner neighbours
   struct PlaneMax {
     uint32_t c, m, s;
   };
   auto reduce = [&](const uint32_t (&c)[ROWS + 2], PlaneMax (&p)[ROWS]) {
     uint32_t a[ROWS + 2];  // max of the two x neighbours
 #pragma unroll
-    for (int r = 0; r < ROWS + 2; ++r)
-      a[r] = max(__shfl_up_sync(0xffffffffu, c[r], 1), __shfl_down_sync(0xffffffffu, c[r], 1));
+    for (int r = 0; r < ROWS + 2; ++r) {
+      const uint32_t before = __shfl_up_sync(0xffffffffu, c[r], 1), after = __shfl_down_sync(0xffffffffu, c[r], 1);
+      a[r] = __vmaxu2(__byte_perm(before, c[r], 0x5432), __byte_perm(c[r], after, 0x5432));
+    }
 #pragma unroll
-    for (int r = 0; r < ROWS; ++r) p[r] = PlaneMax{c[r + 1], max3(a[r + 1], c[r], c[r + 2]), max(a[r], a[r + 2])};
+    for (int r = 0; r < ROWS; ++r)
+      p[r] = PlaneMax{c[r + 1], __vimax3_u16x2(a[r + 1], c[r], c[r + 2]), __vmaxu2(a[r], a[r + 2])};
   };
   uint32_t c[ROWS + 2];
   PlaneMax mid[ROWS], hi[ROWS];
@@ -93,8 +101,8 @@ ridge_map_kernel(const uint32_t* __restrict__ dist, Dims dm, const uint2* __rest
   reduce(c, mid);
 #pragma unroll
   for (int r = 0; r < ROWS; ++r) {
-    face[r] = max(mid[r].m, hi[r].c);
-    edge[r] = max(mid[r].s, hi[r].m);
+    face[r] = __vmaxu2(mid[r].m, hi[r].c);
+    edge[r] = __vmaxu2(mid[r].s, hi[r].m);
     corner[r] = hi[r].s;
   }
   load(z0 + 1, c);
@@ -106,28 +114,34 @@ ridge_map_kernel(const uint32_t* __restrict__ dist, Dims dm, const uint2* __rest
       const uint32_t R = mid[r].c;
       uint32_t v = 0u;
       if (R) {
-        const uint2 t = __ldg(thr + R);  // {face | edge << 16, corner}
-        const bool ridge = max(face[r], hi[r].c) < (t.x & 0xffffu) && max(edge[r], hi[r].m) < (t.x >> 16) &&
-                           max(corner[r], hi[r].s) < t.y;
-        v = 2u * R + (ridge ? 1u : 0u);
+        const uint2 t0 = __ldg(thr + (R & 0xffffu)), t1 = __ldg(thr + (R >> 16));  // {face | edge << 16, corner}
+        const uint32_t tf = __byte_perm(t0.x, t1.x, 0x5410), te = __byte_perm(t0.x, t1.x, 0x7632),
+                       tc = __byte_perm(t0.y, t1.y, 0x5410);
+        // a half is 0 where all three maxima are at most their bounds
+        const uint32_t over = (__vimax3_u16x2(face[r], hi[r].c, tf) ^ tf) | (__vimax3_u16x2(edge[r], hi[r].m, te) ^ te) |
+                              (__vimax3_u16x2(corner[r], hi[r].s, tc) ^ tc);
+        v = 2u * R;
+        if (!(over & 0xffffu) && (R & 0xffffu)) v |= 1u;
+        if (!(over >> 16) && (R >> 16)) v |= 0x10000u;
       }
-      if (xout && y0 + r < dm.h) dst[(long long)z * slice + r * dm.w] = (uint16_t)v;
-      face[r] = max(hi[r].m, mid[r].c);
-      edge[r] = max(hi[r].s, mid[r].m);
+      if (xout && y0 + r < h) dst[(long long)z * slice + r * pairs] = v;
+      face[r] = __vmaxu2(hi[r].m, mid[r].c);
+      edge[r] = __vmaxu2(hi[r].s, mid[r].m);
       corner[r] = mid[r].s;
       mid[r] = hi[r];
     }
   }
 }
 
-// thr[R] = the three search templates of R (lut) packed for the ridge map;
+// thr[R] = the largest values that pass the ridge map's three tests of R: its
+// search templates (lut, at least 1) less 1;
 // tmpl[rho] = the largest |u + o|^2 over the 2-D lattice points |u|^2 <= rho for
 // o = (1, 0) in the low and o = (1, 1) in the high half.
 __global__ void disc_tables_kernel(const uint4* __restrict__ lut, uint32_t n, uint2* __restrict__ thr,
                                    uint32_t* __restrict__ tmpl) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const uint4 t = lut[i];
-    thr[i] = make_uint2(min(t.x, 0xffffu) | (min(t.y, 0xffffu) << 16), min(t.z, 0xffffu));
+    thr[i] = make_uint2((min(t.x, 0x10000u) - 1u) | ((min(t.y, 0x10000u) - 1u) << 16), min(t.z, 0x10000u) - 1u);
     uint32_t face = 0, corner = 0;
     for (uint32_t a = 0; a * a <= i; ++a) {
       const uint32_t b = floor_sqrt(i - a * a);
@@ -192,7 +206,7 @@ __device__ __forceinline__ int cell_of(uint32_t c) { return (int)(c >> 5) * kRow
 // and a third step.
 template <int NZ>
 __global__ void __launch_bounds__(kListThreads, 2)
-disc_list_kernel(const uint16_t* __restrict__ rmap, Dims dm, int H, const uint32_t* __restrict__ tmpl, int npx, int npy,
+disc_list_kernel(const uint16_t* __restrict__ rmap, int pitch, Dims dm, int H, const uint32_t* __restrict__ tmpl, int npx, int npy,
                  uint32_t* __restrict__ hdr, uint2* __restrict__ ent, uint2* __restrict__ pool,
                  unsigned long long pool_cap, Counters* __restrict__ ctr) {
   extern __shared__ uint32_t smem[];
@@ -207,14 +221,14 @@ disc_list_kernel(const uint16_t* __restrict__ rmap, Dims dm, int H, const uint32
   const long long bid = blockIdx.x;
   const int px = (int)(bid % npx), py = (int)((bid / npx) % npy), pz = (int)(bid / ((long long)npx * npy));
   const int z0 = pz * NZ, nz = min(NZ, dm.d - z0);
-  const long long slice = (long long)dm.w * dm.h;
+  const long long slice = (long long)pitch * dm.h;
   const long long plane_hdrs = (long long)npx * npy;
   const long long first_hdr = (long long)z0 * plane_hdrs + (long long)py * npx + px;
   constexpr int kParts = kListThreads / kCols;  // threads per column, each on a part of the planes
   const int cell = tid & (kCols - 1), part = tid / kCols;
   const int x = px * kDiscPX + lane, y = py * kDiscPY + (cell >> 5);
   const bool in = x < dm.w && y < dm.h;
-  const uint16_t* src = rmap + (long long)y * dm.w + x;
+  const uint16_t* src = rmap + (long long)y * pitch + x;
   const int za = max(z0 - H, 0), zb = min(z0 + nz + H, dm.d);
   const int per = (zb - za + kParts - 1) / kParts;
   const int w0 = za + part * per, w1 = min(w0 + per, zb);  // planes this thread walks
@@ -620,16 +634,18 @@ cudaError_t launch_disc_tables(const uint4* lut, uint32_t n, uint2* thr, uint32_
 
 namespace {
 template <int ROWS, int NZ>
-cudaError_t ridge_map_rows(const uint32_t* dist, Dims dm, const uint2* thr, uint16_t* rmap, cudaStream_t s) {
-  const int nxt = (dm.w + kMapX - 1) / kMapX, nyt = (dm.h + ROWS - 1) / ROWS, nzt = (dm.d + NZ - 1) / NZ;
+cudaError_t ridge_map_rows(const uint16_t* dist, Dims dm, const uint2* thr, uint16_t* rmap, cudaStream_t s) {
+  const int pairs = edt_near_pitch(dm.w) / 2;
+  const int nxt = (pairs + kMapPairs - 1) / kMapPairs, nyt = (dm.h + ROWS - 1) / ROWS, nzt = (dm.d + NZ - 1) / NZ;
   const long long warps = (long long)nxt * nyt * nzt;
   ridge_map_kernel<ROWS, NZ><<<(unsigned)((warps + kMapWarps - 1) / kMapWarps), kMapWarps * 32, 0, s>>>(
-      dist, dm, thr, rmap, nxt, nyt, nzt);
+      reinterpret_cast<const uint32_t*>(dist), pairs, dm.h, dm.d, thr, reinterpret_cast<uint32_t*>(rmap), nxt, nyt,
+      nzt);
   return cudaGetLastError();
 }
 }  // namespace
 
-cudaError_t launch_ridge_map(const uint32_t* dist, Dims dm, const uint2* thr, uint16_t* rmap, cudaStream_t s,
+cudaError_t launch_ridge_map(const uint16_t* dist, Dims dm, const uint2* thr, uint16_t* rmap, cudaStream_t s,
                              unsigned long long* launches) {
   ++*launches;
   return dm.n() >= (1ll << 23) ? ridge_map_rows<4, 32>(dist, dm, thr, rmap, s)
@@ -651,7 +667,7 @@ cudaError_t list_planes(const uint16_t* rmap, Dims dm, int H, const uint32_t* tm
   const long long blocks = (long long)npx * npy * ((dm.d + NZ - 1) / NZ);
   cudaError_t e = cudaFuncSetAttribute(disc_list_kernel<NZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  disc_list_kernel<NZ><<<(unsigned)blocks, kListThreads, smem, s>>>(rmap, dm, H, tmpl, npx, npy, hdr, ent, pool,
+  disc_list_kernel<NZ><<<(unsigned)blocks, kListThreads, smem, s>>>(rmap, edt_near_pitch(dm.w), dm, H, tmpl, npx, npy, hdr, ent, pool,
                                                                     pool_cap, ctr);
   return cudaGetLastError();
 }

@@ -248,14 +248,19 @@ edt_x_vec_kernel(const uint8_t* __restrict__ a, const uint8_t* __restrict__ b, D
 // One thread per line; consecutive threads take consecutive x so that every
 // load and store of the line data is a coalesced row.  The envelope stack
 // (position, f) lives in global scratch, k-major, and is cached by L1/L2.
+// Out uint16_t: a map with strides of its own, values beyond 16 bits cut to 0xffff.
+template <class Out>
 __global__ void __launch_bounds__(256)
-edt_line_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, int n, long long stride, int w,
-                long long outer, long long nlines, uint32_t* __restrict__ spos, uint32_t* __restrict__ sf,
-                Counters* __restrict__ ctr, int track_max, const uint8_t* __restrict__ only) {
+edt_line_kernel(const uint32_t* __restrict__ in, Out* __restrict__ out, int n, long long stride, int w,
+                long long outer, long long out_stride, long long out_outer, long long nlines,
+                uint32_t* __restrict__ spos, uint32_t* __restrict__ sf, Counters* __restrict__ ctr, int track_max,
+                const uint8_t* __restrict__ only) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   uint32_t localmax = 0;
   if (t < nlines && (only == nullptr || only[t])) {
     const long long base = (t / w) * outer + (t % w);
+    Out* to = out + (t / w) * out_outer + (t % w);
+    auto put = [&](int q, uint32_t v) { to[(long long)q * out_stride] = (Out)(sizeof(Out) == 2 ? min(v, 0xffffu) : v); };
     int k = -1;
     long long p1 = 0, F1 = 0;  // stack top
     long long p0 = 0, F0 = 0;  // entry below the top (valid when k >= 1)
@@ -288,7 +293,7 @@ edt_line_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, int
       F1 = Fq;
     }
     if (k < 0) {
-      for (int q = 0; q < n; ++q) out[base + (long long)q * stride] = kInfSq;
+      for (int q = 0; q < n; ++q) put(q, kInfSq);
     } else {
       int j = 0;
       long long pj = spos[t];
@@ -315,7 +320,7 @@ edt_line_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, int
         }
         const long long dq = q - pj;
         const uint32_t v = (uint32_t)(dq * dq) + fj;
-        out[base + (long long)q * stride] = v;
+        put(q, v);
         localmax = max(localmax, v);
       }
     }
@@ -824,11 +829,11 @@ __device__ __forceinline__ uint32_t near_group(const uint32_t* col, int m, int h
   return mx;
 }
 
-// The y (Z = false) or z pass over 64 columns and kWinTL outputs per block, the
-// input staged by every thread, with a halo as wide as the largest value needs.
-// in: pairs; strides in pairs.  The z pass writes the 32-bit result at the
-// volume's own pitch.
-template <bool Z>
+// The y or z pass over 64 columns and kWinTL outputs per block, the input
+// staged by every thread, with a halo as wide as the largest value needs.
+// in: pairs; strides in pairs.  WIDE: the 32-bit result at the volume's own
+// pitch, else pairs again.
+template <bool Z, bool WIDE>
 __global__ void __launch_bounds__(kWinThreads)
 edt_near_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, int n, long long stride, int pairs,
                 long long outer, int nxt, int nchunk, int w, long long out_stride, uint8_t* __restrict__ redo,
@@ -880,7 +885,7 @@ edt_near_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, int
   uint32_t far = 0;  // the lane's columns with an output beyond kNearMax
   // a block that stages nothing up to kNearMax holds no output up to it either
   // (columns of the padding stage zeros)
-  const bool some = !Z || top <= kNearMax || (pin && min(least & 0xffffu, x + 1 < w ? least >> 16 : kFar16) <= kNearMax);
+  const bool some = !Z || top <= kNearMax || (pin && min(least & 0xffffu, least >> 16) <= kNearMax);
   if (!__syncthreads_or(some)) {
     if (x < w) redo[orow * w + x] = 1u;
     if (x + 1 < w) redo[orow * w + x + 1] = 1u;
@@ -901,6 +906,8 @@ edt_near_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, int
       else localmax = max(localmax, m0);
       if (m1 > kNearMax) far |= 2u;
       else localmax = max(localmax, m1);
+    }
+    if (WIDE) {
       uint32_t* op = out + orow * w + x + (long long)q * out_stride;
 #pragma unroll
       for (int k = 0; k < kWinGroup; ++k, op += out_stride) {
@@ -1058,8 +1065,8 @@ cudaError_t launch_edt_line(int axis, const uint32_t* in, uint32_t* out, Dims dm
   uint32_t* spos = static_cast<uint32_t*>(scratch);
   uint32_t* sf = spos + (size_t)nlines * n;
   const long long blocks = (nlines + 255) / 256;
-  edt_line_kernel<<<(unsigned)blocks, 256, 0, s>>>(in, out, n, stride, dm.w, outer, nlines, spos, sf, ctr,
-                                                   axis == 2 ? 1 : 0, nullptr);
+  edt_line_kernel<<<(unsigned)blocks, 256, 0, s>>>(in, out, n, stride, dm.w, outer, stride, outer, nlines, spos, sf,
+                                                   ctr, axis == 2 ? 1 : 0, nullptr);
   ++*launches;
   return cudaGetLastError();
 }
@@ -1153,8 +1160,21 @@ cudaError_t launch_edt_redo(int axis, const uint32_t* in, uint32_t* out, Dims dm
   const Lines l = lines_of(axis, dm);
   uint32_t* spos = static_cast<uint32_t*>(scratch);
   uint32_t* sf = spos + (size_t)l.count * l.n;
-  edt_line_kernel<<<(unsigned)((l.count + 255) / 256), 256, 0, s>>>(in, out, l.n, l.stride, dm.w, l.outer, l.count, spos,
-                                                                   sf, ctr, axis == 2 ? 1 : 0, redo);
+  edt_line_kernel<<<(unsigned)((l.count + 255) / 256), 256, 0, s>>>(in, out, l.n, l.stride, dm.w, l.outer, l.stride,
+                                                                   l.outer, l.count, spos, sf, ctr, axis == 2 ? 1 : 0,
+                                                                   redo);
+  ++*launches;
+  return cudaGetLastError();
+}
+
+cudaError_t launch_edt_near_redo(const uint32_t* in, uint16_t* out, Dims dm, void* scratch, const uint8_t* redo,
+                                 Counters* ctr, cudaStream_t s, unsigned long long* launches) {
+  const Lines l = lines_of(2, dm);
+  const long long pitch = edt_near_pitch(dm.w);
+  uint32_t* spos = static_cast<uint32_t*>(scratch);
+  uint32_t* sf = spos + (size_t)l.count * l.n;
+  edt_line_kernel<<<(unsigned)((l.count + 255) / 256), 256, 0, s>>>(in, out, l.n, l.stride, dm.w, l.outer,
+                                                                   pitch * dm.h, pitch, l.count, spos, sf, ctr, 1, redo);
   ++*launches;
   return cudaGetLastError();
 }
@@ -1206,19 +1226,20 @@ cudaError_t launch_edt_near_xy(const uint8_t* a, const uint8_t* b, int mode, Dim
     edt_near_tma_kernel<<<blocks, kWinThreads, 0, s>>>(map, out, dm.h, pairs, nxt, nchunk, ctr,
                                                        wait_cycles < 0 ? kWaitCycles : wait_cycles);
   } else {
-    edt_near_kernel<false><<<blocks, kWinThreads, 0, s>>>(in, out, dm.h, pairs, pairs, (long long)pairs * dm.h, nxt,
+    edt_near_kernel<false, false><<<blocks, kWinThreads, 0, s>>>(in, out, dm.h, pairs, pairs, (long long)pairs * dm.h, nxt,
                                                           nchunk, dm.w, 0, nullptr, ctr);
   }
   return cudaGetLastError();
 }
 
-cudaError_t launch_edt_near_z(const uint16_t* ymap, uint32_t* out, Dims dm, uint8_t* redo, Counters* ctr,
-                              cudaStream_t s, unsigned long long* launches) {
+cudaError_t launch_edt_near_z(const uint16_t* ymap, uint32_t* wide, uint16_t* narrow, Dims dm, uint8_t* redo,
+                              Counters* ctr, cudaStream_t s, unsigned long long* launches) {
   const int pairs = edt_near_pitch(dm.w) / 2;
   const int nxt = (pairs + 31) / 32, nchunk = (dm.d + kWinTL - 1) / kWinTL;
-  edt_near_kernel<true><<<(unsigned)((long long)nxt * nchunk * dm.h), kWinThreads, 0, s>>>(
-      reinterpret_cast<const uint32_t*>(ymap), out, dm.d, (long long)pairs * dm.h, pairs, pairs, nxt, nchunk, dm.w,
-      (long long)dm.w * dm.h, redo, ctr);
+  auto kernel = wide ? edt_near_kernel<true, true> : edt_near_kernel<true, false>;
+  kernel<<<(unsigned)((long long)nxt * nchunk * dm.h), kWinThreads, 0, s>>>(
+      reinterpret_cast<const uint32_t*>(ymap), wide ? wide : reinterpret_cast<uint32_t*>(narrow), dm.d,
+      (long long)pairs * dm.h, pairs, pairs, nxt, nchunk, dm.w, (long long)dm.w * dm.h, redo, ctr);
   ++*launches;
   return cudaGetLastError();
 }

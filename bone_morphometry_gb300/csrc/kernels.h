@@ -65,8 +65,12 @@ int edt_near_pitch(int w);
 cudaError_t launch_edt_near_xy(const uint8_t* a, const uint8_t* b, int mode, Dims dm, uint16_t* xmap, uint16_t* ymap,
                                uint32_t* selbits, Counters* ctr, long long wait_cycles, bool x_pass, cudaStream_t s,
                                unsigned long long* launches);
-cudaError_t launch_edt_near_z(const uint16_t* ymap, uint32_t* out, Dims dm, uint8_t* redo, Counters* ctr,
-                              cudaStream_t s, unsigned long long* launches);
+// wide (32 bits at the volume's pitch) or narrow (16 bits at edt_near_pitch): the one not null.
+cudaError_t launch_edt_near_z(const uint16_t* ymap, uint32_t* wide, uint16_t* narrow, Dims dm, uint8_t* redo,
+                              Counters* ctr, cudaStream_t s, unsigned long long* launches);
+// The flagged lines of a narrow result, from the 32-bit y pass' output.
+cudaError_t launch_edt_near_redo(const uint32_t* in, uint16_t* out, Dims dm, void* scratch, const uint8_t* redo,
+                                 Counters* ctr, cudaStream_t s, unsigned long long* launches);
 
 // Search-template table entries lut[r2] for r2 in [lo, hi]:
 // {scan_cube(1,0,0), scan_cube(1,1,0), scan_cube(1,1,1), f32 bits of 2*sqrt(r2)}.
@@ -127,8 +131,9 @@ size_t disc_header_count(Dims dm);
 // thr / tmpl: n entries by squared radius, from the search templates.
 cudaError_t launch_disc_tables(const uint4* lut, uint32_t n, uint2* thr, uint32_t* tmpl, cudaStream_t s,
                                unsigned long long* launches);
-// The distance ridge as a u16 map: twice the squared distance, plus 1 for ridge voxels.
-cudaError_t launch_ridge_map(const uint32_t* dist, Dims dm, const uint2* thr, uint16_t* rmap, cudaStream_t s,
+// The distance ridge of a 16-bit distance map as one: twice the squared
+// distance, plus 1 for ridge voxels.  Both at edt_near_pitch, the padding 0.
+cudaError_t launch_ridge_map(const uint16_t* dist, Dims dm, const uint2* thr, uint16_t* rmap, cudaStream_t s,
                              unsigned long long* launches);
 // Disc lists: hdr[patch] = count | reach << 16 for every 32 x 8 patch of every
 // plane (disc_header_count), its discs {R << 16 | rho, column | (first row +

@@ -69,3 +69,18 @@ def test_sites_outside_the_first_word(gpu_ctx, w, tiles):
     finally:
         gpu_ctx.set_fill_tile_rows(0)
     assert np.array_equal(got.view(np.uint32), O.local_thickness(vol, 0).thickness.view(np.uint32))
+
+
+@pytest.mark.parametrize("shape", [(5, 6, 15), (4, 9, 16), (7, 5, 17), (9, 7, 59), (5, 33, 60), (6, 4, 61), (33, 8, 119),
+                                   (35, 5, 121), (70, 9, 31), (75, 71, 66), (131, 20, 15)])
+def test_ridge_of_pairs_bitwise(gpu_ctx, shape):
+    """Ridge map at the edges of its 60-voxel warps and padded rows; the last two
+    shapes hold squared distances beyond 65^2 (16-bit map from flagged lines)."""
+    vol = noise(shape, 0.9, sum(shape))
+    if shape[0] > 70:
+        vol[:] = 1
+        vol[0, 0, shape[2] - 1] = 0
+    got, sq = local_thickness(vol, Phase.FOREGROUND, ctx=gpu_ctx, return_squared=True)
+    ref = O.local_thickness(vol, 0)
+    assert np.array_equal(sq, ref.propagated)
+    assert np.array_equal(got.view(np.uint32), ref.thickness.view(np.uint32))
