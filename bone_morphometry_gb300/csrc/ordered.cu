@@ -46,11 +46,15 @@
 // reference's loop is serial (metrics.rs:215-226).
 //
 // Per map, against an earlier form (a serial fold per chunk, a one-CTA scan, a
-// one-warp walker that went through the levels): 0.08 against 0.22 ms on
-// 64 x 56 x 72, 0.30 against 0.50 ms on 33.5 M values, 0.64 against 0.90 ms on
+// one-warp walker that went through the levels): 0.07 against 0.22 ms on
+// 64 x 56 x 72, 0.29 against 0.50 ms on 33.5 M values, 0.63 against 0.90 ms on
 // 512^3.  The second step is bound by the integer ALU pipe, the walker by the
-// latency of its replays (about 1.5 us each; 3.7 us by one warp of 8 values a
-// lane).
+// latency of its replays, some thousand cycles a round of which the 64-bit
+// shifts that make the increments are the largest part.  128^3, bone and marrow
+// phase: 84 and 97 thousand cycles for the sum, 104 and 127 for the squares; 110
+// and 125, 118 and 146 with a round of four barriers per binade of a chunk and a
+// reduction per run of predicted chunks.  The chunks' values in shared memory
+// beforehand gave nothing.
 #include <climits>
 #include <cstdint>
 
@@ -608,97 +612,166 @@ __global__ void __launch_bounds__(256) osum_level_kernel(Level s_in, Level q_in,
   }
 }
 
-// Shared memory of a replay.
+// What a run of values adds to a state in units of its binade's ulp, when the
+// state is even (inc) and when it is odd (inc + d, d = (int)w >> 2); bits 0 and
+// 1 of w: the parity after it.
+struct Step {
+  unsigned long long inc;
+  uint32_t w;
+};
+
+constexpr uint32_t kStay = 2u;  // w of a run that adds nothing
+
+__device__ __forceinline__ unsigned long long after_step(unsigned long long u, const Step& f) {
+  return u + f.inc + (unsigned long long)((u & 1ull) ? (long long)((int)f.w >> 2) : 0ll);
+}
+
+__device__ __forceinline__ Step then(const Step& f, const Step& g) {
+  const int d = (int)g.w >> 2, d0 = f.w & 1u ? d : 0, d1 = f.w & 2u ? d : 0;
+  const uint32_t o0 = (g.w >> (f.w & 1u)) & 1u, o1 = (g.w >> ((f.w >> 1) & 1u)) & 1u;
+  return Step{f.inc + g.inc + (unsigned long long)(long long)d0,
+              ((uint32_t)(((int)f.w >> 2) + d1 - d0) << 2) | (o1 << 1) | o0};
+}
+
+// Inclusive scan over the warp.
+__device__ __forceinline__ void scan_steps(Step& f, int lane) {
+#pragma unroll 1
+  for (int o = 1; o < 32; o <<= 1) {
+    const Step g{__shfl_up_sync(0xffffffffu, f.inc, o), __shfl_up_sync(0xffffffffu, f.w, o)};
+    if (lane >= o) f = then(g, f);
+  }
+}
+
+// Shared memory of a replay; the halves are used in turn.
 struct Replay {
-  unsigned long long total[kChunk / 32];
-  uint32_t parity[kChunk / 32];
-  int first;
-  unsigned long long units;
-  double s;
+  unsigned long long total[2][2][kChunk / 32];  // of the warps' values, in the state's binade and in the next
+  uint32_t ties[2][kChunk / 32];                // bit 0: a tie in the state's binade, bit 1: in the next
+  Step step[kChunk / 32];                       // the warps' values with their ties
+  unsigned long long rest[2];
+  double s[2];
+  int next[2];
+  uint32_t has[kChunk / 32];
+  double first;
 };
 
 // Replays chunk c from state s exactly as the reference adds, by a CTA of kChunk
 // threads that all hold s, a value per thread.  In s's binade every value is an
 // increment; a scan of them gives the state after each value, and the first
 // value that leaves the binade (or the first value at all, s = 0) is added with
-// an f64 addition, the reference's own operation (metrics.rs:223-224); the
-// values after it go on in the new binade.  A tie is rounded to even by the
-// parity before it, from a scan of its own: a value flips the parity or, after
-// a tie, leaves it even.
+// an f64 addition, the reference's own operation (metrics.rs:223-224).  The
+// values after it go on in the next binade, whose increments are scanned beside
+// the first ones: a chunk with one crossing and no tie takes one round of two
+// barriers.  An increment that is a tie depends on the parity before it: where
+// there are any, the warps scan their values as functions of the parity.
 __device__ __noinline__ double replay_chunk(const float* __restrict__ map, long long n, float scale, bool sq,
                                             long long c, double s, Replay& sh) {
+  constexpr int kWarps = kChunk / 32;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const long long at = c * kChunk + tid;
   const float raw = at < n ? map[at] : 0.0f;
   const Term t = term(raw, scale, sq);
-  const bool has = t.M != 0ull, inf = t.k == INT_MAX;
-  const double x = has ? term_value(raw, scale, sq) : 0.0;
-  for (int start = 0; start < kChunk;) {  // the first value not yet added
-    if (!isfinite(s)) return s;           // +inf stays +inf
-    int b;                                // the value added in f64
-    double before = s;
-    if (s == 0.0) {
-      if (tid == 0) sh.first = kChunk;
-      __syncthreads();
-      if (has && tid >= start) atomicMin(&sh.first, tid);
-      __syncthreads();
-      b = sh.first;
-      if (b == kChunk) return s;
-    } else {
-      const int E = binade_of(s), sft = E - 52 - (inf ? 0 : t.k);
-      const unsigned long long u0 = units_of(s);
-      unsigned long long inc = 0;
-      bool tie = false;
-      if (has && tid >= start) {
-        if (inf || sft <= -54 || (sft < 0 && (t.M >> (54 + sft)) != 0ull)) {
-          inc = kSat;  // leaves the binade
-        } else if (sft <= 0) {
-          inc = t.M << -sft;
-        } else if (sft <= 48) {
-          const unsigned long long rem = t.M & ((1ull << sft) - 1ull), half = 1ull << (sft - 1);
-          tie = rem == half;
-          inc = (t.M >> sft) + (rem > half ? 1ull : 0ull);
-        }
-      }
-      if (__syncthreads_or(tie)) {
-        // bit 1: the parity is set (to bit 0), else flipped by bit 0
-        auto then = [](uint32_t f, uint32_t g) { return g & 2u ? g : (f & 2u) | ((f ^ g) & 1u); };
-        uint32_t f = tie ? 2u : (uint32_t)(inc & 1ull);
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const uint32_t g = __shfl_up_sync(0xffffffffu, f, o);
-          if (lane >= o) f = then(g, f);
-        }
-        if (lane == 31) sh.parity[warp] = f;
-        __syncthreads();
-        uint32_t p = 2u | (uint32_t)(u0 & 1ull);  // the parity before the warp
-        for (int w = 0; w < warp; ++w) p = then(p, sh.parity[w]);
-        const uint32_t g = __shfl_up_sync(0xffffffffu, f, 1);
-        if (lane > 0) p = then(p, g);
-        if (tie) inc += (inc + p) & 1ull;
-      }
-      unsigned long long incl = inc;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long g = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += g;
-      }
-      if (lane == 31) sh.total[warp] = incl;
-      __syncthreads();
-      unsigned long long after = u0 + incl;
-      for (int w = 0; w < warp; ++w) after += sh.total[w];
-      b = __syncthreads_count(after <= kTwo53);  // the states only grow
-      if (b == kChunk) {
-        if (tid == kChunk - 1) sh.units = after;
-        __syncthreads();
-        return from_units(sh.units, E);
-      }
-      before = from_units(after - inc, E);
-    }
-    if (tid == b) sh.s = __dadd_rn(before, x);
+  const bool inf = t.k == INT_MAX;
+  int start = 0;     // the first value not yet added
+  __syncthreads();   // the last replay's results have been read
+  if (s == 0.0) {
+    const unsigned has = __ballot_sync(0xffffffffu, t.M != 0ull);
+    if (lane == 0) sh.has[warp] = has;
     __syncthreads();
-    s = sh.s;
+    int b = kChunk;
+#pragma unroll
+    for (int w = kWarps - 1; w >= 0; --w)
+      if (sh.has[w]) b = w * 32 + __ffs(sh.has[w]) - 1;
+    if (b == kChunk) return s;
+    if (tid == b) sh.first = term_value(raw, scale, sq);
+    __syncthreads();
+    s = sh.first;
     start = b + 1;
+  }
+#pragma unroll 1
+  for (int turn = 0; start < kChunk; turn ^= 1) {
+    if (!isfinite(s)) return s;  // +inf stays +inf
+    const int E = binade_of(s), sft = E - 52 - (inf ? 0 : t.k);
+    // a, and what is left below it: nothing, less than, exactly or more than half an ulp
+    unsigned long long a = 0;
+    bool left = false, tie = false;
+    uint32_t up = 0;
+    if (t.M != 0ull && tid >= start) {
+      if (inf || sft <= -54 || (sft < 0 && (t.M >> (54 + sft)) != 0ull)) {
+        a = kSat;  // leaves the binade
+      } else if (sft <= 0) {
+        a = t.M << -sft;
+      } else if (sft <= 48) {
+        a = t.M >> sft;
+        const unsigned long long rem = t.M << (64 - sft);  // M < 2^48: at the top of 64 bits
+        left = rem != 0ull;
+        tie = rem == 1ull << 63;
+        up = rem > 1ull << 63 ? 1u : 0u;
+      } else {
+        left = true;
+      }
+    }
+    const uint32_t odd = (uint32_t)a & 1u;
+    unsigned long long f = a + up, g = (a >> 1) + (odd && left ? 1u : 0u);
+    const uint32_t ties =
+        (__any_sync(0xffffffffu, tie) ? 1u : 0u) | (__any_sync(0xffffffffu, odd && !left) ? 2u : 0u);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long f2 = __shfl_up_sync(0xffffffffu, f, o), g2 = __shfl_up_sync(0xffffffffu, g, o);
+      if (lane >= o) {
+        f += f2;
+        g += g2;
+      }
+    }
+    if (lane == 31) {
+      sh.total[turn][0][warp] = f;
+      sh.total[turn][1][warp] = g;
+      sh.ties[turn][warp] = ties;
+    }
+    __syncthreads();
+    uint32_t all = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) all |= sh.ties[turn][w];
+    Step own{f, kStay};
+    if (all & 1u) {
+      const unsigned long long inc = a + up;
+      const uint32_t p = (uint32_t)(inc & 1ull);
+      own = tie ? (p ? Step{inc + 1ull, (uint32_t)-4} : Step{inc, 4u}) : Step{inc, p | ((p ^ 1u) << 1)};
+      scan_steps(own, lane);
+      if (lane == 31) sh.step[warp] = own;
+      __syncthreads();
+    }
+    unsigned long long u = units_of(s), before = 0;
+    int wb = -1;  // the warp whose values leave the binade: the states only grow
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      const unsigned long long v = all & 1u ? after_step(u, sh.step[w]) : u + sh.total[turn][0][w];
+      if (wb < 0 && v > kTwo53) {
+        wb = w;
+        before = u;
+      }
+      u = v;
+    }
+    if (wb < 0) return from_units(u, E);
+    if (warp == wb) {
+      const unsigned long long after = all & 1u ? after_step(before, own) : before + f;
+      const int b = __popc(__ballot_sync(0xffffffffu, after <= kTwo53));
+      const unsigned long long prev = __shfl_up_sync(0xffffffffu, after, 1);
+      if (lane == b) {
+        sh.s[turn] = __dadd_rn(from_units(lane ? prev : before, E), term_value(raw, scale, sq));
+        sh.next[turn] = wb * 32 + b + 1;
+        sh.rest[turn] = sh.total[turn][1][wb] - g;
+      }
+    }
+    __syncthreads();
+    s = sh.s[turn];
+    start = sh.next[turn];
+    if (!(all & 2u) && isfinite(s) && binade_of(s) == E + 1) {
+      u = units_of(s) + sh.rest[turn];
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w)
+        if (w > wb) u += sh.total[turn][1][w];
+      if (u <= kTwo53) return from_units(u, E + 1);
+    }
   }
   return s;
 }
@@ -710,6 +783,30 @@ __device__ __noinline__ double replay_chunk(const float* __restrict__ map, long 
 // (lane j: chunk c0 + j; identity past the map's end), from lane p to lane e.
 __device__ __noinline__ double walk_block(const float* __restrict__ map, long long n, float scale, bool sq,
                                           long long c0, const Fn& f, int p, int e, double s, int lane, Replay& sh) {
+  // the runs between unpredicted chunks, composed at once: run's lane t holds
+  // the chunks from the one after the last unpredicted before t (or p) up to t
+  const unsigned bad = __ballot_sync(0xffffffffu, f.meta == 0u);
+  const unsigned upto = bad & ((2u << lane) - 1u);
+  const int first = max(p, upto ? 32 - __clz(upto) : 0);
+  Fn run = first <= lane ? f : fn_identity();
+#pragma unroll 1
+  for (int o = 1; o < 32; o <<= 1) {
+    const Fn g = shfl_fn(run, lane - o);
+    if (lane - o >= first) run = compose(g, run);
+  }
+  while (p <= e) {
+    if (!isfinite(s)) break;
+    const unsigned next = bad >> p;  // p <= 31
+    const int q = min(next ? p + __ffs(next) - 1 : 32, e + 1);  // chunks p .. q - 1 are predicted
+    if (q > p) {
+      if (!apply_fn(shfl_fn(run, q - 1), s)) break;
+      p = q;
+      continue;
+    }
+    s = replay_chunk(map, n, scale, sq, c0 + p, s, sh);
+    ++p;
+  }
+  // where a prediction does not hold
   while (p <= e) {
     if (!isfinite(s)) break;
     const int E = s == 0.0 ? INT_MIN : binade_of(s);
