@@ -41,8 +41,6 @@ __device__ __forceinline__ uint32_t floor_sqrt(uint32_t t) {
   return __float_as_uint(__fadd_rz(f * r, 8388608.0f)) & 0x7fffffu;
 }
 
-__device__ __forceinline__ uint32_t max3(uint32_t a, uint32_t b, uint32_t c) { return max(max(a, b), c); }
-
 // ---- ridge map --------------------------------------------------------------
 // Distance ridge (local_thickness.rs:104-167) as a u16 map: twice the squared
 // distance (0 for a non-selected voxel), plus 1 for a ridge voxel.  Two
@@ -415,6 +413,13 @@ constexpr int kPaintAhead = 2;             // entries a lane loads at a time
 static_assert(kPaintAhead == 2, "the loop below picks one of two");
 constexpr int kQueue = 64;                 // discs a warp holds back until 32 are ready
 
+// Bound by issue (66 to 76 % of the cycles at two CTAs an SM).  Of a 64-row tile's
+// warp instructions about half are chords in the marrow phase of the 512^3
+// generator, an eighth in the bone phase; the rest is per tile and list, so
+// lists are taken without divisions or empty halves and the levels pushed down
+// two voxels at a time: both phases of 512^3 4.04 -> 3.88 ms.  Cutting the discs'
+// rows at the columns to the sides too leaves 17 % fewer of them, which saved
+// the painting 0.24 ms and cost the lists 0.28.
 template <int TY>
 __global__ void __launch_bounds__(8 * TY, 64 / TY * 2)
 disc_paint_kernel(const uint32_t* __restrict__ hdr, const uint2* __restrict__ ent, const uint2* __restrict__ pool,
@@ -440,14 +445,14 @@ disc_paint_kernel(const uint32_t* __restrict__ hdr, const uint2* __restrict__ en
   const long long zh = (long long)z * npx * npy;
   if (tid == 0) s_patches = s_discs = s_units = s_next = 0u;
   __syncthreads();
-  // the patches whose discs reach the tile: index << 16 | count
+  // the patches whose discs reach the tile: place << 16 | count
   for (int i = tid; i < nh; i += kPaintThreads) {
-    const int px = px0 + i % nhx, py = py0 + i / nhx;
+    const int ry = i / nhx, rx = i - ry * nhx, px = px0 + rx, py = py0 + ry;
     const uint32_t h = __ldg(hdr + zh + (long long)py * npx + px);
     const int reach = (int)(h >> 16), bx = px * kDiscPX, by = py * kDiscPY;
     if (h != 0u && bx - reach <= x0 + kPaintX - 1 && bx + kDiscPX - 1 + reach >= x0 && by - reach <= y0 + TY - 1 &&
         by + kDiscPY - 1 + reach >= y0) {
-      s_list[atomicAdd(&s_patches, 1u)] = ((uint32_t)i << 16) | (h & 0xffffu);
+      s_list[atomicAdd(&s_patches, 1u)] = ((uint32_t)(ry << 8 | rx) << 16) | (h & 0xffffu);
       atomicAdd(&s_discs, h & 0xffffu);
     }
   }
@@ -495,7 +500,7 @@ disc_paint_kernel(const uint32_t* __restrict__ hdr, const uint2* __restrict__ en
         const uint32_t u = s_unit[next], item = s_list[u >> 16];
         e0 = (u & 0xffffu) * unit;
         count = min(e0 + unit, item & 0xffffu);
-        const int px = px0 + (int)(item >> 16) % nhx, py = py0 + (int)(item >> 16) / nhx;
+        const int px = px0 + (int)((item >> 16) & 255u), py = py0 + (int)(item >> 24);
         list = ent + (zh + (long long)py * npx + px) * kDiscSlots;
         if ((item & 0xffffu) > kDiscSlots) list = pool + __ldg(list).x;
         bx = px * kDiscPX - x0;
@@ -510,8 +515,10 @@ disc_paint_kernel(const uint32_t* __restrict__ hdr, const uint2* __restrict__ en
       e[j] = i < count ? __ldg(list + i) : make_uint2(0u, 0u);
     }
     e0 += 32 * kPaintAhead;
+    // (one round more than the unit has, with nothing in it, where the queue is to be emptied)
+    const int rounds = done ? 1 : count + 32 * kPaintAhead - e0 > 32 ? 2 : 1;
 #pragma unroll 1
-    for (int j = 0; j < kPaintAhead; ++j) {
+    for (int j = 0; j < rounds; ++j) {
       const uint2 d = j ? e[1] : e[0];
       const int cx = bx + (int)(d.y & 31u), cy = by + (int)((d.y >> 5) & 7u);
       const int r = (int)floor_sqrt(d.x & 0xffffu);
@@ -583,19 +590,19 @@ disc_paint_kernel(const uint32_t* __restrict__ hdr, const uint2* __restrict__ en
   // the two cells of level k - 1 at its own place and 2^(k-1) further
   for (int y = warp; y < vy; y += kPaintWarps) {
     const uint32_t* row = lev + y * kPaintStride;
-    uint32_t a = 0u, b = 0u;  // voxels lane and lane + 32
+    uint32_t v = 0u;  // voxels lane (low half) and lane + 32: squared radii fit 16 bits
     for (int k = kmax; k >= 0; --k) {
       const uint32_t* lk = row + k * kPlane;
-      const int s = 1 << k;  // the shift of level k + 1's second cell
-      uint32_t sa = 0u, sb = 0u;
+      const uint32_t own = lk[lane] | (lk[lane + 32] << 16);
+      uint32_t moved = 0u;
       if (k < kmax) {
-        const uint32_t ra = __shfl_sync(0xffffffffu, a, (lane - s) & 31), rb = __shfl_sync(0xffffffffu, b, (lane - s) & 31);
-        sa = lane >= s ? ra : 0u;
-        sb = lane >= s ? rb : ra;
+        const int s = 1 << k;  // the shift of level k + 1's second cell
+        moved = __shfl_sync(0xffffffffu, v, (lane - s) & 31);
+        if (lane < s) moved <<= 16;  // voxel lane + 32 - s
       }
-      a = max3(a, sa, lk[lane]);
-      b = max3(b, sb, lk[lane + 32]);
+      v = __vimax3_u16x2(v, moved, own);
     }
+    const uint32_t a = v & 0xffffu, b = v >> 16;
     const long long at = (long long)y * dm.w + lane;
     if (lane < vx) {
       out[at] = __ldg(dia + a);
