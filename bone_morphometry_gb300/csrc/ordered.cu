@@ -438,6 +438,21 @@ __device__ __noinline__ FnPair ordered_fold(const float* __restrict__ map, long 
                 shfl_fn(warp_reduce_fn(acc_fn(q, has, eq), lane), 0)};
 }
 
+// v << n, 0 for n >= 32.
+__device__ __forceinline__ uint32_t shifted_left(uint32_t v, uint32_t n) {
+  uint32_t r;
+  asm("shl.b32 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(n));
+  return r;
+}
+
+// Sum over the warp (modulo 2^64), in parts whose sums fit 32 bits.
+__device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
+  const uint32_t lo = (uint32_t)v, hi = (uint32_t)(v >> 32);
+  const uint32_t a = __reduce_add_sync(0xffffffffu, lo & 0xffffu), b = __reduce_add_sync(0xffffffffu, lo >> 16);
+  const uint32_t h = __reduce_add_sync(0xffffffffu, hi);
+  return a + ((unsigned long long)b << 16) + ((unsigned long long)h << 32);
+}
+
 // 2. Functions of every chunk, for both sums, and of every block.  One CTA per
 // block; a chunk without values is not read again.
 template <int CPW>
@@ -512,10 +527,13 @@ osum_fn_kernel(const float* __restrict__ map, long long n, float scale, long lon
     uint32_t bits[8], top = 0u, low = ~0u;
 #pragma unroll
     for (int t = 0; t < 8; ++t) {
-      const bool ok = v[t] > 0.0f && isfinite(v[t]);
+      const bool ok = __float_as_uint(v[t]) - 1u < 0x7f7fffffu;  // positive and finite
       bits[t] = ok ? __float_as_uint(__fmul_rn(v[t], scale)) : 0u;
-      top = max(top, bits[t]);
-      low = min(low, bits[t] - 1u);  // (the skipped ones go to the top)
+    }
+#pragma unroll
+    for (int t = 0; t < 8; t += 2) {
+      top = __vimax3_u32(top, bits[t], bits[t + 1]);
+      low = __vimin3_u32(low, bits[t] - 1u, bits[t + 1] - 1u);  // (the skipped ones go to the top)
     }
     top = __reduce_max_sync(0xffffffffu, top) >> 23;
     low = (__reduce_min_sync(0xffffffffu, low) + 1u) >> 23;
@@ -535,12 +553,15 @@ osum_fn_kernel(const float* __restrict__ map, long long n, float scale, long lon
       const uint32_t base = low << 23;
       odd = false;
       auto sum = [&](auto&& shift_q) {
+        uint32_t pair = 0;
 #pragma unroll
         for (int t = 0; t < 8; ++t) {
-          const uint32_t m = bits[t] ? ((bits[t] & 0x7fffffu) | 0x800000u) << ((bits[t] - base) >> 23) : 0u;
+          // (a skipped entry's 0 - base is shifted by 258 or more: 0)
+          const uint32_t m = shifted_left((bits[t] & 0x7fffffu) | 0x800000u, (bits[t] - base) >> 23);
           const uint32_t ta = m + half_a;
           odd = odd || (ta & mask_a) == tie_a;
-          A += ta >> ra;
+          if (t & 1) A += pair + (ta >> ra);  // each below 2^31
+          else pair = ta >> ra;
           shift_q((unsigned long long)m * m + half_q);
         }
       };
@@ -563,11 +584,8 @@ osum_fn_kernel(const float* __restrict__ map, long long n, float scale, long lon
       if (sha < 0) A <<= -sha;
     }
     if (!__any_sync(0xffffffffu, odd)) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        A += __shfl_xor_sync(0xffffffffu, A, o);
-        Q += __shfl_xor_sync(0xffffffffu, Q, o);
-      }
+      A = warp_sum(A);
+      Q = warp_sum(Q);
       fs = plain_fn(A, es);
       fq = plain_fn(Q, eq);
     } else {
