@@ -47,7 +47,7 @@
 //
 // Per map, against an earlier form (a serial fold per chunk, a one-CTA scan, a
 // one-warp walker that went through the levels): 0.07 against 0.22 ms on
-// 64 x 56 x 72, 0.29 against 0.50 ms on 33.5 M values, 0.63 against 0.90 ms on
+// 64 x 56 x 72, 0.26 against 0.50 ms on 33.5 M values, 0.51 against 0.90 ms on
 // 512^3.  The second step is bound by the integer ALU pipe, the walker by the
 // latency of its replays, some thousand cycles a round of which the 64-bit
 // shifts that make the increments are the largest part.  128^3, bone and marrow
@@ -238,8 +238,10 @@ __device__ __forceinline__ unsigned long long to_fixed(float x) {
 }
 
 constexpr int kSumLevels = 4;      // approximate sums: blocks, and groups of 32, 1024 and 32768 blocks
-// Chunks per warp (32 / CPW warps take the 32 chunks of a block): 4, or 1 for
-// maps of fewer than kSmallMap values, which are bound by a warp's latency.
+// Chunks per warp (32 / CPW warps take the 32 chunks of a block): 4 in the first
+// step and 8 in the second (4: 1.07 instead of 1.03 ms for the sums of both
+// phases of 512^3), or 1 for maps of fewer than kSmallMap values, which are bound
+// by a warp's latency.
 constexpr long long kSmallMap = 1ll << 22;
 constexpr float kEmptyChunk = -0.0f;  // approximate sum of a chunk without values (others have no sign)
 
@@ -461,6 +463,8 @@ osum_fn_kernel(const float* __restrict__ map, long long n, float scale, long lon
                const uint32_t* __restrict__ maxbits, const float* __restrict__ cs, const float* __restrict__ cq,
                Sums sums, Walk ws, Walk wq) {
   __shared__ Fn sh[2][32];
+  __shared__ int binade[2][32];
+  static_assert(CPW <= 16, "two warps predict");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long blk = blockIdx.x, b0 = blk * 32;
   const float my_s = b0 + lane < nchunks ? cs[b0 + lane] : kEmptyChunk;
@@ -485,26 +489,26 @@ osum_fn_kernel(const float* __restrict__ map, long long n, float scale, long lon
   };
   float next[8];
   load(0, next);
-  // lane j: chunk j's predicted binades
-  int es_mine = INT_MIN, eq_mine = INT_MIN;
-  if (filled) {
-    const unsigned long long as = to_fixed(my_s), aq = b0 + lane < nchunks ? to_fixed(cq[b0 + lane]) : 0ull;
-    unsigned long long ps = as, pq = aq;  // inclusive scan within the block
+  // the chunks' predicted binades: those of the sum by warp 0, of the squares by warp 1
+  if (warp < 2) {
+    int e = INT_MIN;
+    if (filled) {
+      const float* approx = warp ? cq : cs;
+      const unsigned long long mine = b0 + lane < nchunks ? to_fixed(approx[b0 + lane]) : 0ull;
+      unsigned long long p = mine;  // inclusive scan within the block
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned long long us = __shfl_up_sync(0xffffffffu, ps, o), uq = __shfl_up_sync(0xffffffffu, pq, o);
-      if (lane >= o) {
-        ps += us;
-        pq += uq;
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long u = __shfl_up_sync(0xffffffffu, p, o);
+        if (lane >= o) p += u;
       }
+      p += prefix_of(warp ? sums.q : sums.s, blk, lane);
+      // the approximate sums are of values scaled by 2^(127 - ef): undo it in the binade
+      const int shift = max_exponent_field(*maxbits) - 127;
+      e = predict(p - mine, p, warp ? 2 * shift : shift);
     }
-    ps += prefix_of(sums.s, blk, lane);
-    pq += prefix_of(sums.q, blk, lane);
-    // the approximate sums are of values scaled by 2^(127 - ef): undo it in the binade
-    const int shift = max_exponent_field(*maxbits) - 127;
-    es_mine = predict(ps - as, ps, shift);
-    eq_mine = predict(pq - aq, pq, 2 * shift);
+    binade[warp][lane] = e;
   }
+  __syncthreads();
 #pragma unroll 1
   for (int j = 0; j < CPW; ++j) {
     float v[8];
@@ -522,7 +526,7 @@ osum_fn_kernel(const float* __restrict__ map, long long n, float scale, long lon
       }
       continue;
     }
-    const int es = __shfl_sync(0xffffffffu, es_mine, c), eq = __shfl_sync(0xffffffffu, eq_mine, c);
+    const int es = binade[0][c], eq = binade[1][c];
     // M = 0 (an increment of 0) for the entries that are skipped
     uint32_t bits[8], top = 0u, low = ~0u;
 #pragma unroll
@@ -1103,7 +1107,7 @@ cudaError_t launch_ordered_sums(const float* map, long long n, float scale, cons
     osum_fn_kernel<1><<<blocks, 1024, 0, s>>>(map, n, scale, nchunks, maxbits, p.cs, p.cq, p.sums, p.ws, p.wq);
   } else {
     osum_chunk_kernel<4><<<blocks, 256, 0, s>>>(map, n, scale, nchunks, maxbits, p.cs, p.cq, p.sums);
-    osum_fn_kernel<4><<<blocks, 256, 0, s>>>(map, n, scale, nchunks, maxbits, p.cs, p.cq, p.sums, p.ws, p.wq);
+    osum_fn_kernel<8><<<blocks, 128, 0, s>>>(map, n, scale, nchunks, maxbits, p.cs, p.cq, p.sums, p.ws, p.wq);
   }
   *launches += 3;
   for (int L = 2; L < p.ws.nlev; ++L) {
