@@ -334,6 +334,17 @@ void ordered_sums(bm_ctx* ctx, const float* d_map, long long n, float scale, Pha
   });
 }
 
+// The order statistics of the quantiles of d_map's finite positive values
+// (metrics.rs:242-288), whose number out->acc holds by then, and their readback.
+void queue_quantiles(bm_ctx* ctx, const float* d_map, long long n, const PhaseOut* out, cudaStream_t s) {
+  uint32_t* hist = static_cast<uint32_t*>(ensure(ctx, ctx->qhist, quantile_scratch_words() * 4, "quantile histograms"));
+  QuantileState* dq = static_cast<QuantileState*>(ensure(ctx, ctx->qtargets, sizeof(QuantileState), "quantile ranks"));
+  timed(ctx, KF_QUANTILE, s, "quantiles",
+        [&] { return launch_quantiles(d_map, n, &out->acc.count, hist, dq, s, &ctx->launches); });
+  check(ctx, cudaMemcpyAsync(&readback(ctx).quantile, dq, sizeof(QuantileState), cudaMemcpyDeviceToHost, s),
+        "quantile readback");
+}
+
 // One phase: EDT (+ local thickness unless edt_only, + the reference-order
 // statistics sums when stats).  d_a / d_b are the device inputs for `mode`;
 // results optionally go to d_edt (u32 EDT), d_map (f32 masked diameters) and
@@ -355,6 +366,7 @@ struct Phase {
   int mode;
   cudaStream_t s;
   bool edt_only = false, stats = false;
+  bool quantiles = false;  // needs d_map
   uint32_t* d_edt = nullptr;
   float* d_map = nullptr;
   uint32_t* d_sq = nullptr;
@@ -583,6 +595,7 @@ struct Phase {
       return launch_cleanup(dmap, selbits, nzbits, inbits, dm, scale, cmap, &out->acc, e_lo, s, &ctx->launches);
     });
     if (stats) ordered_sums(ctx, cmap, dm.n(), scale, out, s);
+    if (quantiles) queue_quantiles(ctx, cmap, dm.n(), out, s);
     check(ctx, cudaMemcpyAsync(&readback(ctx).out, out, sizeof(PhaseOut), cudaMemcpyDeviceToHost, s), "stats readback");
   }
 
@@ -648,42 +661,25 @@ int finish_stats(bm_ctx* ctx, const StatsAccum& a, const double* osum, bm_stats*
   return BM_OK;
 }
 
-// Quantiles of the finite positive values of d_map (metrics.rs:242-298):
-// median, P10, P25, P75, P90 by numpy-linear interpolation of exact order
-// statistics, then (q as f32 * scale_f32) as f64; IQR = P75 - P25.
-void quantiles(bm_ctx* ctx, const float* d_map, long long n, unsigned long long count, double scale,
-               bm_stats* out, cudaStream_t s) {
-  static const double kQ[5] = {0.5, 0.1, 0.25, 0.75, 0.9};  // metrics.rs:247-251
-  QuantileState& qs = readback(ctx).quantile;
-  qs = QuantileState{};
-  double frac[5];
-  for (int i = 0; i < 5; ++i) {
-    const double position = kQ[i] * (double)(count - 1);
-    const double lo = std::floor(position), hi = std::ceil(position);
-    qs.rank[2 * i] = (unsigned long long)lo;
-    qs.rank[2 * i + 1] = (unsigned long long)hi;
-    frac[i] = position - lo;
-  }
-  uint32_t* hist = static_cast<uint32_t*>(ensure(ctx, ctx->qhist, quantile_scratch_words() * 4, "quantile histograms"));
-  QuantileState* dq = static_cast<QuantileState*>(ensure(ctx, ctx->qtargets, sizeof(QuantileState), "quantile ranks"));
-  check(ctx, cudaMemcpyAsync(dq, &qs, sizeof qs, cudaMemcpyHostToDevice, s), "ranks upload");
-  timed(ctx, KF_QUANTILE, s, "quantiles", [&] { return launch_quantiles(d_map, n, hist, dq, s, &ctx->launches); });
-  check(ctx, cudaMemcpyAsync(&qs, dq, sizeof qs, cudaMemcpyDeviceToHost, s), "quantile readback");
-  check(ctx, cudaStreamSynchronize(s), "quantiles");
-  double v[kQuantileRanks];
-  for (int r = 0; r < kQuantileRanks; ++r) {
-    if (qs.bits[r] == 0xffffffffu)
-      fail(ctx, BM_ERR_CUDA, "quantile rank %llu beyond the %llu values", qs.rank[r], count);
-    float f;
-    std::memcpy(&f, &qs.bits[r], 4);
-    v[r] = (double)f;
-  }
+// Quantiles (metrics.rs:242-298) from the order statistics that queue_quantiles
+// left: median, P10, P25, P75, P90 by numpy-linear interpolation, then
+// (q as f32 * scale_f32) as f64; IQR = P75 - P25.
+void finish_quantiles(bm_ctx* ctx, const QuantileState& qs, unsigned long long count, double scale, bm_stats* out) {
   const float sf = (float)scale;
   double q[5];
   for (int i = 0; i < 5; ++i) {
-    const double lv = v[2 * i], uv = v[2 * i + 1];
-    const double qv = lv + frac[i] * (uv - lv);  // metrics.rs:289
-    q[i] = (double)((float)qv * sf);             // metrics.rs:290
+    unsigned long long rank[2];
+    const double frac = quantile_ranks(i, count, &rank[0], &rank[1]);
+    double v[2];
+    for (int j = 0; j < 2; ++j) {
+      const uint32_t bits = qs.bits[2 * i + j];
+      if (bits == 0xffffffffu) fail(ctx, BM_ERR_CUDA, "quantile rank %llu beyond the %llu values", rank[j], count);
+      float f;
+      std::memcpy(&f, &bits, 4);
+      v[j] = (double)f;
+    }
+    const double qv = v[0] + frac * (v[1] - v[0]);  // metrics.rs:289
+    q[i] = (double)((float)qv * sf);                // metrics.rs:290
   }
   out->median = q[0];
   out->percentile_10 = q[1];
@@ -700,12 +696,13 @@ int nonzero_stats_impl(bm_ctx* ctx, const float* d_values, size_t n, double scal
   timed(ctx, KF_QUANTILE, s, "moments kernel",
         [&] { return launch_moments(d_values, (long long)n, (float)scale, &po->acc, s, &ctx->launches); });
   ordered_sums(ctx, d_values, (long long)n, (float)scale, po, s);
+  if (flags & BM_FLAG_QUANTILES) queue_quantiles(ctx, d_values, (long long)n, po, s);
   PhaseOut& r = readback(ctx).out;
   check(ctx, cudaMemcpyAsync(&r, po, sizeof(PhaseOut), cudaMemcpyDeviceToHost, s), "stats readback");
   check(ctx, cudaStreamSynchronize(s), "moments kernel");
   const int st = finish_stats(ctx, r.acc, r.osum, out);
   if (st) return st;
-  if (flags & BM_FLAG_QUANTILES) quantiles(ctx, d_values, (long long)n, r.acc.count, scale, out, s);
+  if (flags & BM_FLAG_QUANTILES) finish_quantiles(ctx, readback(ctx).quantile, r.acc.count, scale, out);
   return BM_OK;
 }
 
@@ -1050,9 +1047,9 @@ struct CallFence {
   }
 };
 
-int report_phase(Phase& p, bm_ctx* ctx, cudaStream_t s, bool want_q, const float* map, double spacing, bm_stats* out) {
+int report_phase(const Phase& p, bm_ctx* ctx, double spacing, bm_stats* out) {
   const int st = finish_stats(ctx, p.acc, p.osum, out);
-  if (st == BM_OK && want_q && out) quantiles(ctx, map, p.dm.n(), p.acc.count, spacing, out, s);
+  if (st == BM_OK && p.quantiles) finish_quantiles(ctx, readback(p.ctx).quantile, p.acc.count, spacing, out);
   return st;
 }
 
@@ -1077,6 +1074,8 @@ int tbth_phases(bm_ctx* ctx, const uint8_t* d_bone, const uint8_t* d_roi, Dims d
   Phase bone{ctx, dm, d_bone, d_roi, SEL_BONE_IN_ROI, s};
   Phase marrow{mctx, dm, d_bone, d_roi, SEL_MARROW_IN_ROI, tw ? tw->stream : s};
   bone.stats = marrow.stats = true;
+  bone.quantiles = want_q && th;
+  marrow.quantiles = want_q && sp;
   bone.scale = marrow.scale = (float)spacing;  // metrics.rs:213
   auto map_of = [&](bm_ctx* c, float* caller) {
     return caller || !want_q ? caller : static_cast<float*>(ensure(c, c->qmap, (size_t)N * 4, "quantile map"));
@@ -1098,12 +1097,12 @@ int tbth_phases(bm_ctx* ctx, const uint8_t* d_bone, const uint8_t* d_roi, Dims d
     bone.lists();
     bone.paint();
     bone.finish();
-    int st = report_phase(bone, ctx, s, want_q, bone.d_map, spacing, th);
+    int st = report_phase(bone, ctx, spacing, th);
     if (st) return st;
     marrow.d_map = map_of(ctx, d_spmap);
     run_phase(marrow);
     fence.done = true;
-    return report_phase(marrow, ctx, s, want_q, marrow.d_map, spacing, sp);
+    return report_phase(marrow, ctx, spacing, sp);
   }
   int twin_status = BM_OK;
   auto try_twin = [&](auto&& f) {
@@ -1153,7 +1152,7 @@ int tbth_phases(bm_ctx* ctx, const uint8_t* d_bone, const uint8_t* d_roi, Dims d
     if (!turns) try_twin([&] { marrow.lists(), marrow.paint(); });
     bone.finish();
   }
-  int st = report_phase(bone, ctx, s, want_q, bone.d_map, spacing, th);
+  int st = report_phase(bone, ctx, spacing, th);
   if (st) return st;
   if (marrow.separable && bone.separable) try_twin([&] { marrow.finish(); });
   if (twin_status != BM_OK) {
@@ -1161,7 +1160,7 @@ int tbth_phases(bm_ctx* ctx, const uint8_t* d_bone, const uint8_t* d_roi, Dims d
     throw CallError{twin_status};
   }
   fence.done = true;
-  return report_phase(marrow, ctx, s, want_q, marrow.d_map, spacing, sp);
+  return report_phase(marrow, ctx, spacing, sp);
 }
 
 int tbth_device_impl(bm_ctx* ctx, const uint8_t* d_bone, const uint8_t* d_roi, Dims dm, double spacing,

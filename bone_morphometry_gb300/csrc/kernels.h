@@ -2,6 +2,7 @@
 #pragma once
 
 #include <atomic>
+#include <cmath>
 
 #include "bm_internal.h"
 
@@ -206,7 +207,6 @@ cudaError_t launch_moments(const float* map, long long n, float scale, StatsAccu
 // 0xffffffff when there is none.  scratch: quantile_scratch_words() words.
 constexpr int kQuantileRanks = 10;
 struct QuantileState {
-  unsigned long long rank[kQuantileRanks];   // in
   unsigned long long resid[kQuantileRanks];  // rank inside its high bin
   uint32_t target[kQuantileRanks];           // the distinct high bins
   uint32_t slot[kQuantileRanks];             // each rank's index into target
@@ -214,7 +214,18 @@ struct QuantileState {
   uint32_t bits[kQuantileRanks];             // out
 };
 size_t quantile_scratch_words();
-cudaError_t launch_quantiles(const float* map, long long n, uint32_t* scratch, QuantileState* q, cudaStream_t s,
-                             unsigned long long* launches);
+// count: the number of positive finite values, known when the launch runs.
+cudaError_t launch_quantiles(const float* map, long long n, const unsigned long long* count, uint32_t* scratch,
+                             QuantileState* q, cudaStream_t s, unsigned long long* launches);
+// The two 0-based ranks that quantile i (median, P10, P25, P75, P90) of `count`
+// values lies between, and its place between them (metrics.rs:247-251, 278-288).
+__host__ __device__ inline double quantile_ranks(int i, unsigned long long count, unsigned long long* lo,
+                                                 unsigned long long* hi) {
+  const double p = i == 0 ? 0.5 : i == 1 ? 0.1 : i == 2 ? 0.25 : i == 3 ? 0.75 : 0.9;
+  const double position = p * (double)(count - 1), f = floor(position);
+  *lo = (unsigned long long)f;
+  *hi = (unsigned long long)ceil(position);
+  return position - f;
+}
 
 }  // namespace bm

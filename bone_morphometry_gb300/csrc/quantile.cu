@@ -138,11 +138,20 @@ __device__ __forceinline__ void find_ranks(const uint32_t* __restrict__ bins, in
 
 // High bins of the ranks: q->target = the distinct ones, q->slot / q->resid =
 // each rank's index into them and its rank inside the bin.
-__global__ void __launch_bounds__(1024) select_hi_kernel(const uint32_t* __restrict__ hist, QuantileState* q) {
+__global__ void __launch_bounds__(1024) select_hi_kernel(const uint32_t* __restrict__ hist,
+                                                         const unsigned long long* __restrict__ count,
+                                                         QuantileState* q) {
   __shared__ uint32_t bin[kQuantileRanks];
-  if (threadIdx.x < kQuantileRanks) bin[threadIdx.x] = 0xffffffffu;
+  __shared__ unsigned long long rank[kQuantileRanks];
+  if (threadIdx.x < kQuantileRanks) {
+    bin[threadIdx.x] = 0xffffffffu;
+    const unsigned long long n = *count;
+    unsigned long long r[2] = {~0ull, ~0ull};  // no such rank
+    if (n) quantile_ranks((int)threadIdx.x / 2, n, &r[0], &r[1]);
+    rank[threadIdx.x] = threadIdx.x & 1 ? r[1] : r[0];
+  }
   __syncthreads();
-  find_ranks<32>(hist, kHiBins, q->rank, kQuantileRanks, [&](int r, int b, unsigned long long resid) {
+  find_ranks<32>(hist, kHiBins, rank, kQuantileRanks, [&](int r, int b, unsigned long long resid) {
     bin[r] = (uint32_t)b;
     q->resid[r] = resid;
   });
@@ -325,8 +334,8 @@ cudaError_t launch_moments(const float* map, long long n, float scale, StatsAccu
 
 size_t quantile_scratch_words() { return (size_t)kHiBins + (size_t)kQuantileRanks * kLoBins; }
 
-cudaError_t launch_quantiles(const float* map, long long n, uint32_t* scratch, QuantileState* q, cudaStream_t s,
-                             unsigned long long* launches) {
+cudaError_t launch_quantiles(const float* map, long long n, const unsigned long long* count, uint32_t* scratch,
+                             QuantileState* q, cudaStream_t s, unsigned long long* launches) {
   const uint32_t* words = reinterpret_cast<const uint32_t*>(map);
   uint32_t* lo = scratch + kHiBins;
   const size_t hi_bytes = (size_t)kHiBins * sizeof(uint32_t);
@@ -335,7 +344,7 @@ cudaError_t launch_quantiles(const float* map, long long n, uint32_t* scratch, Q
     e = cudaFuncSetAttribute(hist_hi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hi_bytes);
   if (e != cudaSuccess) return e;
   hist_hi_kernel<<<ctas_for(n, 16384, 152), 1024, hi_bytes, s>>>(words, n, scratch);
-  select_hi_kernel<<<1, 1024, 0, s>>>(scratch, q);
+  select_hi_kernel<<<1, 1024, 0, s>>>(scratch, count, q);
   hist_lo_kernel<<<ctas_for(n, 8192, 152 * 4), 512, 0, s>>>(words, n, q, lo);
   select_lo_kernel<<<kQuantileRanks, 1024, 0, s>>>(lo, q);
   *launches += 4;
