@@ -28,9 +28,9 @@ __device__ __forceinline__ void each_four(const uint32_t* __restrict__ map, long
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x, nth = (long long)gridDim.x * blockDim.x;
   const bool vec = (reinterpret_cast<uintptr_t>(map) & 15u) == 0;
   const long long quads = (n + 3) / 4;
-  // whole warps stay together: f may use warp-wide operations
-  for (long long q0 = tid - (threadIdx.x & 31); q0 < quads; q0 += nth) {
-    const long long i = 4 * (q0 + (threadIdx.x & 31));
+  const int lane = threadIdx.x & 31;
+  auto load = [&](long long q0) {
+    const long long i = 4 * (q0 + lane);
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
     if (vec && i + 4 <= n) {
       v = __ldg(reinterpret_cast<const uint4*>(map + i));
@@ -40,7 +40,17 @@ __device__ __forceinline__ void each_four(const uint32_t* __restrict__ map, long
       if (i + 2 < n) v.z = map[i + 2];
       if (i + 3 < n) v.w = map[i + 3];
     }
+    return v;
+  };
+  // whole warps stay together: f may use warp-wide operations.  Two steps' words
+  // are in flight beside the one in hand.
+  const long long first = tid - lane;
+  uint4 v = load(first), next = load(first + nth);
+  for (long long q0 = first; q0 < quads; q0 += nth) {
+    const uint4 after = load(q0 + 2 * nth);
     f(v.x, v.y, v.z, v.w);
+    v = next;
+    next = after;
   }
 }
 
