@@ -239,10 +239,11 @@ __global__ void __launch_bounds__(1024) select_lo_kernel(const uint32_t* __restr
 // Exact moment sums of f32(raw * scale) over the finite positive raw values
 // (metrics.rs:215-226), same accumulator as the cleanup kernel.  A warp adds
 // its values in fixed point relative to the largest exponent it meets first
-// (span of 18 exponents, no atomics); values outside go to the block's
+// (span of 16 exponents: squares shifted by at most 30 bits, 78 bits each and 96
+// a thread, no atomics); values outside go to the block's
 // per-exponent sums one by one.  At the end the fixed-point totals are split
-// into the per-exponent sums too: 2^20 units of exponent e are one of e + 20.
-constexpr int kMomentSpan = 17;
+// into the per-exponent sums too: 2^15 units of exponent e are one of e + 15.
+constexpr int kMomentSpan = 15;
 
 __global__ void __launch_bounds__(256)
 moments_kernel(const uint32_t* __restrict__ map, long long n, float scale, StatsAccum* __restrict__ acc) {
@@ -255,20 +256,21 @@ moments_kernel(const uint32_t* __restrict__ map, long long n, float scale, Stats
     smax = 0;
   }
   __syncthreads();
-  unsigned long long cnt = 0, fx1 = 0;
-  unsigned __int128 fx2 = 0;
+  uint32_t thread_cnt = 0;
+  unsigned long long fx1 = 0;
+  uint32_t f0 = 0, f1 = 0, f2 = 0;  // the fixed-point sum of squares
   uint32_t mx = 0, base = 0;  // base: the exponent of the fixed-point unit (0: not chosen yet; the same in all lanes)
   each_four(map, n, [&](uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
     const uint32_t raw[4] = {a, b, c, d};
     uint32_t v[4];
-    uint32_t top = 0;
+    uint32_t top;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const bool ok = positive_finite(raw[j]);
       v[j] = ok ? __float_as_uint(__fmul_rn(__uint_as_float(raw[j]), scale)) : 0u;
-      cnt += ok;
-      top = max(top, v[j]);
+      thread_cnt += ok;
     }
+    top = __vimax3_u32(v[0], v[1], max(v[2], v[3]));
     mx = max(mx, top);
     if (base == 0u) {
       const uint32_t e = __reduce_max_sync(0xffffffffu, top) >> 23;
@@ -280,8 +282,11 @@ moments_kernel(const uint32_t* __restrict__ map, long long n, float scale, Stats
       const uint32_t s = e - base;
       const unsigned long long m2 = (unsigned long long)m * m;
       if (base && s <= (uint32_t)kMomentSpan) {
+        const uint32_t w0 = (uint32_t)m2, w1 = (uint32_t)(m2 >> 32), by = 2u * s;
         fx1 += (unsigned long long)m << s;
-        fx2 += (unsigned __int128)m2 << (2 * s);
+        asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, %5;"
+            : "+r"(f0), "+r"(f1), "+r"(f2)
+            : "r"(w0 << by), "r"(__funnelshift_l(w0, w1, by)), "r"(__funnelshift_l(w1, 0u, by)));
       } else if (m) {
         atomicAdd(&s1[e], (unsigned long long)m);
         atomicAdd(&sh[e], m2 >> 24);
@@ -289,7 +294,7 @@ moments_kernel(const uint32_t* __restrict__ map, long long n, float scale, Stats
       }
     }
   });
-  unsigned long long lo = (unsigned long long)fx2, hi = (unsigned long long)(fx2 >> 64);
+  unsigned long long cnt = thread_cnt, lo = (unsigned long long)f1 << 32 | f0, hi = f2;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     fx1 += __shfl_xor_sync(0xffffffffu, fx1, o);
@@ -304,8 +309,7 @@ moments_kernel(const uint32_t* __restrict__ map, long long n, float scale, Stats
     atomicAdd(&scount, cnt);
     atomicMax(&smax, mx);
     if (base) {
-      fx2 = ((unsigned __int128)hi << 64) | lo;
-      const unsigned __int128 rest = fx2 >> (2 * kMomentSpan);
+      const unsigned __int128 rest = (((unsigned __int128)hi << 64) | lo) >> (2 * kMomentSpan);
       atomicAdd(&s1[base], fx1 & ((1ull << kMomentSpan) - 1ull));
       atomicAdd(&s1[base + kMomentSpan], fx1 >> kMomentSpan);
       atomicAdd(&sl[base], lo & 0xffffffull);
