@@ -650,15 +650,16 @@ edt_window_tma_kernel(const __grid_constant__ CUtensorMap tin, uint32_t* __restr
 // up to kNearMax are exact too; it flags the lines that hold others, and the
 // 32-bit passes compute those (launch_edt_far).
 //
-// 512^3, 15 % foreground: 754 us with 32-bit passes, 476 here (x 121, y 129,
-// z 184; the maps' bytes alone take 260 at the copy rate, the rest is issue).
-// 417 x 333 x 379 (rows that no vector load fits): 726 us, 387 here (129, 102,
-// 119).  Where 36 to 94 % of the volume lies beyond 65 voxels of a site, so
+// 512^3, 15 % foreground: 754 us with 32-bit passes, 445 here (x 106, y 129,
+// z 172; the maps' bytes alone take 260 at the copy rate, the rest is issue).
+// 417 x 333 x 379 (rows that no vector load fits): 673 us, 381 here (125, 102,
+// 115).  Where 36 to 94 % of the volume lies beyond 65 voxels of a site, so
 // that the 32-bit passes run as well, 1.23-2.70 ms before and 1.18-2.68 here.
 constexpr uint32_t kNearMax = (kWinHalo + 1) * (kWinHalo + 1);
 constexpr uint32_t kFar16 = 40000;
-constexpr int kReach = 190;
+constexpr int kReach = 190, kReachWords = 6;
 constexpr uint32_t kPair = 0x10001u;
+static_assert(32 * kReachWords >= kReach, "a site beyond the words looked at is at least kReach away");
 static_assert((kReach + 7) * (kReach + 7) <= (int)kFar16 && kReach * kReach > (int)kNearMax, "far rows stay far");
 static_assert(kFar16 + (kWinHalo + 6) * (kWinHalo + 6) < 65536, "the window scan adds distance^2 to kFar16");
 
@@ -675,9 +676,7 @@ edt_x_near_kernel(const uint8_t* __restrict__ a, const uint8_t* __restrict__ b, 
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int nw = dm.nw();
-  uint32_t* mask = smem + (size_t)warp * 3 * nw;
-  int* lastpos = reinterpret_cast<int*>(mask + nw);
-  int* firstpos = lastpos + nw;
+  uint32_t* mask = smem + (size_t)warp * nw;  // the row's sites
   const long long rows = (long long)dm.h * dm.d;
   const bool two = MODE == SEL_BONE_IN_ROI || MODE == SEL_MARROW_IN_ROI;
   unsigned long long sites = 0;
@@ -754,7 +753,6 @@ edt_x_near_kernel(const uint8_t* __restrict__ a, const uint8_t* __restrict__ b, 
       }
     }
     __syncwarp();
-    x_row_scans(mask, lastpos, firstpos, nw, lane);
     const int bit = (lane & 3) * 8;  // first bit of this lane's voxels in their word
     const uint32_t below = (1u << bit) - 1u, above = ~((2u << (bit + 7)) - 1u);  // bit + 7 = 31: above = 0
     uint4* orow = reinterpret_cast<uint4*>(out + row * pitch);
@@ -764,9 +762,14 @@ edt_x_near_kernel(const uint8_t* __restrict__ a, const uint8_t* __restrict__ b, 
       if (x < dm.w) {
         const int c = x >> 5;
         const uint32_t m = mask[c];
-        const uint32_t lo = m & below, hi = m & above;
-        const int left = lo ? c * 32 + 31 - __clz(lo) : (c > 0 ? lastpos[c - 1] : kNoLeft);
-        const int right = hi ? c * 32 + __ffs(hi) - 1 : (c + 1 < nw ? firstpos[c + 1] : kNoRight);
+        // the nearest site on either side, no further than kReachWords words away
+        uint32_t lo = m & below, hi = m & above;
+        int cl = c, cr = c;
+#pragma unroll 1
+        while (lo == 0u && cl > max(c - kReachWords, 0)) lo = mask[--cl];
+#pragma unroll 1
+        while (hi == 0u && cr < min(c + kReachWords, nw - 1)) hi = mask[++cr];
+        const int left = lo ? cl * 32 + 31 - __clz(lo) : kNoLeft, right = hi ? cr * 32 + __ffs(hi) - 1 : kNoRight;
         const uint32_t dl = (uint32_t)min(x - left, kReach) * kPair, dr = (uint32_t)min(right - x - 7, kReach) * kPair;
         const uint4 in8 = s_inside[(m >> bit) & 0xffu];
         auto square = [&](uint32_t inside, uint32_t i) {  // of voxels i and i + 1 of the eight
@@ -834,7 +837,7 @@ __device__ __forceinline__ uint32_t near_group(const uint32_t* col, int m, int h
 // in: pairs; strides in pairs.  WIDE: the 32-bit result at the volume's own
 // pitch, else pairs again.
 template <bool Z, bool WIDE>
-__global__ void __launch_bounds__(kWinThreads)
+__global__ void __launch_bounds__(kWinThreads, 6)
 edt_near_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, int n, long long stride, int pairs,
                 long long outer, int nxt, int nchunk, int w, long long out_stride, uint8_t* __restrict__ redo,
                 Counters* __restrict__ ctr) {
@@ -1185,14 +1188,10 @@ template <int MODE>
 cudaError_t launch_edt_x_near_mode(const uint8_t* a, const uint8_t* b, Dims dm, uint16_t* out, uint32_t* selbits,
                                    Counters* ctr, unsigned blocks, cudaStream_t s) {
   const bool two = MODE == SEL_BONE_IN_ROI || MODE == SEL_MARROW_IN_ROI;
-  const size_t smem = (size_t)kXWarps * 3 * dm.nw() * sizeof(uint32_t);
+  const size_t smem = (size_t)kXWarps * dm.nw() * sizeof(uint32_t);  // at most 32 KB, beside the table's 4
   const bool vec = dm.w % 16 == 0 && (reinterpret_cast<uintptr_t>(a) & 15u) == 0 &&
                    (!two || (reinterpret_cast<uintptr_t>(b) & 15u) == 0);
   auto kernel = vec ? edt_x_near_kernel<MODE, true> : edt_x_near_kernel<MODE, false>;
-  if (smem > 44 * 1024) {  // with the table's 4 KB
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kXMaxSmem);
-    if (e != cudaSuccess) return e;
-  }
   kernel<<<blocks, kXWarps * 32, smem, s>>>(a, b, dm, edt_near_pitch(dm.w), out, selbits, ctr);
   return cudaGetLastError();
 }
