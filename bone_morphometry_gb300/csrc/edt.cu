@@ -652,8 +652,8 @@ edt_window_tma_kernel(const __grid_constant__ CUtensorMap tin, uint32_t* __restr
 //
 // 512^3, 15 % foreground: 754 us with 32-bit passes, 445 here (x 106, y 129,
 // z 172; the maps' bytes alone take 260 at the copy rate, the rest is issue).
-// 417 x 333 x 379 (rows that no vector load fits): 673 us, 381 here (125, 102,
-// 115).  Where 36 to 94 % of the volume lies beyond 65 voxels of a site, so
+// 417 x 333 x 379 (rows at any address): 673 us, 333 here (79, 102, 115; the x
+// pass 125 from single bytes, a ballot per 32).  Where 36 to 94 % of the volume lies beyond 65 voxels of a site, so
 // that the 32-bit passes run as well, 1.23-2.70 ms before and 1.18-2.68 here.
 constexpr uint32_t kNearMax = (kWinHalo + 1) * (kWinHalo + 1);
 constexpr uint32_t kFar16 = 40000;
@@ -663,11 +663,52 @@ static_assert(32 * kReachWords >= kReach, "a site beyond the words looked at is 
 static_assert((kReach + 7) * (kReach + 7) <= (int)kFar16 && kReach * kReach > (int)kNearMax, "far rows stay far");
 static_assert(kFar16 + (kWinHalo + 6) * (kWinHalo + 6) < 65536, "the window scan adds distance^2 to kFar16");
 
+// A byte volume at any address, read as aligned words.
+struct ByteVolume {
+  const uint32_t* words;  // the word that holds the first byte
+  int lead;               // bytes of it before the first
+  long long end;          // one past the last byte, from words
+  __device__ ByteVolume(const uint8_t* p, long long n)
+      : words(reinterpret_cast<const uint32_t*>(p - (reinterpret_cast<uintptr_t>(p) & 3u))),
+        lead((int)(reinterpret_cast<uintptr_t>(p) & 3u)),
+        end(n + lead) {}
+};
+
+// A word that the volume does not fill, from the bytes it has (0 for the others).
+__device__ __noinline__ uint32_t edge_word(const uint32_t* words, int lead, long long end, long long k) {
+  uint32_t w = 0u;
+  for (int j = 0; j < 4; ++j) {
+    const long long i = 4 * k + j;
+    if (i >= lead && i < end) w |= (uint32_t) reinterpret_cast<const uint8_t*>(words)[i] << (8 * j);
+  }
+  return w;
+}
+
+// Bytes at .. at + 15 of the volume (0 past its end).
+__device__ __forceinline__ uint4 load16(const ByteVolume& v, long long at) {
+  const long long k = (at + v.lead) >> 2;
+  const uint32_t by = (uint32_t)(at + v.lead) % 4u * 8u;
+  uint32_t w[5];
+  if (4 * k >= v.lead && 4 * k + 20 <= v.end) {
+#pragma unroll
+    for (int j = 0; j < 5; ++j) w[j] = __ldg(v.words + k + j);
+  } else {
+#pragma unroll 1
+    for (int j = 0; j < 5; ++j) {
+      const uint32_t e = edge_word(v.words, v.lead, v.end, k + j);
+#pragma unroll
+      for (int i = 0; i < 5; ++i) w[i] = i == j ? e : w[i];
+    }
+  }
+  return make_uint4(__funnelshift_r(w[0], w[1], by), __funnelshift_r(w[1], w[2], by), __funnelshift_r(w[2], w[3], by),
+                    __funnelshift_r(w[3], w[4], by));
+}
+
 // The x pass: a warp per row, eight voxels per lane.  A voxel's distance is the
 // least of three: to a site among its lane's eight voxels (a table by their
 // bits), to the nearest site left of them and right of them.
 template <int MODE, bool VEC>
-__global__ void __launch_bounds__(kXWarps * 32, 6)
+__global__ void __launch_bounds__(kXWarps * 32, VEC ? 6 : 5)
 edt_x_near_kernel(const uint8_t* __restrict__ a, const uint8_t* __restrict__ b, Dims dm, int pitch,
                   uint16_t* __restrict__ out, uint32_t* __restrict__ selbits, Counters* __restrict__ ctr) {
   extern __shared__ uint32_t smem[];
@@ -679,6 +720,7 @@ edt_x_near_kernel(const uint8_t* __restrict__ a, const uint8_t* __restrict__ b, 
   uint32_t* mask = smem + (size_t)warp * nw;  // the row's sites
   const long long rows = (long long)dm.h * dm.d;
   const bool two = MODE == SEL_BONE_IN_ROI || MODE == SEL_MARROW_IN_ROI;
+  const ByteVolume ba(a, dm.n()), bb(two ? b : a, dm.n());
   unsigned long long sites = 0;
   {
     const uint32_t t = threadIdx.x;
@@ -698,58 +740,31 @@ edt_x_near_kernel(const uint8_t* __restrict__ a, const uint8_t* __restrict__ b, 
   for (long long row = (long long)blockIdx.x * kXWarps + warp; row < rows;
        row += (long long)gridDim.x * kXWarps) {
     const long long base = row * dm.w;
-    if (VEC) {
-      const uint4* av = reinterpret_cast<const uint4*>(a + base);
-      const uint4* bv = two ? reinterpret_cast<const uint4*>(b + base) : nullptr;
-      const int nvec = dm.w >> 4;  // 16 voxels per uint4
-      for (int v0 = 0; v0 < nvec; v0 += 32) {
-        const int v = v0 + lane;
-        uint32_t s16 = 0, t16 = 0;
-        if (v < nvec) {
-          const uint4 A = av[v];
-          const uint4 B = two ? bv[v] : make_uint4(0u, 0u, 0u, 0u);
-          s16 = sel4<MODE>(A.x, B.x) | (sel4<MODE>(A.y, B.y) << 4) | (sel4<MODE>(A.z, B.z) << 8) |
-                (sel4<MODE>(A.w, B.w) << 12);
-          t16 = ~s16 & 0xffffu;  // all 16 voxels lie inside the row
-        }
-        const uint32_t s_hi = __shfl_down_sync(0xffffffffu, s16, 1);
-        const uint32_t t_hi = __shfl_down_sync(0xffffffffu, t16, 1);
-        if (!(lane & 1) && v < nvec) {
-          const int c = v >> 1;  // word index: voxels 32c .. 32c + 31
-          // a row of 16k voxels with k odd ends on a half word: its upper half is empty
-          const bool full = v + 1 < nvec;
-          const uint32_t tw = t16 | (full ? t_hi << 16 : 0u);
-          mask[c] = tw;
-          selbits[row * nw + c] = s16 | (full ? s_hi << 16 : 0u);
-          sites += __popc(tw);
-        }
+    const int nvec = (dm.w + 15) >> 4;  // 16 voxels per lane
+    for (int v0 = 0; v0 < nvec; v0 += 32) {
+      const int v = v0 + lane;
+      uint32_t s16 = 0, t16 = 0;
+      if (v < nvec) {
+        const long long at = base + 16 * v;
+        const uint4 A = VEC ? __ldg(reinterpret_cast<const uint4*>(a + at)) : load16(ba, at);
+        const uint4 B = !two  ? make_uint4(0u, 0u, 0u, 0u)
+                        : VEC ? __ldg(reinterpret_cast<const uint4*>(b + at))
+                              : load16(bb, at);
+        const uint32_t inside = dm.w - 16 * v >= 16 ? 0xffffu : (1u << (dm.w - 16 * v)) - 1u;  // voxels of this row
+        s16 = (sel4<MODE>(A.x, B.x) | (sel4<MODE>(A.y, B.y) << 4) | (sel4<MODE>(A.z, B.z) << 8) |
+               (sel4<MODE>(A.w, B.w) << 12)) & inside;
+        t16 = ~s16 & inside;
       }
-    } else {
-      constexpr int kAhead = 8;  // words whose bytes are in flight
-      for (int c0 = 0; c0 < nw; c0 += kAhead) {
-        uint32_t av[kAhead], bv[kAhead];
-#pragma unroll
-        for (int j = 0; j < kAhead; ++j) {
-          const int x = (c0 + j) * 32 + lane;
-          av[j] = x < dm.w ? a[base + x] : 0u;
-          bv[j] = two && x < dm.w ? b[base + x] : 0u;
-        }
-        uint32_t sw = 0, tw = 0;
-#pragma unroll
-        for (int j = 0; j < kAhead; ++j) {
-          const bool in = (c0 + j) * 32 + lane < dm.w;
-          const bool s = in && (MODE == SEL_FOREGROUND    ? av[j] != 0
-                                : MODE == SEL_BACKGROUND  ? av[j] == 0
-                                : MODE == SEL_BONE_IN_ROI ? bv[j] != 0 && av[j] != 0
-                                                          : bv[j] != 0 && av[j] == 0);
-          const uint32_t t = __ballot_sync(0xffffffffu, in && !s), u = __ballot_sync(0xffffffffu, s);
-          if (lane == j) tw = t, sw = u;
-        }
-        if (lane < kAhead && c0 + lane < nw) {
-          mask[c0 + lane] = tw;
-          selbits[row * nw + c0 + lane] = sw;
-          sites += __popc(tw);
-        }
+      const uint32_t s_hi = __shfl_down_sync(0xffffffffu, s16, 1);
+      const uint32_t t_hi = __shfl_down_sync(0xffffffffu, t16, 1);
+      if (!(lane & 1) && v < nvec) {
+        const int c = v >> 1;  // word index: voxels 32c .. 32c + 31
+        // an odd number of 16-voxel groups ends on a half word: its upper half is empty
+        const bool full = v + 1 < nvec;
+        const uint32_t tw = t16 | (full ? t_hi << 16 : 0u);
+        mask[c] = tw;
+        selbits[row * nw + c] = s16 | (full ? s_hi << 16 : 0u);
+        sites += __popc(tw);
       }
     }
     __syncwarp();
