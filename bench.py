@@ -52,16 +52,16 @@ UNIT = "Gvoxel/s"
 # Algorithmic bytes per voxel of each kernel family for one phase (reads +
 # writes a perfect kernel must make; bitmask words count 1/8 byte per voxel).
 ALGO_BYTES_PER_VOXEL = {
-    "edt_x": 2.0 + 4.0 + 0.125,        # bone + roi in, u32 out, selection bits out
-    "edt_y": 8.0,                      # u32 in, u32 out
-    "edt_z": 8.0,
-    "ridge": 4.0,                      # u32 distance map in (ridge records counted separately)
-    "fill": 4.0,                       # u32 squared-thickness map out
-    "fill_rank": 0.0,                  # per-r^2 tables only
-    "fill_bin": 0.0,                   # per-ridge work (ridge records in, bin entries out)
+    "edt_x": 2.0 + 2.0 + 0.125,        # bone + roi in, 16-bit map out, selection bits out
+    "edt_y": 4.0,                      # 16-bit map in, 16-bit map out
+    "edt_z": 4.0,
+    "ridge": 4.0,                      # 16-bit distance map in, 16-bit ridge map out
+    "fill_bin": 2.0,                   # ridge map in (the disc lists are counted separately)
+    "fill": 4.0 + 0.125,               # f32 diameter map and nonzero bits out
+    "fill_rank": 0.0,                  # tile fill only: per-r^2 tables
     "templates": 0.0,
-    "fill_sites": 0.0,                 # per-ridge work (sphere points of each ridge)
-    "cleanup_final": 4.0 + 0.25 + 4.0,  # r^2 map in, two bitmasks in, f32 map out (the statistics read it)
+    "fill_sites": 0.0,                 # tile fill only: per-ridge work
+    "cleanup_final": 4.0 + 0.5 + 4.0,  # diameter map in, bitmasks in and out, f32 map out (the statistics read it)
     "stats_order": 8.0,                # f32 map read twice (chunk sums, chunk functions)
     "count_roi": 2.0,
 }
