@@ -801,155 +801,18 @@ __global__ void count_roi_kernel(const uint8_t* __restrict__ bone, const uint8_t
   }
 }
 
-// ROI voxels, ROI-clipped bone voxels, and those of them with a 6-neighbour
-// outside the volume or outside the ROI (metrics.rs:166-202).
-__global__ void volume_counts_kernel(const uint8_t* __restrict__ bone, const uint8_t* __restrict__ roi, Dims dm,
-                                     unsigned long long* __restrict__ out) {
-  unsigned long long c_roi = 0, c_bone = 0, c_edge = 0;
-  const long long n = dm.n();
-  const long long sl = (long long)dm.w * dm.h;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const bool r = roi[i] != 0;
-    c_roi += r;
-    if (r && bone[i] != 0) {
-      ++c_bone;
-      const int z = (int)(i / sl);
-      const long long rem = i - (long long)z * sl;
-      const int y = (int)(rem / dm.w), x = (int)(rem - (long long)y * dm.w);
-      const bool edge = x == 0 || y == 0 || z == 0 || x == dm.w - 1 || y == dm.h - 1 || z == dm.d - 1 ||
-                        roi[i - 1] == 0 || roi[i + 1] == 0 || roi[i - dm.w] == 0 || roi[i + dm.w] == 0 ||
-                        roi[i - sl] == 0 || roi[i + sl] == 0;
-      c_edge += edge;
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    c_roi += __shfl_xor_sync(0xffffffffu, c_roi, o);
-    c_bone += __shfl_xor_sync(0xffffffffu, c_bone, o);
-    c_edge += __shfl_xor_sync(0xffffffffu, c_edge, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    if (c_roi) atomicAdd(&out[0], c_roi);
-    if (c_bone) atomicAdd(&out[1], c_bone);
-    if (c_edge) atomicAdd(&out[2], c_edge);
-  }
-}
-
-// The same counts four voxels per thread, for 4-byte aligned volumes of less
-// than 2^32 voxels.  The six neighbours of a word are the words at offsets that
-// need not be aligned, but each offset's alignment is the same for every word:
-// two loads and a funnel shift (the second load is a cache hit), made only
-// where the word holds ROI-clipped bone.  The words within a slice of either
-// end of the volume check their bounds; voxels on the volume's faces are looked
-// at one by one.  430 x 389 x 401: 611 us with one voxel per thread and byte
-// loads, 92 us here (six neighbours from L1 and L2: bound by issue and latency).
-constexpr uint32_t kHigh = 0x80808080u;
-
-// The high bit of every byte that is not 0 (the other bits are arbitrary).
-__device__ __forceinline__ uint32_t nonzero_high(uint32_t v) { return ((v & ~kHigh) + ~kHigh) | v; }
-
-// Word k of a volume of n bytes, 0 outside it.
-__device__ __noinline__ uint32_t word_or_zero(const uint8_t* p, long long k, long long n) {
-  if (k < 0 || 4 * k >= n) return 0u;
-  if (4 * k + 4 <= n) return reinterpret_cast<const uint32_t*>(p)[k];
-  uint32_t v = 0u;
-  for (long long j = 4 * k; j < n; ++j) v |= (uint32_t)p[j] << (8 * (j & 3));
-  return v;
-}
-
-constexpr int kCountWords = 4;  // words a thread has in flight
-
-__global__ void __launch_bounds__(256)
-volume_counts4_kernel(const uint8_t* __restrict__ bone, const uint8_t* __restrict__ roi, Dims dm, VoxelDecoder vd,
-                      unsigned long long* __restrict__ out) {
-  const long long n = dm.n();
-  const int sl = dm.w * dm.h;  // <= 2^30
-  const uint32_t* R = reinterpret_cast<const uint32_t*>(roi);
-  const uint32_t* B = reinterpret_cast<const uint32_t*>(bone);
-  const int whole = (int)(n / 4), margin = sl / 4 + 2;  // whole words; words within reach of an end of the volume
-  // 2^32 voxels over at least 2^15 threads: the counts of one fit 32 bits
-  uint32_t c_roi = 0, c_bone = 0, c_edge = 0;
-  auto faces = [&](int q, uint32_t inner) -> uint32_t {  // inner without the voxels on the volume's faces
-    int x, y, z;
-    vd(4u * (uint32_t)q, x, y, z);
-    if (x != 0 && x + 4 < dm.w && y != 0 && y != dm.h - 1 && z != 0 && z != dm.d - 1) return inner;
-    for (int j = 0; j < 4; ++j) {
-      if (x == 0 || x == dm.w - 1 || y == 0 || y == dm.h - 1 || z == 0 || z == dm.d - 1) inner &= ~(0xffu << (8 * j));
-      if (++x == dm.w) {
-        x = 0;
-        if (++y == dm.h) y = 0, ++z;
-      }
-    }
-    return inner;
-  };
-  const int step = (int)(gridDim.x * blockDim.x) * kCountWords;
-  for (int q0 = (int)(blockIdx.x * blockDim.x * kCountWords + threadIdx.x); q0 <= whole; q0 += step) {
-    uint32_t in[kCountWords], both[kCountWords];
-#pragma unroll
-    for (int j = 0; j < kCountWords; ++j) {
-      const int q = q0 + j * (int)blockDim.x;
-      in[j] = q < whole ? __ldg(R + q) : q == whole ? word_or_zero(roi, q, n) : 0u;
-      both[j] = q < whole ? __ldg(B + q) : q == whole ? word_or_zero(bone, q, n) : 0u;
-    }
-#pragma unroll
-    for (int j = 0; j < kCountWords; ++j) {
-      in[j] = nonzero_high(in[j]) & kHigh;
-      both[j] = nonzero_high(both[j]) & in[j];
-      c_roi += __popc(in[j]);
-      c_bone += __popc(both[j]);
-    }
-#pragma unroll
-    for (int j = 0; j < kCountWords; ++j) {
-      const int q = q0 + j * (int)blockDim.x;
-      if (!both[j]) continue;
-      uint32_t inner = ~0u;
-      if (q >= margin && q + margin < whole) {
-        auto near = [&](int o) {
-          const uint32_t* p = R + (q + (o >> 2));
-          inner &= nonzero_high(__funnelshift_r(__ldg(p), __ldg(p + 1), (uint32_t)(o & 3) * 8u));
-        };
-        near(-1), near(1), near(-dm.w), near(dm.w), near(-sl), near(sl);
-      } else {
-#pragma unroll 1
-        for (int k = 0; k < 6; ++k) {
-          const int d = k < 2 ? 1 : k < 4 ? dm.w : sl, o = k & 1 ? d : -d;
-          const long long i = (long long)q + (o >> 2);
-          inner &= nonzero_high(__funnelshift_r(word_or_zero(roi, i, n), word_or_zero(roi, i + 1, n),
-                                                (uint32_t)(o & 3) * 8u));
-        }
-      }
-      c_edge += __popc(both[j] & ~faces(q, inner));
-    }
-  }
-  unsigned long long t_roi = c_roi, t_bone = c_bone, t_edge = c_edge;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    t_roi += __shfl_xor_sync(0xffffffffu, t_roi, o);
-    t_bone += __shfl_xor_sync(0xffffffffu, t_bone, o);
-    t_edge += __shfl_xor_sync(0xffffffffu, t_edge, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    if (t_roi) atomicAdd(&out[0], t_roi);
-    if (t_bone) atomicAdd(&out[1], t_bone);
-    if (t_edge) atomicAdd(&out[2], t_edge);
-  }
-}
-
 int volume_metrics_impl(bm_ctx* ctx, const uint8_t* d_bone, const uint8_t* d_roi, Dims dm, const double* sp,
                         bm_volume_metrics* out, cudaStream_t s) {
   for (int i = 0; i < 3; ++i)
     if (!std::isfinite(sp[i]) || sp[i] <= 0.0)
       fail(ctx, BM_ERR_SPACING, "voxel spacings must be finite and positive; got [%g, %g, %g]", sp[0], sp[1], sp[2]);
   unsigned long long* dc = reinterpret_cast<unsigned long long*>(phase_out(ctx));
+  const size_t bits = (size_t)dm.nw() * dm.h * dm.d * sizeof(uint32_t);
+  uint32_t* rbits = static_cast<uint32_t*>(ensure(ctx, ctx->selbits, bits, "ROI bits"));
+  uint32_t* bbits = static_cast<uint32_t*>(ensure(ctx, ctx->nzbits, bits, "bone bits"));
   check(ctx, cudaMemsetAsync(dc, 0, 24, s), "memset");
-  timed(ctx, KF_COUNT_ROI, s, "volume counts", [&] {
-    if (((reinterpret_cast<uintptr_t>(d_bone) | reinterpret_cast<uintptr_t>(d_roi)) & 3u) == 0)
-      volume_counts4_kernel<<<152 * 8, 256, 0, s>>>(d_bone, d_roi, dm, VoxelDecoder::of(dm), dc);
-    else
-      volume_counts_kernel<<<152 * 8, 256, 0, s>>>(d_bone, d_roi, dm, dc);
-    ++ctx->launches;
-    return cudaGetLastError();
-  });
+  timed(ctx, KF_COUNT_ROI, s, "volume counts",
+        [&] { return launch_volume_counts(d_bone, d_roi, dm, rbits, bbits, dc, s, &ctx->launches); });
   unsigned long long* hc = readback(ctx).counts;
   check(ctx, cudaMemcpyAsync(hc, dc, 24, cudaMemcpyDeviceToHost, s), "count readback");
   check(ctx, cudaStreamSynchronize(s), "volume counts");

@@ -73,6 +73,12 @@ cudaError_t launch_edt_near_z(const uint16_t* ymap, uint32_t* wide, uint16_t* na
 cudaError_t launch_edt_near_redo(const uint32_t* in, uint16_t* out, Dims dm, void* scratch, const uint8_t* redo,
                                  Counters* ctr, cudaStream_t s, unsigned long long* launches);
 
+// out (zeroed): ROI voxels, ROI-clipped bone voxels, and those of them with a
+// 6-neighbour outside the volume or the ROI (metrics.rs:166-202).  rbits, bbits:
+// a row-padded bitmask each (nw * h * d words).
+cudaError_t launch_volume_counts(const uint8_t* bone, const uint8_t* roi, Dims dm, uint32_t* rbits, uint32_t* bbits,
+                                 unsigned long long* out, cudaStream_t s, unsigned long long* launches);
+
 // Search-template table entries lut[r2] for r2 in [lo, hi]:
 // {scan_cube(1,0,0), scan_cube(1,1,0), scan_cube(1,1,1), f32 bits of 2*sqrt(r2)}.
 cudaError_t launch_lut(uint4* lut, uint32_t lo, uint32_t hi, cudaStream_t s, unsigned long long* launches);

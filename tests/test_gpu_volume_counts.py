@@ -16,7 +16,8 @@ def counts(bone, roi):
     return int(b.sum()), int(r.sum()), int((b & ~inner).sum())
 
 
-@pytest.mark.parametrize("shape", [(2, 2, 2), (3, 5, 3), (2, 3, 4), (7, 6, 5), (9, 10, 33), (5, 40, 64), (21, 19, 130)])
+@pytest.mark.parametrize("shape", [(2, 2, 2), (3, 5, 3), (2, 3, 4), (7, 6, 5), (9, 10, 33), (5, 40, 64), (21, 19, 130), (9, 8, 32), (17, 3, 31),
+                                   (3, 4, 511), (3, 2, 529), (2, 5, 1100)])
 @pytest.mark.parametrize("offset", [0, 1, 2])
 @pytest.mark.parametrize("p", [0.3, 0.97])
 def test_volume_counts(gpu_ctx, shape, offset, p):
