@@ -512,8 +512,9 @@ struct Phase {
     const size_t count = disc_header_count(dm);
     hdr = static_cast<uint32_t*>(ensure(ctx, ctx->dischdr, count * 4, "disc lists"));
     ent = static_cast<uint2*>(ensure(ctx, ctx->discent, count * kDiscSlots * sizeof(uint2), "disc lists"));
-    const size_t pool_cap = disc_pool_entries(dm);
-    pool = static_cast<uint2*>(ensure(ctx, ctx->discpool, pool_cap * sizeof(uint2), "disc lists"));
+    pool = static_cast<uint2*>(
+        ensure(ctx, ctx->discpool, disc_pool_entries(dm, hc.rmax) * sizeof(uint2), "disc lists"));
+    const size_t pool_cap = ctx->discpool.bytes / sizeof(uint2);
     const uint2* thr = static_cast<const uint2*>(ctx->discthr.ptr);
     const uint32_t* tmpl = static_cast<const uint32_t*>(ctx->disctmpl.ptr);
     timed(ctx, KF_RIDGE, s, "ridge map", [&] {
@@ -602,10 +603,27 @@ struct Phase {
   void finish() {
     check(ctx, cudaStreamSynchronize(s), "local thickness");
     if (separable && readback(ctx).out.ctr.disc_overflow) {
-      // the lists' pool ran out: again with the tile fill, in the lists' memory
-      for (Buffer* b : {&ctx->ridgemap, &ctx->discent, &ctx->discpool}) release(*b);
+      // the lists' pool ran out: again with one of the size that they wanted, or,
+      // where there is no memory for it, with the tile fill in the lists' memory
+      const unsigned long long wanted = readback(ctx).out.ctr.disc_pool;
       check(ctx, cudaMemsetAsync(&out->acc, 0, sizeof(StatsAccum), s), "memset");
-      tile_fill();
+      check(ctx, cudaMemsetAsync(&out->ctr.disc_pool, 0, sizeof(out->ctr.disc_pool), s), "memset");
+      check(ctx, cudaMemsetAsync(&out->ctr.disc_overflow, 0, sizeof(out->ctr.disc_overflow), s), "memset");
+      bool room = true;
+      try {
+        ensure(ctx, ctx->discpool, (wanted + wanted / 8) * sizeof(uint2), "disc lists");
+      } catch (const CallError&) {
+        ctx->last_error.clear();
+        room = false;
+      }
+      if (room) {
+        lists();
+        paint();
+      } else {
+        separable = false;
+        for (Buffer* b : {&ctx->ridgemap, &ctx->discent, &ctx->discpool}) release(*b);
+        tile_fill();
+      }
       check(ctx, cudaStreamSynchronize(s), "local thickness");
     }
     const PhaseOut& r = readback(ctx).out;

@@ -299,10 +299,10 @@ extern "C" {
 
 uint64_t bm_footprint_bytes(size_t width, size_t height, size_t depth) {
   // per voxel: inputs 2; per phase (the two phases run side by side, each on
-  // its own buffers): three u32 maps 12 (x/y pass, z pass), envelope scratch 8,
-  // u16 ridge map 2, disc lists 12.5, f32 thickness map 4 (read by the
+  // its own buffers): x, y and z pass maps 8, envelope scratch 8, u16 ridge map
+  // 2, disc lists 12 and their pool (4.5 at radius 40), f32 thickness map 4 (read by the
   // statistics' ordered sums, ~0.2 more of their scratch), quantile map 4,
-  // bitmasks ~1; the tile fill (radii above 127) takes a chain map 4, ridge
+  // bitmasks ~1; the tile fill (radii above 127) takes 4 more for the maps, a chain map 4, ridge
   // records <= 8 and bin entries ~5 in place of the ridge map and the lists;
   // tables 2 x 64 MiB
   const uint64_t n = (uint64_t)width * height * depth;

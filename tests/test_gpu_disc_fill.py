@@ -66,3 +66,23 @@ def test_plane_runs_bitwise(gpu_ctx, d, w):
     got, sq = local_thickness(vol, Phase.FOREGROUND, ctx=gpu_ctx, return_squared=True)
     assert np.array_equal(sq, ref.propagated)
     assert np.array_equal(got.view(np.uint32), ref.thickness.view(np.uint32))
+
+
+def test_lists_that_outgrow_their_pool():
+    """Balls that overlap at random want more list entries than their radius
+    suggests: the first call fills again in a larger pool, the second at once."""
+    from bone_morphometry_gb300 import Context
+
+    ctx = Context(0)
+    vol = (np.random.default_rng(11).random((90, 100, 130)) < 0.9995).astype(np.uint8)
+    ref = O.local_thickness(vol, 0)
+    launches = []
+    for _ in range(2):
+        before = ctx.launches
+        got, sq = local_thickness(vol, Phase.FOREGROUND, ctx=ctx, return_squared=True)
+        launches.append(ctx.launches - before)
+        assert np.array_equal(sq, ref.propagated)
+        assert np.array_equal(got.view(np.uint32), ref.thickness.view(np.uint32))
+    ctx.close()
+    # 3 launches make the tables of a new context, 5 fill again
+    assert launches[0] == launches[1] + 3 + 5
