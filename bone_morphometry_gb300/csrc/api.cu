@@ -947,7 +947,7 @@ int tbth_phases(bm_ctx* ctx, const uint8_t* d_bone, const uint8_t* d_roi, Dims d
   // (its own stream and buffers), so that their kernels overlap on the GPU.
   // Results and errors are reported in the reference's order (bone first).
   // Side by side only while one phase cannot fill the GPU: on 1024^3 the two
-  // phases' kernels compete (174 ms against 159 ms one after the other), on
+  // phases' kernels compete (59.9 ms against 55.9 ms one after the other), on
   // 512^3 and below they fill each other's gaps.
   bm_ctx* tw = phases_side_by_side(ctx, dm) ? twin_of(ctx) : nullptr;
   bm_ctx* mctx = tw ? tw : ctx;

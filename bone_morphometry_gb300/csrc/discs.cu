@@ -20,7 +20,7 @@
 //
 // On a 192^3 crop of the 512^3 workload's generator (marrow phase) a ball
 // centre meets 5.6 planes per selected voxel and 58.7 rows; the lists hold
-// 0.69 discs and the tiles paint 10.7 rows per selected voxel.  Nothing depends
+// 0.85 discs with 7.4 rows per selected voxel.  Nothing depends
 // on the order of the balls, so there is no sort by radius, no list of balls
 // per tile and no barrier between radii, and the non-selected voxels on a
 // ball's sphere (rho = 0 at the end) come out of the same passes.

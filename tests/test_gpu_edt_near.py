@@ -86,7 +86,7 @@ def test_ridge_of_pairs_bitwise(gpu_ctx, shape):
     assert np.array_equal(got.view(np.uint32), ref.thickness.view(np.uint32))
 
 
-@pytest.mark.parametrize("offset", [0, 1, 2, 3])
+@pytest.mark.parametrize("offset", [0, 1, 2, 3, 4, 8, 11, 12, 15])
 @pytest.mark.parametrize("shape", [(2, 2, 2), (2, 3, 5), (3, 2, 15), (3, 5, 16), (2, 4, 17), (3, 3, 31), (2, 2, 33), (4, 3, 511), (3, 2, 529)])
 def test_rows_at_any_address(gpu_ctx, shape, offset):
     """Rows that start at any byte: words that hang over either end of the volume."""
@@ -95,7 +95,7 @@ def test_rows_at_any_address(gpu_ctx, shape, offset):
     vol = noise(shape, 0.8, sum(shape))
     vol.flat[0] = 0
     vol.flat[-1] = 1
-    t = torch.full((vol.size + 8,), 1, dtype=torch.uint8, device="cuda")
+    t = torch.full((vol.size + 16,), 1, dtype=torch.uint8, device="cuda")
     t[offset : offset + vol.size] = torch.from_numpy(vol).cuda().flatten()
     view = t[offset : offset + vol.size].view(shape)
     got = edt(view, Phase.FOREGROUND, ctx=gpu_ctx)

@@ -18,7 +18,7 @@ def counts(bone, roi):
 
 @pytest.mark.parametrize("shape", [(2, 2, 2), (3, 5, 3), (2, 3, 4), (7, 6, 5), (9, 10, 33), (5, 40, 64), (21, 19, 130), (9, 8, 32), (17, 3, 31),
                                    (3, 4, 511), (3, 2, 529), (2, 5, 1100)])
-@pytest.mark.parametrize("offset", [0, 1, 2])
+@pytest.mark.parametrize("offset", [0, 1, 2, 7, 8, 13])
 @pytest.mark.parametrize("p", [0.3, 0.97])
 def test_volume_counts(gpu_ctx, shape, offset, p):
     import torch
@@ -29,7 +29,7 @@ def test_volume_counts(gpu_ctx, shape, offset, p):
     bone.flat[0] = roi.flat[0] = 1
 
     def on_gpu(a):  # at a byte offset from an aligned address
-        t = torch.zeros(a.size + 16, dtype=torch.uint8, device="cuda")
+        t = torch.zeros(a.size + 32, dtype=torch.uint8, device="cuda")
         t[offset:offset + a.size] = torch.from_numpy(a.reshape(-1)).cuda()
         return t[offset:offset + a.size].view(a.shape)
 
