@@ -137,6 +137,7 @@ SIGNATURES = {
     "bm_ctx_set_site_method": (_i, [_vp, _i]),
     "bm_ctx_set_fill_tile_rows": (_i, [_vp, _i]),
     "bm_ctx_set_wait_cycles": (_i, [_vp, ctypes.c_longlong]),
+    "bm_ctx_fail_allocation": (_i, [_vp, ctypes.c_char_p, _i]),
     "bm_tiff_read": (_i, [ctypes.c_char_p, ctypes.c_uint, _i, _vp, _sz, ctypes.POINTER(_sz), ctypes.POINTER(_sz),
                           ctypes.POINTER(_sz)]),
 }
@@ -233,6 +234,10 @@ class Context:
         """Cycle limit of the device-side bounded waits (-1: the default, ~2 s;
         0: give up at once, to exercise the timeout path)."""
         self.call("bm_ctx_set_wait_cycles", int(cycles))
+
+    def fail_allocation(self, what: str = "", skip: int = 0) -> None:
+        """For tests: after ``skip`` more, this context's next allocation of the buffer ``what`` fails, once."""
+        self.call("bm_ctx_fail_allocation", what.encode(), int(skip))
 
     def kernel_times(self) -> dict:
         """{family: (launches, total_ms)} of the kernels timed since profile(True)."""

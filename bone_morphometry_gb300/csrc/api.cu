@@ -50,6 +50,13 @@ void check(bm_ctx* ctx, cudaError_t e, const char* what) {
   fail(ctx, st, "%s: %s", what, cudaGetErrorString(e));
 }
 
+// Whether this allocation is the one that bm_ctx_fail_allocation asked to fail.
+bool refused(bm_ctx* ctx, const char* what) {
+  if (ctx->fail_what.empty() || ctx->fail_what != what || ctx->fail_skip-- > 0) return false;
+  ctx->fail_what.clear();
+  return true;
+}
+
 void* ensure(bm_ctx* ctx, Buffer& b, size_t bytes, const char* what) {
   if (bytes == 0) bytes = 16;
   if (b.bytes >= bytes) return b.ptr;
@@ -59,7 +66,7 @@ void* ensure(bm_ctx* ctx, Buffer& b, size_t bytes, const char* what) {
     b.bytes = 0;
   }
   void* p = nullptr;
-  cudaError_t e = cudaMalloc(&p, bytes);
+  cudaError_t e = refused(ctx, what) ? cudaErrorMemoryAllocation : cudaMalloc(&p, bytes);
   if (e != cudaSuccess) {
     cudaGetLastError();
     fail(ctx, BM_ERR_OOM, "device allocation of %zu bytes for %s failed: %s", bytes, what, cudaGetErrorString(e));
@@ -510,10 +517,10 @@ struct Phase {
     if (!separable) return;
     uint16_t* rmap = static_cast<uint16_t*>(ensure(ctx, ctx->ridgemap, narrow_bytes(), "ridge map"));
     const size_t count = disc_header_count(dm);
-    hdr = static_cast<uint32_t*>(ensure(ctx, ctx->dischdr, count * 4, "disc lists"));
+    hdr = static_cast<uint32_t*>(ensure(ctx, ctx->dischdr, count * 4, "disc headers"));
     ent = static_cast<uint2*>(ensure(ctx, ctx->discent, count * kDiscSlots * sizeof(uint2), "disc lists"));
     pool = static_cast<uint2*>(
-        ensure(ctx, ctx->discpool, disc_pool_entries(dm, hc.rmax) * sizeof(uint2), "disc lists"));
+        ensure(ctx, ctx->discpool, disc_pool_entries(dm, hc.rmax) * sizeof(uint2), "disc pool"));
     const size_t pool_cap = ctx->discpool.bytes / sizeof(uint2);
     const uint2* thr = static_cast<const uint2*>(ctx->discthr.ptr);
     const uint32_t* tmpl = static_cast<const uint32_t*>(ctx->disctmpl.ptr);
@@ -611,7 +618,7 @@ struct Phase {
       check(ctx, cudaMemsetAsync(&out->ctr.disc_overflow, 0, sizeof(out->ctr.disc_overflow), s), "memset");
       bool room = true;
       try {
-        ensure(ctx, ctx->discpool, (wanted + wanted / 8) * sizeof(uint2), "disc lists");
+        ensure(ctx, ctx->discpool, (wanted + wanted / 8) * sizeof(uint2), "disc pool");
       } catch (const CallError&) {
         ctx->last_error.clear();
         room = false;
@@ -1001,7 +1008,10 @@ int tbth_phases(bm_ctx* ctx, const uint8_t* d_bone, const uint8_t* d_roi, Dims d
     marrow.d_map = map_of(tw, d_spmap);
     marrow.wait_edt();
   });
-  if (twin_status == BM_OK && !(bone.separable && marrow.separable)) {
+  // Decided here, once: a phase may turn to the tile fill later, in finish, when
+  // its lists' pool cannot grow.
+  const bool queued = bone.separable && marrow.separable;
+  if (twin_status == BM_OK && !queued) {
     // the tile fill waits for its own counts: a host thread for each phase
     std::thread thread([&] {
       try_twin([&] {
@@ -1035,7 +1045,7 @@ int tbth_phases(bm_ctx* ctx, const uint8_t* d_bone, const uint8_t* d_roi, Dims d
   }
   int st = report_phase(bone, ctx, spacing, th);
   if (st) return st;
-  if (marrow.separable && bone.separable) try_twin([&] { marrow.finish(); });
+  if (queued) try_twin([&] { marrow.finish(); });
   if (twin_status != BM_OK) {
     ctx->last_error = tw->last_error;
     throw CallError{twin_status};
@@ -1294,6 +1304,15 @@ int bm_ctx_set_wait_cycles(bm_ctx* ctx, long long cycles) {
   return guarded(ctx, [&]() -> int {
     ctx->wait_cycles = cycles < 0 ? -1 : cycles;
     if (ctx->twin) ctx->twin->wait_cycles = ctx->wait_cycles;
+    return BM_OK;
+  });
+}
+
+int bm_ctx_fail_allocation(bm_ctx* ctx, const char* what, int skip) {
+  return guarded(ctx, [&]() -> int {
+    if (skip < 0) fail(ctx, BM_ERR_INVALID, "skip must not be negative; got %d", skip);
+    ctx->fail_what = what ? what : "";
+    ctx->fail_skip = skip;
     return BM_OK;
   });
 }

@@ -197,6 +197,8 @@ struct bm_ctx {
   cudaStream_t stream = nullptr;
   void* pinned = nullptr;      // page-locked readback area (bm::Readback)
   cudaEvent_t counted = nullptr;  // the ROI counts have been copied
+  std::string fail_what;       // the buffer whose allocation is to fail (bm_ctx_fail_allocation), and
+  int fail_skip = 0;           // how many of them succeed before
   // second context (own stream and buffers) that runs the marrow phase of
   // bm_tbth_tbsp while this one runs the bone phase; created on first use
   bm_ctx* twin = nullptr;

@@ -313,6 +313,13 @@ int bm_ctx_set_fill_tile_rows(bm_ctx* ctx, int rows);
  * call returns BM_ERR_TIMEOUT with the context still usable.  For tests. */
 int bm_ctx_set_wait_cycles(bm_ctx* ctx, long long cycles);
 
+/* Fault injection on the host, for tests of the out-of-memory paths: of this
+ * context's (not its inner second context's) allocations of the buffer named
+ * `what`, the one after the next `skip` fails once, as though cudaMalloc had
+ * returned out of memory.  what NULL or empty: none.  The names are those that
+ * the error messages give ("disc pool", "distance map", ...). */
+int bm_ctx_fail_allocation(bm_ctx* ctx, const char* what, int skip);
+
 /* Kernel launches issued by this context since creation (library kernels only). */
 uint64_t bm_ctx_launch_count(const bm_ctx* ctx);
 

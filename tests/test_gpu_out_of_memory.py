@@ -1,0 +1,48 @@
+"""Calls whose device allocations fail part way, injected on the host
+(Context.fail_allocation): they fall back or report BM_ERR_OOM, and the context
+stays usable.  Maps bit for bit against the oracle."""
+
+import numpy as np
+import pytest
+
+import oracle as O
+from refstats import assert_reference_stats
+from bone_morphometry_gb300 import Context, analyze_thickness
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def ctx():
+    c = Context(0)
+    yield c
+    c.close()
+
+
+def random_balls(shape=(90, 100, 130), seed=11):
+    """Balls that overlap at random: more list entries than their radius suggests."""
+    return (np.random.default_rng(seed).random(shape) < 0.9995).astype(np.uint8)
+
+
+def assert_maps(res, bone, roi, spacing):
+    for sel, got, gmap in ((True, res.thickness, res.thickness_map), (False, res.spacing, res.spacing_map)):
+        ref = O.local_thickness(O.phase_inside(bone, roi, sel), O.FOREGROUND)
+        assert np.array_equal(gmap.view(np.uint32), ref.thickness.view(np.uint32))
+        assert_reference_stats(got, ref.thickness, spacing)
+
+
+@pytest.mark.parametrize("concurrent", [True, False])
+def test_bone_phase_whose_pool_cannot_grow(ctx, concurrent):
+    """The bone phase turns to the tile fill at its end, the marrow phase beside it does not."""
+    bone = random_balls()
+    roi = np.ones_like(bone)
+    ctx.set_concurrent_phases(concurrent)
+    ctx.fail_allocation("disc pool", 1)
+    ctx.profile(True)
+    res = analyze_thickness(bone, roi, 12.5, ctx=ctx, return_maps=True)
+    times = ctx.kernel_times()
+    ctx.profile(False)
+    assert times["fill_rank"][0] > 0  # the tile fill ran
+    assert_maps(res, bone, roi, 12.5)
+    # the injection is spent: the lists again
+    assert_maps(analyze_thickness(bone, roi, 12.5, ctx=ctx, return_maps=True), bone, roi, 12.5)
