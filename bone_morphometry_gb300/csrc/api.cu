@@ -146,44 +146,45 @@ Dims check_dims(bm_ctx* ctx, size_t w, size_t h, size_t d) {
 
 const char* phase_name(int phase) { return phase == BM_PHASE_BACKGROUND ? "background" : "foreground"; }
 
+// The tables by squared radius: search templates, diameters, and those of the
+// separable fill.  All are made before any takes its place in the context, so
+// that a failure on the way leaves the context with the tables that it had.
 void ensure_lut(bm_ctx* ctx, uint32_t rmax) {
   if (ctx->lut_max >= rmax && ctx->lut.ptr) return;
   // grow to at least twice the current size so repeated growth stays amortised
   uint32_t target = rmax;
   if (ctx->lut.ptr && target < ctx->lut_max * 2u) target = ctx->lut_max * 2u;
   if (target < 1024) target = 1024;
-  const size_t bytes = ((size_t)target + 1) * sizeof(uint4);
-  void* p = nullptr;
-  cudaError_t e = cudaMalloc(&p, bytes);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    fail(ctx, BM_ERR_OOM, "device allocation of %zu bytes for the template table failed", bytes);
-  }
+  const size_t n = (size_t)target + 1, nd = std::min<size_t>(target, kDiscMaxR2) + 1;
+  struct Tables {
+    Buffer lut, dia, thr, tmpl;
+    ~Tables() {
+      for (Buffer* b : {&lut, &dia, &thr, &tmpl}) release(*b);
+    }
+  } t;
+  uint4* lut = static_cast<uint4*>(ensure(ctx, t.lut, n * sizeof(uint4), "template table"));
+  float* dia = static_cast<float*>(ensure(ctx, t.dia, n * sizeof(float), "diameter table"));
+  uint2* thr = static_cast<uint2*>(ensure(ctx, t.thr, nd * sizeof(uint2), "disc tables"));
+  uint32_t* tmpl = static_cast<uint32_t*>(ensure(ctx, t.tmpl, nd * sizeof(uint32_t), "disc tables"));
   uint32_t lo = 0;
   if (ctx->lut.ptr) {
-    check(ctx, cudaMemcpyAsync(p, ctx->lut.ptr, ((size_t)ctx->lut_max + 1) * sizeof(uint4), cudaMemcpyDeviceToDevice,
+    check(ctx, cudaMemcpyAsync(lut, ctx->lut.ptr, ((size_t)ctx->lut_max + 1) * sizeof(uint4), cudaMemcpyDeviceToDevice,
                                ctx->stream),
           "template table copy");
     lo = ctx->lut_max + 1;
   }
   timed(ctx, KF_TEMPLATES, ctx->stream, "template kernel",
-        [&] { return launch_lut(static_cast<uint4*>(p), lo, target, ctx->stream, &ctx->launches); });
-  check(ctx, cudaStreamSynchronize(ctx->stream), "template kernel");
-  release(ctx->lut);
-  ctx->lut.ptr = p;
-  ctx->lut.bytes = bytes;
-  ctx->lut_max = target;
-  float* dia = static_cast<float*>(ensure(ctx, ctx->lutf, ((size_t)target + 1) * sizeof(float), "diameter table"));
-  check(ctx, launch_dia_table(static_cast<const uint4*>(p), target + 1, dia, ctx->stream, &ctx->launches),
-        "diameter table");
-  const uint32_t nd = (target < kDiscMaxR2 ? target : kDiscMaxR2) + 1;
-  uint2* thr = static_cast<uint2*>(ensure(ctx, ctx->discthr, (size_t)nd * sizeof(uint2), "disc tables"));
-  uint32_t* tmpl = static_cast<uint32_t*>(ensure(ctx, ctx->disctmpl, (size_t)nd * sizeof(uint32_t), "disc tables"));
-  timed(ctx, KF_TEMPLATES, ctx->stream, "disc tables", [&] {
-    return launch_disc_tables(static_cast<const uint4*>(p), nd, thr, tmpl, ctx->stream, &ctx->launches);
-  });
+        [&] { return launch_lut(lut, lo, target, ctx->stream, &ctx->launches); });
+  check(ctx, launch_dia_table(lut, (uint32_t)n, dia, ctx->stream, &ctx->launches), "diameter table");
+  timed(ctx, KF_TEMPLATES, ctx->stream, "disc tables",
+        [&] { return launch_disc_tables(lut, (uint32_t)nd, thr, tmpl, ctx->stream, &ctx->launches); });
   // the phase that reads the tables may run on another stream
   check(ctx, cudaStreamSynchronize(ctx->stream), "template tables");
+  std::swap(ctx->lut, t.lut);
+  std::swap(ctx->lutf, t.dia);
+  std::swap(ctx->discthr, t.thr);
+  std::swap(ctx->disctmpl, t.tmpl);
+  ctx->lut_max = target;
 }
 
 void ensure_surf(bm_ctx* ctx, uint32_t rmax);

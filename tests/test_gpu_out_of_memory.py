@@ -7,7 +7,7 @@ import pytest
 
 import oracle as O
 from refstats import assert_reference_stats
-from bone_morphometry_gb300 import Context, analyze_thickness
+from bone_morphometry_gb300 import BoneMorphometryError, Context, Phase, _lib, analyze_thickness, local_thickness
 
 pytestmark = pytest.mark.gpu
 
@@ -46,3 +46,28 @@ def test_bone_phase_whose_pool_cannot_grow(ctx, concurrent):
     assert_maps(res, bone, roi, 12.5)
     # the injection is spent: the lists again
     assert_maps(analyze_thickness(bone, roi, 12.5, ctx=ctx, return_maps=True), bone, roi, 12.5)
+
+
+def assert_thickness(ctx, vol):
+    ref = O.local_thickness(vol, O.FOREGROUND)
+    got, sq = local_thickness(vol, Phase.FOREGROUND, ctx=ctx, return_squared=True)
+    assert np.array_equal(sq, ref.propagated)
+    assert np.array_equal(got.view(np.uint32), ref.thickness.view(np.uint32))
+
+
+@pytest.mark.parametrize("what,skip", [("template table", 0), ("diameter table", 0), ("disc tables", 0),
+                                       ("disc tables", 1)])
+def test_tables_by_radius_after_a_failed_allocation(ctx, what, skip):
+    """A context's first tables, and their growth: the call reports it and the next ones are exact."""
+    rng = np.random.default_rng(3)
+    small = (rng.random((20, 24, 40)) < 0.8).astype(np.uint8)
+    large = np.ones((90, 12, 20), np.uint8)  # squared radii to 7921: the tables grow
+    large[0, 0, 0] = 0
+    for vol in (small, large):
+        ctx.fail_allocation(what, skip)
+        with pytest.raises(BoneMorphometryError) as e:
+            local_thickness(vol, Phase.FOREGROUND, ctx=ctx)
+        assert e.value.status == _lib.BM_ERR_OOM and what in str(e.value)
+        if vol is large:
+            assert_thickness(ctx, small)
+        assert_thickness(ctx, vol)
