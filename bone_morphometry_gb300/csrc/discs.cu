@@ -24,6 +24,7 @@
 // on the order of the balls, so there is no sort by radius, no list of balls
 // per tile and no barrier between radii, and the non-selected voxels on a
 // ball's sphere (rho = 0 at the end) come out of the same passes.
+#include "disc_place.h"
 #include "kernels.h"
 
 namespace bm {
@@ -386,7 +387,7 @@ disc_list_kernel(const uint16_t* __restrict__ rmap, int pitch, Dims dm, int H, c
         if (cnt > kDiscSlots) {
           const unsigned long long first = atomicAdd(&ctr->disc_pool, (unsigned long long)cnt);
           if (first + cnt <= pool_cap) {
-            list[0].x = (uint32_t)first;
+            list[0] = disc_place(first);
             s_dst[k] = pool + first;
             s_count[k] = 0u;
             atomicOr(&s_full, 1u << k);
@@ -502,7 +503,7 @@ disc_paint_kernel(const uint32_t* __restrict__ hdr, const uint2* __restrict__ en
         count = min(e0 + unit, item & 0xffffu);
         const int px = px0 + (int)((item >> 16) & 255u), py = py0 + (int)(item >> 24);
         list = ent + (zh + (long long)py * npx + px) * kDiscSlots;
-        if ((item & 0xffffu) > kDiscSlots) list = pool + __ldg(list).x;
+        if ((item & 0xffffu) > kDiscSlots) list = pool + disc_first(__ldg(list));
         bx = px * kDiscPX - x0;
         by = py * kDiscPY - y0;
       }
