@@ -511,17 +511,32 @@ struct Phase {
     separable = hc.rmax <= kDiscMaxR2 && !tiles_asked();
   }
 
+  // No memory for the lists: the tile fill in the memory that they hold.  None of
+  // their kernels may be in flight.
+  void leave_separable() {
+    ctx->last_error.clear();
+    separable = false;
+    for (Buffer* b : {&ctx->ridgemap, &ctx->dischdr, &ctx->discent, &ctx->discpool}) release(*b);
+  }
+
   // Local thickness, after wait_edt: lists, then paint, queued to their end (but
   // for the tile fill's own waits).
   void lists() {
     ensure_lut(ctx, hc.rmax);
     if (!separable) return;
-    uint16_t* rmap = static_cast<uint16_t*>(ensure(ctx, ctx->ridgemap, narrow_bytes(), "ridge map"));
-    const size_t count = disc_header_count(dm);
-    hdr = static_cast<uint32_t*>(ensure(ctx, ctx->dischdr, count * 4, "disc headers"));
-    ent = static_cast<uint2*>(ensure(ctx, ctx->discent, count * kDiscSlots * sizeof(uint2), "disc lists"));
-    pool = static_cast<uint2*>(
-        ensure(ctx, ctx->discpool, disc_pool_entries(dm, hc.rmax) * sizeof(uint2), "disc pool"));
+    uint16_t* rmap = nullptr;
+    try {
+      rmap = static_cast<uint16_t*>(ensure(ctx, ctx->ridgemap, narrow_bytes(), "ridge map"));
+      const size_t count = disc_header_count(dm);
+      hdr = static_cast<uint32_t*>(ensure(ctx, ctx->dischdr, count * 4, "disc headers"));
+      ent = static_cast<uint2*>(ensure(ctx, ctx->discent, count * kDiscSlots * sizeof(uint2), "disc lists"));
+      pool = static_cast<uint2*>(
+          ensure(ctx, ctx->discpool, disc_pool_entries(dm, hc.rmax) * sizeof(uint2), "disc pool"));
+    } catch (const CallError& e) {
+      if (e.status != BM_ERR_OOM) throw;
+      leave_separable();
+      return;
+    }
     const size_t pool_cap = ctx->discpool.bytes / sizeof(uint2);
     const uint2* thr = static_cast<const uint2*>(ctx->discthr.ptr);
     const uint32_t* tmpl = static_cast<const uint32_t*>(ctx->disctmpl.ptr);
@@ -617,21 +632,14 @@ struct Phase {
       check(ctx, cudaMemsetAsync(&out->acc, 0, sizeof(StatsAccum), s), "memset");
       check(ctx, cudaMemsetAsync(&out->ctr.disc_pool, 0, sizeof(out->ctr.disc_pool), s), "memset");
       check(ctx, cudaMemsetAsync(&out->ctr.disc_overflow, 0, sizeof(out->ctr.disc_overflow), s), "memset");
-      bool room = true;
       try {
         ensure(ctx, ctx->discpool, (wanted + wanted / 8) * sizeof(uint2), "disc pool");
-      } catch (const CallError&) {
-        ctx->last_error.clear();
-        room = false;
-      }
-      if (room) {
         lists();
-        paint();
-      } else {
-        separable = false;
-        for (Buffer* b : {&ctx->ridgemap, &ctx->discent, &ctx->discpool}) release(*b);
-        tile_fill();
+      } catch (const CallError& e) {
+        if (e.status != BM_ERR_OOM) throw;
+        leave_separable();
       }
+      paint();
       check(ctx, cudaStreamSynchronize(s), "local thickness");
     }
     const PhaseOut& r = readback(ctx).out;

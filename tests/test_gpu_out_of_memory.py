@@ -71,3 +71,29 @@ def test_tables_by_radius_after_a_failed_allocation(ctx, what, skip):
         if vol is large:
             assert_thickness(ctx, small)
         assert_thickness(ctx, vol)
+
+
+LIST_BUFFERS = ["ridge map", "disc headers", "disc lists", "disc pool"]
+
+
+@pytest.mark.parametrize("what", LIST_BUFFERS)
+def test_no_memory_for_the_lists(ctx, what):
+    """The first allocation of any of the lists' buffers fails: the tile fill."""
+    vol = random_balls((40, 50, 70))
+    ctx.fail_allocation(what)
+    ctx.profile(True)
+    assert_thickness(ctx, vol)
+    assert ctx.kernel_times()["fill_rank"][0] > 0
+    ctx.profile(True)
+    assert_thickness(ctx, vol)  # the injection is spent: the lists
+    assert ctx.kernel_times()["fill_rank"][0] == 0
+    ctx.profile(False)
+
+
+@pytest.mark.parametrize("shape", [(40, 50, 70), (90, 100, 130)])
+def test_no_memory_for_one_phases_lists(ctx, shape):
+    """The bone phase's pool only; phases launched in turns (below 2^20 voxels) or one after the other."""
+    bone = random_balls(shape)
+    roi = np.ones_like(bone)
+    ctx.fail_allocation("disc pool")
+    assert_maps(analyze_thickness(bone, roi, 7.0, ctx=ctx, return_maps=True), bone, roi, 7.0)
