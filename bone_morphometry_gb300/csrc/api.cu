@@ -374,7 +374,7 @@ struct Phase {
   int mode;
   cudaStream_t s;
   bool edt_only = false, stats = false;
-  bool quantiles = false;  // needs d_map
+  bool quantiles = false;  // with stats
   uint32_t* d_edt = nullptr;
   float* d_map = nullptr;
   uint32_t* d_sq = nullptr;
@@ -385,16 +385,18 @@ struct Phase {
   StatsAccum acc;
   double osum[2] = {0.0, 0.0};
 
-  uint32_t* A = nullptr;        // x pass output (kept for the chain passes), y pass input
-  uint32_t* B = nullptr;        // y pass output
+  // x pass output (kept for the chain passes), y pass input; then the ridge map;
+  // then the f32 map, where the caller wants none
+  uint32_t* A = nullptr;
+  uint32_t* B = nullptr;        // y pass output; then the fill's diameters
   uint32_t* E = nullptr;        // z pass output
-  void* scratch = nullptr;      // envelope scratch of the flagged lines
   uint32_t* selbits = nullptr;  // selection bits
   PhaseOut* out = nullptr;
   uint8_t* yflags = nullptr;    // per-line flags of the windowed passes
   uint8_t* zflags = nullptr;
   bool near = false;            // the 16-bit passes first
   bool separable = false;
+  bool left_separable = false;  // there was no memory for the lists
   uint32_t* hdr = nullptr;      // disc lists
   uint2* ent = nullptr;
   uint2* pool = nullptr;
@@ -404,29 +406,56 @@ struct Phase {
   size_t bits_bytes() const { return (size_t)dm.nw() * dm.h * dm.d * sizeof(uint32_t); }
 
   size_t narrow_bytes() const { return (size_t)edt_near_pitch(dm.w) * dm.h * dm.d * 2; }
+  size_t map_bytes() const { return std::max(voxels() * 4, near ? narrow_bytes() : 0); }
+  size_t lists_bytes() const { return disc_header_count(dm) * kDiscSlots * sizeof(uint2); }
+  size_t flag_bytes() const { return (size_t)dm.w * (dm.h + dm.d); }  // lines along y and z
 
   // A forced site method or tile height asks for the tile fill.
   bool tiles_asked() const { return ctx->site_method != BM_SITES_AUTO || ctx->fill_rows != 0; }
 
+  // What the separable fill leaves of a budgeted phase's bytes for its pool.
+  size_t pool_room() const {
+    if (!ctx->budgeted) return SIZE_MAX;
+    const size_t limit = phase_limit_bytes(voxels());
+    const size_t held = 2 * std::max(voxels() * 4, narrow_bytes()) + narrow_bytes() + lists_bytes() +
+                        disc_header_count(dm) * 4 + 3 * bits_bytes() + ordered_sum_scratch_bytes(dm.n()) +
+                        quantile_scratch_words() * 4 + sizeof(PhaseOut) + flag_bytes();
+    return held < limit ? limit - held : 0;
+  }
+
+  // The 16-bit rows are padded to 16 voxels and the lists to 32 x 8 columns: of
+  // a volume a few voxels wide they would take many times its size (two voxels
+  // wide 48 and 200 bytes a voxel).  Such a volume keeps them while they are
+  // small: 512 x 512 x 2 local thickness 442 us, 770 with the tile fill.
+  bool narrow_fits() const {
+    constexpr size_t kSmall = 1ull << 30;
+    if (edt_only) return narrow_bytes() <= std::max(voxels() * 4, kSmall);
+    return lists_bytes() <= std::max(voxels() * 24, kSmall) && pool_room() > 0;
+  }
+
   // Buffers, and everything the phase accumulates into zeroed.
   void prepare() {
-    const size_t N = voxels();
     // the 16-bit passes, but where the caller has asked for the tile fill (its
     // chain passes read the 32-bit maps)
-    near = edt_only || !tiles_asked();
-    A = static_cast<uint32_t*>(ensure(ctx, ctx->dist, near ? narrow_bytes() : N * 4, "distance map"));
-    B = static_cast<uint32_t*>(ensure(ctx, ctx->dist2, std::max(N * 4, near ? narrow_bytes() : 0), "distance map"));
-    scratch = ensure(ctx, ctx->stack, edt_scratch_bytes(dm), "envelope scratch");
+    near = (edt_only || !tiles_asked()) && narrow_fits();
+    A = static_cast<uint32_t*>(ensure(ctx, ctx->dist, edt_only && near ? narrow_bytes() : map_bytes(), "distance map"));
+    B = static_cast<uint32_t*>(ensure(ctx, ctx->dist2, map_bytes(), "distance map"));
     selbits = static_cast<uint32_t*>(ensure(ctx, ctx->selbits, bits_bytes(), "selection bits"));
-    const size_t ny = (size_t)dm.w * dm.d, nz = (size_t)dm.w * dm.h;
-    out = phase_out(ctx, ny + nz);
+    out = phase_out(ctx, flag_bytes());
     yflags = reinterpret_cast<uint8_t*>(out + 1);
-    zflags = yflags + ny;
+    zflags = yflags + (size_t)dm.w * dm.d;
     // local thickness keeps the x pass output (the chain passes read it): the z
     // pass then writes its own map, in 16 bits for the separable fill
     E = d_edt ? d_edt
-              : static_cast<uint32_t*>(ensure(ctx, ctx->edtmap, near ? narrow_bytes() : N * 4, "distance map"));
-    check(ctx, cudaMemsetAsync(out, 0, sizeof(PhaseOut) + ny + nz, s), "memset");
+              : static_cast<uint32_t*>(ensure(ctx, ctx->edtmap, near ? narrow_bytes() : voxels() * 4, "distance map"));
+    check(ctx, cudaMemsetAsync(out, 0, sizeof(PhaseOut) + flag_bytes(), s), "memset");
+  }
+
+  // Envelope scratch of the flagged lines, in the memory that the disc lists take
+  // after them (allocated at their size where they may follow).
+  void* line_scratch() {
+    const size_t lists_follow = near && !edt_only && !left_separable ? lists_bytes() : 0;
+    return ensure(ctx, ctx->discent, std::max(edt_scratch_bytes(dm), lists_follow), "envelope scratch");
   }
 
   // The x and y passes of planes z0 .. z1-1: both work within a plane, so a slab
@@ -459,11 +488,12 @@ struct Phase {
     A = static_cast<uint32_t*>(ensure(ctx, ctx->dist, voxels() * 4, "distance map"));
     timed(ctx, KF_EDT_X, s, "edt x pass",
           [&] { return launch_edt_x(a, b, mode, sd, A + off, sel, &out->ctr, s, &ctx->launches); });
+    void* lines = line_scratch();
     timed(ctx, KF_EDT_Y, s, "edt y pass", [&] {
       const cudaError_t e =
           launch_edt_window(1, A + off, B + off, sd, flags, &out->ctr, ctx->wait_cycles, only, s, &ctx->launches);
       if (e != cudaSuccess) return e;
-      return launch_edt_redo(1, A + off, B + off, sd, scratch, flags, &out->ctr, s, &ctx->launches);
+      return launch_edt_redo(1, A + off, B + off, sd, lines, flags, &out->ctr, s, &ctx->launches);
     });
   }
 
@@ -489,11 +519,12 @@ struct Phase {
       // the flagged lines, from 32-bit x and y passes
       const unsigned long long sites = hc.sites;
       if (near) wide_xy(dm, d_a, d_b, selbits, 0, yflags, zflags);
+      void* lines = line_scratch();
       timed(ctx, KF_EDT_Z, s, "edt z lines", [&] {
         if (near && !d_edt)
-          return launch_edt_near_redo(B, reinterpret_cast<uint16_t*>(E), dm, scratch, zflags, &out->ctr, s,
+          return launch_edt_near_redo(B, reinterpret_cast<uint16_t*>(E), dm, lines, zflags, &out->ctr, s,
                                       &ctx->launches);
-        return launch_edt_redo(2, B, E, dm, scratch, zflags, &out->ctr, s, &ctx->launches);
+        return launch_edt_redo(2, B, E, dm, lines, zflags, &out->ctr, s, &ctx->launches);
       });
       read_counters();
       check(ctx, cudaStreamSynchronize(s), "edt");
@@ -508,7 +539,7 @@ struct Phase {
            phase_name(phase));
     }
     // The separable fill (discs.cu) up to radius 127, where its packed discs end.
-    separable = hc.rmax <= kDiscMaxR2 && !tiles_asked();
+    separable = near && !edt_only && hc.rmax <= kDiscMaxR2;
   }
 
   // No memory for the lists: the tile fill in the memory that they hold.  None of
@@ -516,7 +547,8 @@ struct Phase {
   void leave_separable() {
     ctx->last_error.clear();
     separable = false;
-    for (Buffer* b : {&ctx->ridgemap, &ctx->dischdr, &ctx->discent, &ctx->discpool}) release(*b);
+    left_separable = true;
+    for (Buffer* b : {&ctx->dischdr, &ctx->discent, &ctx->discpool}) release(*b);
   }
 
   // Local thickness, after wait_edt: lists, then paint, queued to their end (but
@@ -524,14 +556,17 @@ struct Phase {
   void lists() {
     ensure_lut(ctx, hc.rmax);
     if (!separable) return;
-    uint16_t* rmap = nullptr;
+    // a budgeted context's phase holds either fill's buffers
+    if (ctx->budgeted)
+      for (Buffer* b : {&ctx->chainmap, &ctx->ridges, &ctx->ridgebits, &ctx->bincounts, &ctx->binoffsets, &ctx->binentries})
+        release(*b);
+    uint16_t* rmap = reinterpret_cast<uint16_t*>(A);  // the y pass has read it
     try {
-      rmap = static_cast<uint16_t*>(ensure(ctx, ctx->ridgemap, narrow_bytes(), "ridge map"));
       const size_t count = disc_header_count(dm);
       hdr = static_cast<uint32_t*>(ensure(ctx, ctx->dischdr, count * 4, "disc headers"));
-      ent = static_cast<uint2*>(ensure(ctx, ctx->discent, count * kDiscSlots * sizeof(uint2), "disc lists"));
-      pool = static_cast<uint2*>(
-          ensure(ctx, ctx->discpool, disc_pool_entries(dm, hc.rmax) * sizeof(uint2), "disc pool"));
+      ent = static_cast<uint2*>(ensure(ctx, ctx->discent, lists_bytes(), "disc lists"));
+      const size_t first = disc_pool_entries(dm, hc.rmax) * sizeof(uint2);
+      pool = static_cast<uint2*>(ensure(ctx, ctx->discpool, std::min(first, pool_room()), "disc pool"));
     } catch (const CallError& e) {
       if (e.status != BM_ERR_OOM) throw;
       leave_separable();
@@ -565,13 +600,14 @@ struct Phase {
   // The whole transform in 32 bits, for the tile fill after the 16-bit passes.
   void widen() {
     E = static_cast<uint32_t*>(ensure(ctx, ctx->edtmap, voxels() * 4, "distance map"));
-    check(ctx, cudaMemsetAsync(yflags, 0, (size_t)dm.w * (dm.d + dm.h), s), "memset");
+    check(ctx, cudaMemsetAsync(yflags, 0, flag_bytes(), s), "memset");
     wide_xy(dm, d_a, d_b, selbits, 0, yflags, nullptr);
+    void* lines = line_scratch();
     timed(ctx, KF_EDT_Z, s, "edt z pass", [&] {
       const cudaError_t e =
           launch_edt_window(2, B, E, dm, zflags, &out->ctr, ctx->wait_cycles, nullptr, s, &ctx->launches);
       if (e != cudaSuccess) return e;
-      return launch_edt_redo(2, B, E, dm, scratch, zflags, &out->ctr, s, &ctx->launches);
+      return launch_edt_redo(2, B, E, dm, lines, zflags, &out->ctr, s, &ctx->launches);
     });
     read_counters();
     check(ctx, cudaStreamSynchronize(s), "edt");
@@ -580,6 +616,8 @@ struct Phase {
   }
 
   void tile_fill() {
+    if (ctx->budgeted)
+      for (Buffer* b : {&ctx->dischdr, &ctx->discpool}) release(*b);
     if (near) widen();
     const uint4* lut = static_cast<const uint4*>(ctx->lut.ptr);
     const float* dia = static_cast<const float*>(ctx->lutf.ptr);
@@ -613,8 +651,8 @@ struct Phase {
     std::memcpy(&tb, &two_s, 4);
     const int e2s = (int)(tb >> 23);
     e_lo = (e2s >= 1 && e2s + kFixedSpan <= 254) ? e2s : 4096;  // 4096: no fixed-point path
-    // the statistics' ordered sums read the f32 map: keep one when the caller wants none
-    float* cmap = (stats && !d_map) ? static_cast<float*>(ensure(ctx, ctx->ordmap, voxels() * 4, "thickness map")) : d_map;
+    // the statistics' sums and quantiles read the f32 map: kept in A when the caller wants none
+    float* cmap = stats && !d_map ? reinterpret_cast<float*>(A) : d_map;
     timed(ctx, KF_CLEAN_FINAL, s, "cleanup", [&] {
       return launch_cleanup(dmap, selbits, nzbits, inbits, dm, scale, cmap, &out->acc, e_lo, s, &ctx->launches);
     });
@@ -627,13 +665,16 @@ struct Phase {
     check(ctx, cudaStreamSynchronize(s), "local thickness");
     if (separable && readback(ctx).out.ctr.disc_overflow) {
       // the lists' pool ran out: again with one of the size that they wanted, or,
-      // where there is no memory for it, with the tile fill in the lists' memory
+      // where there is no memory (or no room in the budget) for it, with the tile
+      // fill in the lists' memory
       const unsigned long long wanted = readback(ctx).out.ctr.disc_pool;
       check(ctx, cudaMemsetAsync(&out->acc, 0, sizeof(StatsAccum), s), "memset");
       check(ctx, cudaMemsetAsync(&out->ctr.disc_pool, 0, sizeof(out->ctr.disc_pool), s), "memset");
       check(ctx, cudaMemsetAsync(&out->ctr.disc_overflow, 0, sizeof(out->ctr.disc_overflow), s), "memset");
       try {
-        ensure(ctx, ctx->discpool, (wanted + wanted / 8) * sizeof(uint2), "disc pool");
+        const size_t room = pool_room();
+        if (wanted * sizeof(uint2) > room) throw CallError{BM_ERR_OOM};
+        ensure(ctx, ctx->discpool, std::min<size_t>((wanted + wanted / 8) * sizeof(uint2), room), "disc pool");
         lists();
       } catch (const CallError& e) {
         if (e.status != BM_ERR_OOM) throw;
@@ -872,6 +913,7 @@ bm_ctx* twin_of(bm_ctx* ctx) {
   t->site_method = ctx->site_method;
   t->fill_rows = ctx->fill_rows;
   t->wait_cycles = ctx->wait_cycles;
+  t->budgeted = ctx->budgeted;
   ctx->twin = t;
   return t;
 }
@@ -974,9 +1016,8 @@ int tbth_phases(bm_ctx* ctx, const uint8_t* d_bone, const uint8_t* d_roi, Dims d
   bone.quantiles = want_q && th;
   marrow.quantiles = want_q && sp;
   bone.scale = marrow.scale = (float)spacing;  // metrics.rs:213
-  auto map_of = [&](bm_ctx* c, float* caller) {
-    return caller || !want_q ? caller : static_cast<float*>(ensure(c, c->qmap, (size_t)N * 4, "quantile map"));
-  };
+  bone.d_map = d_thmap;
+  marrow.d_map = d_spmap;
   if (tw) {
     check(ctx, cudaEventRecord(ctx->inputs_ready, s), "event record");
     check(ctx, cudaStreamWaitEvent(tw->stream, ctx->inputs_ready, 0), "stream wait");
@@ -988,7 +1029,6 @@ int tbth_phases(bm_ctx* ctx, const uint8_t* d_bone, const uint8_t* d_roi, Dims d
   if (tw) on_twin(ctx, tw, [&] { marrow.z(); });
   check_roi_counts(ctx, N, flags);
 
-  bone.d_map = map_of(ctx, d_thmap);
   bone.wait_edt();
   if (!tw) {
     bone.lists();
@@ -996,7 +1036,6 @@ int tbth_phases(bm_ctx* ctx, const uint8_t* d_bone, const uint8_t* d_roi, Dims d
     bone.finish();
     int st = report_phase(bone, ctx, spacing, th);
     if (st) return st;
-    marrow.d_map = map_of(ctx, d_spmap);
     run_phase(marrow);
     fence.done = true;
     return report_phase(marrow, ctx, spacing, sp);
@@ -1014,7 +1053,6 @@ int tbth_phases(bm_ctx* ctx, const uint8_t* d_bone, const uint8_t* d_roi, Dims d
     }
   };
   try_twin([&] {
-    marrow.d_map = map_of(tw, d_spmap);
     marrow.wait_edt();
   });
   // Decided here, once: a phase may turn to the tile fill later, in finish, when
@@ -1149,12 +1187,12 @@ void set_thread_error(const char* msg) { g_create_error = msg; }
 // The per-call working buffers of a context (released by bm_ctx_trim; the
 // cached tables stay).
 std::vector<Buffer*> work_buffers(bm_ctx* ctx) {
-  return {&ctx->in_a,      &ctx->in_b,       &ctx->dist,        &ctx->dist2,   &ctx->stack,  &ctx->edtmap,
+  return {&ctx->in_a,      &ctx->in_b,       &ctx->dist,        &ctx->dist2,   &ctx->edtmap,
           &ctx->chainmap,  &ctx->fillmap,    &ctx->selbits,     &ctx->ridgebits, &ctx->ridges, &ctx->phaseout,
           &ctx->outmap,    &ctx->outmap2,     &ctx->occ,     &ctx->rank,   &ctx->rvals,
           &ctx->bincounts, &ctx->binoffsets, &ctx->binentries,  &ctx->scanscratch, &ctx->qhist,
-          &ctx->qtargets,  &ctx->qmap,       &ctx->rgeo,        &ctx->ordmap,  &ctx->ordscratch,
-          &ctx->tileorder, &ctx->ridgemap,   &ctx->dischdr,     &ctx->discent, &ctx->discpool,
+          &ctx->qtargets,  &ctx->qmap,       &ctx->rgeo,        &ctx->ordscratch,
+          &ctx->tileorder, &ctx->dischdr,     &ctx->discent, &ctx->discpool,
           &ctx->nzbits,    &ctx->inbits};
 }
 

@@ -142,6 +142,11 @@ struct Buffer {
   size_t bytes = 0;
 };
 
+// What one phase of bm_tbth_tbsp holds at most in a budgeted context, from which
+// bm_footprint_bytes follows (the tile fill: five u32 maps, envelope scratch 8,
+// ridge records <= 8, bin entries ~5, masks and sums ~1 bytes a voxel, and its bins).
+inline uint64_t phase_limit_bytes(uint64_t voxels) { return voxels * 46u + (32ull << 20); }
+
 struct Counters {  // device-side counters of one phase
   unsigned long long sites;     // non-selected voxels
   unsigned long long selected;  // selected voxels
@@ -197,6 +202,7 @@ struct bm_ctx {
   cudaStream_t stream = nullptr;
   void* pinned = nullptr;      // page-locked readback area (bm::Readback)
   cudaEvent_t counted = nullptr;  // the ROI counts have been copied
+  bool budgeted = false;       // a server's worker: a phase stays within phase_limit_bytes
   std::string fail_what;       // the buffer whose allocation is to fail (bm_ctx_fail_allocation), and
   int fail_skip = 0;           // how many of them succeed before
   // second context (own stream and buffers) that runs the marrow phase of
@@ -220,7 +226,6 @@ struct bm_ctx {
   bm::Buffer in_a, in_b;       // staged host inputs
   bm::Buffer dist, dist2;      // u32 EDT ping/pong
   bm::Buffer edtmap, chainmap; // u32 z-pass output kept apart from the x pass's, and the site-chain map
-  bm::Buffer stack;            // EDT line scratch
   bm::Buffer fillmap;          // u32 propagated r^2
   bm::Buffer selbits, ridgebits; // row-padded bitmasks: selected voxels, ridge voxels
   bm::Buffer nzbits, inbits;   // the r^2 map's nonzero voxels, and those without a zero 26-neighbour
@@ -234,10 +239,11 @@ struct bm_ctx {
   bm::Buffer bincounts, binoffsets, binentries, scanscratch;
   // cached sphere lattice-point table for r2 in [0, surf_max]
   bm::Buffer surf_off, surf_pts;
-  // separable fill: u16 ridge map, list headers and disc lists; cached tables by squared radius
-  bm::Buffer ridgemap, dischdr, discent, discpool, discthr, disctmpl;
-  bm::Buffer qhist, qtargets, qmap;  // quantile histograms, targets, map scratch
-  bm::Buffer ordmap, ordscratch;  // f32 map for the ordered sums, and their scratch
+  // separable fill: list headers and disc lists (before them: scratch of the
+  // distance transform's flagged lines); cached tables by squared radius
+  bm::Buffer dischdr, discent, discpool, discthr, disctmpl;
+  bm::Buffer qhist, qtargets, qmap;  // quantile histograms, targets; values of bm_nonzero_stats
+  bm::Buffer ordscratch;       // the ordered sums' scratch
   bm::Buffer tileorder;        // the fill's tile order (heaviest first) and its bucket counts
   uint32_t surf_max = 0;
 

@@ -32,6 +32,8 @@ double now_s() {
   return duration<double>(steady_clock::now().time_since_epoch()).count();
 }
 
+constexpr double kNoBudget = 1e300;
+
 struct Job {
   bm_specimen sp{};
   unsigned flags = 0;
@@ -98,6 +100,7 @@ class Pool {
       c->site_method = settings.site_method;
       c->fill_rows = settings.fill_rows;
       c->split_phases = settings.split_phases;
+      c->budgeted = budget < kNoBudget;
       ctxs_.push_back(c);
     }
     if (status_ == BM_OK)
@@ -298,15 +301,10 @@ struct bm_server {
 extern "C" {
 
 uint64_t bm_footprint_bytes(size_t width, size_t height, size_t depth) {
-  // per voxel: inputs 2; per phase (the two phases run side by side, each on
-  // its own buffers): x, y and z pass maps 8, envelope scratch 8, u16 ridge map
-  // 2, disc lists 12 and their pool (4.5 at radius 40), f32 thickness map 4 (read by the
-  // statistics' ordered sums, ~0.2 more of their scratch), quantile map 4,
-  // bitmasks ~1; the tile fill (radii above 127) takes 4 more for the maps, a chain map 4, ridge
-  // records <= 8 and bin entries ~5 in place of the ridge map and the lists;
-  // tables 2 x 64 MiB
+  // inputs 2 bytes a voxel; the two phases side by side, each on its own buffers
+  // (1 byte for rounding); tables 64 MiB
   const uint64_t n = (uint64_t)width * height * depth;
-  return n * 95u + (128ull << 20);
+  return n * 3u + 2u * phase_limit_bytes(n) + (64ull << 20);
 }
 
 int bm_ctx_set_workers(bm_ctx* ctx, int workers) {
@@ -336,7 +334,7 @@ int bm_batch_tbth_tbsp(bm_ctx* ctx, const bm_specimen* items, size_t n, int devi
   }
   if (!ctx->pool) {
     int st = BM_OK;
-    ctx->pool = pool_create(ctx->device, ctx->workers, 1e300, want, &st);
+    ctx->pool = pool_create(ctx->device, ctx->workers, kNoBudget, want, &st);
     if (!ctx->pool) return st;
   }
   std::vector<Job> jobs(n);

@@ -73,7 +73,7 @@ def test_tables_by_radius_after_a_failed_allocation(ctx, what, skip):
         assert_thickness(ctx, vol)
 
 
-LIST_BUFFERS = ["ridge map", "disc headers", "disc lists", "disc pool"]
+LIST_BUFFERS = ["disc headers", "disc lists", "disc pool"]
 
 
 @pytest.mark.parametrize("what", LIST_BUFFERS)
