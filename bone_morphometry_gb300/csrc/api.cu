@@ -385,8 +385,8 @@ struct Phase {
   StatsAccum acc;
   double osum[2] = {0.0, 0.0};
 
-  // x pass output (kept for the chain passes), y pass input; then the ridge map;
-  // then the f32 map, where the caller wants none
+  // x pass output (kept for the chain passes), y pass input; then the ridge map,
+  // or the flagged lines in 32 bits; then the f32 map, where the caller wants none
   uint32_t* A = nullptr;
   uint32_t* B = nullptr;        // y pass output; then the fill's diameters
   uint32_t* E = nullptr;        // z pass output
@@ -522,7 +522,7 @@ struct Phase {
       void* lines = line_scratch();
       timed(ctx, KF_EDT_Z, s, "edt z lines", [&] {
         if (near && !d_edt)
-          return launch_edt_near_redo(B, reinterpret_cast<uint16_t*>(E), dm, lines, zflags, &out->ctr, s,
+          return launch_edt_near_redo(B, reinterpret_cast<uint16_t*>(E), A, dm, lines, zflags, &out->ctr, s,
                                       &ctx->launches);
         return launch_edt_redo(2, B, E, dm, lines, zflags, &out->ctr, s, &ctx->launches);
       });
@@ -598,7 +598,16 @@ struct Phase {
   }
 
   // The whole transform in 32 bits, for the tile fill after the 16-bit passes.
+  // Beyond the separable fill's radius the flagged lines are in A already, and the
+  // chain passes, which read the x and y passes' maps, do not run.
   void widen() {
+    if (hc.rmax > kDiscMaxR2) {
+      timed(ctx, KF_EDT_Z, s, "edt z lines", [&] {
+        return launch_edt_widen(reinterpret_cast<const uint16_t*>(E), A, dm, zflags, s, &ctx->launches);
+      });
+      E = A;
+      return;
+    }
     E = static_cast<uint32_t*>(ensure(ctx, ctx->edtmap, voxels() * 4, "distance map"));
     check(ctx, cudaMemsetAsync(yflags, 0, flag_bytes(), s), "memset");
     wide_xy(dm, d_a, d_b, selbits, 0, yflags, nullptr);
@@ -632,8 +641,9 @@ struct Phase {
     timed(ctx, KF_RIDGE, s, "ridge kernel",
           [&] { return launch_ridges(E, selbits, dm, lut, ridges, &out->ctr, occ, rbits, s, &ctx->launches); });
     // E is the context's map: the chain passes may reuse it
-    uint32_t* F = fill_phase(ctx, dm, ridges, &out->ctr, selected, hc.rmax, occ, selbits, A, B, E, rbits,
-                             d_sq ? d_sq : B, s);
+    static_assert(kChainMaxR2 <= kDiscMaxR2, "no chain passes after a widened transform");
+    uint32_t* F = fill_phase(ctx, dm, ridges, &out->ctr, selected, hc.rmax, occ, selbits, E == A ? nullptr : A, B, E,
+                             rbits, d_sq ? d_sq : B, s);
     float* dmap = reinterpret_cast<float*>(F == d_sq ? B : F);
     timed(ctx, KF_CLEAN_FINAL, s, "diameters",
           [&] { return launch_diameters(F, dm, dia, dmap, nzbits, s, &ctx->launches); });

@@ -249,11 +249,12 @@ edt_x_vec_kernel(const uint8_t* __restrict__ a, const uint8_t* __restrict__ b, D
 // One thread per line; consecutive threads take consecutive x so that every
 // load and store of the line data is a coalesced row.  The envelope stack
 // (position, f) lives in global scratch, k-major, and is cached by L1/L2.
-// Out uint16_t: a map with strides of its own, values beyond 16 bits cut to 0xffff.
+// Out uint16_t: a map with strides of its own, values beyond 16 bits cut to
+// 0xffff, beside the whole values in wide (at in's strides).
 template <class Out>
 __global__ void __launch_bounds__(256)
-edt_line_kernel(const uint32_t* __restrict__ in, Out* __restrict__ out, int n, long long stride, int w,
-                long long outer, long long out_stride, long long out_outer, long long nlines,
+edt_line_kernel(const uint32_t* __restrict__ in, Out* __restrict__ out, uint32_t* __restrict__ wide, int n,
+                long long stride, int w, long long outer, long long out_stride, long long out_outer, long long nlines,
                 uint32_t* __restrict__ spos, uint32_t* __restrict__ sf, Counters* __restrict__ ctr, int track_max,
                 const uint8_t* __restrict__ only) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -261,7 +262,10 @@ edt_line_kernel(const uint32_t* __restrict__ in, Out* __restrict__ out, int n, l
   if (t < nlines && (only == nullptr || only[t])) {
     const long long base = (t / w) * outer + (t % w);
     Out* to = out + (t / w) * out_outer + (t % w);
-    auto put = [&](int q, uint32_t v) { to[(long long)q * out_stride] = (Out)(sizeof(Out) == 2 ? min(v, 0xffffu) : v); };
+    auto put = [&](int q, uint32_t v) {
+      to[(long long)q * out_stride] = (Out)(sizeof(Out) == 2 ? min(v, 0xffffu) : v);
+      if (sizeof(Out) == 2) wide[base + (long long)q * stride] = v;
+    };
     int k = -1;
     long long p1 = 0, F1 = 0;  // stack top
     long long p0 = 0, F0 = 0;  // entry below the top (valid when k >= 1)
@@ -968,6 +972,22 @@ edt_near_tma_kernel(const __grid_constant__ CUtensorMap tin, uint32_t* __restric
   }
 }
 
+// The lines along z that redo does not flag, from 16 to 32 bits (a thread per
+// line and kWidenZ planes; bytes alone bound it).
+constexpr int kWidenZ = 64;
+__global__ void __launch_bounds__(256)
+edt_widen_kernel(const uint16_t* __restrict__ narrow, uint32_t* __restrict__ wide, Dims dm, int pitch,
+                 const uint8_t* __restrict__ redo) {
+  const int x = blockIdx.x * 256 + threadIdx.x, y = blockIdx.y, z0 = blockIdx.z * kWidenZ;
+  if (x >= dm.w || redo[(long long)y * dm.w + x]) return;
+  const uint16_t* from = narrow + ((long long)z0 * dm.h + y) * pitch + x;
+  uint32_t* to = wide + ((long long)z0 * dm.h + y) * dm.w + x;
+  const int planes = min(kWidenZ, dm.d - z0);
+#pragma unroll 8
+  for (int z = 0; z < planes; ++z)
+    to[(long long)z * dm.w * dm.h] = from[(long long)z * pitch * dm.h];
+}
+
 }  // namespace
 
 size_t edt_scratch_bytes(Dims dm) {
@@ -1043,7 +1063,7 @@ cudaError_t launch_edt_line(int axis, const uint32_t* in, uint32_t* out, Dims dm
   uint32_t* spos = static_cast<uint32_t*>(scratch);
   uint32_t* sf = spos + (size_t)nlines * n;
   const long long blocks = (nlines + 255) / 256;
-  edt_line_kernel<<<(unsigned)blocks, 256, 0, s>>>(in, out, n, stride, dm.w, outer, stride, outer, nlines, spos, sf,
+  edt_line_kernel<<<(unsigned)blocks, 256, 0, s>>>(in, out, nullptr, n, stride, dm.w, outer, stride, outer, nlines, spos, sf,
                                                    ctr, axis == 2 ? 1 : 0, nullptr);
   ++*launches;
   return cudaGetLastError();
@@ -1138,21 +1158,29 @@ cudaError_t launch_edt_redo(int axis, const uint32_t* in, uint32_t* out, Dims dm
   const Lines l = lines_of(axis, dm);
   uint32_t* spos = static_cast<uint32_t*>(scratch);
   uint32_t* sf = spos + (size_t)l.count * l.n;
-  edt_line_kernel<<<(unsigned)((l.count + 255) / 256), 256, 0, s>>>(in, out, l.n, l.stride, dm.w, l.outer, l.stride,
-                                                                   l.outer, l.count, spos, sf, ctr, axis == 2 ? 1 : 0,
-                                                                   redo);
+  edt_line_kernel<<<(unsigned)((l.count + 255) / 256), 256, 0, s>>>(in, out, nullptr, l.n, l.stride, dm.w, l.outer,
+                                                                   l.stride, l.outer, l.count, spos, sf, ctr,
+                                                                   axis == 2 ? 1 : 0, redo);
   ++*launches;
   return cudaGetLastError();
 }
 
-cudaError_t launch_edt_near_redo(const uint32_t* in, uint16_t* out, Dims dm, void* scratch, const uint8_t* redo,
+cudaError_t launch_edt_near_redo(const uint32_t* in, uint16_t* out, uint32_t* wide, Dims dm, void* scratch, const uint8_t* redo,
                                  Counters* ctr, cudaStream_t s, unsigned long long* launches) {
   const Lines l = lines_of(2, dm);
   const long long pitch = edt_near_pitch(dm.w);
   uint32_t* spos = static_cast<uint32_t*>(scratch);
   uint32_t* sf = spos + (size_t)l.count * l.n;
-  edt_line_kernel<<<(unsigned)((l.count + 255) / 256), 256, 0, s>>>(in, out, l.n, l.stride, dm.w, l.outer,
+  edt_line_kernel<<<(unsigned)((l.count + 255) / 256), 256, 0, s>>>(in, out, wide, l.n, l.stride, dm.w, l.outer,
                                                                    pitch * dm.h, pitch, l.count, spos, sf, ctr, 1, redo);
+  ++*launches;
+  return cudaGetLastError();
+}
+
+cudaError_t launch_edt_widen(const uint16_t* narrow, uint32_t* wide, Dims dm, const uint8_t* redo, cudaStream_t s,
+                             unsigned long long* launches) {
+  const dim3 grid((unsigned)((dm.w + 255) / 256), (unsigned)dm.h, (unsigned)((dm.d + kWidenZ - 1) / kWidenZ));
+  edt_widen_kernel<<<grid, 256, 0, s>>>(narrow, wide, dm, edt_near_pitch(dm.w), redo);
   ++*launches;
   return cudaGetLastError();
 }

@@ -69,9 +69,13 @@ cudaError_t launch_edt_near_xy(const uint8_t* a, const uint8_t* b, int mode, Dim
 // wide (32 bits at the volume's pitch) or narrow (16 bits at edt_near_pitch): the one not null.
 cudaError_t launch_edt_near_z(const uint16_t* ymap, uint32_t* wide, uint16_t* narrow, Dims dm, uint8_t* redo,
                               Counters* ctr, cudaStream_t s, unsigned long long* launches);
-// The flagged lines of a narrow result, from the 32-bit y pass' output.
-cudaError_t launch_edt_near_redo(const uint32_t* in, uint16_t* out, Dims dm, void* scratch, const uint8_t* redo,
-                                 Counters* ctr, cudaStream_t s, unsigned long long* launches);
+// The flagged lines of a narrow result, from the 32-bit y pass' output; in 32
+// bits in wide too.
+cudaError_t launch_edt_near_redo(const uint32_t* in, uint16_t* out, uint32_t* wide, Dims dm, void* scratch,
+                                 const uint8_t* redo, Counters* ctr, cudaStream_t s, unsigned long long* launches);
+// The other lines of a narrow result into wide.
+cudaError_t launch_edt_widen(const uint16_t* narrow, uint32_t* wide, Dims dm, const uint8_t* redo, cudaStream_t s,
+                             unsigned long long* launches);
 
 // out (zeroed): ROI voxels, ROI-clipped bone voxels, and those of them with a
 // 6-neighbour outside the volume or the ROI (metrics.rs:166-202).  rbits, bbits:
