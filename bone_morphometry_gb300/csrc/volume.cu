@@ -1,7 +1,7 @@
 // Voxel counts of volume_metrics (metrics.rs:123-132, 166-202).
 //
-// The first kernel packs the ROI and the ROI-clipped bone into bitmasks, one
-// warp per row and 16 voxels per lane, at any address, and counts both; the
+// The first kernel packs the ROI and the ROI-clipped bone into bitmasks, 16
+// voxels per lane and rows of a warp (or less), at any address, and counts both; the
 // second finds the boundary voxels 32 at a time from seven words.  The inputs
 // are read once (2 bytes a voxel); the masks, an eighth of that, stay in L2.
 // 430 x 389 x 401: 611 us a voxel per thread with byte loads, 92 four voxels per
@@ -39,17 +39,23 @@ __device__ __forceinline__ void add_block(uint32_t v, unsigned long long* out) {
   }
 }
 
+// 2^LG lanes take a row (an even number, of which pairs make a word), so that a
+// warp takes several rows of a narrow volume: 512 x 512 x 2 73 us with a warp per
+// row, 20 here, 512 x 512 x 128 74 and 32.
+template <int LG>
 __global__ void __launch_bounds__(kPackWarps * 32)
 pack_rows_kernel(const uint8_t* __restrict__ bone, const uint8_t* __restrict__ roi, Dims dm,
                  uint32_t* __restrict__ rbits, uint32_t* __restrict__ bbits, unsigned long long* __restrict__ out) {
   const ByteVolume vr(roi, dm.n()), vb(bone, dm.n());
   const int lane = threadIdx.x & 31, nw = dm.nw(), nvec = (dm.w + 15) >> 4;
+  constexpr int kSeg = 1 << LG;
   const long long rows = (long long)dm.h * dm.d;
   uint32_t n_roi = 0, n_bone = 0;  // 2^32 voxels over many threads: 32 bits hold a thread's
-  for (long long row = (long long)blockIdx.x * kPackWarps + (threadIdx.x >> 5); row < rows;
-       row += (long long)gridDim.x * kPackWarps) {
-    for (int v0 = 0; v0 < nvec; v0 += 32) {
-      const int v = v0 + lane;
+  for (long long row0 = (long long)blockIdx.x * kPackWarps + (threadIdx.x >> 5); (row0 << (5 - LG)) < rows;
+       row0 += (long long)gridDim.x * kPackWarps) {
+    const long long row = (row0 << (5 - LG)) + (lane >> LG);
+    for (int v0 = 0; v0 < nvec; v0 += kSeg) {
+      const int v = LG == 5 || row < rows ? v0 + (lane & (kSeg - 1)) : nvec;
       uint32_t r = 0, b = 0;
       if (v < nvec) {
         const long long at = row * dm.w + 16 * v;
@@ -97,11 +103,24 @@ boundary_kernel(const uint32_t* __restrict__ rbits, const uint32_t* __restrict__
 
 }  // namespace
 
+namespace {
+// The fewest lanes that hold a row.
+template <int LG>
+void pack_rows(const uint8_t* bone, const uint8_t* roi, Dims dm, uint32_t* rbits, uint32_t* bbits,
+               unsigned long long* out, cudaStream_t s) {
+  if constexpr (LG < 5) {
+    if (dm.w > 16 << LG) return pack_rows<LG + 1>(bone, roi, dm, rbits, bbits, out, s);
+  }
+  constexpr long long kRows = kPackWarps << (5 - LG);  // of a block
+  long long blocks = ((long long)dm.h * dm.d + kRows - 1) / kRows;
+  if (blocks > 152 * 12) blocks = 152 * 12;
+  pack_rows_kernel<LG><<<(unsigned)blocks, kPackWarps * 32, 0, s>>>(bone, roi, dm, rbits, bbits, out);
+}
+}  // namespace
+
 cudaError_t launch_volume_counts(const uint8_t* bone, const uint8_t* roi, Dims dm, uint32_t* rbits, uint32_t* bbits,
                                  unsigned long long* out, cudaStream_t s, unsigned long long* launches) {
-  long long blocks = ((long long)dm.h * dm.d + kPackWarps - 1) / kPackWarps;
-  if (blocks > 152 * 12) blocks = 152 * 12;
-  pack_rows_kernel<<<(unsigned)blocks, kPackWarps * 32, 0, s>>>(bone, roi, dm, rbits, bbits, out);
+  pack_rows<1>(bone, roi, dm, rbits, bbits, out, s);
   const int plane = dm.nw() * dm.h;
   boundary_kernel<<<dim3((unsigned)((plane + kPackWarps * 32 - 1) / (kPackWarps * 32)),
                          (unsigned)((dm.d + kEdgeZ - 1) / kEdgeZ)),
