@@ -515,7 +515,7 @@ struct Phase {
   void wait_edt() {
     check(ctx, cudaStreamSynchronize(s), "edt");
     hc = readback(ctx).ctr;
-    if (hc.z_redo && !hc.status) {
+    if (hc.z_redo && !hc.status && hc.sites) {  // (without a site every line is flagged: refused below)
       // the flagged lines, from 32-bit x and y passes
       const unsigned long long sites = hc.sites;
       if (near) wide_xy(dm, d_a, d_b, selbits, 0, yflags, zflags);

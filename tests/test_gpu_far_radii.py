@@ -7,7 +7,8 @@ import numpy as np
 import pytest
 
 import oracle as O
-from bone_morphometry_gb300 import Phase, analyze_thickness, local_thickness
+from bone_morphometry_gb300 import (BoneMorphometryError, Phase, _lib, analyze_thickness,
+                                    euclidean_distance_transform_squared, local_thickness)
 from refstats import assert_reference_stats
 
 pytestmark = pytest.mark.gpu
@@ -56,3 +57,13 @@ def test_far_phase_beside_a_near_one(gpu_ctx, concurrent):
         ref = O.local_thickness(O.phase_inside(bone, roi, sel), O.FOREGROUND)
         assert np.array_equal(gmap.view(np.uint32), ref.thickness.view(np.uint32))
         assert_reference_stats(got, ref.thickness, 3.0)
+
+
+@pytest.mark.parametrize("call", [local_thickness, euclidean_distance_transform_squared])
+def test_all_selected_is_refused_after_one_transform(gpu_ctx, call):
+    vol = np.ones((20, 30, 40), np.uint8)
+    before = gpu_ctx.launches
+    with pytest.raises(BoneMorphometryError) as e:
+        call(vol, Phase.FOREGROUND, ctx=gpu_ctx)
+    assert e.value.status == _lib.BM_ERR_ALL_SELECTED
+    assert gpu_ctx.launches - before == 3  # x, y and z in 16 bits
