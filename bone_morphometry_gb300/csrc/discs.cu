@@ -24,6 +24,7 @@
 // on the order of the balls, so there is no sort by radius, no list of balls
 // per tile and no barrier between radii, and the non-selected voxels on a
 // ball's sphere (rho = 0 at the end) come out of the same passes.
+#include "disc_cuts.h"
 #include "disc_place.h"
 #include "kernels.h"
 
@@ -32,10 +33,11 @@ namespace bm {
 namespace {
 
 __device__ __forceinline__ uint32_t floor_sqrt(uint32_t t) {
-  // t < 2^22.  sqrt(t + 1/2) is at least 1/(4 sqrt t) away from every whole
-  // number, far more than the error of the hardware reciprocal root (2^-22
-  // relative), so its floor is floor(sqrt(t)).  The conversions go through the
-  // f32 mantissa (2^23 + t), which leaves one special-function operation.
+  // t <= kDiscMaxR2 = 127^2.  sqrt(t + 1/2) is at least 1/(4 * 127) = 2e-3 away
+  // from every whole number, far more than the error of the hardware reciprocal
+  // root (2^-22 relative: 3e-5), so its floor is floor(sqrt(t)).  The conversions
+  // go through the f32 mantissa (2^23 + t), which leaves one special-function
+  // operation.
   const float f = __uint_as_float(0x4b000000u | t) - 8388607.5f;
   float r;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(f));
@@ -162,15 +164,6 @@ constexpr int kWalk = 6;                   // planes a thread walks per step
 constexpr int kCentres = 4096;             // ball centres a CTA keeps from its first walk
 // centres and runs a warp holds back until 32 are ready
 constexpr int kCentreQueue = 32 + 32 * kWalk, kRunQueue = 64;
-
-// The last t with a disc (or chord) of squared radius rho - t^2 not covered by
-// that of the neighbour one step up, rho' - (t - 1)^2, gain = rho' - rho: covered
-// where gain >= 1 - 2 t, or (not strict: an equal value) where gain > 1 - 2 t.
-__device__ __forceinline__ int cut_above(int gain, bool larger) {
-  return larger ? -((gain - 1) >> 1) - 1 : (1 - gain) >> 1;
-}
-// The first t not covered by the neighbour one step down: covered where gain >= 1 + 2 t.
-__device__ __forceinline__ int cut_below(int gain) { return (gain + 1) >> 1; }
 
 // Cell of patch column c in a plane of the padded table.
 __device__ __forceinline__ int cell_of(uint32_t c) { return (int)(c >> 5) * kRowPad + kRowPad + (int)(c & 31u) + 1; }
