@@ -378,9 +378,9 @@ disc_list_kernel(const uint16_t* __restrict__ rmap, int pitch, Dims dm, int H, c
         uint32_t h = cnt | (cnt ? floor_sqrt(r) << 16 : 0u);
         s_dst[k] = nullptr;
         if (cnt > kDiscSlots) {
-          const unsigned long long first = atomicAdd(&ctr->disc_pool, (unsigned long long)cnt);
+          const unsigned long long first = atomicAdd(&ctr->disc_pool, (unsigned long long)disc_segment(cnt));
           if (first + cnt <= pool_cap) {
-            list[0] = disc_place(first);
+            list[0].x = disc_place(first);
             s_dst[k] = pool + first;
             s_count[k] = 0u;
             atomicOr(&s_full, 1u << k);
@@ -496,7 +496,7 @@ disc_paint_kernel(const uint32_t* __restrict__ hdr, const uint2* __restrict__ en
         count = min(e0 + unit, item & 0xffffu);
         const int px = px0 + (int)((item >> 16) & 255u), py = py0 + (int)(item >> 24);
         list = ent + (zh + (long long)py * npx + px) * kDiscSlots;
-        if ((item & 0xffffu) > kDiscSlots) list = pool + disc_first(__ldg(list));
+        if ((item & 0xffffu) > kDiscSlots) list = pool + disc_first(__ldg(&list->x));
         bx = px * kDiscPX - x0;
         by = py * kDiscPY - y0;
       }

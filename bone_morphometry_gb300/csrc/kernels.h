@@ -150,7 +150,7 @@ cudaError_t launch_ridge_map(const uint16_t* dist, Dims dm, const uint2* thr, ui
 // plane (disc_header_count), its discs {R << 16 | rho, column | (first row +
 // 128) << 8 | (last row + 128) << 16} (rows from the centre's) at
 // ent[patch * kDiscSlots].  A patch with more than kDiscSlots discs has them at
-// pool[disc_first(ent[patch * kDiscSlots])]; a pool that is too small (disc_pool_entries:
+// pool[disc_first(ent[patch * kDiscSlots].x)]; a pool that is too small (disc_pool_entries:
 // a first estimate) sets ctr->disc_overflow and leaves lists out; ctr->disc_pool,
 // 0 beforehand, has the entries wanted in either case.
 size_t disc_pool_entries(Dims dm, uint32_t rmax);

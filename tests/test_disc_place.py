@@ -11,10 +11,13 @@ PROGRAM = r"""
 #include <cstdio>
 #include "disc_place.h"
 int main() {
-  const unsigned long long places[] = {0ull, 1ull, 0xfffffffeull, 0xffffffffull, 0x100000000ull, 0x100000001ull,
-                                       9332000000ull, 0x123456789abull};
+  const unsigned long long places[] = {0ull, 4ull, 0xfffffffcull, 0x100000000ull, 0x100000004ull, 9332000000ull,
+                                       0x3fffffffcull};
   for (unsigned long long p : places)
     if (bm::disc_first(bm::disc_place(p)) != p) return 1;
+  // segments keep the next place a multiple of 4, and hold their list
+  for (unsigned n = 1; n < 70000; ++n)
+    if (bm::disc_segment(n) % 4 != 0 || bm::disc_segment(n) < n || bm::disc_segment(n) > n + 3) return 2;
   return 0;
 }
 """
@@ -30,5 +33,5 @@ def test_places_beyond_32_bits(tmp_path):
 
 def test_kernels_keep_the_place_whole():
     text = open(os.path.join(build.CSRC, "discs.cu")).read()
-    assert "disc_place(first)" in text and "disc_first(__ldg(list))" in text
-    assert "(uint32_t)first" not in text
+    assert "disc_place(first)" in text and "disc_first(__ldg(&list->x))" in text
+    assert "(uint32_t)first" not in text and "disc_segment(cnt)" in text
