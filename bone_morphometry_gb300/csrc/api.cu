@@ -362,9 +362,9 @@ void queue_quantiles(bm_ctx* ctx, const float* d_map, long long n, const PhaseOu
 // where the inputs arrive so), z; wait_edt, whose largest radius sizes and
 // chooses what follows; fill; finish, which waits for the results.  The two
 // phases of a call are stepped in turn by one host thread, each on its own
-// context.  64^3 device inputs: 272 us, against 383 with a thread started per
-// call, pageable readbacks and a wait for the ROI counts before either phase
-// (128^3 host inputs with quantiles: 547 against 688).
+// context.  A thread started per call, pageable readbacks and a wait for the ROI
+// counts before either phase took 111 us more of a 64 x 56 x 72 call (235 us now)
+// and 141 more of a 128^3 one from host inputs with quantiles (450).
 struct Phase {
   // set by the caller
   bm_ctx* ctx;
@@ -1087,12 +1087,13 @@ int tbth_phases(bm_ctx* ctx, const uint8_t* d_bone, const uint8_t* d_roi, Dims d
     bone.paint();
     bone.finish();
   } else {
-    // Small volumes in turns and the marrow phase, whose balls are larger as a
-    // rule, first: neither phase's kernels wait for all the other's launches (64^3
-    // 240 us, 268 with the bone phase queued whole and first).  Where kernels
-    // outlast launches the bone phase first, so that the phases are at different
-    // kernels (128^3 536 us, 543 in turns; 512^3 10.10 ms, 10.32).
-    const bool turns = N < (1ll << 20);
+    // In turns and the marrow phase, whose balls are larger as a rule, first:
+    // neither phase's kernels wait for all the other's launches (64^3 242 us, 255
+    // with the bone phase queued whole and first; 128^3 364 and 375; 256^3 1306 and
+    // 1332; 300 x 310 x 290 2.01 and 2.03 ms).  Where kernels outlast launches the
+    // bone phase first, so that the phases are at different kernels (400 x 410 x 390
+    // 4.41 ms, 4.49 in turns; 512^3 9.17 and 9.33).
+    const bool turns = N < (1ll << 25);
     if (turns) try_twin([&] { marrow.lists(); });
     bone.lists();
     if (turns) try_twin([&] { marrow.paint(); });

@@ -652,7 +652,10 @@ cudaError_t ridge_map_rows(const uint16_t* dist, Dims dm, const uint2* thr, uint
 cudaError_t launch_ridge_map(const uint16_t* dist, Dims dm, const uint2* thr, uint16_t* rmap, cudaStream_t s,
                              unsigned long long* launches) {
   ++*launches;
-  return dm.n() >= (1ll << 23) ? ridge_map_rows<4, 32>(dist, dm, thr, rmap, s)
+  // 4 rows and 32 planes a warp load fewer halos, 2 and 4 give more warps; both
+  // phases: 128^3 59 and 27 us, 187 x 203 x 251 67 and 59, 301 x 190 x 253 80 and 83,
+  // 320^3 142 and 162, 512^3 411 and 574.
+  return dm.n() >= (3ll << 22) ? ridge_map_rows<4, 32>(dist, dm, thr, rmap, s)
                                : ridge_map_rows<2, 4>(dist, dm, thr, rmap, s);
 }
 
@@ -718,6 +721,11 @@ cudaError_t launch_disc_paint(const uint32_t* hdr, const uint2* ent, const uint2
                               unsigned long long* launches) {
   ++*launches;
   const int H = halo_of(rmax);
+  // Tiles of 64 rows take a list that reaches two of 32 once, those of 32 are twice
+  // as many.  Both phases: 64^3 28.0 and 26.7 us, 90 x 97 x 95 45.3 and 41.0, 128^3
+  // 61.4 and 63.2; 320^3 (smoothing of 4 voxels) 0.80 and 0.88 ms, 512^3 (5) 3.44 and
+  // 3.81.  With smaller balls 32 rows stay ahead a little longer (smoothing of 3.5:
+  // 160^3 122 and 115 us, 256^3 380 and 376, 320^3 728 and 718).
   return dm.n() >= (1ll << 22) ? paint_rows<64>(hdr, ent, pool, dm, H, dia, dmap, nzbits, fillmap, s)
                                : paint_rows<32>(hdr, ent, pool, dm, H, dia, dmap, nzbits, fillmap, s);
 }
