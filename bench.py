@@ -228,8 +228,8 @@ def workload_config(workload: str, shape, world: int) -> dict:
     return {"workload": "%s: %s" % (workload, WORKLOADS[workload]["desc"]),
             "shape_whd": [w, h, d], "voxels_per_specimen": n_vox, "phases": ["Tb.Th", "Tb.Sp"],
             "parallelism": "replicas" if world > 1 else "single GPU",
-            "l2": "inputs (%d MiB) and u32 maps (%d MiB each) larger than the 129 MB L2"
-                  % (2 * n_vox >> 20, 4 * n_vox >> 20)}
+            "l2": "inputs (%d MiB) and maps (%d MiB of 16 bits, %d MiB of 32 bits a voxel) larger than the 129 MB L2"
+                  % (2 * n_vox >> 20, 2 * n_vox >> 20, 4 * n_vox >> 20)}
 
 
 def run_reference(args, rank, world):

@@ -653,13 +653,15 @@ edt_window_tma_kernel(const __grid_constant__ CUtensorMap tin, uint32_t* __restr
 // on either side (a candidate beyond them adds at least 65^2).  A minimum of at
 // most kNearMax can only have come from exact candidates, so the z pass' outputs
 // up to kNearMax are exact too; it flags the lines that hold others, and the
-// 32-bit passes compute those (launch_edt_far).
+// 32-bit passes compute those (launch_edt_x, launch_edt_window, then
+// launch_edt_redo or launch_edt_near_redo).
 //
 // 512^3, 15 % foreground: 754 us with 32-bit passes, 445 here (x 106, y 129,
 // z 172; the maps' bytes alone take 260 at the copy rate, the rest is issue).
 // 417 x 333 x 379 (rows at any address): 673 us, 333 here (79, 102, 115; the x
-// pass 125 from single bytes, a ballot per 32).  Where 36 to 94 % of the volume lies beyond 65 voxels of a site, so
-// that the 32-bit passes run as well, 1.23-2.70 ms before and 1.18-2.68 here.
+// pass 125 from single bytes, a ballot per 32).  Where 36 to 94 % of the volume
+// lies beyond 65 voxels of a site, so that the 32-bit passes run as well, 1.23-2.70
+// ms before and 1.18-2.68 here; small volumes all of which lie beyond lose 20 us.
 constexpr uint32_t kNearMax = (kWinHalo + 1) * (kWinHalo + 1);
 constexpr uint32_t kFar16 = 40000;
 constexpr int kReach = 190, kReachWords = 6;
