@@ -71,3 +71,18 @@ def test_wide_thin_volume_takes_no_lists():
         got = local_thickness(vol, Phase.FOREGROUND, ctx=ctx)
         assert before - free_bytes() <= footprint_bytes(shape)
     assert np.array_equal(got.view(np.uint32), O.local_thickness(vol, O.FOREGROUND).thickness.view(np.uint32))
+
+
+def test_a_worker_that_changes_between_fills():
+    """One worker: the separable fill, the tile fill (radii above 127), the first again."""
+    near = (np.random.default_rng(8).random((40, 50, 60)) < 0.9).astype(np.uint8)
+    far = np.ones((20, 20, 300), np.uint8)
+    far[10, 10, :120:4] = 0
+    order = (near, far, near, far, near)
+    with closing(Context(0)) as ctx:
+        alone = [analyze_thickness(v, np.ones_like(v), 5.0, ctx=ctx) for v in order]
+    with Server(workers=1, hbm_budget_bytes=20e9) as srv:
+        for v, a in zip(order, alone):
+            r = srv.result(srv.submit(v, np.ones_like(v), 5.0))
+            assert r.status == 0
+            assert repr(r.thickness) == repr(a.thickness) and repr(r.spacing) == repr(a.spacing)
