@@ -654,8 +654,10 @@ cudaError_t launch_ridge_map(const uint16_t* dist, Dims dm, const uint2* thr, ui
   ++*launches;
   // 4 rows and 32 planes a warp load fewer halos, 2 and 4 give more warps; both
   // phases: 128^3 59 and 27 us, 187 x 203 x 251 67 and 59, 301 x 190 x 253 80 and 83,
-  // 320^3 142 and 162, 512^3 411 and 574.
-  return dm.n() >= (3ll << 22) ? ridge_map_rows<4, 32>(dist, dm, thr, rmap, s)
+  // 320^3 142 and 162, 512^3 411 and 574.  The line lies below where the two meet
+  // for a call alone: fewer halos are less work, which counts where specimens
+  // overlap (16 of 96 to 384 voxels an edge 9.11 ms, 9.17 with the line at 3 * 2^22).
+  return dm.n() >= (1ll << 23) ? ridge_map_rows<4, 32>(dist, dm, thr, rmap, s)
                                : ridge_map_rows<2, 4>(dist, dm, thr, rmap, s);
 }
 
