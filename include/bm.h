@@ -287,13 +287,13 @@ int bm_ctx_set_concurrent_phases(bm_ctx* ctx, int on);
 /* How the sphere fill finds the non-selected voxels a ridge ball reaches
  * (local_thickness.rs:169-202 paints them too).  BM_SITES_AUTO (the default)
  * lets the separable fill paint them with the others, up to a largest radius
- * of 127 voxels; beyond, and with the other two settings, the tile fill paints
- * the selected voxels and BM_SITES_SPHERES tests every lattice point of every
- * ridge sphere, BM_SITES_CHAINS pushes the ridge r^2 backwards along the
- * distance transform's tied argmins (two window passes over the volume, two
- * more u32 maps of device memory), BM_SITES_AUTO picks chains when the spheres'
- * lattice points would take the site test more than 0.2 half-warp steps per
- * voxel of the volume.  Results are identical either way. */
+ * of 127 voxels and while its lists have memory; otherwise, and with the other
+ * two settings, the tile fill paints the selected voxels and BM_SITES_SPHERES
+ * tests every lattice point of every ridge sphere, BM_SITES_CHAINS pushes the
+ * ridge r^2 backwards along the distance transform's tied argmins (two window
+ * passes over the volume, two more u32 maps of device memory), BM_SITES_AUTO
+ * picks chains when the spheres' lattice points would take the site test more
+ * than 0.2 half-warp steps per voxel of the volume.  Results are identical either way. */
 enum { BM_SITES_AUTO = 0, BM_SITES_SPHERES = 1, BM_SITES_CHAINS = 2 };
 int bm_ctx_set_site_method(bm_ctx* ctx, int method);
 
